@@ -13,6 +13,7 @@
 #include "../../include/gmoe.h"
 #include "kernels.h"
 #include "synth.h"
+#include "hostflow.h"
 
 void k_count_add(long n);
 
@@ -52,12 +53,12 @@ static struct {
     float *x, *hn, *y, *hqs, *logits, *topw, *uw, *act, *aqs, *down, *gate, *up, *bias;
     int8_t *hq, *aq;
     int *ecnt, *uexp, *hqsum, *top, *nu, *ue, *estart, *ustart, *utok, *slot, *tp, *aqsum, *ntiles_a, *ntiles_b, *gu_dots, *dn_dots;
-    unsigned *mask; int *err, *h_err;
+    unsigned *mask; int *err, *h_err;      /* the kernels' error word, in page-locked host memory: the device's and the host's pointer to it */
     MoeTile *tiles_a, *tiles_b;
     ExpertPtrs *tab_call;      /* the used experts of one gpre_moe call */
     ExpertMaps *maps_call, *h_maps; int8_t *hq_sorted; TMap4 bmap_hq, bmap_aq;
     struct { const void *key; ExpertMaps m; } *map_cache;   /* tensor maps of experts seen by gpre_moe, by code pointer */
-    MoeTile *h_tiles; ExpertPtrs *h_tab;   /* host staging for the reference-shaped calls */
+    ExpertPtrs *h_tab;         /* host staging of a layer's pointer table */
     double t_experts;          /* GPU seconds in gfull_moe, reported by gfull_report */
     float *ring; int ring_nb, ring_n;
     unsigned prof_mask; cudaEvent_t *pev; int pev_n, pev_cap; unsigned char *pev_stage; long *pev_launch;
@@ -65,6 +66,19 @@ static struct {
     /* tensor-core router (k_router_umma.cu) */
     void *hA; float *hnorm, *rpart; int *flagged, *nflagged, *rdone; TMap amap; int router_mode;
 } S;
+
+/* The tables of a reference-shaped call are written into one page-locked block, from which one kernel distributes them to their places
+ * on the card (instead of a dozen small copies, each of which costs as much as the kernel). */
+static struct { uint8_t *h; size_t cap, used; cudaEvent_t taken; int pending; TableSegs seg; } CT;
+static int tables_begin(const char *who) {
+    if (CT.pending && cudaEventSynchronize(CT.taken) != cudaSuccess) return fail(who, "the stream reports an earlier error");
+    CT.pending = 0; CT.used = 0; CT.seg.n = 0; return 0;
+}
+static void *tables_add(void *dst, size_t bytes) {      /* bytes: a multiple of 4 */
+    void *p = CT.h + CT.used; const int i = CT.seg.n++;
+    CT.seg.dst[i] = dst; CT.seg.src[i] = p; CT.seg.words[i] = (unsigned)(bytes / 4);
+    CT.used += (bytes + 15) & ~(size_t)15; return p;
+}
 
 /* ------------------------------------------------------------------------------------------------------------ */
 static int dmalloc(void **p, size_t bytes) { return cudaMalloc(p, bytes ? bytes : 16) == cudaSuccess ? 0 : -1; }
@@ -133,7 +147,7 @@ static int init_common(const char *who, int maxtok, int topk) {
     size_t P = (size_t)maxtok * TOPK, T = (size_t)maxtok;
     S.maxtok = maxtok; S.maxp = (int)P; S.mask_words = (maxtok + 31) / 32;
     ALLOC(x, T * HID * 4); ALLOC(hn, T * HID * 4); ALLOC(y, T * HID * 4); ALLOC(hT, (T + 15) / 16 * 16 * HID * 8);
-    ALLOC(hq, T * HID); ALLOC(hqs, T * 4); ALLOC(hqsum, T * 4);
+    ALLOC(hq, T * HID); ALLOC(hqs, T * 8); S.hqsum = (int *)S.hqs + T;      /* one block: both arrays cross to the card in one copy */
     ALLOC(logits, T * NEXP * 4); ALLOC(top, P * 4); ALLOC(topw, P * 4); ALLOC(bias, NEXP * 4);
     ALLOC(ecnt, NEXP * 4); ALLOC(uexp, P * 4);
     ALLOC(mask, ((size_t)2 * NEXP * S.mask_words + NEXP) * 4); ALLOC(nu, 16); ALLOC(ue, NEXP * 4); ALLOC(estart, NEXP * 4);
@@ -141,18 +155,20 @@ static int init_common(const char *who, int maxtok, int topk) {
     ALLOC(tiles_a, (P / 8 + NEXP) * sizeof(MoeTile)); ALLOC(tiles_b, (P / 8 + NEXP) * sizeof(MoeTile));
     ALLOC(ntiles_a, 16); ALLOC(ntiles_b, 16);
     ALLOC(act, P * FFN * 4); ALLOC(gate, P * FFN * 4); ALLOC(up, P * FFN * 4); ALLOC(aq, P * FFN); ALLOC(aqs, P * 4); ALLOC(aqsum, P * 4); ALLOC(down, P * HID * 4);
-    ALLOC(tab_call, NEXP * sizeof(ExpertPtrs)); ALLOC(err, 16); ALLOC(maps_call, NEXP * sizeof(ExpertMaps)); ALLOC(hq_sorted, P * HID);
+    ALLOC(tab_call, NEXP * sizeof(ExpertPtrs)); ALLOC(maps_call, NEXP * sizeof(ExpertMaps)); ALLOC(hq_sorted, P * HID);
     ALLOC(wire, WIRE_BYTES(P)); CU(who, cudaMemset(S.wire, 0, WIRE_BYTES(P))); ALLOC(dsp_call, NEXP * sizeof(void *));
     ALLOC(hA, T * HID * 4); ALLOC(hnorm, T * 4); ALLOC(rpart, (size_t)8 * T * NEXP * 4); ALLOC(flagged, T * 4); ALLOC(nflagged, 16); ALLOC(rdone, T * 4); CU(who, cudaMemset(S.rdone, 0, T * 4));
     CU(who, cudaMemset(S.hA, 0, T * HID * 4)); CU(who, cudaMemset(S.nflagged, 0, 16));
     if (tmap_init(who)) return -1;
     if (tmap_f16_2d(who, &S.amap, S.hA, 2 * HID, T, (uint64_t)2 * HID * 2, 64, 128)) return -1;
     if (bmaps(who, P)) return -1;
-    CU(who, cudaMemset(S.err, 0, 16));
-    CU(who, cudaHostAlloc((void **)&S.h_err, 16, cudaHostAllocDefault)); *S.h_err = 0;
-    S.h_tiles = malloc(2 * (P / 8 + NEXP) * sizeof(MoeTile)); S.h_tab = malloc(NEXP * sizeof(ExpertPtrs));
+    CU(who, cudaHostAlloc((void **)&S.h_err, 16, cudaHostAllocMapped)); *S.h_err = 0;
+    CU(who, cudaHostGetDevicePointer((void **)&S.err, S.h_err, 0));
+    CT.cap = P * 12 + (P / 8 + NEXP) * sizeof(MoeTile) + T * 8 + NEXP * (sizeof(ExpertMaps) + sizeof(ExpertPtrs) + 16) + 4096;
+    CU(who, cudaHostAlloc((void **)&CT.h, CT.cap, cudaHostAllocMapped)); CU(who, cudaEventCreateWithFlags(&CT.taken, cudaEventDisableTiming));
+    S.h_tab = malloc(NEXP * sizeof(ExpertPtrs));
     S.h_maps = aligned_alloc(64, NEXP * sizeof(ExpertMaps)); S.map_cache = aligned_alloc(64, MAP_CACHE * sizeof *S.map_cache);
-    if (!S.h_tiles || !S.h_tab || !S.h_maps || !S.map_cache) return fail(who, "out of host memory");
+    if (!S.h_tab || !S.h_maps || !S.map_cache) return fail(who, "out of host memory");
     memset(S.map_cache, 0, MAP_CACHE * sizeof *S.map_cache);
     S.ready = 1;
     fprintf(stderr, "%s: %s, chunks up to %d tokens, %.0f MB of device workspace, weights resident in HBM\n", who, pr.name, maxtok,
@@ -453,22 +469,39 @@ static const float *bias_dev(const float *bias) {
     cudaMemcpyAsync(S.bias, bias, NEXP * 4, cudaMemcpyHostToDevice, S.st);
     return S.bias;
 }
-static double finish(const char *who) {
-    cudaMemcpyAsync(S.h_err, S.err, 4, cudaMemcpyDeviceToHost, S.st);
+/* waits for the stream: 0, or -1 when a kernel or the runtime reported an error */
+static int check_done(const char *who) {
     cudaError_t e = cudaStreamSynchronize(S.st);
-    if (e == cudaSuccess && *S.h_err) {
-        const int code = *S.h_err;
-        *S.h_err = 0; cudaMemsetAsync(S.err, 0, 4, S.st);
+    const int code = e == cudaSuccess ? *(volatile int *)S.h_err : 0;
+    if (code) {
+        *S.h_err = 0;
         /* a down pass that no combine followed leaves escape bits behind; they are only ever OR-ed into */
         cudaMemsetAsync(S.wire, 0, WIRE_BYTES((size_t)S.maxp), S.st);
         fail(who, "a kernel gave up waiting (code %d: %s); results are invalid", code,
              code == 41 ? "a rank did not arrive at the expert-parallel rendezvous" : code == 31 ? "router operand ring" : "barrier inside an expert kernel");
-        return -1.0;
+        return -1;
     }
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) { fail(who, "%s", cudaGetErrorString(e)); return -1.0; }
+    return e == cudaSuccess ? 0 : fail(who, "%s", cudaGetErrorString(e));
+}
+static double finish(const char *who) {      /* and the seconds between the call's two events */
+    if (check_done(who)) return -1.0;
     float ms = 0; cudaEventElapsedTime(&ms, S.e0, S.e1);
     return ms * 1e-3;
+}
+
+/* hidden rows between a caller's host array and the card (hostflow.h) */
+static int rows_in(const char *who, float *dev, const float *x, int nb) {
+    Flow f; memset(&f, 0, sizeof f);
+    f.rows = nb; f.src = x; f.row = HID * 4; f.dst = dev;
+    const cudaError_t e = flow_run(&f, S.st);
+    return e == cudaSuccess ? 0 : fail(who, "copy of %d rows to the card: %s", nb, cudaGetErrorString(e));
+}
+static int rows_out(const char *who, float *y, const float *dev, int nb) {
+    Flow f; memset(&f, 0, sizeof f);
+    f.rows = nb; f.nout = 1; f.osrc[0] = dev; f.odst[0] = y; f.orow[0] = HID * 4;
+    const cudaError_t e = flow_run(&f, S.st);
+    return e == cudaSuccess ? 0 : fail(who, "copy of %d rows from the card: %s", nb, cudaGetErrorString(e));
 }
 
 /* ---- the layer loop as a CUDA graph: one launch per call instead of a dozen per layer -------------------------------------
@@ -535,12 +568,12 @@ static int layers_enqueue(int nb, int l0, int nl, const float *bd) { return laye
 
 double gmoe_moe(int L, const float *x, int nb, float *y, const float *bias) {
     if (check_call("gmoe", L, nb)) return -1.0;
-    CUD("gmoe", cudaMemcpyAsync(S.hn, x, (size_t)nb * HID * 4, cudaMemcpyHostToDevice, S.st));
+    if (rows_in("gmoe", S.hn, x, nb)) return -1.0;
     const float *bd = bias_dev(bias);
     cudaEventRecord(S.e0, S.st);
     run_layer(L, nb, 0, bd);
     cudaEventRecord(S.e1, S.st);
-    CUD("gmoe", cudaMemcpyAsync(y, S.y, (size_t)nb * HID * 4, cudaMemcpyDeviceToHost, S.st));
+    if (rows_out("gmoe", y, S.y, nb)) return -1.0;
     S.nb_cur = nb;
     return finish("gmoe");
 }
@@ -585,9 +618,9 @@ double gmoe_forward(float *x, int nb, int l0, int nl, const float *bias) {   /* 
     for (int L = l0; L < l0 + nl; L++) if (check_call("gmoe", L, nb)) return -1.0;
     const float *bd = bias_dev(bias);
     cudaEventRecord(S.e0, S.st);
-    CUD("gmoe", cudaMemcpyAsync(S.x, x, (size_t)nb * HID * 4, cudaMemcpyHostToDevice, S.st));
+    if (rows_in("gmoe", S.x, x, nb)) return -1.0;
     if (layers_enqueue(nb, l0, nl, bd)) return -1.0;
-    CUD("gmoe", cudaMemcpyAsync(x, S.x, (size_t)nb * HID * 4, cudaMemcpyDeviceToHost, S.st));
+    if (rows_out("gmoe", x, S.x, nb)) return -1.0;
     cudaEventRecord(S.e1, S.st);
     S.nb_cur = nb;
     return finish("gmoe");
@@ -599,7 +632,7 @@ static struct {
     cudaStream_t in, out; int ready, seq, done;          /* seq: chunks submitted, done: chunks waited for */
     float *xin[2], *xout[2]; size_t cap;                /* staging slots on the card, cap floats each */
     cudaEvent_t mark, start[2], loaded[2], taken[2], ran[2], stored[2];
-    int *h_err;                                          /* pinned: the kernels' error word as each chunk left it */
+    int bad;                                             /* chunks still to be reported as invalid after a kernel's error */
 } PIPE;
 static int pipe_setup(int nb) {
     if (!PIPE.ready) {
@@ -610,8 +643,6 @@ static int pipe_setup(int nb) {
             CU("gmoe", cudaEventCreateWithFlags(&PIPE.loaded[k], cudaEventDisableTiming)); CU("gmoe", cudaEventCreateWithFlags(&PIPE.taken[k], cudaEventDisableTiming));
             CU("gmoe", cudaEventCreateWithFlags(&PIPE.ran[k], cudaEventDisableTiming));
         }
-        if (cudaHostAlloc((void **)&PIPE.h_err, 2 * sizeof(int), cudaHostAllocDefault) != cudaSuccess) return fail("gmoe", "no pinned memory");
-        PIPE.h_err[0] = PIPE.h_err[1] = 0;
         CU("gmoe", cudaEventRecord(PIPE.mark, PIPE.in));
         PIPE.ready = 1;
     }
@@ -649,7 +680,6 @@ int gmoe_forward_submit(const float *x_in, float *x_out, int nb, int l0, int nl,
     CU("gmoe", cudaEventRecord(PIPE.ran[k], S.st));
     CU("gmoe", cudaStreamWaitEvent(PIPE.out, PIPE.ran[k], 0));
     CU("gmoe", cudaMemcpyAsync(x_out, PIPE.xout[k], bytes, cudaMemcpyDeviceToHost, PIPE.out));
-    CU("gmoe", cudaMemcpyAsync(&PIPE.h_err[k], S.err, 4, cudaMemcpyDeviceToHost, PIPE.out));
     CU("gmoe", cudaEventRecord(PIPE.stored[k], PIPE.out));
     S.nb_cur = nb; PIPE.seq++;
     return 0;
@@ -660,12 +690,14 @@ double gmoe_forward_wait(void) {
     PIPE.done++;
     cudaError_t e = cudaEventSynchronize(PIPE.stored[k]);
     if (e != cudaSuccess) { fail("gmoe", "%s", cudaGetErrorString(e)); return -1.0; }
-    if (PIPE.h_err[k]) {
-        const int code = PIPE.h_err[k];
-        PIPE.h_err[k] = 0; cudaStreamSynchronize(S.st); cudaMemsetAsync(S.err, 0, 4, S.st); cudaMemsetAsync(S.wire, 0, WIRE_BYTES((size_t)S.maxp), S.st);
+    const int code = *(volatile int *)S.h_err;
+    if (code) {      /* whichever outstanding chunk raised it, all of them are reported */
+        cudaStreamSynchronize(S.st); *S.h_err = 0; cudaMemsetAsync(S.wire, 0, WIRE_BYTES((size_t)S.maxp), S.st);
+        PIPE.bad = PIPE.seq - PIPE.done;
         fail("gmoe", "a kernel gave up waiting (code %d); results are invalid", code);
         return -1.0;
     }
+    if (PIPE.bad > 0) { PIPE.bad--; fail("gmoe", "a kernel gave up waiting while this chunk was outstanding; results are invalid"); return -1.0; }
     float ms = 0.0f;
     if (cudaEventElapsedTime(&ms, PIPE.mark, PIPE.stored[k]) != cudaSuccess) { fail("gmoe", "event timing"); return -1.0; }
     return (double)ms * 1e-3;
@@ -726,66 +758,89 @@ static void host_buffer_seen(const void *p, size_t len) {
 }
 
 /* ---- the reference-shaped calls: grouping supplied by the host ---------------------------------------------------- */
-static int upload_grouping(const char *who, int nb, int nu, const uint32_t *loc, const int *regs, const int *ustart,
-                           const int *ptok, const float *pw, const int *tp) {
+/* Checks the call's tables and writes them into the block that the card reads (tables_begin has been called; tables_send distributes it). */
+static int stage_grouping(const char *who, int nb, int nu, const uint32_t *loc, const int *regs, const int *ustart,
+                          const int *ptok, const float *pw, const int *tp) {
+    const int np = ustart[nu], um = use_umma(nb), tn = um ? UMMA_TN : tile_tn(nb);
+    if (np != nb * TOPK) return fail(who, "%d pairs for %d tokens (need %d per token)", np, nb, TOPK);
+    if (ustart[0] != 0) return fail(who, "ustart[0] = %d", ustart[0]);
+    const float **dsp = tables_add(S.dsp_call, NEXP * sizeof(void *));
+    ExpertPtrs *tab = tables_add(S.tab_call, (size_t)nu * sizeof(ExpertPtrs));
+    ExpertMaps *maps = um ? tables_add(S.maps_call, (size_t)nu * sizeof(ExpertMaps)) : NULL;
+    for (int u = 0; u < nu; u++) {
+        if (ustart[u + 1] <= ustart[u]) return fail(who, "used expert %d has no pairs", u);
+        if (resolve(who, loc + u * 12, regs, &tab[u])) return -1;
+        dsp[u] = tab[u].ds;
+        if (!um) continue;
+        /* tensor maps of this expert: encoded the first time its codes are seen */
+        size_t hsh = ((uintptr_t)tab[u].gc >> 8) % MAP_CACHE;
+        if (S.map_cache[hsh].key != (const void *)tab[u].gc) {
+            if (expert_maps(who, &tab[u], &S.map_cache[hsh].m)) return -1;
+            S.map_cache[hsh].key = tab[u].gc;
+        }
+        memcpy(&maps[u], &S.map_cache[hsh].m, sizeof(ExpertMaps));
+    }
+    for (int u = nu; u < NEXP; u++) dsp[u] = NULL;
+    int bad = 0, nt = 0;
+    for (int a = 0; a < np; a++) bad |= (unsigned)ptok[a] >= (unsigned)nb;
+    if (bad) { for (int a = 0; a < np; a++) if (ptok[a] < 0 || ptok[a] >= nb) return fail(who, "ptok[%d] = %d", a, ptok[a]); }
+    for (int i = 0; i < np; i++) bad |= (unsigned)tp[i] >= (unsigned)np;
+    if (bad) { for (int i = 0; i < np; i++) if (tp[i] < 0 || tp[i] >= np) return fail(who, "tp[%d] = %d", i, tp[i]); }
+    for (int u = 0; u < nu; u++) nt += (ustart[u + 1] - ustart[u] + tn - 1) / tn;
+    MoeTile *t = tables_add(um ? S.tiles_b : S.tiles_a, (size_t)nt * sizeof(MoeTile));
+    for (int u = 0; u < nu; u++) for (int p = ustart[u]; p < ustart[u + 1]; p += tn) {   /* gpu_pre.m:329-333 */
+        const MoeTile m = {u, p, ustart[u + 1] - p < tn ? ustart[u + 1] - p : tn, u}; *t++ = m;
+    }
+    *(int *)tables_add(um ? S.ntiles_b : S.ntiles_a, 4) = nt; *(int *)tables_add(S.nu, 4) = nu;
+    memcpy(tables_add(S.ustart, (size_t)(nu + 1) * 4), ustart, (size_t)(nu + 1) * 4);
+    memcpy(tables_add(S.utok, (size_t)np * 4), ptok, (size_t)np * 4);
+    memcpy(tables_add(S.uw, (size_t)np * 4), pw, (size_t)np * 4);
+    memcpy(tables_add(S.tp, (size_t)np * 4), tp, (size_t)np * 4);
+    return 0;
+}
+static int tables_send(const char *who) {
+    k_tables(S.st, &CT.seg);
+    CU(who, cudaEventRecord(CT.taken, S.st)); CT.pending = 1;
+    return 0;
+}
+static int grouping_args(const char *who, int nb, int nu) {
     if (!S.ready) return fail(who, "not initialised");
     if (S.ep_on) return fail(who, "expert parallelism is set up: use the gmoe_ep_* entry points");
     if (nb < 1 || nb > S.maxtok) return fail(who, "%d tokens outside 1..%d", nb, S.maxtok);
     if (nu < 1 || nu > NEXP) return fail(who, "%d used experts outside 1..%d", nu, NEXP);
-    int np = ustart[nu];
-    if (np != nb * TOPK) return fail(who, "%d pairs for %d tokens (need %d per token)", np, nb, TOPK);
-    if (ustart[0] != 0) return fail(who, "ustart[0] = %d", ustart[0]);
-    int tn = tile_tn(nb), nt = 0, ntb = 0;
-    MoeTile *h_tb = S.h_tiles + ((size_t)S.maxp / 8 + NEXP);
-    for (int u = 0; u < nu; u++) {
-        if (ustart[u + 1] <= ustart[u]) return fail(who, "used expert %d has no pairs", u);
-        if (resolve(who, loc + u * 12, regs, &S.h_tab[u])) return -1;
-        {   /* tensor maps of this expert: encoded the first time its codes are seen */
-            size_t hsh = ((uintptr_t)S.h_tab[u].gc >> 8) % MAP_CACHE;
-            if (S.map_cache[hsh].key != (const void *)S.h_tab[u].gc) {
-                if (expert_maps(who, &S.h_tab[u], &S.map_cache[hsh].m)) return -1;
-                S.map_cache[hsh].key = S.h_tab[u].gc;
-            }
-            S.h_maps[u] = S.map_cache[hsh].m;
-        }
-        for (int p = ustart[u]; p < ustart[u + 1]; p += tn) {   /* gpu_pre.m:329-333 */
-            MoeTile m = {u, p, ustart[u + 1] - p < tn ? ustart[u + 1] - p : tn, u}; S.h_tiles[nt++] = m;
-        }
-        for (int p = ustart[u]; p < ustart[u + 1]; p += UMMA_TN) {
-            MoeTile m = {u, p, ustart[u + 1] - p < UMMA_TN ? ustart[u + 1] - p : UMMA_TN, u}; h_tb[ntb++] = m;
-        }
-    }
-    for (int a = 0; a < np; a++) if (ptok[a] < 0 || ptok[a] >= nb) return fail(who, "ptok[%d] = %d", a, ptok[a]);
-    for (int i = 0; i < np; i++) if (tp[i] < 0 || tp[i] >= np) return fail(who, "tp[%d] = %d", i, tp[i]);
-    for (int u = 0; u < NEXP; u++) S.h_dsp[u] = u < nu ? S.h_tab[u].ds : NULL;
-    CU(who, cudaMemcpyAsync(S.dsp_call, S.h_dsp, NEXP * sizeof(void *), cudaMemcpyHostToDevice, S.st));
-    CU(who, cudaMemcpyAsync(S.tab_call, S.h_tab, (size_t)nu * sizeof(ExpertPtrs), cudaMemcpyHostToDevice, S.st));
-    CU(who, cudaMemcpyAsync(S.maps_call, S.h_maps, (size_t)nu * sizeof(ExpertMaps), cudaMemcpyHostToDevice, S.st));
-    CU(who, cudaMemcpyAsync(S.tiles_a, S.h_tiles, (size_t)nt * sizeof(MoeTile), cudaMemcpyHostToDevice, S.st));
-    CU(who, cudaMemcpyAsync(S.ntiles_a, &nt, 4, cudaMemcpyHostToDevice, S.st));
-    CU(who, cudaMemcpyAsync(S.tiles_b, h_tb, (size_t)ntb * sizeof(MoeTile), cudaMemcpyHostToDevice, S.st));
-    CU(who, cudaMemcpyAsync(S.ntiles_b, &ntb, 4, cudaMemcpyHostToDevice, S.st));
-    CU(who, cudaMemcpyAsync(S.ustart, ustart, (size_t)(nu + 1) * 4, cudaMemcpyHostToDevice, S.st));
-    CU(who, cudaMemcpyAsync(S.nu, &nu, 4, cudaMemcpyHostToDevice, S.st));
-    CU(who, cudaMemcpyAsync(S.utok, ptok, (size_t)np * 4, cudaMemcpyHostToDevice, S.st));
-    CU(who, cudaMemcpyAsync(S.uw, pw, (size_t)np * 4, cudaMemcpyHostToDevice, S.st));
-    CU(who, cudaMemcpyAsync(S.tp, tp, (size_t)np * 4, cudaMemcpyHostToDevice, S.st));
-    CU(who, cudaStreamSynchronize(S.st));   /* the host staging arrays are reused by the next call */
     return 0;
+}
+static void run_call_experts(int nb, const float *init, float *out) {
+    if (use_umma(nb)) k_gather_rows(S.st, S.hq, S.utok, S.hq_sorted, nb * TOPK);
+    run_experts(S.tab_call, S.maps_call, (const float *const *)S.dsp_call, NULL, nb, 7);
+    run_combine((const float *const *)S.dsp_call, nb, init, out);
+}
+/* The experts only see the rows' int8 form, so that is what crosses to the card: a quarter of the bytes, made by the host threads that would
+ * otherwise copy the rows into page-locked memory (same bits as the device's prep, hostio.c). */
+typedef struct { int nb, nu; const uint32_t *loc; const int *regs, *ustart, *ptok; const float *pw; const int *tp; int bad; } CallTables;
+static int stage_call(void *p) {
+    CallTables *c = p;
+    return c->bad = stage_grouping("gpre", c->nb, c->nu, c->loc, c->regs, c->ustart, c->ptok, c->pw, c->tp);
 }
 double gpre_moe(const float *x, int nb, int nu, const uint32_t *loc, const int *regs, const int *next,
                 const int *ustart, const int *ptok, const float *pw, const int *tp, float *y) {
     (void)next;
-    if (upload_grouping("gpre", nb, nu, loc, regs, ustart, ptok, pw, tp)) return -1.0;
+    if (grouping_args("gpre", nb, nu) || tables_begin("gpre")) return -1.0;
+    CallTables c = {nb, nu, loc, regs, ustart, ptok, pw, tp, 0};
     host_buffer_seen(x, (size_t)nb * HID * 4); host_buffer_seen(y, (size_t)nb * HID * 4);
-    CUD("gpre", cudaMemcpyAsync(S.hn, x, (size_t)nb * HID * 4, cudaMemcpyHostToDevice, S.st));
+    if (S.keep && rows_in("gpre", S.hn, x, nb)) return -1.0;
+    Flow f; memset(&f, 0, sizeof f);
+    f.rows = nb; f.src = x; f.row = HID * 4; f.dst = S.hq; f.quant = 1;
+    f.hqs = tables_add(S.hqs, (size_t)nb * 4); f.hqsum = tables_add(S.hqsum, (size_t)nb * 4);
+    f.meanwhile = stage_call; f.mctx = &c;                      /* the tables are checked and written while helper threads read x */
+    const cudaError_t e = flow_run(&f, S.st);
+    if (c.bad) return -1.0;
+    if (e != cudaSuccess) { fail("gpre", "copy of %d rows to the card: %s", nb, cudaGetErrorString(e)); return -1.0; }
     cudaEventRecord(S.e0, S.st);
-    k_norm_prep(S.st, S.hn, NULL, S.hn, S.hq, S.hqs, S.hqsum, nb);
-    if (use_umma(nb)) k_gather_rows(S.st, S.hq, S.utok, S.hq_sorted, nb * TOPK);
-    run_experts(S.tab_call, S.maps_call, (const float *const *)S.dsp_call, NULL, nb, 7);
-    run_combine((const float *const *)S.dsp_call, nb, NULL, S.y);
+    if (tables_send("gpre")) return -1.0;
+    run_call_experts(nb, NULL, S.y);
     cudaEventRecord(S.e1, S.st);
-    CUD("gpre", cudaMemcpyAsync(y, S.y, (size_t)nb * HID * 4, cudaMemcpyDeviceToHost, S.st));
+    if (rows_out("gpre", y, S.y, nb)) return -1.0;
     S.nb_cur = nb;
     return finish("gpre");
 }
@@ -793,22 +848,20 @@ void gfull_begin(const float *x, int nb, int pos0) {
     (void)pos0;
     if (!S.ready || nb < 1 || nb > S.maxtok) { fail("gfull", "gfull_begin with %d tokens", nb); return; }
     host_buffer_seen(x, (size_t)nb * HID * 4);
-    cudaMemcpyAsync(S.x, x, (size_t)nb * HID * 4, cudaMemcpyHostToDevice, S.st); S.nb_cur = nb;
+    rows_in("gfull", S.x, x, nb); S.nb_cur = nb;
 }
 void gfull_moe(int nu, const uint32_t *loc, const int *regs, const int *ustart, const int *ptok, const float *pw, const int *tp) {
     int nb = S.nb_cur;
-    if (upload_grouping("gfull", nb, nu, loc, regs, ustart, ptok, pw, tp)) return;
+    if (grouping_args("gfull", nb, nu) || tables_begin("gfull") || stage_grouping("gfull", nb, nu, loc, regs, ustart, ptok, pw, tp) || tables_send("gfull")) return;
     cudaEventRecord(S.e0, S.st);
-    if (use_umma(nb)) k_gather_rows(S.st, S.hq, S.utok, S.hq_sorted, nb * TOPK);
-    run_experts(S.tab_call, S.maps_call, (const float *const *)S.dsp_call, NULL, nb, 7);            /* hq/hqs/hqsum were left by gmoe_post_norm */
-    run_combine((const float *const *)S.dsp_call, nb, S.x, S.x);
+    run_call_experts(nb, S.x, S.x);            /* hq/hqs/hqsum were left by gmoe_post_norm */
     cudaEventRecord(S.e1, S.st);
     S.fwd_timed = 1;
 }
 void gfull_read(float *x, const uint16_t **ko) {
     if (ko) *ko = NULL;
     if (!S.ready) { fail("gfull", "not initialised"); return; }
-    if (x) { host_buffer_seen(x, (size_t)S.nb_cur * HID * 4); cudaMemcpyAsync(x, S.x, (size_t)S.nb_cur * HID * 4, cudaMemcpyDeviceToHost, S.st); }
+    if (x && S.nb_cur > 0) { host_buffer_seen(x, (size_t)S.nb_cur * HID * 4); if (rows_out("gfull", x, S.x, S.nb_cur)) return; }
     cudaError_t e = cudaStreamSynchronize(S.st);
     if (e != cudaSuccess) fail("gfull", "%s", cudaGetErrorString(e));
     else if (S.fwd_timed) { float ms = 0; cudaEventElapsedTime(&ms, S.e0, S.e1); S.t_experts += ms * 1e-3; S.fwd_timed = 0; }
@@ -912,6 +965,10 @@ int gmoe_rope_table(const float *cs, int positions) {
     CU("gmoe", cudaMemcpyAsync(AT.cs, cs, (size_t)positions * 64 * 4, cudaMemcpyHostToDevice, S.st)); CU("gmoe", cudaStreamSynchronize(S.st));
     AT.positions = positions; return 0;
 }
+static int rope_rows(void *ctx, int r, int n) {
+    k_qk_rope(S.st, AT.qkv + (size_t)r * 3072, AT.pos + r, n, *(int *)ctx, AT.norms, AT.norms + 128, AT.cs, AT.positions, AT.q + (size_t)r * 2048, (uint16_t *)AT.kc + (size_t)r * 512, (uint16_t *)AT.vc + (size_t)r * 512, S.err);
+    return 0;
+}
 double gmoe_qk_rope(const float *qkv, const int *pos, int nb, int glob, const float *qn, const float *kn, float *q, uint16_t *kc, uint16_t *vc) {
     if (!S.ready) { fail("gmoe", "not initialised"); return -1.0; }
     if (nb < 1 || nb > S.maxtok) { fail("gmoe", "gmoe_qk_rope: %d tokens outside 1..%d", nb, S.maxtok); return -1.0; }
@@ -927,17 +984,16 @@ double gmoe_qk_rope(const float *qkv, const int *pos, int nb, int glob, const fl
             dmalloc((void **)&AT.pos, T * 4) || dmalloc((void **)&AT.norms, 256 * 4)) { fail("gmoe", "no device memory for the attention head of %d tokens", S.maxtok); return -1.0; }
         AT.cap = S.maxtok;
     }
-    CUD("gmoe", cudaMemcpyAsync(AT.qkv, qkv, (size_t)nb * 3072 * 4, cudaMemcpyHostToDevice, S.st));
-    CUD("gmoe", cudaMemcpyAsync(AT.pos, pos, (size_t)nb * 4, cudaMemcpyHostToDevice, S.st));
-    CUD("gmoe", cudaMemcpyAsync(AT.norms, qn, 128 * 4, cudaMemcpyHostToDevice, S.st));
-    CUD("gmoe", cudaMemcpyAsync(AT.norms + 128, kn, 128 * 4, cudaMemcpyHostToDevice, S.st));
-    cudaEventRecord(S.e0, S.st);
-    k_qk_rope(S.st, AT.qkv, AT.pos, nb, glob, AT.norms, AT.norms + 128, AT.cs, AT.positions, AT.q, AT.kc, AT.vc, S.err);
-    cudaEventRecord(S.e1, S.st);
-    CUD("gmoe", cudaMemcpyAsync(q, AT.q, (size_t)nb * 2048 * 4, cudaMemcpyDeviceToHost, S.st));
-    CUD("gmoe", cudaMemcpyAsync(kc, AT.kc, (size_t)nb * 512 * 2, cudaMemcpyDeviceToHost, S.st));
-    CUD("gmoe", cudaMemcpyAsync(vc, AT.vc, (size_t)nb * 512 * 2, cudaMemcpyDeviceToHost, S.st));
-    return finish("gmoe");
+    if (tables_begin("gmoe")) return -1.0;
+    memcpy(tables_add(AT.pos, (size_t)nb * 4), pos, (size_t)nb * 4);
+    float *nn = tables_add(AT.norms, 256 * 4); memcpy(nn, qn, 128 * 4); memcpy(nn + 128, kn, 128 * 4);
+    if (tables_send("gmoe")) return -1.0;
+    Flow f; memset(&f, 0, sizeof f);
+    f.rows = nb; f.src = qkv; f.row = 3072 * 4; f.dst = AT.qkv; f.compute = rope_rows; f.ctx = &glob; f.timed = 1;
+    f.nout = 3; f.osrc[0] = AT.q; f.odst[0] = q; f.orow[0] = 2048 * 4; f.osrc[1] = AT.kc; f.odst[1] = kc; f.orow[1] = 512 * 2; f.osrc[2] = AT.vc; f.odst[2] = vc; f.orow[2] = 512 * 2;
+    const cudaError_t e = flow_run(&f, S.st);
+    if (e != cudaSuccess) { fail("gmoe", "gmoe_qk_rope of %d tokens: %s", nb, cudaGetErrorString(e)); return -1.0; }
+    return check_done("gmoe") ? -1.0 : f.secs;
 }
 
 /* ---- the attention projections (gpu_pre.m:200-256): every layer's q,k,v (group 2L) and o (group 2L+1) resident on the card.
@@ -948,9 +1004,11 @@ double gmoe_qk_rope(const float *qkv, const int *pos, int nb, int glob, const fl
 static struct {
     uint8_t *hcodes; float *hscales;            /* staged on the host until gpre_dense_done */
     uint8_t *codes; float *scales;              /* on the card: [rows][512] codes, [rows] scales */
-    int rows, staged; ExpertMaps maps;          /* maps.down: the 3-D map of the tcgen05 kernel (rows a multiple of 256) */
+    int rows, staged; ExpertMaps *maps;         /* on the card: maps->down = the 3-D map of the tcgen05 kernel (rows a multiple of 256) */
+    ExpertPtrs *tab;                            /* on the card */
 } DG[DGRP];
 static float *DY; static int DY_tok, DY_rows, dense_bad;
+static float *DH_qs; static int *DH_qsum;       /* one call's row scales and sums on the host */
 static TMap4 bmap_tok;                          /* the tokens' int8 rows [maxtok][2048] as the B operand */
 void gpre_dense_add(int g, const uint8_t *codes, const float *scales, int rows, int cols) {
     if (!S.ready) { fail("gpre", "gpre_dense_add before gpre_init"); dense_bad = 1; return; }
@@ -977,12 +1035,17 @@ int gpre_dense_done(int maxtok) {
         CU("gpre", cudaMemcpy(DG[g].codes, DG[g].hcodes, cb, cudaMemcpyHostToDevice));
         CU("gpre", cudaMemcpy(DG[g].scales, DG[g].hscales, sb, cudaMemcpyHostToDevice));
         free(DG[g].hcodes); free(DG[g].hscales); DG[g].hcodes = NULL; DG[g].hscales = NULL; DG[g].staged = 0;
+        ExpertPtrs tab; ExpertMaps maps; memset(&tab, 0, sizeof tab); memset(&maps, 0, sizeof maps);
+        tab.dc = DG[g].codes; tab.ds = DG[g].scales;
+        if (dmalloc((void **)&DG[g].tab, sizeof tab) || dmalloc((void **)&DG[g].maps, sizeof maps)) return fail("gpre", "no room for the attention projections of group %d", g);
+        CU("gpre", cudaMemcpy(DG[g].tab, &tab, sizeof tab, cudaMemcpyHostToDevice));
         if (DG[g].rows % 256 == 0) {   /* [rows/2 row pairs][2 parities][512 bytes], box = 128 row pairs x 1 parity x 128 bytes */
             cuuint64_t gdim[3] = {HID / 4, 2, (cuuint64_t)DG[g].rows / 2}, gstride[2] = {HID / 4, HID / 2};
             cuuint32_t box[3] = {128, 1, 128}, estr[3] = {1, 1, 1};
-            CUresult r = g_encode((CUtensorMap *)&DG[g].maps.down, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, DG[g].codes, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CUresult r = g_encode((CUtensorMap *)&maps.down, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, DG[g].codes, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (r != CUDA_SUCCESS) return fail("gpre", "cuTensorMapEncodeTiled failed (%d) for the projections of group %d", (int)r, g);
+            CU("gpre", cudaMemcpy(DG[g].maps, &maps, sizeof maps, cudaMemcpyHostToDevice));
         }
     }
     if (!ymax) return fail("gpre", "gpre_dense_done: no matrices were added");
@@ -990,33 +1053,40 @@ int gpre_dense_done(int maxtok) {
         cudaFree(DY); DY = NULL;
         if (dmalloc((void **)&DY, (size_t)maxtok * ymax * 4)) return fail("gpre", "no room for the attention projections' results");
         DY_tok = maxtok; DY_rows = ymax;
+        float *hq = realloc(DH_qs, (size_t)maxtok * 8);
+        if (!hq) { DY_tok = 0; return fail("gpre", "out of host memory"); }
+        DH_qs = hq; DH_qsum = (int *)hq + maxtok;
     }
     for (int i = 0; i < 4; i++) if (tmap_bytes_2d("gpre", &bmap_tok.m[i], S.hq, HID, (uint64_t)S.maxtok, HID, 128, 32 * (i + 1))) return -1;
+    return 0;
+}
+/* A call is cut into chunks of 256 tokens, whose rows cross the link in both directions while other chunks are multiplied: 14 us of kernel
+ * against 57 us for the 3.1 MB of q,k,v results, so a chunk need not fill the card. */
+#define DENSE_CHUNK 256
+typedef struct { int g, nb; } DenseCall;
+static int dense_rows(void *ctx, int r, int n) {
+    const DenseCall *c = ctx;
+    const int ys = DG[c->g].rows, um = n > 128 && ys % 256 == 0;
+    ExpertArgs a; memset(&a, 0, sizeof a);
+    a.tab = DG[c->g].tab; a.maps = DG[c->g].maps; a.err = S.err; a.dense_p0 = r; a.dense_n = n;
+    a.aq = S.hq; a.aqs = S.hqs; a.aqsum = S.hqsum; a.down = DY; a.down_stride = ys; a.dense_mblocks = ys / 256;
+    if (um) k_dense_umma(S.st, &a, &bmap_tok); else k_dense_mma(S.st, &a, ys);
     return 0;
 }
 double gpre_dense(int g, const float *x, int nb, float *y) {
     if (!S.ready || !DY) { fail("gpre", "gpre_dense before gpre_dense_done"); return -1.0; }
     if (g < 0 || g >= DGRP || !DG[g].codes) { fail("gpre", "gpre_dense: group %d has no matrices on the card", g); return -1.0; }
     if (nb < 1 || nb > DY_tok) { fail("gpre", "gpre_dense: %d tokens outside 1..%d", nb, DY_tok); return -1.0; }
-    const int ys = DG[g].rows, um = nb >= 512 && ys % 256 == 0, tn = um ? UMMA_TN : 32, nt = (nb + tn - 1) / tn;
-    memset(S.h_tab, 0, sizeof(ExpertPtrs));
-    S.h_tab[0].dc = DG[g].codes; S.h_tab[0].ds = DG[g].scales;
-    for (int i = 0; i < nt; i++) { MoeTile t = {0, i * tn, nb - i * tn < tn ? nb - i * tn : tn, 0}; S.h_tiles[i] = t; }
-    CUD("gpre", cudaMemcpyAsync(S.hn, x, (size_t)nb * HID * 4, cudaMemcpyHostToDevice, S.st));
-    CUD("gpre", cudaMemcpyAsync(S.tab_call, S.h_tab, sizeof(ExpertPtrs), cudaMemcpyHostToDevice, S.st));
-    CUD("gpre", cudaMemcpyAsync(S.maps_call, &DG[g].maps, sizeof(ExpertMaps), cudaMemcpyHostToDevice, S.st));
-    CUD("gpre", cudaMemcpyAsync(S.tiles_a, S.h_tiles, (size_t)nt * sizeof(MoeTile), cudaMemcpyHostToDevice, S.st));
-    CUD("gpre", cudaMemcpyAsync(S.ntiles_a, &nt, 4, cudaMemcpyHostToDevice, S.st));
-    cudaEventRecord(S.e0, S.st);
-    k_norm_prep(S.st, S.hn, NULL, S.hn, S.hq, S.hqs, S.hqsum, nb);          /* prep of maple.c:184-194 per token */
-    ExpertArgs a; memset(&a, 0, sizeof a);
-    a.tab = S.tab_call; a.maps = S.maps_call; a.tiles = S.tiles_a; a.ntiles = S.ntiles_a; a.max_tiles = nt; a.err = S.err;
-    a.aq = S.hq; a.aqs = S.hqs; a.aqsum = S.hqsum; a.down = DY; a.down_stride = ys; a.dense_mblocks = ys / 256;
-    if (um) k_dense_umma(S.st, &a, &bmap_tok); else k_dense_mma(S.st, &a, ys);
-    cudaEventRecord(S.e1, S.st);
-    CUD("gpre", cudaMemcpyAsync(y, DY, (size_t)nb * ys * 4, cudaMemcpyDeviceToHost, S.st));
+    if (S.keep && rows_in("gpre", S.hn, x, nb)) return -1.0;
+    DenseCall d = {g, nb};
+    Flow f; memset(&f, 0, sizeof f);
+    f.rows = nb; f.chunk = DENSE_CHUNK; f.src = x; f.row = HID * 4; f.dst = S.hq; f.quant = 1; f.hqs = DH_qs; f.hqsum = DH_qsum; f.dst_qs = S.hqs; f.qs_pitch = (size_t)S.maxtok;
+    f.compute = dense_rows; f.ctx = &d; f.timed = 1;
+    f.nout = 1; f.osrc[0] = DY; f.odst[0] = y; f.orow[0] = (size_t)DG[g].rows * 4;
+    const cudaError_t e = flow_run(&f, S.st);
+    if (e != cudaSuccess) { fail("gpre", "gpre_dense of %d tokens: %s", nb, cudaGetErrorString(e)); return -1.0; }
     S.nb_cur = nb;
-    return finish("gpre");
+    return check_done("gpre") ? -1.0 : f.secs;
 }
 int gpu_head_init(const uint16_t *w, int rows, int cols) { (void)w; (void)rows; (void)cols; return -1; }
 int gpu_head_init_i8(const int8_t *w, const float *scale, int rows, int cols) { (void)w; (void)scale; (void)rows; (void)cols; return -1; }
@@ -1249,9 +1319,7 @@ int gmoe_ep_timeout_selftest(int ms) {
         cudaMemcpy(tab, h_tab, sizeof h_tab, cudaMemcpyHostToDevice) == cudaSuccess) {
         EpXchArgs a = {NULL, (int *const *)tab, xch, epoch, 0, 2, (unsigned long long)(ms > 0 ? ms : 1) * 1000000ull, S.err};
         k_ep_exchange(S.st, &a);
-        if (cudaMemcpyAsync(S.h_err, S.err, 4, cudaMemcpyDeviceToHost, S.st) == cudaSuccess && cudaStreamSynchronize(S.st) == cudaSuccess) {
-            code = *S.h_err; *S.h_err = 0; cudaMemsetAsync(S.err, 0, 4, S.st); cudaStreamSynchronize(S.st);
-        }
+        if (cudaStreamSynchronize(S.st) == cudaSuccess) { code = *(volatile int *)S.h_err; *S.h_err = 0; }
     }
     cudaFree(xch); cudaFree(tab); cudaFree(epoch);
     return code < 0 ? fail("gmoe", "rendezvous self-test: %s", cudaGetErrorString(cudaGetLastError())) : code;

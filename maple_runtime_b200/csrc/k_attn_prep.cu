@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(256) qk_rope_kernel(const float *__restrict__ 
     float4 c4 = make_float4(0.f, 0.f, 0.f, 0.f), s4 = c4;
     if (!glob) {
         int p = pos[b];
-        if (p < 0 || p >= cs_positions) { if (lane == 0) atomicExch(err, 51); p = 0; }      // a position outside the table: flagged, not read
+        if (p < 0 || p >= cs_positions) { if (lane == 0) *(volatile int *)err = 51; p = 0; }      // a position outside the table: flagged, not read
         if (lane < 16) {
             const float4 *t = reinterpret_cast<const float4 *>(cs + ((size_t)p * 32 + 4 * (lane & 7)) * 2);      // (cos, sin) of four pairs
             const float4 t0 = t[0], t1 = t[1];

@@ -43,8 +43,10 @@ __global__ void __launch_bounds__(128) expert_mma_kernel(ExpertArgs a) {
     constexpr int TN = NBLK * 8, KB = KCH * 256;            // tokens per tile, bytes of one int8 activation vector
     extern __shared__ __align__(16) uint8_t smem[];          // [KCH][4][TN][4][16]
     const int tile_i = blockIdx.y;
-    const int ntiles = *a.ntiles;
-    const MoeTile tile = a.tiles[tile_i < a.max_tiles ? tile_i : 0];      // read beside the count, not after it
+    const bool dense = !GATEUP && KCH == 8;
+    const int ntiles = dense ? gridDim.y : *a.ntiles;
+    const MoeTile tile = dense ? MoeTile{0, a.dense_p0 + tile_i * TN, min(TN, a.dense_n - tile_i * TN), 0}
+                               : a.tiles[tile_i < a.max_tiles ? tile_i : 0];      // read beside the count, not after it
     if (tile_i >= ntiles) return;
     const ExpertPtrs ep = a.tab[tile.ex];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -190,10 +192,10 @@ extern "C" void k_down_mma(cudaStream_t st, const ExpertArgs *a, int tn) {
 // The attention projections (gpu_pre.m:200-256 gpre_dense*): the same int8 x 2-bit product with one matrix instead of 256
 // experts and every token in it: K = 2048, two 16-row blocks per warp, 128 rows per CTA, tiles of 32 tokens.
 extern "C" void k_dense_mma(cudaStream_t st, const ExpertArgs *a, int rows) {
-    if (a->max_tiles <= 0 || rows <= 0) return;
+    if (a->dense_n <= 0 || rows <= 0) return;
     const size_t smem = (size_t)8 * 4 * 32 * 64 + 32 * 8;
     static bool attr_done = false;
     if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<8, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
-    launch_k(expert_mma_kernel<8, 4, false>, dim3(rows / 128, a->max_tiles), 128, smem, st, *a);
+    launch_k(expert_mma_kernel<8, 4, false>, dim3(rows / 128, (a->dense_n + 31) / 32), 128, smem, st, *a);
     k_count_add(1);
 }

@@ -95,7 +95,10 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
     tc_fence_after();
     const uint32_t tb = sh->tmem_base;
     bool live = true;
-    const int nitems = *a.ntiles * MB;
+    const int ntiles = DENSE ? (a.dense_n + UM_TN - 1) / UM_TN : *a.ntiles, nitems = ntiles * MB;
+    auto tile_at = [&](const int i) {
+        return DENSE ? MoeTile{0, a.dense_p0 + i * UM_TN, min(UM_TN, a.dense_n - i * UM_TN), 0} : a.tiles[i];
+    };
 
     if (warp < 8) {
         // ---------------- decode: this warp's 32 rows of both halves, every second block, from the shared-memory ring ----------------
@@ -140,11 +143,11 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
         // ---------------- weight TMA (one lane): per stage the 128 rows of half 0 and the 128 of half 1, 512 columns ----------------
         if (lane == 0) {
             uint32_t wcnt = 0;
-            MoeTile tnext = blockIdx.x < nitems ? a.tiles[blockIdx.x / MB] : MoeTile{0, 0, 0, 0};      // one item ahead: no load latency at an item's start
+            MoeTile tnext = blockIdx.x < nitems ? tile_at(blockIdx.x / MB) : MoeTile{0, 0, 0, 0};      // one item ahead: no load latency at an item's start
             for (int item = blockIdx.x; item < nitems && live; item += gridDim.x) {
                 const MoeTile tile = tnext;
                 if (item + (int)gridDim.x < nitems) {
-                    tnext = a.tiles[(item + gridDim.x) / MB];
+                    tnext = tile_at((item + gridDim.x) / MB);
                     const ExpertMaps *en = a.maps + tnext.ex;              // the next item's expert: its maps are in the descriptor cache when its copies start
                     if (GATEUP) { tma_prefetch_map(&en->gate); tma_prefetch_map(&en->up); } else tma_prefetch_map(&en->down);
                 }
@@ -169,10 +172,10 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
         // ---------------- B TMA (one lane): per 128-column block one box of the pair-ordered int8 activations ----------------
         if (lane == 0) {
             uint32_t bcnt = 0;
-            MoeTile tnext = blockIdx.x < nitems ? a.tiles[blockIdx.x / MB] : MoeTile{0, 0, 0, 0};
+            MoeTile tnext = blockIdx.x < nitems ? tile_at(blockIdx.x / MB) : MoeTile{0, 0, 0, 0};
             for (int item = blockIdx.x; item < nitems && live; item += gridDim.x) {
                 const MoeTile tile = tnext;
-                if (item + (int)gridDim.x < nitems) tnext = a.tiles[(item + gridDim.x) / MB];
+                if (item + (int)gridDim.x < nitems) tnext = tile_at((item + gridDim.x) / MB);
                 // only as many rows as the tile has pairs, in steps of 32 (the MMA reads (cnt + 15) & ~15 <= that many)
                 const int bi = tile.cnt > 0 ? (tile.cnt - 1) >> 5 : 0;
                 for (int kb = 0; kb < KB && live; kb++, bcnt++) {
@@ -191,10 +194,10 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
         const uint32_t sfull0 = smem_u32(&sh->s_full[0]), sempty0 = smem_u32(&sh->s_empty[0]);
         const uint32_t bfull0 = smem_u32(&sh->b_full[0]), bempty0 = smem_u32(&sh->b_empty[0]);
         uint32_t as = 0, ap = 0, bs = 0, bp = 0, icnt = 0;
-        int cnt_next = blockIdx.x < nitems ? a.tiles[blockIdx.x / MB].cnt : 0;
+        int cnt_next = blockIdx.x < nitems ? tile_at(blockIdx.x / MB).cnt : 0;
         for (int item = blockIdx.x; item < nitems && live; item += gridDim.x, icnt++) {
             const int cnt = __shfl_sync(0xffffffffu, cnt_next, 0);
-            if (item + (int)gridDim.x < nitems) cnt_next = a.tiles[(item + gridDim.x) / MB].cnt;
+            if (item + (int)gridDim.x < nitems) cnt_next = tile_at((item + gridDim.x) / MB).cnt;
             const uint32_t idesc = idesc_i8_u8s8((uint32_t)((cnt + 15) & ~15));
             const uint32_t buf = icnt % NACC, d = tb + buf * (2 * UM_TN) + h * UM_TN;
             if (!mbar_wait(&sh->acc_empty[buf], ((icnt / NACC) & 1) ^ 1, abortp)) { live = false; break; }
@@ -227,8 +230,8 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
         // to shared memory when the item starts), so that an item starts without a dependent global read in front of it.
         const int stride = gridDim.x;
         constexpr int HN = UM_TN / 32;
-        MoeTile t1 = blockIdx.x < nitems ? a.tiles[blockIdx.x / MB] : MoeTile{0, 0, 0, 0};
-        MoeTile t2 = (int)blockIdx.x + stride < nitems ? a.tiles[(blockIdx.x + stride) / MB] : MoeTile{0, 0, 0, 0};
+        MoeTile t1 = blockIdx.x < nitems ? tile_at(blockIdx.x / MB) : MoeTile{0, 0, 0, 0};
+        MoeTile t2 = (int)blockIdx.x + stride < nitems ? tile_at((blockIdx.x + stride) / MB) : MoeTile{0, 0, 0, 0};
         ExpertPtrs ep1 = a.tab[t1.ex];
         float h_qs[HN]; int h_qsum[HN]; unsigned long long h_dst[HN];
         auto header_load = [&](const MoeTile &t) {      // the values of tokens lane, lane + 32, lane + 64 of tile t (clamped to its pairs)
@@ -262,7 +265,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
             }
             __syncwarp();
             t1 = t2; ep1 = a.tab[t1.ex];
-            if (item + 2 * stride < nitems) t2 = a.tiles[(item + 2 * stride) / MB];
+            if (item + 2 * stride < nitems) t2 = tile_at((item + 2 * stride) / MB);
             if (item + stride < nitems) header_load(t1);                     // in flight while this item's pieces are worked on
             if (!mbar_wait(&sh->acc_full[buf], (icnt / NACC) & 1, abortp)) { live = false; break; }
             tc_fence_after();
@@ -442,7 +445,7 @@ static void launch(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) {
 extern "C" void k_gateup_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->max_tiles > 0) launch<16, 0>(st, a, bmap); }
 extern "C" void k_down_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->max_tiles > 0) launch<4, 1>(st, a, bmap); }
 /* dense projections: tab[ex].ds / maps[ex].down of a matrix of 256 * a->dense_mblocks rows x 2048 columns, B rows = the tokens' int8 rows */
-extern "C" void k_dense_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->max_tiles > 0) launch<16, 2>(st, a, bmap); }
+extern "C" void k_dense_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->dense_n > 0) launch<16, 2>(st, a, bmap); }
 
 // ---- rows of the per-token int8 matrix copied into pair (expert-grouped) order: the B operand the TMA can tile ----
 __global__ void __launch_bounds__(256) gather_rows_kernel(const int8_t *__restrict__ src, const int *__restrict__ rows, int8_t *__restrict__ dst, int np) {

@@ -156,7 +156,7 @@ __global__ void __maxnreg__(224) router_tile_kernel(const uint8_t *__restrict__ 
         }
     }
     __syncthreads();
-    if (tid == 0 && sh.abort) atomicExch(err, 31);      // a wait ran out: the host reports it and the logits are not to be used
+    if (tid == 0 && sh.abort) *(volatile int *)err = 31;      // a wait ran out: the host reports it and the logits are not to be used
 }
 
 extern "C" void k_router_pack(cudaStream_t st, const uint16_t *router, void *router_t) {
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(256, 2) router_small_kernel(const uint8_t *__r
         float *dst = logits + (size_t)(b0 + tok) * NEXP + e;
         dst[0] = bias ? __fadd_rn(l0, bias[e]) : l0; dst[1] = bias ? __fadd_rn(l1, bias[e + 1]) : l1;
     }
-    if (tid == 0 && !ok) atomicExch(err, 31);
+    if (tid == 0 && !ok) *(volatile int *)err = 31;
 }
 extern "C" void k_router_pack_small(cudaStream_t st, const uint16_t *router, void *router_s) {
     router_pack_w_small_kernel<<<NEXP * HID / 4 / 256, 256, 0, st>>>(router, (uint2 *)router_s);

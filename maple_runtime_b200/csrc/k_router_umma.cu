@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(192, 1) router_umma_kernel(const __grid_consta
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tb, 256);
-        if (lane == 0 && sh.abort_flag) atomicExch(err, 31);
+        if (lane == 0 && sh.abort_flag) *(volatile int *)err = 31;
     }
 }
 

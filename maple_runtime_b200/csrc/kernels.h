@@ -30,6 +30,7 @@ typedef struct {
     float *down;             /* [np][2048], or [np][down_stride] when down_stride != 0 (the dense projections: several matrices side by side) */
     int down_stride;
     int dense_mblocks;       /* k_dense_umma: 256-row blocks of the matrix */
+    int dense_p0, dense_n;   /* k_dense_*: the first token and the token count; there is no tile list, tile t is tokens dense_p0 + t * (tile size) .. */
     /* decode path: the down kernel quantises the fp32 SiLU outputs itself (no separate pass): act_for_down [np][512] in, and the
      * int8 rows, scales and sums it computed are also stored here for later inspection */
     const float *act_for_down; int8_t *aq_out; float *aqs_out; int *aqsum_out;
@@ -44,6 +45,11 @@ typedef struct {
 } ExpertArgs;
 
 void k_count_reset(void); long k_count(void);
+
+/* n arrays of 4-byte words copied to dst from page-locked host memory (16-byte aligned), by one kernel */
+#define TABLE_SEGS 16
+typedef struct { void *dst[TABLE_SEGS]; const void *src[TABLE_SEGS]; unsigned words[TABLE_SEGS]; int n; } TableSegs;
+void k_tables(cudaStream_t st, const TableSegs *t);
 
 void k_norm_prep(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, int nb);
 /* the same, and the normalised rows once more in the decode router's layout (hS, nb*HID*4 bytes): k_router_logits_small then takes relaid = 1 */
