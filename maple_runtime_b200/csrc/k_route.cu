@@ -310,10 +310,119 @@ static void launch_group_cta(cudaStream_t st, const GroupArgs *g) {
     if (!attr_done) { cudaFuncSetAttribute(group_cta_kernel<MAXTOK, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr_done = true; }
     launch_k(group_cta_kernel<MAXTOK, NT>, 1, NT, smem, st, *g);
 }
+// 257 to GROUP_CLUSTER_MAX tokens: one launch of one cluster of CTAS CTAs.  CTA r owns its share of the tokens (in whole
+// words of 32) and keeps their bits in its shared memory; the counts are exchanged through distributed shared memory, after which every CTA
+// scans the experts for itself and its threads place one token each.  Bound by latency: what counts is the number of launches (a launch costs
+// the host 3.9 us; clearing, marking and placing as three kernels took 16.4 us per call at 1000 tokens, 10.2 us like this) and of trips through
+// global memory (inside a layer of 2048 tokens, against the router setting the bits and the place kernel reading them: 4 us less).  Eight
+// CTAs are what every GPU has to allow; from 513 tokens on sixteen share the scattered stores (2048 tokens: 14.4 -> 11.9 us).
+#define GC_WORDS 8
+template <int GC_CTAS>
+__global__ void __launch_bounds__(NEXP) group_cluster_kernel(GroupArgs g) {
+    __shared__ unsigned s_mask[NEXP][GC_WORDS + 1];           // + 1: a warp's 32 experts of one word lie in 32 banks
+    __shared__ unsigned short s_pre[NEXP][GC_WORDS + 1];      // the pairs of the CTA's expert in front of word w
+    __shared__ int s_cnt[NEXP], s_start[NEXP];
+    __shared__ int w_cnt[8], w_used[8], w_ta[8], w_tb[8];
+    const int e = threadIdx.x, lane = e & 31, wid = e >> 5, nb = g.nb;
+    const int per = (((nb + 31) / 32 + GC_CTAS - 1) / GC_CTAS) * 32, tok = blockIdx.x * per + e;      // per <= 32 GC_WORDS = one token per thread
+    const bool mine = e < per && tok < nb;
+    const bool wide = (((uintptr_t)g.top | (uintptr_t)g.topw | (uintptr_t)g.tp | (uintptr_t)g.slot) & 15) == 0;      // the caller's arrays may lie anywhere
+    int x[TOPK]; float w[TOPK];
+    if (mine) {
+        const int *tr = g.top + (size_t)tok * TOPK; const float *wr = g.topw + (size_t)tok * TOPK;
+        if (wide) {
+            const int4 a = reinterpret_cast<const int4 *>(tr)[0], b = reinterpret_cast<const int4 *>(tr)[1];
+            const float4 c = reinterpret_cast<const float4 *>(wr)[0], d = reinterpret_cast<const float4 *>(wr)[1];
+            x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+            w[0] = c.x; w[1] = c.y; w[2] = c.z; w[3] = c.w; w[4] = d.x; w[5] = d.y; w[6] = d.z; w[7] = d.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < TOPK; k++) { x[k] = tr[k]; w[k] = wr[k]; }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k <= GC_WORDS; k++) (&s_mask[0][0])[e + k * NEXP] = 0u;
+    __syncthreads();
+    if (mine)
+#pragma unroll
+        for (int k = 0; k < TOPK; k++) atomicOr(&s_mask[x[k]][wid], 1u << lane);
+    __syncthreads();
+    int own = 0;
+#pragma unroll
+    for (int k = 0; k < GC_WORDS; k++) { s_pre[e][k] = (unsigned short)own; own += __popc(s_mask[e][k]); }
+    s_cnt[e] = own;
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    int cnt = 0, before = 0;
+#pragma unroll
+    for (int r = 0; r < GC_CTAS; r++) {
+        uint32_t at; int v;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(&s_cnt[e])), "r"(r));
+        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+        cnt += v; if (r < (int)blockIdx.x) before += v;
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // this CTA has read the others' counts
+    const int used = cnt > 0, na = (cnt + g.tn_a - 1) / g.tn_a, nt = (cnt + g.tn_b - 1) / g.tn_b;
+    int c = cnt, u = used, a = na, b = nt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int tc = __shfl_up_sync(0xffffffffu, c, o), tu = __shfl_up_sync(0xffffffffu, u, o);
+        const int t1 = __shfl_up_sync(0xffffffffu, a, o), t2 = __shfl_up_sync(0xffffffffu, b, o);
+        if (lane >= o) { c += tc; u += tu; a += t1; b += t2; }
+    }
+    if (lane == 31) { w_cnt[wid] = c; w_used[wid] = u; w_ta[wid] = a; w_tb[wid] = b; }
+    __syncthreads();
+    int oc = 0, ou = 0, oa = 0, ob = 0;
+    for (int k = 0; k < wid; k++) { oc += w_cnt[k]; ou += w_used[k]; oa += w_ta[k]; ob += w_tb[k]; }
+    const int start = oc + c - cnt, uidx = ou + u - used, ta0 = oa + a - na, tb0 = ob + b - nt;
+    s_start[e] = start + before;
+    __syncthreads();
+    if (mine) {
+        int sl[TOPK];
+#pragma unroll
+        for (int k = 0; k < TOPK; k++) sl[k] = s_start[x[k]] + s_pre[x[k]][wid] + __popc(s_mask[x[k]][wid] & ((1u << lane) - 1u));
+#pragma unroll
+        for (int k = 0; k < TOPK; k++) { g.utok[sl[k]] = tok; g.uw[sl[k]] = w[k]; if (g.uexp) g.uexp[sl[k]] = x[k]; }
+        int *sp = g.slot + (size_t)tok * TOPK, *tq = g.tp + (size_t)tok * TOPK;
+        if (wide) { reinterpret_cast<int4 *>(sp)[0] = make_int4(sl[0], sl[1], sl[2], sl[3]); reinterpret_cast<int4 *>(sp)[1] = make_int4(sl[4], sl[5], sl[6], sl[7]); }
+        else {
+#pragma unroll
+            for (int k = 0; k < TOPK; k++) sp[k] = sl[k];
+        }
+#pragma unroll
+        for (int i = 1; i < TOPK; i++)
+#pragma unroll
+            for (int k = TOPK - 1; k >= 1; k--) if (k >= i && sl[k] < sl[k - 1]) { const int t = sl[k]; sl[k] = sl[k - 1]; sl[k - 1] = t; }
+        if (wide) { reinterpret_cast<int4 *>(tq)[0] = make_int4(sl[0], sl[1], sl[2], sl[3]); reinterpret_cast<int4 *>(tq)[1] = make_int4(sl[4], sl[5], sl[6], sl[7]); }
+        else {
+#pragma unroll
+            for (int k = 0; k < TOPK; k++) tq[k] = sl[k];
+        }
+    }
+    if (blockIdx.x == GC_CTAS - 1) {                           // the CTA with the fewest tokens writes the experts' tables
+        if (g.ecnt) g.ecnt[e] = cnt;
+        g.estart[e] = used ? start : -1;
+        if (used) {
+            g.ue[uidx] = e; g.ustart[uidx] = start;
+            for (int t = 0; t < na; t++) { const MoeTile m = {uidx, start + t * g.tn_a, min(g.tn_a, cnt - t * g.tn_a), e}; g.tiles_a[ta0 + t] = m; }
+            for (int t = 0; t < nt; t++) { const MoeTile m = {uidx, start + t * g.tn_b, min(g.tn_b, cnt - t * g.tn_b), e}; g.tiles_b[tb0 + t] = m; }
+        }
+        if (e == NEXP - 1) { const int nu = uidx + used; *g.nu = nu; g.ustart[nu] = start + cnt; *g.ntiles_a = ta0 + na; *g.ntiles_b = tb0 + nt; }
+    }
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");        // the others have read this CTA's counts: it may go
+}
 extern "C" void k_group(cudaStream_t st, const GroupArgs *g) {
     if (g->nb <= 0) return;
     if (g->nb <= 256) { launch_group_cta<256, 256>(st, g); g_launches++; return; }
     const int np = g->nb * TOPK;
+    if (g->nb <= GROUP_CLUSTER_MAX) {
+        if (g->nb <= 512) launch_cluster(group_cluster_kernel<8>, 8, NEXP, st, *g);
+        else {
+            static bool attr_done = false;
+            if (!attr_done) { cudaFuncSetAttribute(group_cluster_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); attr_done = true; }
+            launch_cluster(group_cluster_kernel<16>, 16, NEXP, st, *g);
+        }
+        g_launches++; return;
+    }
     if (!g->marked) {
         const int zw = NEXP * g->mask_words + NEXP;                                           // bit words + the 256 counters behind them
         launch_k(zero_words_kernel, (zw + 1023) / 1024, 1024, 0, st, g->mask, zw);

@@ -66,6 +66,7 @@ void k_topk(cudaStream_t st, const float *logits, int *top, float *topw, int nb)
 /* norm + int8 as k_norm_prep, and the normalised rows once more as two fp16 terms per value (hA: [nb][4096] fp16, hi then lo) with the
  * rows' Euclidean norms (hnorm [nb]): the A operand of the tensor-core router */
 void k_norm_prep_split(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, void *hA, float *hnorm, int nb);
+#define GROUP_CLUSTER_MAX 4096      /* up to here k_group makes its own bits; above it the routing kernels may set them (GroupArgs.marked) */
 typedef struct {
     const int *top; const float *topw; int nb;
     unsigned *mask;          /* [mask_words][256] bit words (bit b % 32 of word b / 32: token b chose the expert), then 256 counters */

@@ -12,3 +12,12 @@ static inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 blo
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
+// the same as one cluster of `ctas` CTAs
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_cluster(void (*kernel)(KArgs...), unsigned ctas, dim3 block, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof cfg);
+    cudaLaunchAttribute at; memset(&at, 0, sizeof at);
+    at.id = cudaLaunchAttributeClusterDimension; at.val.clusterDim.x = ctas; at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = ctas; cfg.blockDim = block; cfg.stream = st; cfg.attrs = &at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
