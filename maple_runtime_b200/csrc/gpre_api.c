@@ -353,7 +353,9 @@ int gmoe_profile_read(double *secs, long *launches) {
 /* ---- the stages ------------------------------------------------------------------------------------------------ */
 static int tile_tn(int nb) { return nb <= 256 ? 8 : 32; }
 
-static int use_umma(int nb) { return S.path == 2 || (S.path == 0 && nb >= 512); }
+/* Which expert kernels: up to 256 tokens the mma.sync kernels on tiles of 8, above that the tcgen05 kernels.  At 301 tokens gate+up, SiLU and down
+ * take 123 us per layer on the mma.sync kernels' tiles of 32 and 76 us on the tcgen05 kernels; at 256 the two are level. */
+static int use_umma(int nb) { return S.path == 2 || (S.path == 0 && nb > 256); }
 static void fill_expert_args(ExpertArgs *a, const ExpertPtrs *tab, const ExpertMaps *maps, const int *ue, int nb) {
     memset(a, 0, sizeof *a);
     a->tab = tab; a->maps = maps; a->ue = ue; a->ptok = S.utok; a->err = S.err;
@@ -365,7 +367,7 @@ static void fill_expert_args(ExpertArgs *a, const ExpertPtrs *tab, const ExpertM
     if (S.keep) { a->gu_dots = S.gu_dots; a->dn_dots = S.dn_dots; }
 }
 static void run_group_m(int nb, int marked) {
-    GroupArgs g; memset(&g, 0, sizeof g); g.marked = marked && nb > 256;
+    GroupArgs g; memset(&g, 0, sizeof g); g.marked = marked && nb > GROUP_CLUSTER_MAX;
     g.top = S.top; g.topw = S.topw; g.nb = nb; g.mask = S.mask; g.mask_words = S.mask_words; g.nu = S.nu; g.ue = S.ue; g.estart = S.estart;
     g.ustart = S.ustart; g.utok = S.utok; g.slot = S.slot; g.tp = S.tp; g.uw = S.uw; g.ecnt = S.ecnt; g.uexp = S.uexp;
     g.tiles_a = S.tiles_a; g.tiles_b = S.tiles_b; g.ntiles_a = S.ntiles_a; g.ntiles_b = S.ntiles_b; g.tn_a = tile_tn(nb); g.tn_b = UMMA_TN;
@@ -403,8 +405,9 @@ static void run_combine(const float *const *dsp, int nb, const float *init, floa
     if (use_umma(nb)) k_combine_wire(S.st, S.wire, S.maxp, dsp, S.uw, S.tp, init, out, nb);
     else k_combine(S.st, S.down, S.uw, S.tp, init, out, nb);
 }
-/* router logits: batches past the decode sizes take the tiled kernel, decode batches the one-wait kernel, both on re-laid rows */
-#define ROUTER_TILE_MIN 257
+/* router logits: large batches take the tiled kernel, small ones the one-wait kernel, both on re-laid rows.  The tiled kernel takes 38 us for any
+ * batch from 257 to 511 tokens (at most 64 CTAs), the other 28.6 at 301, 33.1 at 400 and 40.2 at 511. */
+#define ROUTER_TILE_MIN 417
 static void run_router_relaid(const LayerDev *l, const float *bias, int nb, int relaid) {   /* relaid: the norm kernel already wrote S.hT */
     if (nb >= ROUTER_TILE_MIN) k_router_logits_tile(S.st, l->router_t, S.hn, S.hT, bias, S.logits, nb, S.err);
     else k_router_logits_small(S.st, l->router_s, S.hn, S.hT, relaid, bias, S.logits, nb, S.err);
@@ -421,7 +424,7 @@ static void run_router_tensor_m(const LayerDev *l, const float *bias, int nb, in
     r.amap = S.amap; r.wmap = l->wmap; r.part = S.rpart; r.nb = nb; r.ntok_cap = S.maxtok; r.err = S.err;
     r.bias = bias; r.hnorm = S.hnorm; r.wnorm = l->wnorm; r.hn = S.hn; r.router_s = l->router_s;
     r.logits = S.logits; r.top = S.top; r.topw = S.topw; r.flagged = S.flagged; r.nflagged = S.nflagged; r.done = S.rdone;
-    if (mark && nb > 256) { r.mask = S.mask; r.mask_words = S.mask_words; }      /* the grouping's bits and counters come out of the routing kernels */
+    if (mark && nb > GROUP_CLUSTER_MAX) { r.mask = S.mask; r.mask_words = S.mask_words; }      /* the grouping's bits and counters come out of the routing kernels */
     k_router_tensor(S.st, &r);
 }
 static void run_router_tensor(const LayerDev *l, const float *bias, int nb) { run_router_tensor_m(l, bias, nb, 0); }
