@@ -11,6 +11,7 @@
 #include "launch.cuh"
 #include "dev_math.cuh"
 #include "topk.cuh"
+#include "silu_row.cuh"
 
 static long g_launches = 0;
 extern "C" void k_count_reset(void) { g_launches = 0; }
@@ -467,26 +468,10 @@ extern "C" void k_actq(cudaStream_t st, const float *act, int8_t *aq, float *aqs
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// SiLU*up + int8 in one pass (maple.c:825-832) for the tensor-core path, whose GEMM stores gate and up: one warp per
-// pair, 16 values per lane: columns 128 i + 4 lane .. + 3 for i = 0..3, so that every load and store instruction of the warp covers
-// one contiguous run of the row.  act (optional) receives the fp32 activations for stage comparisons.
-//
-// The int8 row, its scale and its sum are the reference's bits in both variants.  EXACT evaluates every element with the libm-equal
-// expf in double (dev_math.cuh).  The other variant evaluates act ~ g / (1 + 2^(-g log2 e)) u with the hardware's approximate
-// exponential and reciprocal (relative error below SQ_EPS for every g <= 7 that does not underflow) and falls back to the exact
-// evaluation only where the approximation could change a result:
-//   * the row maximum: every element within 2 SQ_EPS of the approximate maximum is evaluated exactly, the exact maximum is among them;
-//   * a rounded value: t = act * inv lands within |t| (2 SQ_EPS + 2^-22) of a rounding boundary (about one element in two thousand).
+// SiLU*up + int8 in one pass (maple.c:825-832) for the tensor-core path, whose GEMM stores gate and up: one warp per pair.  EXACT evaluates
+// every element with the libm-equal expf in double (dev_math.cuh) and can also store the fp32 activations (act, optional) for stage
+// comparisons; the other variant is silu_row.cuh.  The results are the reference's bits in both.
 // ------------------------------------------------------------------------------------------------------------
-#define SQ_EPS 1.2e-5f
-__device__ __forceinline__ float silu_mul_approx(float g, float u) {
-    g = g < 7.0f ? g : 7.0f;
-    u = u < -7.0f ? -7.0f : (u > 7.0f ? 7.0f : u);
-    float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-    return g * r * u;
-}
 template <bool EXACT>
 __global__ void __launch_bounds__(256, 4) silu_quant_kernel(const float *__restrict__ gate, const float *__restrict__ up, float *__restrict__ act,
                                                          int8_t *__restrict__ aq, float *__restrict__ aqs, int *__restrict__ aqsum, int np, const int *__restrict__ np_dev) {
@@ -498,15 +483,16 @@ __global__ void __launch_bounds__(256, 4) silu_quant_kernel(const float *__restr
     if (a >= np) return;
     const float4 *gr = reinterpret_cast<const float4 *>(gate + (size_t)a * FFN) + lane;
     const float4 *ur = reinterpret_cast<const float4 *>(up + (size_t)a * FFN) + lane;
-    float gv[16], uv[16], v[16];
+    float4 g4[4], u4[4]; float s; int tot; uint32_t pk[4] = {0, 0, 0, 0};
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float4 g = gr[32 * i], u = ur[32 * i];
-        gv[4 * i] = g.x; gv[4 * i + 1] = g.y; gv[4 * i + 2] = g.z; gv[4 * i + 3] = g.w;
-        uv[4 * i] = u.x; uv[4 * i + 1] = u.y; uv[4 * i + 2] = u.z; uv[4 * i + 3] = u.w;
-    }
-    float mx = 0.0f;
+    for (int i = 0; i < 4; i++) { g4[i] = gr[32 * i]; u4[i] = ur[32 * i]; }
     if (EXACT) {
+        float gv[16], uv[16], v[16], mx = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            gv[4 * i] = g4[i].x; gv[4 * i + 1] = g4[i].y; gv[4 * i + 2] = g4[i].z; gv[4 * i + 3] = g4[i].w;
+            uv[4 * i] = u4[i].x; uv[4 * i + 1] = u4[i].y; uv[4 * i + 2] = u4[i].z; uv[4 * i + 3] = u4[i].w;
+        }
 #pragma unroll
         for (int i = 0; i < 16; i++) { v[i] = dev_silu_mul_tab(gv[i], uv[i], tab); mx = fmaxf(mx, fabsf(v[i])); }
         if (act) {
@@ -516,38 +502,16 @@ __global__ void __launch_bounds__(256, 4) silu_quant_kernel(const float *__restr
         }
 #pragma unroll
         for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    } else {
-        float mxa = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 16; i++) { v[i] = silu_mul_approx(gv[i], uv[i]); mxa = fmaxf(mxa, fabsf(v[i])); }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) mxa = fmaxf(mxa, __shfl_xor_sync(0xffffffffu, mxa, o));
-        const float thr = mxa * (1.0f - 2.5f * SQ_EPS) - 1e-30f;      // every element that can be the exact maximum
-#pragma unroll
-        for (int i = 0; i < 16; i++) if (!(fabsf(v[i]) < thr)) mx = fmaxf(mx, fabsf(dev_silu_mul_tab(gv[i], uv[i], tab)));
-#pragma unroll
-        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    }
-    const float s = mx > 0.0f ? __fdiv_rn(mx, 127.0f) : 1.0f, inv = __fdiv_rn(1.0f, s);
-    int tot = 0; uint32_t pk[4] = {0, 0, 0, 0};
-    if (EXACT) {
+        s = mx > 0.0f ? __fdiv_rn(mx, 127.0f) : 1.0f;
+        const float inv = __fdiv_rn(1.0f, s);
+        tot = 0;
 #pragma unroll
         for (int i = 0; i < 16; i++) { int qi = __float2int_rn(__fmul_rn(v[i], inv)); tot += qi; pk[i >> 2] |= (uint32_t)(qi & 0xFF) << (8 * (i & 3)); }
-    } else {
-        const float slack = 1e-36f * inv;                                // elements the approximation flushed to zero
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const float t = __fmul_rn(v[i], inv), big = __fadd_rn(t, 12582912.0f), r = __fsub_rn(big, 12582912.0f);      // r = t rounded to an integer, half to even
-            int qi = __float_as_int(big) - 0x4B400000;
-            if (!(0.5f - fabsf(__fsub_rn(t, r)) > fabsf(t) * (2.0f * SQ_EPS + 2.4e-7f) + slack))
-                qi = __float2int_rn(__fmul_rn(dev_silu_mul_tab(gv[i], uv[i], tab), inv));
-            tot += qi; pk[i >> 2] |= (uint32_t)(qi & 0xFF) << (8 * (i & 3));
-        }
-    }
+        for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    } else silu_quant_row(g4, u4, gate + (size_t)a * FFN, up + (size_t)a * FFN, tab, lane, pk, s, tot);
 #pragma unroll
     for (int i = 0; i < 4; i++) reinterpret_cast<uint32_t *>(aq + (size_t)a * FFN)[32 * i + lane] = pk[i];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
     if (lane == 0) { aqs[a] = s; aqsum[a] = tot; }
 }
 extern "C" void k_silu_quant(cudaStream_t st, const float *gate, const float *up, float *act, int8_t *aq, float *aqs, int *aqsum, int np, const int *np_dev) {
