@@ -5,6 +5,8 @@
 // operand without touching shared memory.  This is the path for decode batches (a few tokens per expert, bound by
 // the weight stream) and the fallback for any token count.
 //
+// Launched programmatically (launch.cuh): while the last gate+up CTAs run, the first down CTAs already hold their weights.
+//
 // Arithmetic = maple.c:425-458 (tdot_multi): tot = sum(code * q) over the row, out = (float)(tot - qsum) * qs * s[r].
 // Integer sums are exact, so any summation order gives the reference's int32.
 //
@@ -35,6 +37,10 @@ __device__ __forceinline__ uint4 ldg_stream(const uint8_t *p) {   // weights are
     return v;
 }
 
+__device__ __forceinline__ MoeTile ldcg_tile(const MoeTile *t) {
+    const int4 v = __ldcg(reinterpret_cast<const int4 *>(t)); return MoeTile{v.x, v.y, v.z, v.w};
+}
+
 // KCH: K-chunks of 256 columns (8 for gate/up K=2048, 2 for down K=512).  NBLK: 8-token blocks per tile.
 // GATEUP: rows block A = gate rows, block B = up rows of the same index, epilogue = SiLU*up;
 // otherwise A and B are two consecutive 16-row blocks of the down matrix, epilogue = scale only.
@@ -43,11 +49,12 @@ __global__ void __launch_bounds__(128) expert_mma_kernel(ExpertArgs a) {
     constexpr int TN = NBLK * 8, KB = KCH * 256;            // tokens per tile, bytes of one int8 activation vector
     extern __shared__ __align__(16) uint8_t smem[];          // [KCH][4][TN][4][16]
     const int tile_i = blockIdx.y;
+    if (GATEUP) { pdl_wait(); pdl_trigger(); }       // the tiles are its predecessor's; the down kernel's are two kernels old, so that its weights come in before its wait
     const bool dense = !GATEUP && KCH == 8;
-    const int ntiles = dense ? gridDim.y : *a.ntiles;
+    const int ntiles = dense ? gridDim.y : __ldcg(a.ntiles);
     const MoeTile tile = dense ? MoeTile{0, a.dense_p0 + tile_i * TN, min(TN, a.dense_n - tile_i * TN), 0}
-                               : a.tiles[tile_i < a.max_tiles ? tile_i : 0];      // read beside the count, not after it
-    if (tile_i >= ntiles) return;
+                               : ldcg_tile(a.tiles + (tile_i < a.max_tiles ? tile_i : 0));      // read beside the count, not after it
+    if (tile_i >= ntiles) { if (!GATEUP) { pdl_wait(); pdl_trigger(); } return; }
     const ExpertPtrs ep = a.tab[tile.ex];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
 
@@ -64,6 +71,7 @@ __global__ void __launch_bounds__(128) expert_mma_kernel(ExpertArgs a) {
         wq[p][2] = ldg_stream(wb + p * 64); wq[p][3] = ldg_stream(wb + 8 * (KB / 4) + p * 64);
     }
 
+    if (!GATEUP) { pdl_wait(); pdl_trigger(); }
     // stage the tile's activation vectors (16-byte pieces) in fragment order
     if (GATEUP || !a.act_for_down) {
         const int8_t *src = GATEUP ? a.hq : a.aq;
@@ -177,7 +185,7 @@ static void launch(cudaStream_t st, const ExpertArgs *a) {
     static bool attr_done = false;
     if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<KCH, NBLK, GATEUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
     dim3 grid(GATEUP ? 8 : 16, a->max_tiles);
-    launch_k(expert_mma_kernel<KCH, NBLK, GATEUP>, grid, 128, smem, st, *a);
+    launch_pdl(expert_mma_kernel<KCH, NBLK, GATEUP>, grid, 128, smem, st, *a);
     k_count_add(1);
 }
 extern "C" void k_gateup_mma(cudaStream_t st, const ExpertArgs *a, int tn) {

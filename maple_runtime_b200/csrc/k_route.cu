@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(WPC * 32) norm_prep_kernel(const float *__rest
                                                              float *__restrict__ qs, int *__restrict__ qsum, float *__restrict__ hS,
                                                              __half *__restrict__ hA, float *__restrict__ hnorm, int nb) {
     const int lane = threadIdx.x & 31, b = blockIdx.x * WPC + (threadIdx.x >> 5);
+    pdl_wait(); pdl_trigger();
     if (b >= nb) return;
     const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)b * HID) + lane;
     float4 v[16];
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(WPC * 32) norm_prep_kernel(const float *__rest
 static void norm_launch(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, __half *hA, float *hnorm, int nb) {
     if (nb <= 0) return;
     if (nb > 256) launch_k(norm_prep_kernel<8>, (nb + 7) / 8, 256, 0, st, x, w, hn, q, qs, qsum, hS, hA, hnorm, nb);
-    else launch_k(norm_prep_kernel<1>, nb, 32, 0, st, x, w, hn, q, qs, qsum, hS, hA, hnorm, nb);
+    else launch_pdl(norm_prep_kernel<1>, nb, 32, 0, st, x, w, hn, q, qs, qsum, hS, hA, hnorm, nb);
     g_launches++;
 }
 extern "C" void k_norm_prep(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, int nb) {
@@ -135,6 +136,7 @@ __global__ void __launch_bounds__(256) topk_kernel(const float *__restrict__ log
     __shared__ unsigned long long tab[32];                  // the expf table beside the arithmetic (lane-varying index)
     if (threadIdx.x < 32) tab[threadIdx.x] = DEV_EXP_TAB[threadIdx.x];
     __syncthreads();
+    pdl_wait(); pdl_trigger();
     const int lane = threadIdx.x & 31;
     const int b = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (b >= nb) return;
@@ -150,7 +152,7 @@ __global__ void __launch_bounds__(256) topk_kernel(const float *__restrict__ log
 }
 extern "C" void k_topk(cudaStream_t st, const float *logits, int *top, float *topw, int nb) {
     if (nb <= 0) return;
-    launch_k(topk_kernel, (nb + 7) / 8, 256, 0, st, logits, top, topw, nb); g_launches++;
+    launch_pdl(topk_kernel, (nb + 7) / 8, 256, 0, st, logits, top, topw, nb); g_launches++;
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -254,6 +256,7 @@ __global__ void __launch_bounds__(NT) group_cta_kernel(GroupArgs g) {
     __shared__ int w_cnt[8], w_used[8], w_ta[8], w_tb[8];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nb = g.nb, np = nb * TOPK;
     for (int i = tid; i < NEXP * WORDS; i += NT) gs_smem[i] = 0u;
+    pdl_wait(); pdl_trigger();
     __syncthreads();
     for (int i = tid; i < np; i += NT) { const int t = i >> 3; atomicOr(&s_mask[g.top[i]][t >> 5], 1u << (t & 31)); }
     __syncthreads();
@@ -309,7 +312,7 @@ static void launch_group_cta(cudaStream_t st, const GroupArgs *g) {
     const int smem = NEXP * (MAXTOK / 32) * 4 + MAXTOK * TOPK * 4 + NEXP * (MAXTOK / 32) * 2;
     static bool attr_done = false;
     if (!attr_done) { cudaFuncSetAttribute(group_cta_kernel<MAXTOK, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr_done = true; }
-    launch_k(group_cta_kernel<MAXTOK, NT>, 1, NT, smem, st, *g);
+    launch_pdl(group_cta_kernel<MAXTOK, NT>, 1, NT, smem, st, *g);
 }
 // 257 to GROUP_CLUSTER_MAX tokens: one launch of one cluster of CTAS CTAs.  CTA r owns its share of the tokens (in whole
 // words of 32) and keeps their bits in its shared memory; the counts are exchanged through distributed shared memory, after which every CTA
@@ -528,6 +531,7 @@ extern "C" void k_silu_quant(cudaStream_t st, const float *gate, const float *up
 __global__ void __launch_bounds__(256) combine_kernel(const float *__restrict__ down, const float *__restrict__ uw, const int *__restrict__ tp,
                                                       const float *__restrict__ init, float *__restrict__ out, int nb) {
     const int i = blockIdx.x * 256 + threadIdx.x, b = i >> 9, c = (i & 511) * 4;
+    pdl_wait(); pdl_trigger();
     if (b >= nb) return;
     float4 acc = init ? *reinterpret_cast<const float4 *>(init + (size_t)b * HID + c) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -540,5 +544,5 @@ __global__ void __launch_bounds__(256) combine_kernel(const float *__restrict__ 
 }
 extern "C" void k_combine(cudaStream_t st, const float *down, const float *uw, const int *tp, const float *init, float *out, int nb) {
     if (nb <= 0) return;
-    launch_k(combine_kernel, (nb * 512 + 255) / 256, 256, 0, st, down, uw, tp, init, out, nb); g_launches++;
+    launch_pdl(combine_kernel, (nb * 512 + 255) / 256, 256, 0, st, down, uw, tp, init, out, nb); g_launches++;
 }

@@ -235,9 +235,11 @@ __global__ void __launch_bounds__(256, 2) router_small_kernel(const uint8_t *__r
     __syncthreads();
     if (tid == 0) {
         mbar_expect_tx(&bar, (uint32_t)(ntok * HID * 4 + RS_WB));
+        bulk_load(smem_u32(rs_sm + RS_HB), WS + (size_t)e0 * HID * 2, RS_WB, &bar);      // the layer's weights: no kernel of the layer loop writes them
+        pdl_wait();
         bulk_load(smem_u32(rs_sm), hS + (size_t)b0 * HID * 4, (uint32_t)(ntok * HID * 4), &bar);
-        bulk_load(smem_u32(rs_sm + RS_HB), WS + (size_t)e0 * HID * 2, RS_WB, &bar);
     }
+    pdl_wait(); pdl_trigger();
     const bool ok = mbar_wait(&bar, 0, &abort_flag);
     float acc0 = 0.0f, acc1 = 0.0f, odd0 = 0.0f, odd1 = 0.0f;       // odd0/odd1: the second chain of the step order (columns 16m + 8 + j)
     if (ok && tok < ntok) {
@@ -284,7 +286,7 @@ extern "C" void k_router_logits_small(cudaStream_t st, const void *router_s, con
     }
     if (!relaid) launch_k(router_pack_h_small_kernel, nb * 2, 256, 0, st, hn, (float4 *)hS, nb);
     const dim3 grid(NEXP / RS_EXP, (nb + RS_TOK - 1) / RS_TOK);
-    if (g_step_order && nb == 1) launch_k(router_small_kernel<true>, grid, 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err);
-    else launch_k(router_small_kernel<false>, grid, 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err);
+    if (g_step_order && nb == 1) launch_pdl(router_small_kernel<true>, grid, 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err);
+    else launch_pdl(router_small_kernel<false>, grid, 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err);
     k_count_add(relaid ? 1 : 2);
 }
