@@ -360,14 +360,19 @@ static void fill_expert_args(ExpertArgs *a, const ExpertPtrs *tab, const ExpertM
     memset(a, 0, sizeof *a);
     a->tab = tab; a->maps = maps; a->ue = ue; a->ptok = S.utok; a->err = S.err;
     if (use_umma(nb)) { a->tiles = S.tiles_b; a->ntiles = S.ntiles_b; a->max_tiles = nb * TOPK / UMMA_TN + NEXP; }
-    else { a->tiles = S.tiles_a; a->ntiles = S.ntiles_a; a->max_tiles = nb * TOPK / tile_tn(nb) + NEXP; }
+    else { a->tiles = S.tiles_a; a->ntiles = S.ntiles_a; a->max_tiles = nb * TOPK / tile_tn(nb) + NEXP; if (a->max_tiles > nb * TOPK) a->max_tiles = nb * TOPK; }
     a->hq = S.hq; a->hqs = S.hqs; a->hqsum = S.hqsum; a->act = S.act;
     a->aq = S.aq; a->aqs = S.aqs; a->aqsum = S.aqsum; a->down = S.down; a->wire = S.wire; a->wire_cap = S.maxp;
     if (S.keep || use_umma(nb)) { a->gate = S.gate; a->up = S.up; }          /* the tensor-core GEMM always stores gate and up */
     if (S.keep) { a->gu_dots = S.gu_dots; a->dn_dots = S.dn_dots; }
 }
-static void run_group_m(int nb, int marked) {
-    GroupArgs g; memset(&g, 0, sizeof g); g.marked = marked && nb > GROUP_CLUSTER_MAX;
+static void run_group_l(int nb, int marked, const float *logits);
+static void run_group_m(int nb, int marked) { run_group_l(nb, marked, NULL); }
+/* logits: up to TOPK_IN_MAX tokens, the top-8 comes from them in the same kernel */
+static void run_group_l(int nb, int marked, const float *logits) {
+    GroupArgs g; memset(&g, 0, sizeof g);
+    if (logits) { g.logits = logits; g.top_out = S.top; g.topw_out = S.topw; }
+    g.marked = marked && nb > GROUP_CLUSTER_MAX;
     g.top = S.top; g.topw = S.topw; g.nb = nb; g.mask = S.mask; g.mask_words = S.mask_words; g.nu = S.nu; g.ue = S.ue; g.estart = S.estart;
     g.ustart = S.ustart; g.utok = S.utok; g.slot = S.slot; g.tp = S.tp; g.uw = S.uw; g.ecnt = S.ecnt; g.uexp = S.uexp;
     g.tiles_a = S.tiles_a; g.tiles_b = S.tiles_b; g.ntiles_a = S.ntiles_a; g.ntiles_b = S.ntiles_b; g.tn_a = tile_tn(nb); g.tn_b = UMMA_TN;
@@ -529,7 +534,25 @@ static int graphs_on(void) {
 }
 int gmoe_set_graph(int on) { g_graph_on = on != 0; return 0; }
 static int run_layer_ep(int L, int nb, const float *bias);
+/* Layers of a decode batch (nb <= 256) without the per-stage hooks of run_layer: the combine of a layer and the norm of the next are one kernel, and
+ * so are top-8 and grouping of up to TOPK_IN_MAX tokens. */
+static int decode_path(int nb) { return nb <= 256 && !use_umma(nb) && !tensor_router(nb) && !S.keep && !S.prof_mask; }
+static void decode_body(const LayerDev *l, int nb, const float *bias) {
+    k_router_logits_small(S.st, l->router_s, S.hn, S.hT, 1, bias, S.logits, nb, S.err);
+    if (nb > TOPK_IN_MAX) k_topk(S.st, S.logits, S.top, S.topw, nb);
+    run_group_l(nb, 0, nb > TOPK_IN_MAX ? NULL : S.logits);
+    run_experts(l->tab, l->maps, (const float *const *)l->dsp, S.ue, nb, 7);
+}
+static void decode_layers(int nb, int l0, int nl, const float *bias) {
+    k_norm_prep_relaid(S.st, S.x, S.ly[l0].post_ln, S.hn, S.hq, S.hqs, S.hqsum, (float *)S.hT, nb);
+    for (int L = l0; L < l0 + nl; L++) {
+        decode_body(&S.ly[L], nb, bias);
+        if (L + 1 < l0 + nl) k_edge(S.st, S.down, S.uw, S.tp, S.x, S.ly[L + 1].post_ln, S.hn, S.hq, S.hqs, S.hqsum, (float *)S.hT, nb);
+        else k_combine(S.st, S.down, S.uw, S.tp, S.x, S.x, nb);
+    }
+}
 static int layers_run(int nb, int l0, int nl, const float *bd, int ep) {
+    if (!ep && nl > 0 && decode_path(nb)) { decode_layers(nb, l0, nl, bd); return 0; }
     for (int L = l0; L < l0 + nl; L++) { if (ep) { if (run_layer_ep(L, nb, bd)) return -1; } else run_layer(L, nb, 1, bd); }
     return 0;
 }

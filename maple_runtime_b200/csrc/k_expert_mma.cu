@@ -44,7 +44,8 @@ __device__ __forceinline__ MoeTile ldcg_tile(const MoeTile *t) {
 // KCH: K-chunks of 256 columns (8 for gate/up K=2048, 2 for down K=512).  NBLK: 8-token blocks per tile.
 // GATEUP: rows block A = gate rows, block B = up rows of the same index, epilogue = SiLU*up;
 // otherwise A and B are two consecutive 16-row blocks of the down matrix, epilogue = scale only.
-template <int KCH, int NBLK, bool GATEUP>
+// PF: chunks of weights in flight per thread.
+template <int KCH, int NBLK, bool GATEUP, int PF>
 __global__ void __launch_bounds__(128) expert_mma_kernel(ExpertArgs a) {
     constexpr int TN = NBLK * 8, KB = KCH * 256;            // tokens per tile, bytes of one int8 activation vector
     extern __shared__ __align__(16) uint8_t smem[];          // [KCH][4][TN][4][16]
@@ -62,8 +63,7 @@ __global__ void __launch_bounds__(128) expert_mma_kernel(ExpertArgs a) {
     const int r0 = blockIdx.x * rows_per_cta + warp * (GATEUP ? 16 : 32);
     const uint8_t *wa = (GATEUP ? ep.gc : ep.dc) + (size_t)(r0 + g) * (KB / 4) + t * 16;
     const uint8_t *wb = GATEUP ? ep.uc + (size_t)(r0 + g) * (KB / 4) + t * 16 : wa + 16 * (KB / 4);
-    // the weight stream starts before anything else: the first two chunks are on their way while the activations are staged
-    constexpr int PF = 2;                                   // chunks in flight (more costs occupancy and loses)
+    // the weight stream starts before anything else: the first PF chunks are on their way while the activations are staged
     uint4 wq[PF][4];
 #pragma unroll
     for (int p = 0; p < PF; p++) if (p < KCH) {
@@ -179,22 +179,26 @@ __global__ void __launch_bounds__(128) expert_mma_kernel(ExpertArgs a) {
         }
 }
 
-template <int KCH, int NBLK, bool GATEUP>
+template <int KCH, int NBLK, bool GATEUP, int PF>
 static void launch(cudaStream_t st, const ExpertArgs *a) {
     const size_t smem = (size_t)KCH * 4 * NBLK * 8 * 64 + (GATEUP ? 0 : NBLK * 8 * 8);   // + scale and code sum per pair when down quantises itself
     static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<KCH, NBLK, GATEUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
+    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<KCH, NBLK, GATEUP, PF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
     dim3 grid(GATEUP ? 8 : 16, a->max_tiles);
-    launch_pdl(expert_mma_kernel<KCH, NBLK, GATEUP>, grid, 128, smem, st, *a);
+    launch_pdl(expert_mma_kernel<KCH, NBLK, GATEUP, PF>, grid, 128, smem, st, *a);
     k_count_add(1);
 }
+// Two chunks in flight leave room for six CTAs per SM, which is what a long list of tiles wants (four chunks: 64 tokens 34.5 instead of 31 us).
+// Where the whole list is resident at once at one or two CTAs per SM, all eight chunks go out together: one trip to memory instead of four
+// (1 token 22.1 -> 20.9 us per layer; from 4 tokens on the two are level).
+#define PF8_TILES 24
 extern "C" void k_gateup_mma(cudaStream_t st, const ExpertArgs *a, int tn) {
     if (a->max_tiles <= 0) return;
-    if (tn == 8) launch<8, 1, true>(st, a); else launch<8, 4, true>(st, a);
+    if (tn != 8) launch<8, 4, true, 2>(st, a); else if (a->max_tiles <= PF8_TILES) launch<8, 1, true, 8>(st, a); else launch<8, 1, true, 2>(st, a);
 }
 extern "C" void k_down_mma(cudaStream_t st, const ExpertArgs *a, int tn) {
     if (a->max_tiles <= 0) return;
-    if (tn == 8) launch<2, 1, false>(st, a); else launch<2, 4, false>(st, a);
+    if (tn == 8) launch<2, 1, false, 2>(st, a); else launch<2, 4, false, 2>(st, a);
 }
 
 // The attention projections (gpu_pre.m:200-256 gpre_dense*): the same int8 x 2-bit product with one matrix instead of 256
@@ -203,7 +207,7 @@ extern "C" void k_dense_mma(cudaStream_t st, const ExpertArgs *a, int rows) {
     if (a->dense_n <= 0 || rows <= 0) return;
     const size_t smem = (size_t)8 * 4 * 32 * 64 + 32 * 8;
     static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<8, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
-    launch_k(expert_mma_kernel<8, 4, false>, dim3(rows / 128, (a->dense_n + 31) / 32), 128, smem, st, *a);
+    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<8, 4, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
+    launch_k(expert_mma_kernel<8, 4, false, 2>, dim3(rows / 128, (a->dense_n + 31) / 32), 128, smem, st, *a);
     k_count_add(1);
 }

@@ -134,6 +134,7 @@ extern "C" void k_norm_prep_split(cudaStream_t st, const float *x, const uint16_
 // ------------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) topk_kernel(const float *__restrict__ logits, int *__restrict__ top, float *__restrict__ topw, int nb) {
     __shared__ unsigned long long tab[32];                  // the expf table beside the arithmetic (lane-varying index)
+    __shared__ __align__(16) float s_row[8][NEXP];
     if (threadIdx.x < 32) tab[threadIdx.x] = DEV_EXP_TAB[threadIdx.x];
     __syncthreads();
     pdl_wait(); pdl_trigger();
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(256) topk_kernel(const float *__restrict__ log
     float4 v0 = lr[0], v1 = lr[1];
     float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
     int isel; float wsel, tsum;
-    exact_topk_warp(p, lane, tab, isel, wsel, tsum);
+    exact_topk_warp(p, lane, tab, s_row[threadIdx.x >> 5], isel, wsel, tsum);
     if (lane < TOPK) {
         top[b * TOPK + lane] = isel;
         topw[b * TOPK + lane] = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));
@@ -245,7 +246,8 @@ __global__ void __launch_bounds__(NEXP) group_place_kernel(const unsigned *__res
 // MAXTOK tokens at most, NT threads (the first 256 own one expert each).  Used up to 256 tokens; a 2048-token instance (160 KB of
 // shared memory, 1024 threads) works but one SM takes longer over 16,384 pairs than the three kernels of the general path below.
 #define GS_MAXTOK 256
-template <int MAXTOK, int NT>
+// TOPK_IN (up to TOPK_IN_MAX tokens): the softmax and top-8 of token w by warp w come first, which saves their kernel.
+template <int MAXTOK, int NT, bool TOPK_IN>
 __global__ void __launch_bounds__(NT) group_cta_kernel(GroupArgs g) {
     constexpr int WORDS = MAXTOK / 32;
     extern __shared__ __align__(16) unsigned gs_smem[];
@@ -254,18 +256,38 @@ __global__ void __launch_bounds__(NT) group_cta_kernel(GroupArgs g) {
     unsigned short (*s_wpre)[WORDS] = reinterpret_cast<unsigned short (*)[WORDS]>(s_slot + MAXTOK * TOPK); // [NEXP][WORDS] pairs before word w
     __shared__ int s_start[NEXP];
     __shared__ int w_cnt[8], w_used[8], w_ta[8], w_tb[8];
+    __shared__ int s_top[TOPK_IN ? TOPK_IN_MAX * TOPK : 1]; __shared__ float s_topw[TOPK_IN ? TOPK_IN_MAX * TOPK : 1];
+    __shared__ __align__(16) float s_row[TOPK_IN ? 8 : 1][NEXP];
+    __shared__ unsigned long long tab[TOPK_IN ? 32 : 1];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nb = g.nb, np = nb * TOPK;
+    if (TOPK_IN && tid < 32) tab[tid] = DEV_EXP_TAB[tid];
     for (int i = tid; i < NEXP * WORDS; i += NT) gs_smem[i] = 0u;
-    pdl_wait(); pdl_trigger();
     __syncthreads();
-    for (int i = tid; i < np; i += NT) { const int t = i >> 3; atomicOr(&s_mask[g.top[i]][t >> 5], 1u << (t & 31)); }
+    pdl_wait(); pdl_trigger();
+    if (TOPK_IN) {
+        if (wid < nb) {
+            const int t = wid;
+            const float4 *lr = reinterpret_cast<const float4 *>(g.logits + (size_t)t * NEXP + lane * 8);
+            const float4 v0 = __ldcg(lr), v1 = __ldcg(lr + 1);
+            float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+            int isel; float wsel, tsum;
+            exact_topk_warp(p, lane, tab, s_row[wid], isel, wsel, tsum);
+            if (lane < TOPK) {
+                const float w = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));
+                s_top[t * TOPK + lane] = isel; s_topw[t * TOPK + lane] = w;
+                g.top_out[t * TOPK + lane] = isel; g.topw_out[t * TOPK + lane] = w;
+            }
+        }
+        __syncthreads();
+    }
+    auto expert = [&](const int i) { return TOPK_IN ? s_top[i] : g.top[i]; };
+    for (int i = tid; i < np; i += NT) { const int t = i >> 3; atomicOr(&s_mask[expert(i)][t >> 5], 1u << (t & 31)); }
     __syncthreads();
     if (tid < NEXP) {
         const int e = tid;
         int cnt = 0;
 #pragma unroll 8
         for (int w = 0; w < WORDS; w++) { s_wpre[e][w] = (unsigned short)cnt; cnt += __popc(s_mask[e][w]); }
-        if (g.ecnt) g.ecnt[e] = cnt;
         const int used = cnt > 0, na = (cnt + g.tn_a - 1) / g.tn_a, nb_ = (cnt + g.tn_b - 1) / g.tn_b;
         int c = cnt, u = used, a = na, b = nb_;
 #pragma unroll
@@ -279,8 +301,9 @@ __global__ void __launch_bounds__(NT) group_cta_kernel(GroupArgs g) {
         int oc = 0, ou = 0, oa = 0, ob = 0;
         for (int w = 0; w < wid; w++) { oc += w_cnt[w]; ou += w_used[w]; oa += w_ta[w]; ob += w_tb[w]; }
         const int start = oc + c - cnt, uidx = ou + u - used, ta0 = oa + a - na, tb0 = ob + b - nb_;
-        g.estart[e] = used ? start : -1;
         s_start[e] = start;
+        if (g.ecnt) g.ecnt[e] = cnt;
+        g.estart[e] = used ? start : -1;
         if (used) {
             g.ue[uidx] = e; g.ustart[uidx] = start;
             for (int t = 0; t < na; t++) { MoeTile m = {uidx, start + t * g.tn_a, min(g.tn_a, cnt - t * g.tn_a), e}; g.tiles_a[ta0 + t] = m; }
@@ -290,12 +313,13 @@ __global__ void __launch_bounds__(NT) group_cta_kernel(GroupArgs g) {
     }
     __syncthreads();
     for (int i = tid; i < np; i += NT) {                             // every pair finds its place
-        const int x = g.top[i], t = i >> 3, w = t >> 5;
+        const int x = expert(i), t = i >> 3, w = t >> 5;
         const int r = s_start[x] + s_wpre[x][w] + __popc(s_mask[x][w] & ((1u << (t & 31)) - 1u));
-        g.utok[r] = t; g.uw[r] = g.topw[i]; if (g.uexp) g.uexp[r] = x; s_slot[i] = r;
+        s_slot[i] = r;
+        g.utok[r] = t; g.uw[r] = TOPK_IN ? s_topw[i] : g.topw[i]; if (g.uexp) g.uexp[r] = x;
     }
     __syncthreads();
-    for (int t = tid; t < nb; t += NT) {                             // tp: the token's eight slots ascending
+    for (int t = tid; t < nb; t += NT) {                         // tp: the token's eight slots ascending
         int sl[TOPK];
 #pragma unroll
         for (int k = 0; k < TOPK; k++) { sl[k] = s_slot[t * TOPK + k]; g.slot[t * TOPK + k] = sl[k]; }
@@ -307,12 +331,12 @@ __global__ void __launch_bounds__(NT) group_cta_kernel(GroupArgs g) {
         for (int k = 0; k < TOPK; k++) g.tp[t * TOPK + k] = sl[k];
     }
 }
-template <int MAXTOK, int NT>
+template <int MAXTOK, int NT, bool TOPK_IN>
 static void launch_group_cta(cudaStream_t st, const GroupArgs *g) {
     const int smem = NEXP * (MAXTOK / 32) * 4 + MAXTOK * TOPK * 4 + NEXP * (MAXTOK / 32) * 2;
     static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(group_cta_kernel<MAXTOK, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr_done = true; }
-    launch_pdl(group_cta_kernel<MAXTOK, NT>, 1, NT, smem, st, *g);
+    if (!attr_done) { cudaFuncSetAttribute(group_cta_kernel<MAXTOK, NT, TOPK_IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr_done = true; }
+    launch_pdl(group_cta_kernel<MAXTOK, NT, TOPK_IN>, 1, NT, smem, st, *g);
 }
 // 257 to GROUP_CLUSTER_MAX tokens: one launch of one cluster of CTAS CTAs.  CTA r owns its share of the tokens (in whole
 // words of 32) and keeps their bits in its shared memory; the counts are exchanged through distributed shared memory, after which every CTA
@@ -416,7 +440,10 @@ __global__ void __launch_bounds__(NEXP) group_cluster_kernel(GroupArgs g) {
 }
 extern "C" void k_group(cudaStream_t st, const GroupArgs *g) {
     if (g->nb <= 0) return;
-    if (g->nb <= 256) { launch_group_cta<256, 256>(st, g); g_launches++; return; }
+    if (g->nb <= 256) {
+        if (g->logits) launch_group_cta<32, 256, true>(st, g); else if (g->nb <= 32) launch_group_cta<32, 256, false>(st, g); else launch_group_cta<256, 256, false>(st, g);
+        g_launches++; return;
+    }
     const int np = g->nb * TOPK;
     if (g->nb <= GROUP_CLUSTER_MAX) {
         if (g->nb <= 512) launch_cluster(group_cluster_kernel<8>, 8, NEXP, st, *g);
@@ -522,6 +549,88 @@ extern "C" void k_silu_quant(cudaStream_t st, const float *gate, const float *up
     if (act) launch_k(silu_quant_kernel<true>, (np + 7) / 8, 256, 0, st, gate, up, act, aq, aqs, aqsum, np, np_dev);
     else launch_k(silu_quant_kernel<false>, (np + 7) / 8, 256, 0, st, gate, up, (float *)NULL, aq, aqs, aqsum, np, np_dev);
     g_launches++;
+}
+
+// ------------------------------------------------------------------------------------------------------------
+// Decode batches, between two layers: the combine of the one (maple.c:834, as combine_kernel) and the RMSNorm + int8 of the next (as
+// norm_prep_kernel, its sums in the same order) for one token per CTA: one launch and one trip of the hidden row less.  Thread tid holds float4
+// tid and tid + 256 of the row.
+// ------------------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) edge_kernel(const float *down, const float *uw, const int *tp, float *x, const uint16_t *__restrict__ w,
+                                                   float *hn, int8_t *q, float *qs, int *qsum, float *hS) {
+    __shared__ double s_term[16 * 32];
+    __shared__ float s_k, s_mx[8]; __shared__ int s_sum[8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c = blockIdx.x;
+    const uint2 ln[2] = {reinterpret_cast<const uint2 *>(w)[tid], reinterpret_cast<const uint2 *>(w)[tid + 256]};      // weights: read before the wait
+    pdl_wait(); pdl_trigger();
+    int slot[TOPK]; float uv[TOPK];
+#pragma unroll
+    for (int k = 0; k < TOPK; k++) slot[k] = tp[c * TOPK + k];
+#pragma unroll
+    for (int k = 0; k < TOPK; k++) uv[k] = uw[slot[k]];
+    float4 v[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = tid + 256 * k;
+        float4 d[TOPK];
+        v[k] = __ldcg(reinterpret_cast<const float4 *>(x) + (size_t)c * 512 + i);
+#pragma unroll
+        for (int t = 0; t < TOPK; t++) d[t] = __ldcg(reinterpret_cast<const float4 *>(down) + (size_t)slot[t] * 512 + i);
+#pragma unroll
+        for (int t = 0; t < TOPK; t++) {
+            v[k].x = __fmaf_rn(uv[t], d[t].x, v[k].x); v[k].y = __fmaf_rn(uv[t], d[t].y, v[k].y);
+            v[k].z = __fmaf_rn(uv[t], d[t].z, v[k].z); v[k].w = __fmaf_rn(uv[t], d[t].w, v[k].w);
+        }
+        reinterpret_cast<float4 *>(x)[(size_t)c * 512 + i] = v[k];
+        s_term[(warp + 8 * k) * 32 + lane] = ((double)v[k].x * (double)v[k].x + (double)v[k].y * (double)v[k].y) + ((double)v[k].z * (double)v[k].z + (double)v[k].w * (double)v[k].w);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        double ss = 0.0;
+#pragma unroll
+        for (int i = 0; i < 16; i++) ss += s_term[i * 32 + lane];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) s_k = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn((float)(ss / (double)HID), 1e-6f)));
+    }
+    __syncthreads();
+    const float kk = s_k;
+    float mx = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = tid + 256 * k, col = 4 * i;
+        v[k].x = __fmul_rn(__fmul_rn(v[k].x, kk), __uint_as_float(ln[k].x << 16)); v[k].y = __fmul_rn(__fmul_rn(v[k].y, kk), __uint_as_float(ln[k].x & 0xFFFF0000u));
+        v[k].z = __fmul_rn(__fmul_rn(v[k].z, kk), __uint_as_float(ln[k].y << 16)); v[k].w = __fmul_rn(__fmul_rn(v[k].w, kk), __uint_as_float(ln[k].y & 0xFFFF0000u));
+        mx = fmaxf(fmaxf(mx, fmaxf(fabsf(v[k].x), fabsf(v[k].y))), fmaxf(fabsf(v[k].z), fabsf(v[k].w)));
+        reinterpret_cast<float4 *>(hn)[(size_t)c * 512 + i] = v[k];
+        float *p = hS + (size_t)c * HID + (col >> 5) * 32 + (col & 7) * 4 + ((col >> 3) & 3);
+        p[0] = v[k].x; p[4] = v[k].y; p[8] = v[k].z; p[12] = v[k].w;
+    }
+    mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));      // >= 0: the bits order like the values
+    if (lane == 0) s_mx[warp] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 8; k++) mx = fmaxf(mx, s_mx[k]);
+    const float s = mx > 0.0f ? __fdiv_rn(mx, 127.0f) : 1.0f, inv = __fdiv_rn(1.0f, s);
+    int tot = 0;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int q0 = __float2int_rn(__fmul_rn(v[k].x, inv)), q1 = __float2int_rn(__fmul_rn(v[k].y, inv)), q2 = __float2int_rn(__fmul_rn(v[k].z, inv)), q3 = __float2int_rn(__fmul_rn(v[k].w, inv));
+        tot += (q0 + q1) + (q2 + q3);
+        reinterpret_cast<uint32_t *>(q)[(size_t)c * 512 + tid + 256 * k] = (uint32_t)(q0 & 0xFF) | ((uint32_t)(q1 & 0xFF) << 8) | ((uint32_t)(q2 & 0xFF) << 16) | ((uint32_t)(q3 & 0xFF) << 24);
+    }
+    tot = __reduce_add_sync(0xffffffffu, tot);
+    if (lane == 0) s_sum[warp] = tot;
+    __syncthreads();
+    if (tid == 0) {
+        int t = 0;
+        for (int k = 0; k < 8; k++) t += s_sum[k];
+        qs[c] = s; qsum[c] = t;
+    }
+}
+extern "C" void k_edge(cudaStream_t st, const float *down, const float *uw, const int *tp, float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb) {
+    if (nb <= 0) return;
+    launch_pdl(edge_kernel, nb, 256, 0, st, down, uw, tp, x, w, hn, q, qs, qsum, hS); g_launches++;
 }
 
 // ------------------------------------------------------------------------------------------------------------

@@ -283,12 +283,12 @@ __global__ void __launch_bounds__(256) router_fix_kernel(const uint8_t *__restri
         if (tid == 0) s_last = atomicAdd(&done[f], 1) == (int)gridDim.x - 1;
         __syncthreads();
         if (s_last && tid < 32) {
-            __threadfence();
+            __threadfence();                                              // hrow is read no more: it is the scratch of the top-8
             const float4 *lr = reinterpret_cast<const float4 *>(logits + (size_t)b * NEXP + lane * 8);
             const float4 v0 = __ldcg(lr), v1 = __ldcg(lr + 1);              // the other CTAs' values: read past L1
             float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
             int isel; float wsel, tsum;
-            exact_topk_warp(p, lane, tab, isel, wsel, tsum);
+            exact_topk_warp(p, lane, tab, hrow, isel, wsel, tsum);
             if (lane < TOPK) {
                 top[b * TOPK + lane] = isel; topw[b * TOPK + lane] = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));
                 if (mask) { atomicOr(&mask[(size_t)(b >> 5) * NEXP + isel], 1u << (b & 31)); atomicAdd(&mask[(size_t)NEXP * mask_words + isel], 1u); }

@@ -66,6 +66,7 @@ void k_topk(cudaStream_t st, const float *logits, int *top, float *topw, int nb)
 /* norm + int8 as k_norm_prep, and the normalised rows once more as two fp16 terms per value (hA: [nb][4096] fp16, hi then lo) with the
  * rows' Euclidean norms (hnorm [nb]): the A operand of the tensor-core router */
 void k_norm_prep_split(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, void *hA, float *hnorm, int nb);
+#define TOPK_IN_MAX 8               /* one token per warp; a second one per warp takes 1.5 us longer than a kernel of its own (13 tokens) */
 #define GROUP_CLUSTER_MAX 4096      /* up to here k_group makes its own bits; above it the routing kernels may set them (GroupArgs.marked) */
 typedef struct {
     const int *top; const float *topw; int nb;
@@ -73,6 +74,7 @@ typedef struct {
     int mask_words;
     int *nu, *ue, *estart, *ustart, *utok, *slot, *tp; float *uw;
     int marked;              /* 1: the routing kernels have already set the bits and counters in mask */
+    const float *logits; int *top_out; float *topw_out;      /* optional, up to TOPK_IN_MAX tokens: the top-8 is computed first, from the logits, and also stored here */
     int *ecnt, *uexp;        /* optional: pairs per expert [256], expert of every pair [np] (expert parallel) */
     MoeTile *tiles_a, *tiles_b; int *ntiles_a, *ntiles_b; int tn_a, tn_b;   /* two tile lists: sizes tn_a and tn_b */
 } GroupArgs;
@@ -81,6 +83,8 @@ void k_group(cudaStream_t st, const GroupArgs *g);
 void k_actq(cudaStream_t st, const float *act, int8_t *aq, float *aqs, int *aqsum, const int *np_dev, int np_max);
 /* SiLU*up then per-pair int8 from stored gate and up (the tensor-core path); act may be NULL */
 void k_silu_quant(cudaStream_t st, const float *gate, const float *up, float *act, int8_t *aq, float *aqs, int *aqsum, int np, const int *np_dev);
+/* decode batches, between two layers: x += the pairs' weighted rows, then norm + int8 of x as k_norm_prep_relaid */
+void k_edge(cudaStream_t st, const float *down, const float *uw, const int *tp, float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb);
 void k_combine(cudaStream_t st, const float *down, const float *uw, const int *tp, const float *init, float *out, int nb);
 
 /* register-decode + mma.sync grouped kernels (any token count; the decode-batch path); tn = 8 or 32 */

@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <stdint.h>
+#include <string.h>
 #include "kernels.h"
 #include "../../include/gmoe.h"
 
@@ -60,11 +61,10 @@ extern "C" int gmoe_group_noalloc(const int *top, const float *topw, int nb, int
         g_na_dev[dev] = static_cast<NaScratch *>(p);
     }
     NaScratch *s = g_na_dev[dev];
-    GroupArgs g;
+    GroupArgs g; memset(&g, 0, sizeof g);
     g.top = top; g.topw = topw; g.nb = nb; g.marked = 0;
     g.mask = s->mask; g.mask_words = (nb + 31) / 32;
     g.nu = nu; g.ue = ue; g.estart = s->estart; g.ustart = ustart; g.utok = utok; g.slot = s->slot; g.tp = tp; g.uw = uw;
-    g.ecnt = NULL; g.uexp = NULL;
     g.tiles_a = s->tiles_a; g.tiles_b = s->tiles_b; g.ntiles_a = s->ntiles_a; g.ntiles_b = s->ntiles_b; g.tn_a = 8; g.tn_b = UMMA_TN;
     k_group(static_cast<cudaStream_t>(stream), &g);   // one kernel with its masks in shared memory (up to 256 tokens one CTA, above that a cluster of eight)
     e = cudaGetLastError();

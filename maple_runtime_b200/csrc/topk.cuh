@@ -2,11 +2,13 @@
 // 8l..8l+7.  p = expf(l - max); the sum runs over the experts in index order (a chain through the lanes); p /= sum; eight rounds of
 // "first strict maximum" (lowest index wins a tie).  Lanes 0..7 return the k-th selected expert and its probability, every lane the sum
 // of the eight in selection order: weight_k = wsel / (tsum + 1e-20f).  tab: the expf table of dev_math.cuh (or a shared-memory copy).
+// row: 256 floats of shared memory of this warp, 16-byte aligned: every lane walks the chain of additions over all experts from there (a chain
+// handed from lane to lane pays a shuffle per eight additions: 1 us instead of 0.6).
 #pragma once
 #include "dev_math.cuh"
 
 template <typename TabT>
-__device__ __forceinline__ void exact_topk_warp(float (&p)[8], const int lane, const TabT *tab, int &isel, float &wsel, float &tsum) {
+__device__ __forceinline__ void exact_topk_warp(float (&p)[8], const int lane, const TabT *tab, float *row, int &isel, float &wsel, float &tsum) {
     float mx = -1e30f;
 #pragma unroll
     for (int i = 0; i < 8; i++) mx = p[i] > mx ? p[i] : mx;
@@ -14,13 +16,15 @@ __device__ __forceinline__ void exact_topk_warp(float (&p)[8], const int lane, c
     for (int o = 16; o; o >>= 1) { float t = __shfl_xor_sync(0xffffffffu, mx, o); mx = t > mx ? t : mx; }
 #pragma unroll
     for (int i = 0; i < 8; i++) p[i] = dev_expf_tab(__fsub_rn(p[i], mx), tab);
+    __syncwarp();
+    reinterpret_cast<float4 *>(row)[2 * lane] = make_float4(p[0], p[1], p[2], p[3]);
+    reinterpret_cast<float4 *>(row)[2 * lane + 1] = make_float4(p[4], p[5], p[6], p[7]);
+    __syncwarp();
     float run = 0.0f;
-    for (int l = 0; l < 32; l++) {
-        if (lane == l) {
-#pragma unroll
-            for (int i = 0; i < 8; i++) run = __fadd_rn(run, p[i]);
-        }
-        run = __shfl_sync(0xffffffffu, run, l);
+#pragma unroll 8
+    for (int i = 0; i < 64; i++) {
+        const float4 v = reinterpret_cast<const float4 *>(row)[i];
+        run = __fadd_rn(run, v.x); run = __fadd_rn(run, v.y); run = __fadd_rn(run, v.z); run = __fadd_rn(run, v.w);
     }
 #pragma unroll
     for (int i = 0; i < 8; i++) p[i] = __fdiv_rn(p[i], run);
