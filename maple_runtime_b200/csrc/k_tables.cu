@@ -28,3 +28,15 @@ extern "C" void k_tables(cudaStream_t st, const TableSegs *t) {
     launch_k(tables_kernel, dim3(ctas, (unsigned)t->n), 256, 0, st, *t);
     k_count_add(1);
 }
+
+__global__ void __launch_bounds__(256) rows_kernel(uint4 *__restrict__ dst, const uint4 *__restrict__ src, unsigned n) {
+    const unsigned i = blockIdx.x * 256 + threadIdx.x;
+    pdl_wait(); pdl_trigger();
+    if (i < n) dst[i] = src[i];
+}
+extern "C" void k_rows(cudaStream_t st, void *dst, const void *src, size_t bytes) {
+    const unsigned n = (unsigned)(bytes / 16);
+    if (!n) return;
+    launch_pdl(rows_kernel, (n + 255) / 256, 256, 0, st, static_cast<uint4 *>(dst), static_cast<const uint4 *>(src), n);
+    k_count_add(1);
+}

@@ -51,6 +51,9 @@ void k_count_reset(void); long k_count(void);
 typedef struct { void *dst[TABLE_SEGS]; const void *src[TABLE_SEGS]; unsigned words[TABLE_SEGS]; int n; } TableSegs;
 void k_tables(cudaStream_t st, const TableSegs *t);
 
+/* bytes (a multiple of 16) from src to dst, either of which may be page-locked host memory */
+void k_rows(cudaStream_t st, void *dst, const void *src, size_t bytes);
+
 void k_norm_prep(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, int nb);
 /* the same, and the normalised rows once more in the decode router's layout (hS, nb*HID*4 bytes): k_router_logits_small then takes relaid = 1 */
 void k_norm_prep_relaid(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb);
