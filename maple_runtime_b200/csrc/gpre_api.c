@@ -14,6 +14,7 @@
 #include "kernels.h"
 #include "synth.h"
 #include "hostflow.h"
+#include "hostio.h"
 
 void k_count_add(long n);
 
@@ -610,13 +611,13 @@ double gmoe_moe(int L, const float *x, int nb, float *y, const float *bias) {
     if (nb <= INPLACE_MAXTOK && decode_path(nb)) {
         const size_t n = (size_t)nb * HID;
         const float *bias_d = bias_dev(bias);
-        memcpy(S.h_rows, x, n * 4);
+        hio_copy_shared(S.h_rows, x, n * 4);
         cudaEventRecord(S.e0, S.st);
         if (layers_enqueue(nb, L, 0, bias_d)) return -1.0;
         cudaEventRecord(S.e1, S.st);
         S.nb_cur = nb;
         const double t = finish("gmoe");
-        if (t >= 0) memcpy(y, S.h_rows + (size_t)INPLACE_MAXTOK * HID, n * 4);
+        if (t >= 0) hio_copy_shared(y, S.h_rows + (size_t)INPLACE_MAXTOK * HID, n * 4);
         return t;
     }
     if (rows_in("gmoe", S.hn, x, nb)) return -1.0;

@@ -11,9 +11,7 @@
 
 #define SLOTS 6
 #define SLOT_BYTES (3u << 20)             /* 256 tokens of the widest row (12 KB) */
-#define PIECE_BYTES (24u << 10)           /* a thread's unit of work: about 1.5 us, so that the calling thread is never away from the chunks for long */
 #define CHUNK_MIN (512u << 10)            /* a chunk costs about 10 us of calls into the driver: as long as half a megabyte on the link */
-#define POOL_BYTES (160u << 10)           /* below this the calling thread alone is done before a helper has seen the job */
 #define STREAM_BYTES (8u << 20)           /* results larger than this are stored past the caches */
 #define MAXCHUNKS 256
 
@@ -72,7 +70,7 @@ static void drain_piece(void *p, int i) {
 /* a chunk's host work: at once when it is small, else as a job of the pool */
 static int start_part(Part *c, hio_fn fn, size_t row_bytes, unsigned *ticket) {
     const size_t bytes = (size_t)c->n * row_bytes;
-    c->per = bytes < POOL_BYTES ? c->n : (int)(PIECE_BYTES / row_bytes) + 1;
+    c->per = bytes < HIO_POOL_BYTES ? c->n : (int)(HIO_PIECE_BYTES / row_bytes) + 1;
     const int pieces = (c->n + c->per - 1) / c->per;
     if (pieces <= 1) { fn(c, 0); return 0; }
     *ticket = hio_submit(fn, c, pieces);

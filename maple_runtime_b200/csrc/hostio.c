@@ -171,3 +171,14 @@ void hio_copy(void *dst, const void *src, size_t bytes, int stream) {
     if (avx2 < 0) avx2 = __builtin_cpu_supports("avx2") != 0;
     if (stream && avx2) copy_stream(dst, src, bytes); else memcpy(dst, src, bytes);
 }
+typedef struct { uint8_t *d; const uint8_t *s; size_t n; } Shared;
+static void shared_piece(void *p, int i) {
+    const Shared *c = p;
+    const size_t a = (size_t)i * HIO_PIECE_BYTES, n = c->n - a < HIO_PIECE_BYTES ? c->n - a : HIO_PIECE_BYTES;
+    memcpy(c->d + a, c->s + a, n);
+}
+void hio_copy_shared(void *dst, const void *src, size_t bytes) {
+    if (bytes < HIO_POOL_BYTES) { memcpy(dst, src, bytes); return; }
+    Shared c = {dst, src, bytes};
+    hio_wait(hio_submit(shared_piece, &c, (int)((bytes + HIO_PIECE_BYTES - 1) / HIO_PIECE_BYTES)));
+}

@@ -16,4 +16,8 @@ void hio_wait(unsigned ticket);           /* helps until the job is done */
 void hio_quant_rows(const float *x, int rows, int8_t *q, float *qs, int *qsum);
 /* memcpy whose stores go past the caches when `stream` is set (a destination that is larger than them) */
 void hio_copy(void *dst, const void *src, size_t bytes, int stream);
+/* memcpy of a large buffer by the pool (by the calling thread alone below HIO_POOL_BYTES, where it is done before a helper has seen the job) */
+#define HIO_POOL_BYTES (160u << 10)
+#define HIO_PIECE_BYTES (24u << 10)       /* a thread's unit of work: about 1.5 us */
+void hio_copy_shared(void *dst, const void *src, size_t bytes);
 #endif
