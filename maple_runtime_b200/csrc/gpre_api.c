@@ -364,7 +364,7 @@ static int tile_tn(int nb) { return nb <= 256 ? 8 : 32; }
 static int use_umma(int nb) { return S.path == 2 || (S.path == 0 && nb > 256); }
 static void fill_expert_args(ExpertArgs *a, const ExpertPtrs *tab, const ExpertMaps *maps, const int *ue, int nb) {
     memset(a, 0, sizeof *a);
-    a->tab = tab; a->maps = maps; a->ue = ue; a->ptok = S.utok; a->err = S.err;
+    a->call_maps = maps == S.maps_call; a->tab = tab; a->maps = maps; a->ue = ue; a->ptok = S.utok; a->err = S.err;
     if (use_umma(nb)) { a->tiles = S.tiles_b; a->ntiles = S.ntiles_b; a->max_tiles = nb * TOPK / UMMA_TN + NEXP; }
     else { a->tiles = S.tiles_a; a->ntiles = S.ntiles_a; a->max_tiles = nb * TOPK / tile_tn(nb) + NEXP; if (a->max_tiles > nb * TOPK) a->max_tiles = nb * TOPK; }
     a->hq = S.hq; a->hqs = S.hqs; a->hqsum = S.hqsum; a->act = S.act;

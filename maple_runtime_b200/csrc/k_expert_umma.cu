@@ -61,6 +61,10 @@ struct __align__(16) UmShared {
     __align__(16) unsigned long long m_dst[8][UM_TN];                             // expert parallel, down: where each token's compact row lives (a peer's memory)
 };
 
+__device__ __forceinline__ MoeTile ldcg_tile(const MoeTile *t) {
+    const int4 v = __ldcg(reinterpret_cast<const int4 *>(t)); return MoeTile{v.x, v.y, v.z, v.w};
+}
+
 template <int KB, int MODE>
 __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const __grid_constant__ TMap4 bmap) {
     extern __shared__ __align__(1024) uint8_t um_smem_raw[];
@@ -95,9 +99,12 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
     tc_fence_after();
     const uint32_t tb = sh->tmem_base;
     bool live = true;
-    const int ntiles = DENSE ? (a.dense_n + UM_TN - 1) / UM_TN : *a.ntiles, nitems = ntiles * MB;
+    // launched programmatically: the weights start to come in before the wait (the tile list is two kernels old), everything else after it
+    if (warp != 8) pdl_wait();
+    pdl_trigger();
+    const int ntiles = DENSE ? (a.dense_n + UM_TN - 1) / UM_TN : __ldcg(a.ntiles), nitems = ntiles * MB;
     auto tile_at = [&](const int i) {
-        return DENSE ? MoeTile{0, a.dense_p0 + i * UM_TN, min(UM_TN, a.dense_n - i * UM_TN), 0} : a.tiles[i];
+        return DENSE ? MoeTile{0, a.dense_p0 + i * UM_TN, min(UM_TN, a.dense_n - i * UM_TN), 0} : ldcg_tile(a.tiles + i);
     };
 
     if (warp < 8) {
@@ -439,7 +446,8 @@ static void launch(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) {
         int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaFuncSetAttribute(expert_umma_kernel<KB, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     }
-    launch_k(expert_umma_kernel<KB, MODE>, sms, 640, smem, st, *a, *bmap);
+    if (a->call_maps || MODE == 2) launch_k(expert_umma_kernel<KB, MODE>, sms, 640, smem, st, *a, *bmap);
+    else launch_pdl(expert_umma_kernel<KB, MODE>, sms, 640, smem, st, *a, *bmap);
     k_count_add(1);
 }
 extern "C" void k_gateup_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->max_tiles > 0) launch<16, 0>(st, a, bmap); }
@@ -449,6 +457,7 @@ extern "C" void k_dense_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *
 
 // ---- rows of the per-token int8 matrix copied into pair (expert-grouped) order: the B operand the TMA can tile ----
 __global__ void __launch_bounds__(256) gather_rows_kernel(const int8_t *__restrict__ src, const int *__restrict__ rows, int8_t *__restrict__ dst, int np) {
+    pdl_wait(); pdl_trigger();
     // 8 pairs per CTA: each thread moves one 16-byte piece of four rows, all four loads in flight together
     const int p0 = blockIdx.x * 8 + (threadIdx.x >> 7) * 4, c = threadIdx.x & 127;
     int r[4]; uint4 v[4];
@@ -461,6 +470,6 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const int8_t *__restri
 }
 extern "C" void k_gather_rows(cudaStream_t st, const int8_t *src, const int *rows, int8_t *dst, int np) {
     if (np <= 0) return;
-    launch_k(gather_rows_kernel, (np + 7) / 8, 256, 0, st, src, rows, dst, np);
+    launch_pdl(gather_rows_kernel, (np + 7) / 8, 256, 0, st, src, rows, dst, np);
     k_count_add(1);
 }

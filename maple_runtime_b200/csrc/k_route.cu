@@ -354,6 +354,7 @@ __global__ void __launch_bounds__(NEXP) group_cluster_kernel(GroupArgs g) {
     const int e = threadIdx.x, lane = e & 31, wid = e >> 5, nb = g.nb;
     const int per = (((nb + 31) / 32 + GC_CTAS - 1) / GC_CTAS) * 32, tok = blockIdx.x * per + e;      // per <= 32 GC_WORDS = one token per thread
     const bool mine = e < per && tok < nb;
+    pdl_wait(); pdl_trigger();
     const bool wide = (((uintptr_t)g.top | (uintptr_t)g.topw | (uintptr_t)g.tp | (uintptr_t)g.slot) & 15) == 0;      // the caller's arrays may lie anywhere
     int x[TOPK]; float w[TOPK];
     if (mine) {
@@ -508,6 +509,7 @@ __global__ void __launch_bounds__(256, 4) silu_quant_kernel(const float *__restr
     __shared__ unsigned long long tab[32];
     if (threadIdx.x < 32) tab[threadIdx.x] = DEV_EXP_TAB[threadIdx.x];
     __syncthreads();
+    pdl_wait(); pdl_trigger();
     if (np_dev) np = min(np, *np_dev);
     const int lane = threadIdx.x & 31, a = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (a >= np) return;

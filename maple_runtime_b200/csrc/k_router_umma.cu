@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(192, 1) router_umma_kernel(const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tb = sh.tmem_base;
+    pdl_wait(); pdl_trigger();
     if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) *nflagged = 0;      // the selection kernel counts its flagged tokens from zero
     if (mask) {     // and sets the grouping's bits and counters: cleared here, one word per thread
         const int w = (blockIdx.y * gridDim.x + blockIdx.x) * 192 + tid;
@@ -167,13 +168,10 @@ __global__ void __launch_bounds__(192, 1) router_umma_kernel(const __grid_consta
 __global__ void __launch_bounds__(256) router_select_kernel(const float *__restrict__ part, int ntok_cap, const float *__restrict__ bias,
                                                             const float *__restrict__ hnorm, const float *__restrict__ wnorm,
                                                             float *__restrict__ logits, int *__restrict__ top, float *__restrict__ topw,
-                                                            int *__restrict__ flagged, int *__restrict__ nflagged, const uint8_t *__restrict__ router_s,
+                                                            int *__restrict__ flagged, int *__restrict__ nflagged,
                                                             unsigned *__restrict__ mask, int mask_words, int nb) {
-    {   // the flagged tokens' recomputation reads the layer's re-laid router rows (1 MB) right after this kernel: pull them into L2 now
-        const unsigned line = blockIdx.x * 256u + threadIdx.x;
-        if (line < NEXP * HID * 2 / 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(router_s + (size_t)line * 128));
-    }
     const int lane = threadIdx.x & 31, b = blockIdx.x * 8 + (threadIdx.x >> 5);
+    pdl_wait(); pdl_trigger();
     if (b >= nb) return;
     float l[8];
     {
@@ -242,58 +240,93 @@ __global__ void __launch_bounds__(256) router_select_kernel(const float *__restr
     }
 }
 
-// The flagged tokens over again as the reference computes them (maple.c:870-889, 117-121, 910-923).  grid (8 expert eighths, y): CTA
-// (x, y) walks flagged tokens y, y + gridDim.y, ... and computes 32 experts of each: 256 threads = 8 lanes x 32 experts, the eight strided
-// multiply-add chains per expert and their pairwise adds.  The last of a token's eight CTAs to finish (a counter per flagged slot, reset
-// by that CTA) runs the exact softmax + top-8 on the token's finished row.
+// The flagged tokens over again as the reference computes them (maple.c:870-889, 117-121, 910-923).  grid (8 expert eighths, RF_GROUPS): CTA
+// (x, y) walks flagged tokens y, y + RF_GROUPS, ... four at a time and computes 32 experts of each: 256 threads = 8 lanes x 32 experts, the
+// eight strided multiply-add chains per expert and their pairwise adds.  The last of a group's eight CTAs to finish (a counter per group
+// of four, reset by that CTA) runs the exact softmax + top-8 on the four finished rows, a warp each.
+// Bound by latency: list -> token -> hidden row -> 256 chained multiply-adds -> counter -> softmax + top-8.  So the CTA's 32 router rows come
+// into shared memory before it waits for the selection, four tokens' chains run side by side in a thread, and 144 CTAs cover 72 tokens (2% of
+// 2048 are flagged: 45) in one round.
 // WS: the router rows re-laid as [expert][column / 32][lane j][4 steps] bf16 (k_router_pack_small, k_router_tile.cu).
+#define RF_GROUPS 18
+#define RF_TOK 4
+#define RF_WPITCH (HID * 2 + 64)         /* rows 16 banks apart: the experts of a warp meet no bank twice */
+#define RF_SMEM (32 * RF_WPITCH + RF_TOK * HID * 4)
+__device__ __forceinline__ void rf_bulk(uint32_t dst_smem, const void *src, uint32_t bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst_smem), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
 __global__ void __launch_bounds__(256) router_fix_kernel(const uint8_t *__restrict__ WS, const float *__restrict__ hn, const float *__restrict__ bias,
                                                          float *__restrict__ logits, int *__restrict__ top, float *__restrict__ topw,
                                                          const int *__restrict__ flagged, const int *__restrict__ nflagged, int *__restrict__ done,
-                                                         unsigned *__restrict__ mask, int mask_words, int nb) {
-    __shared__ __align__(16) float hrow[HID];
+                                                         unsigned *__restrict__ mask, int mask_words, int nb, int *err) {
+    extern __shared__ __align__(128) uint8_t rf_sm[];
+    float *hrow = reinterpret_cast<float *>(rf_sm + 32 * RF_WPITCH);       // [RF_TOK][HID]
     __shared__ unsigned long long tab[32];
-    __shared__ int s_last;
-    const int tid = threadIdx.x, j = tid & 7, pos = tid >> 3, lane = tid & 31;
+    __shared__ uint64_t bar; __shared__ int s_last, abort_flag;
+    const int tid = threadIdx.x, j = tid & 7, pos = tid >> 3, lane = tid & 31, warp = tid >> 5, e = blockIdx.x * 32 + pos;
     if (tid < 32) tab[tid] = DEV_EXP_TAB[tid];
-    const int total = min(*nflagged, nb);
-    for (int f = blockIdx.y; f < total; f += gridDim.y) {
-        const int b = flagged[f];
+    if (tid == 0) {
+        mbar_init(&bar, 1); abort_flag = 0; mbar_init_fence();
+        mbar_expect_tx(&bar, 32 * HID * 2);
+        for (int r = 0; r < 32; r++) rf_bulk(smem_u32(rf_sm) + r * RF_WPITCH, WS + (size_t)(blockIdx.x * 32 + r) * (HID * 2), HID * 2, &bar);
+    }
+    const float be = bias ? bias[e] : 0.0f;
+    __syncthreads();
+    const bool ok = mbar_wait(&bar, 0, &abort_flag);
+    pdl_wait(); pdl_trigger();
+    const int total = ok ? min(*nflagged, nb) : 0;
+    if (!ok && tid == 0) *(volatile int *)err = 31;
+    for (int f0 = blockIdx.y; f0 < total; f0 += RF_GROUPS * RF_TOK) {
+        int b[RF_TOK];                                                      // the group's tokens; past the end the first one again, not stored
+#pragma unroll
+        for (int t = 0; t < RF_TOK; t++) { const int f = f0 + t * RF_GROUPS; b[t] = flagged[f < total ? f : f0]; }
+        const int n = (min(total, f0 + RF_GROUPS * RF_TOK) - f0 + RF_GROUPS - 1) / RF_GROUPS;
         __syncthreads();
-        for (int i = tid; i < HID / 4; i += 256) reinterpret_cast<float4 *>(hrow)[i] = reinterpret_cast<const float4 *>(hn + (size_t)b * HID)[i];
+#pragma unroll
+        for (int t = 0; t < RF_TOK; t++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) reinterpret_cast<float4 *>(hrow)[t * (HID / 4) + tid + 256 * i] = reinterpret_cast<const float4 *>(hn + (size_t)b[t] * HID)[tid + 256 * i];
         __syncthreads();
-        const int e = blockIdx.x * 32 + pos;
-        const uint8_t *wp = WS + (size_t)e * (HID * 2) + j * 8;
-        float acc = 0.0f;
-#pragma unroll 16
+        const uint8_t *wp = rf_sm + pos * RF_WPITCH + j * 8;
+        float acc[RF_TOK] = {};
+#pragma unroll 8
         for (int i4 = 0; i4 < 64; i4++) {
             const uint2 a = *reinterpret_cast<const uint2 *>(wp + i4 * 64);
-            acc = __fmaf_rn(__uint_as_float(a.x << 16), hrow[32 * i4 + j], acc);
-            acc = __fmaf_rn(__uint_as_float(a.x & 0xFFFF0000u), hrow[32 * i4 + 8 + j], acc);
-            acc = __fmaf_rn(__uint_as_float(a.y << 16), hrow[32 * i4 + 16 + j], acc);
-            acc = __fmaf_rn(__uint_as_float(a.y & 0xFFFF0000u), hrow[32 * i4 + 24 + j], acc);
+            const float w0 = __uint_as_float(a.x << 16), w1 = __uint_as_float(a.x & 0xFFFF0000u), w2 = __uint_as_float(a.y << 16), w3 = __uint_as_float(a.y & 0xFFFF0000u);
+#pragma unroll
+            for (int t = 0; t < RF_TOK; t++) {
+                const float *h = hrow + t * HID + 32 * i4 + j;
+                acc[t] = __fmaf_rn(w0, h[0], acc[t]); acc[t] = __fmaf_rn(w1, h[8], acc[t]); acc[t] = __fmaf_rn(w2, h[16], acc[t]); acc[t] = __fmaf_rn(w3, h[24], acc[t]);
+            }
         }
-        float l = acc;      // (l0+l4)+(l1+l5) then +((l2+l6)+(l3+l7)): the same on every lane of the expert
-        l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 4));
-        l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
-        l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 2));
-        if (j == 0) logits[(size_t)b * NEXP + e] = bias ? __fadd_rn(l, bias[e]) : l;
+#pragma unroll
+        for (int t = 0; t < RF_TOK; t++) {
+            float l = acc[t];      // (l0+l4)+(l1+l5) then +((l2+l6)+(l3+l7)): the same on every lane of the expert
+            l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 4));
+            l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
+            l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 2));
+            if (j == 0 && t < n) logits[(size_t)b[t] * NEXP + e] = bias ? __fadd_rn(l, be) : l;
+        }
         __threadfence();
         __syncthreads();
-        if (tid == 0) s_last = atomicAdd(&done[f], 1) == (int)gridDim.x - 1;
+        if (tid == 0) s_last = atomicAdd(&done[f0], 1) == (int)gridDim.x - 1;
         __syncthreads();
-        if (s_last && tid < 32) {
-            __threadfence();                                              // hrow is read no more: it is the scratch of the top-8
-            const float4 *lr = reinterpret_cast<const float4 *>(logits + (size_t)b * NEXP + lane * 8);
+        if (s_last && warp < n) {
+            __threadfence();
+            int bt = b[0];
+#pragma unroll
+            for (int t = 1; t < RF_TOK; t++) if (warp == t) bt = b[t];
+            const float4 *lr = reinterpret_cast<const float4 *>(logits + (size_t)bt * NEXP + lane * 8);
             const float4 v0 = __ldcg(lr), v1 = __ldcg(lr + 1);              // the other CTAs' values: read past L1
             float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
             int isel; float wsel, tsum;
-            exact_topk_warp(p, lane, tab, hrow, isel, wsel, tsum);
+            exact_topk_warp(p, lane, tab, hrow + warp * HID, isel, wsel, tsum);      // hrow is read no more: it is the scratch of the top-8
             if (lane < TOPK) {
-                top[b * TOPK + lane] = isel; topw[b * TOPK + lane] = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));
-                if (mask) { atomicOr(&mask[(size_t)(b >> 5) * NEXP + isel], 1u << (b & 31)); atomicAdd(&mask[(size_t)NEXP * mask_words + isel], 1u); }
+                top[bt * TOPK + lane] = isel; topw[bt * TOPK + lane] = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));
+                if (mask) { atomicOr(&mask[(size_t)(bt >> 5) * NEXP + isel], 1u << (bt & 31)); atomicAdd(&mask[(size_t)NEXP * mask_words + isel], 1u); }
             }
-            if (lane == 0) done[f] = 0;
+            if (tid == 0) done[f0] = 0;
         }
     }
 }
@@ -302,9 +335,9 @@ extern "C" void k_router_tensor(cudaStream_t st, const RouterTensorArgs *r) {
     if (r->nb <= 0) return;
     static bool attr_done = false;
     const int smem = RU_STAGES * RU_STAGE_BYTES + 1024;
-    if (!attr_done) { cudaFuncSetAttribute(router_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr_done = true; }
-    launch_k(router_umma_kernel, dim3(RU_KS, (r->nb + 127) / 128), 192, smem, st, r->amap, r->wmap, r->part, r->nb, r->ntok_cap, r->err, r->nflagged, r->mask, NEXP * r->mask_words + NEXP);
-    launch_k(router_select_kernel, (r->nb + 7) / 8, 256, 0, st, r->part, r->ntok_cap, r->bias, r->hnorm, r->wnorm, r->logits, r->top, r->topw, r->flagged, r->nflagged, (const uint8_t *)r->router_s, r->mask, r->mask_words, r->nb);
-    launch_k(router_fix_kernel, dim3(8, 74), 256, 0, st, (const uint8_t *)r->router_s, r->hn, r->bias, r->logits, r->top, r->topw, r->flagged, r->nflagged, r->done, r->mask, r->mask_words, r->nb);
+    if (!attr_done) { cudaFuncSetAttribute(router_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); cudaFuncSetAttribute(router_fix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RF_SMEM); attr_done = true; }
+    launch_pdl(router_umma_kernel, dim3(RU_KS, (r->nb + 127) / 128), 192, smem, st, r->amap, r->wmap, r->part, r->nb, r->ntok_cap, r->err, r->nflagged, r->mask, NEXP * r->mask_words + NEXP);
+    launch_pdl(router_select_kernel, (r->nb + 7) / 8, 256, 0, st, r->part, r->ntok_cap, r->bias, r->hnorm, r->wnorm, r->logits, r->top, r->topw, r->flagged, r->nflagged, r->mask, r->mask_words, r->nb);
+    launch_pdl(router_fix_kernel, dim3(8, RF_GROUPS), 256, RF_SMEM, st, (const uint8_t *)r->router_s, r->hn, r->bias, r->logits, r->top, r->topw, r->flagged, r->nflagged, r->done, r->mask, r->mask_words, r->nb, r->err);
     k_count_add(3);
 }

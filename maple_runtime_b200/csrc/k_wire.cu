@@ -40,12 +40,13 @@ __global__ void __launch_bounds__(CW_WARPS * 32, 1) combine_wire_kernel(uint8_t 
 #pragma unroll
         for (int it = 0; it < CW_EX / CW_WARPS; it++) p[it] = dsp[warp + CW_WARPS * it];
         const int npair = (b_end - b_begin) * TOPK;
-        int slot[(CW_MAXTOK * TOPK + CW_WARPS * 32 - 1) / (CW_WARPS * 32)];
-#pragma unroll
-        for (int it = 0; it < (int)(sizeof slot / sizeof slot[0]); it++) { const int i = tid + it * CW_WARPS * 32; slot[it] = i < npair ? tp[b_begin * TOPK + i] : -1; }
 #pragma unroll
         for (int it = 0; it < CW_EX / CW_WARPS; it++)
             v[it] = p[it] ? reinterpret_cast<const float4 *>(p[it] + rb * CW_ROWS)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        pdl_wait(); pdl_trigger();                                     // the scales are weights: read while the down kernel still runs elsewhere
+        int slot[(CW_MAXTOK * TOPK + CW_WARPS * 32 - 1) / (CW_WARPS * 32)];
+#pragma unroll
+        for (int it = 0; it < (int)(sizeof slot / sizeof slot[0]); it++) { const int i = tid + it * CW_WARPS * 32; slot[it] = i < npair ? tp[b_begin * TOPK + i] : -1; }
 #pragma unroll
         for (int it = 0; it < (int)(sizeof slot / sizeof slot[0]); it++) if (slot[it] >= 0) {
             const int4 rec = *reinterpret_cast<const int4 *>(recs + (size_t)slot[it] * WIRE_REC);

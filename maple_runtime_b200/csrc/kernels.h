@@ -41,6 +41,7 @@ typedef struct {
     /* the tcgen05 down kernel stores compact rows (see WIRE_* below) instead of fp32 ones: wire [np] rows, or in expert parallel
      * peer_wire[rank] = that rank's buffer */
     uint8_t *wire; uint8_t *const *peer_wire; int wire_cap;   /* wire_cap: pairs each such buffer is laid out for */
+    int call_maps;           /* 1: maps were written by a kernel of the same call: nothing is read through them before that kernel is complete */
     int *err;                /* set to 1 by a kernel whose bounded wait ran out */
 } ExpertArgs;
 

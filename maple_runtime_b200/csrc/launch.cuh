@@ -1,11 +1,13 @@
 // launch.cuh -- one way to launch every kernel of the layer loop (cudaLaunchKernelEx), so that launch attributes have one place to live.
 //
-// launch_pdl: programmatic dependent launch, for the kernels of decode batches.  Such a kernel is placed on the SMs while its predecessor in
+// launch_pdl: programmatic dependent launch, for the kernels of the layer loop.  Such a kernel is placed on the SMs while its predecessor in
 // the stream finishes; it does its own set-up and reads of weights, then calls pdl_wait() before it touches any memory that a predecessor
 // wrote or still reads, and pdl_trigger() after that: its own successor may then be placed.  Since a kernel triggers only after its wait,
 // everything before its predecessor is complete when it starts: what was written two kernels ago may be read before pdl_wait (past L1).
-// The kernels of prefill chunks do not trigger at their start: their successors' CTAs would take shared and tensor memory from the kernel that
-// is still running (24 layers of 2048 tokens: 4.69 ms against 4.37 ms).
+// Not every kernel gains: norm and SiLU of prefill chunks and their combine, placed early, end up unevenly spread over the SMs that happen to be
+// free first (4096 tokens: combine 324 against 308 us per layer, SiLU 308 against 302; 512 tokens: norm 110 against 108); they are launched plainly.
+// (Triggering before the wait, so that several kernels ahead are placed, was slower for prefill chunks: their CTAs take shared and tensor memory
+// from the kernel that is still running.)
 #pragma once
 #include <cuda_runtime.h>
 #include <string.h>
@@ -28,12 +30,13 @@ static inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 b
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #endif
-// the same as one cluster of `ctas` CTAs
+// the same, programmatically too, as one cluster of `ctas` CTAs
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_cluster(void (*kernel)(KArgs...), unsigned ctas, dim3 block, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof cfg);
-    cudaLaunchAttribute at; memset(&at, 0, sizeof at);
-    at.id = cudaLaunchAttributeClusterDimension; at.val.clusterDim.x = ctas; at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.gridDim = ctas; cfg.blockDim = block; cfg.stream = st; cfg.attrs = &at; cfg.numAttrs = 1;
+    cudaLaunchAttribute at[2]; memset(at, 0, sizeof at);
+    at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = ctas; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = ctas; cfg.blockDim = block; cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
