@@ -93,9 +93,12 @@ extern "C" void k_combine_wire(cudaStream_t st, uint8_t *wire, int np_cap, const
         int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaFuncSetAttribute(combine_wire_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     }
-    int groups = sms / (HID / CW_ROWS); if (groups < 1) groups = 1;      // one wave of CTAs: 16 row blocks x groups
+    /* whole waves of CTAs (16 row blocks x groups, one CTA per SM), every CTA with as many tokens as the last wave's: 4096 tokens are 18 groups of 228
+     * (1.95 waves) instead of 15 of 288 (1.62) */
+    const int fit = sms / (HID / CW_ROWS) > 0 ? sms / (HID / CW_ROWS) : 1, least = (nb + CW_MAXTOK - 1) / CW_MAXTOK, waves = (least + fit - 1) / fit;
+    int groups = waves * sms / (HID / CW_ROWS); if (groups < 1) groups = 1;
     int per = (nb + groups - 1) / groups; if (per < CW_WARPS) per = CW_WARPS;
-    if (per > CW_MAXTOK) per = CW_MAXTOK;                                  /* more tokens than one wave holds: more groups */
+    if (per > CW_MAXTOK) per = CW_MAXTOK;
     groups = (nb + per - 1) / per;
     launch_k(combine_wire_kernel, dim3(HID / CW_ROWS, groups), CW_WARPS * 32, smem, st, wire, np_cap, dsp, uw, tp, init, out, nb, per);
     k_count_add(1);
