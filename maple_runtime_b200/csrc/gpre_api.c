@@ -28,6 +28,8 @@ void k_count_add(long n);
 /* Up to so many tokens (0.8 MB) kernels read and write a caller's page-locked rows in place: 0.5 MB takes 11 us like this and 9 us by a copy, but a
  * copy is a link of its own in the chain of a call (submit, wait for the event, move to its place), 25 us and more with its neighbours. */
 #define INPLACE_MAXTOK 96
+#define INPLACE_WIDE 3072
+#define H_ROWS_OUT (S.h_rows + (size_t)INPLACE_MAXTOK * INPLACE_WIDE)
 
 static char g_err[512];
 static int fail(const char *who, const char *fmt, ...) {
@@ -56,7 +58,7 @@ static struct {
     const float **dsp_call, *h_dsp[NEXP];   /* down-scale pointers of one gpre_moe call's experts; host staging */
     float *x, *hn, *y, *hqs, *logits, *topw, *uw, *act, *aqs, *down, *gate, *up, *bias;
     int8_t *hq, *aq;
-    float *h_rows;             /* page-locked: a decode batch's rows in, and behind them its rows out */
+    float *h_rows;             /* page-locked: a decode batch's rows in, and behind them its rows out (INPLACE_WIDE values per token each) */
     int *ecnt, *uexp, *hqsum, *top, *nu, *ue, *estart, *ustart, *utok, *slot, *tp, *aqsum, *ntiles_a, *ntiles_b, *gu_dots, *dn_dots;
     unsigned *mask; int *err, *h_err;      /* the kernels' error word, in page-locked host memory: the device's and the host's pointer to it */
     MoeTile *tiles_a, *tiles_b;
@@ -169,9 +171,9 @@ static int init_common(const char *who, int maxtok, int topk) {
     if (bmaps(who, P)) return -1;
     CU(who, cudaHostAlloc((void **)&S.h_err, 16, cudaHostAllocMapped)); *S.h_err = 0;
     CU(who, cudaHostGetDevicePointer((void **)&S.err, S.h_err, 0));
-    CT.cap = P * 12 + (P / 8 + NEXP) * sizeof(MoeTile) + T * 8 + NEXP * (sizeof(ExpertMaps) + sizeof(ExpertPtrs) + 16) + 4096;
+    CT.cap = (size_t)INPLACE_MAXTOK * (HID + 8) + P * 12 + (P / 8 + NEXP) * sizeof(MoeTile) + T * 8 + NEXP * (sizeof(ExpertMaps) + sizeof(ExpertPtrs) + 16) + 4096;
     CU(who, cudaHostAlloc((void **)&CT.h, CT.cap, cudaHostAllocMapped)); CU(who, cudaEventCreateWithFlags(&CT.taken, cudaEventDisableTiming));
-    CU(who, cudaHostAlloc((void **)&S.h_rows, (size_t)2 * INPLACE_MAXTOK * HID * 4, cudaHostAllocMapped));
+    CU(who, cudaHostAlloc((void **)&S.h_rows, (size_t)2 * INPLACE_MAXTOK * INPLACE_WIDE * 4, cudaHostAllocMapped));
     S.h_tab = malloc(NEXP * sizeof(ExpertPtrs));
     S.h_maps = aligned_alloc(64, NEXP * sizeof(ExpertMaps)); S.map_cache = aligned_alloc(64, MAP_CACHE * sizeof *S.map_cache);
     if (!S.h_tab || !S.h_maps || !S.map_cache) return fail(who, "out of host memory");
@@ -561,7 +563,7 @@ static void decode_layers(int nb, int l0, int nl, const float *bias) {
 static void decode_moe(int nb, int L, const float *bias) {
     k_norm_prep_relaid(S.st, S.h_rows, NULL, S.hn, S.hq, S.hqs, S.hqsum, (float *)S.hT, nb);
     decode_body(&S.ly[L], nb, bias);
-    k_combine(S.st, S.down, S.uw, S.tp, NULL, S.h_rows + (size_t)INPLACE_MAXTOK * HID, nb);
+    k_combine(S.st, S.down, S.uw, S.tp, NULL, H_ROWS_OUT, nb);
 }
 /* nl = 0: decode_moe of layer l0 */
 static int layers_run(int nb, int l0, int nl, const float *bd, int ep) {
@@ -617,7 +619,7 @@ double gmoe_moe(int L, const float *x, int nb, float *y, const float *bias) {
         cudaEventRecord(S.e1, S.st);
         S.nb_cur = nb;
         const double t = finish("gmoe");
-        if (t >= 0) hio_copy_shared(y, S.h_rows + (size_t)INPLACE_MAXTOK * HID, n * 4);
+        if (t >= 0) hio_copy_shared(y, H_ROWS_OUT, n * 4);
         return t;
     }
     if (rows_in("gmoe", S.hn, x, nb)) return -1.0;
@@ -1046,6 +1048,18 @@ double gmoe_qk_rope(const float *qkv, const int *pos, int nb, int glob, const fl
     if (!qkv || !pos || !qn || !kn || !q || !kc || !vc) { fail("gmoe", "gmoe_qk_rope: null argument"); return -1.0; }
     if (!glob && !AT.cs) { fail("gmoe", "gmoe_qk_rope on a local layer before gmoe_rope_table"); return -1.0; }
     if (!glob) for (int b = 0; b < nb; b++) if (pos[b] < 0 || pos[b] >= AT.positions) { fail("gmoe", "gmoe_qk_rope: position %d of token %d outside the table (%d positions)", pos[b], b, AT.positions); return -1.0; }
+    if (nb <= INPLACE_MAXTOK) {      /* rows through page-locked memory that the kernel reads and writes in place: one launch, no copies */
+        RopeArgs prm;
+        memcpy(prm.qn, qn, sizeof prm.qn); memcpy(prm.kn, kn, sizeof prm.kn); memcpy(prm.pos, pos, (size_t)nb * sizeof *pos);
+        float *oq = H_ROWS_OUT; uint16_t *ok = (uint16_t *)(oq + (size_t)nb * 2048), *ov = ok + (size_t)nb * 512;
+        hio_copy_shared(S.h_rows, qkv, (size_t)nb * 3072 * 4);
+        cudaEventRecord(S.e0, S.st);
+        k_qk_rope_small(S.st, S.h_rows, &prm, nb, glob, AT.cs, AT.positions, oq, ok, ov, S.err);
+        cudaEventRecord(S.e1, S.st);
+        const double t = finish("gmoe");
+        if (t >= 0) { hio_copy_shared(q, oq, (size_t)nb * 2048 * 4); memcpy(kc, ok, (size_t)nb * 1024); memcpy(vc, ov, (size_t)nb * 1024); }
+        return t;
+    }
     if (nb > AT.cap) {
         cudaStreamSynchronize(S.st);
         cudaFree(AT.qkv); cudaFree(AT.q); cudaFree(AT.kc); cudaFree(AT.vc); cudaFree(AT.pos); cudaFree(AT.norms); AT.cap = 0;
@@ -1144,12 +1158,35 @@ static int dense_rows(void *ctx, int r, int n) {
     if (um) k_dense_umma(S.st, &a, &bmap_tok); else k_dense_mma(S.st, &a, ys);
     return 0;
 }
+#define QUANT_ROWS 3              /* rows per piece of work: 24 KB */
+typedef struct { const float *x; int nb; int8_t *q; float *qs; int *qsum; } QuantJob;
+static void quant_piece(void *p, int i) {
+    const QuantJob *j = p;
+    const int r = i * QUANT_ROWS, n = j->nb - r < QUANT_ROWS ? j->nb - r : QUANT_ROWS;
+    hio_quant_rows(j->x + (size_t)r * HID, n, j->q + (size_t)r * HID, j->qs + r, j->qsum + r);
+}
 double gpre_dense(int g, const float *x, int nb, float *y) {
     if (!S.ready || !DY) { fail("gpre", "gpre_dense before gpre_dense_done"); return -1.0; }
     if (g < 0 || g >= DGRP || !DG[g].codes) { fail("gpre", "gpre_dense: group %d has no matrices on the card", g); return -1.0; }
     if (nb < 1 || nb > DY_tok) { fail("gpre", "gpre_dense: %d tokens outside 1..%d", nb, DY_tok); return -1.0; }
     if (S.keep && rows_in("gpre", S.hn, x, nb)) return -1.0;
     DenseCall d = {g, nb};
+    if (nb <= INPLACE_MAXTOK && DG[g].rows <= INPLACE_WIDE) {      /* three kernels in a row: int8 rows in, the product, its rows out */
+        if (tables_begin("gpre")) return -1.0;
+        QuantJob j = {x, nb, tables_add(S.hq, (size_t)nb * HID), tables_add(S.hqs, (size_t)nb * 4), tables_add(S.hqsum, (size_t)nb * 4)};
+        if ((size_t)nb * HID * 4 < HIO_POOL_BYTES) { for (int i = 0; i * QUANT_ROWS < nb; i++) quant_piece(&j, i); }
+        else hio_wait(hio_submit(quant_piece, &j, (nb + QUANT_ROWS - 1) / QUANT_ROWS));
+        const size_t bytes = (size_t)nb * DG[g].rows * 4;
+        cudaEventRecord(S.e0, S.st);
+        k_tables(S.st, &CT.seg);             /* no event behind it: the call waits for the stream anyway, and the product is launched programmatically */
+        dense_rows(&d, 0, nb);
+        k_rows(S.st, H_ROWS_OUT, DY, bytes);
+        cudaEventRecord(S.e1, S.st);
+        S.nb_cur = nb;
+        const double t = finish("gpre");
+        if (t >= 0) hio_copy_shared(y, H_ROWS_OUT, bytes);
+        return t;
+    }
     Flow f; memset(&f, 0, sizeof f);
     f.rows = nb; f.chunk = DENSE_CHUNK; f.src = x; f.row = HID * 4; f.dst = S.hq; f.quant = 1; f.hqs = DH_qs; f.hqsum = DH_qsum; f.dst_qs = S.hqs; f.qs_pitch = (size_t)S.maxtok;
     f.compute = dense_rows; f.ctx = &d; f.timed = 1;

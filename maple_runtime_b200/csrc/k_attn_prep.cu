@@ -19,9 +19,14 @@ extern "C" void k_count_add(long n);
 
 // One warp per (token, group of four heads): groups 0-3 the query heads, 4 the key heads, 5 the value heads; the four rows of a group are
 // loaded together, so that a lane has four 16-byte loads in flight.
+// SMALL: the norms and positions come in the launch's parameters (their own copies to the card would cost more than the kernel), qkv, q, kc and vc
+// may be page-locked host memory: every value is read and written once, in runs of 256 bytes and more.
+template <bool SMALL>
 __global__ void __launch_bounds__(256) qk_rope_kernel(const float *__restrict__ qkv, const int *__restrict__ pos, int nb, int glob,
                                                       const float *__restrict__ qn, const float *__restrict__ kn, const float *__restrict__ cs, int cs_positions,
-                                                      float *__restrict__ q, __half *__restrict__ kc, __half *__restrict__ vc, int *err) {
+                                                      float *__restrict__ q, __half *__restrict__ kc, __half *__restrict__ vc, int *err, const __grid_constant__ RopeArgs prm) {
+    __shared__ __align__(16) float s_norm[SMALL ? 2 * AP_HD : 4];
+    if (SMALL) { s_norm[threadIdx.x] = threadIdx.x < AP_HD ? prm.qn[threadIdx.x] : prm.kn[threadIdx.x - AP_HD]; __syncthreads(); }
     const int lane = threadIdx.x & 31, item = blockIdx.x * 8 + (threadIdx.x >> 5);
     const int b = item / 6, grp = item % 6;
     if (b >= nb) return;
@@ -37,10 +42,10 @@ __global__ void __launch_bounds__(256) qk_rope_kernel(const float *__restrict__ 
         }
         return;
     }
-    const float4 w = reinterpret_cast<const float4 *>(grp < 4 ? qn : kn)[lane];
+    const float4 w = SMALL ? reinterpret_cast<const float4 *>(s_norm + (grp < 4 ? 0 : AP_HD))[lane] : reinterpret_cast<const float4 *>(grp < 4 ? qn : kn)[lane];
     float4 c4 = make_float4(0.f, 0.f, 0.f, 0.f), s4 = c4;
     if (!glob) {
-        int p = pos[b];
+        int p = SMALL ? prm.pos[b] : pos[b];
         if (p < 0 || p >= cs_positions) { if (lane == 0) *(volatile int *)err = 51; p = 0; }      // a position outside the table: flagged, not read
         if (lane < 16) {
             const float4 *t = reinterpret_cast<const float4 *>(cs + ((size_t)p * 32 + 4 * (lane & 7)) * 2);      // (cos, sin) of four pairs
@@ -73,6 +78,12 @@ extern "C" void k_qk_rope(cudaStream_t st, const float *qkv, const int *pos, int
                           float *q, void *kc, void *vc, int *err) {
     if (nb <= 0) return;
     const int items = nb * 6;
-    launch_k(qk_rope_kernel, (items + 7) / 8, 256, 0, st, qkv, pos, nb, glob, qn, kn, cs, cs_positions, q, (__half *)kc, (__half *)vc, err);
+    static const RopeArgs none = {};
+    launch_k(qk_rope_kernel<false>, (items + 7) / 8, 256, 0, st, qkv, pos, nb, glob, qn, kn, cs, cs_positions, q, (__half *)kc, (__half *)vc, err, none);
+    k_count_add(1);
+}
+extern "C" void k_qk_rope_small(cudaStream_t st, const float *qkv, const RopeArgs *prm, int nb, int glob, const float *cs, int cs_positions, float *q, void *kc, void *vc, int *err) {
+    if (nb <= 0) return;
+    launch_k(qk_rope_kernel<true>, (nb * 6 + 7) / 8, 256, 0, st, qkv, (const int *)NULL, nb, glob, (const float *)NULL, (const float *)NULL, cs, cs_positions, q, (__half *)kc, (__half *)vc, err, *prm);
     k_count_add(1);
 }

@@ -10,6 +10,7 @@
 extern "C" void k_count_add(long n);
 
 __global__ void __launch_bounds__(256) tables_kernel(const __grid_constant__ TableSegs t) {
+    pdl_trigger();                                                       // a successor launched programmatically waits for the whole kernel all the same
     const unsigned words = t.words[blockIdx.y], step = gridDim.x * 256;
     const uint32_t *src = static_cast<const uint32_t *>(t.src[blockIdx.y]);
     uint32_t *dst = static_cast<uint32_t *>(t.dst[blockIdx.y]);

@@ -115,6 +115,10 @@ void k_gather_rows(cudaStream_t st, const int8_t *src, const int *rows, int8_t *
  * = q 2048 | k 512 | v 512; pos [nb]; qn, kn [128] fp32; cs [cs_positions][32][2] (cos, sin); q [nb][2048] fp32; kc, vc [nb][512] fp16 */
 void k_qk_rope(cudaStream_t st, const float *qkv, const int *pos, int nb, int glob, const float *qn, const float *kn, const float *cs, int cs_positions,
                float *q, void *kc, void *vc, int *err);
+/* the same for up to ROPE_SMALL tokens, norms and positions by value; qkv, q, kc, vc may be page-locked host memory */
+#define ROPE_SMALL 96
+typedef struct { float qn[128], kn[128]; int pos[ROPE_SMALL]; } RopeArgs;
+void k_qk_rope_small(cudaStream_t st, const float *qkv, const RopeArgs *prm, int nb, int glob, const float *cs, int cs_positions, float *q, void *kc, void *vc, int *err);
 
 /* ---- router on the tensor cores (k_router_umma.cu): logits, top-8 and weights of nb tokens.  Tokens whose nine largest logits are
  * too close to call are recomputed in the reference's exact order of operations, so the indices are the reference's for every token;
