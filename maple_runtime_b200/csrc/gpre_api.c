@@ -418,12 +418,12 @@ static void run_combine(const float *const *dsp, int nb, const float *init, floa
     if (use_umma(nb)) k_combine_wire(S.st, S.wire, S.maxp, dsp, S.uw, S.tp, init, out, nb);
     else k_combine(S.st, S.down, S.uw, S.tp, init, out, nb);
 }
-/* router logits: large batches take the tiled kernel, small ones the one-wait kernel, both on re-laid rows.  The tiled kernel takes 38 us for any
- * batch from 257 to 511 tokens (at most 64 CTAs), the other 28.6 at 301, 33.1 at 400 and 40.2 at 511. */
+/* router logits: large batches take the tiled kernel, small ones the kernels that read the norm's re-laid rows in place (k_router_logits_small chooses).
+ * The line: a layer takes 103.6 us with the latter and 112 with the former at 400 tokens, 105.1 and 104.5 at 420, 110 and 108.7 at 511. */
 #define ROUTER_TILE_MIN 417
 static void run_router_relaid(const LayerDev *l, const float *bias, int nb, int relaid) {   /* relaid: the norm kernel already wrote S.hT */
     if (nb >= ROUTER_TILE_MIN) k_router_logits_tile(S.st, l->router_t, S.hn, S.hT, bias, S.logits, nb, S.err);
-    else k_router_logits_small(S.st, l->router_s, S.hn, S.hT, relaid, bias, S.logits, nb, S.err);
+    else k_router_logits_small(S.st, l->router_s, l->router_t, S.hn, S.hT, relaid, bias, S.logits, nb, S.err);
 }
 static void run_router(const LayerDev *l, const float *bias, int nb) { run_router_relaid(l, bias, nb, 0); }
 /* Which router: 0 = by size (tensor cores from 512 tokens on), 1 = always the exact-order kernels, 2 = tensor cores for every size. */
@@ -546,7 +546,7 @@ static int run_layer_ep(int L, int nb, const float *bias);
  * so are top-8 and grouping of up to TOPK_IN_MAX tokens. */
 static int decode_path(int nb) { return nb <= 256 && !use_umma(nb) && !tensor_router(nb) && !S.keep && !S.prof_mask; }
 static void decode_body(const LayerDev *l, int nb, const float *bias) {
-    k_router_logits_small(S.st, l->router_s, S.hn, S.hT, 1, bias, S.logits, nb, S.err);
+    k_router_logits_small(S.st, l->router_s, l->router_t, S.hn, S.hT, 1, bias, S.logits, nb, S.err);
     if (nb > TOPK_IN_MAX) k_topk(S.st, S.logits, S.top, S.topw, nb);
     run_group_l(nb, 0, nb > TOPK_IN_MAX ? NULL : S.logits);
     run_experts(l->tab, l->maps, (const float *const *)l->dsp, S.ue, nb, 7);

@@ -197,7 +197,7 @@ extern "C" void k_router_logits_tile(cudaStream_t st, const void *router_t, cons
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Decode batches (up to 256 tokens).  The arithmetic is a handful of microseconds of dependent multiply-adds (256 per chain), so
+// Decode batches (up to 144 tokens on 148 SMs).  The arithmetic is a handful of microseconds of dependent multiply-adds (256 per chain), so
 // the kernel is about latency: a CTA owns 8 tokens x 8 experts, fetches all 2048 columns of both in two bulk copies (64 KB of
 // hidden values, 32 KB of bf16 weights, both pre-laid as [column / 32][lane j][4 steps] so that the eight lanes of a position
 // read consecutive 16-byte (8-byte) pieces), waits once, and runs the 64 x 4 steps without another synchronisation.  Two CTAs
@@ -270,6 +270,132 @@ __global__ void __launch_bounds__(256, 2) router_small_kernel(const uint8_t *__r
     }
     if (tid == 0 && !ok) *(volatile int *)err = 31;
 }
+// ---------------------------------------------------------------------------------------------------------------------
+// A few hundred tokens.  The kernel above runs one wave per 74 of them (a multiply-add costs it three quarters of a shared-memory read and an unpacking);
+// the prefill kernel's CTAs are too few to fill the SMs, its one warp per scheduler issues every 2.5 cycles, and it wants its rows copied once more.  Here a
+// warp is 8 lanes x 4 positions of TT tokens x 8 experts, small enough for two warps per scheduler at 300 tokens; a CTA is four of them on the same 4 TT
+// tokens and 32 experts, and a fifth that fills a ring of three stages of 256 columns.  Rows and weights are read as they lie: rows in the decode layout that
+// the norm left, weights in the tile layout.  Kernel above -> here, per layer of the stack: 160 tokens 84.8 -> 83.1, 256 108.2 -> 105.6, 301 103.3 -> 98.7,
+// 416 112.5 -> 104.9 us.  (TT = 4 with 16 experts per position, two warps per CTA: 103 at 301, 107 at 400.)
+// ---------------------------------------------------------------------------------------------------------------------
+#define RM_COLS 256
+#define RM_NCH (HID / RM_COLS)
+#define RM_ROW (RM_COLS * 4)
+#define RM_WB (2 * 2 * RP_GRP)            /* two chunks of the tile layout x two groups of 16 experts */
+#define RM_STAGES 3
+template <int TT>
+__global__ void __launch_bounds__(160) router_mid_kernel(const uint8_t *__restrict__ WT, const uint8_t *__restrict__ hS, const float *__restrict__ bias,
+                                                         float *__restrict__ logits, int nb, int *err) {
+    extern __shared__ __align__(128) uint8_t rm_ring[];
+    __shared__ uint64_t full[RM_STAGES], empty[RM_STAGES]; __shared__ int abort_flag, late;
+    constexpr int HB = 4 * TT * RM_ROW, STAGE = HB + RM_WB;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, j = lane & 7, tg = lane >> 3;
+    const int tok0 = blockIdx.y * 4 * TT, g0 = blockIdx.x * 2;            // first token, first group of 16 experts
+    if (tid == 0) {
+        for (int s = 0; s < RM_STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); }
+        abort_flag = late = 0; mbar_init_fence();
+    }
+    __syncthreads();
+    if (warp == 4) {                                                       // lane 0 copies the weights, lane t row t of the tile (a row past the end is the last one again)
+        auto issue_w = [&](int ch) {
+            const int s = ch % RM_STAGES;
+            mbar_expect_tx(&full[s], STAGE);
+            const uint8_t *w = WT + (size_t)(g0 / 8) * RP_NCH * RP_WB + (g0 % 8) * RP_GRP;
+            for (int h = 0; h < 2; h++) bulk_load(smem_u32(rm_ring) + s * STAGE + HB + h * 2 * RP_GRP, w + (size_t)(2 * ch + h) * RP_WB, 2 * RP_GRP, &full[s]);
+        };
+        auto issue_h = [&](int ch) {
+            const int s = ch % RM_STAGES;
+            bulk_load(smem_u32(rm_ring) + s * STAGE + lane * RM_ROW, hS + (size_t)min(tok0 + lane, nb - 1) * HID * 4 + ch * RM_ROW, RM_ROW, &full[s]);
+        };
+        if (lane == 0) for (int ch = 0; ch < RM_STAGES; ch++) issue_w(ch);   // the layer's weights: no kernel of the layer loop writes them
+        __syncwarp();
+        pdl_wait(); pdl_trigger();
+        if (lane < 4 * TT) for (int ch = 0; ch < RM_STAGES; ch++) issue_h(ch);
+        int ch = RM_STAGES;
+        for (; ch < RM_NCH; ch++) {
+            const bool go = mbar_wait(&empty[ch % RM_STAGES], (ch / RM_STAGES - 1) & 1, &abort_flag);
+            if (!__all_sync(0xffffffffu, go)) break;
+            if (lane == 0) issue_w(ch);
+            __syncwarp();
+            if (lane < 4 * TT) issue_h(ch);
+        }
+        // after a wait that ran out the copies still in flight land first (again with a limit)
+        if (ch < RM_NCH && lane == 0) for (int c = ch - RM_STAGES; c < ch; c++) mbar_wait(&full[c % RM_STAGES], (c / RM_STAGES) & 1, &late);
+    } else {
+        pdl_wait(); pdl_trigger();
+        uint64_t acc[TT][4];                                               // [token][expert pair], halves = experts 2m, 2m+1
+#pragma unroll
+        for (int a = 0; a < TT; a++)
+#pragma unroll
+            for (int m = 0; m < 4; m++) acc[a][m] = 0ull;
+        bool live = true;
+        for (int ch = 0; ch < RM_NCH; ch++) {
+            const int s = ch % RM_STAGES;
+            if (!mbar_wait(&full[s], (ch / RM_STAGES) & 1, &abort_flag)) live = false;
+            live = __all_sync(0xffffffffu, live);
+            if (!live) break;
+            const uint8_t *hp = rm_ring + s * STAGE + tg * TT * RM_ROW + j * 16, *wp = rm_ring + s * STAGE + HB + (warp >> 1) * RP_GRP + (warp & 1) * 128 + j * 16;
+            // a step's weights are read one step ahead, its rows four (the last read of a chunk wraps to its start and goes unused)
+            float4 hv[TT], hn4[TT];
+#pragma unroll
+            for (int a = 0; a < TT; a++) hn4[a] = *reinterpret_cast<const float4 *>(hp + a * RM_ROW);
+            uint4 n0 = *reinterpret_cast<const uint4 *>(wp);
+#pragma unroll 2
+            for (int i4 = 0; i4 < RM_COLS / 32; i4++) {
+#pragma unroll
+                for (int a = 0; a < TT; a++) { hv[a] = hn4[a]; hn4[a] = *reinterpret_cast<const float4 *>(hp + a * RM_ROW + (i4 + 1) % 8 * 128); }
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const uint32_t wu[4] = {n0.x, n0.y, n0.z, n0.w};
+                    const int t = (4 * i4 + k + 1) % 32;
+                    n0 = *reinterpret_cast<const uint4 *>(wp + (t >> 4) * 2 * RP_GRP + (t & 15) * 256);
+                    uint64_t wv[4];
+#pragma unroll
+                    for (int m = 0; m < 4; m++) wv[m] = pair64(wu[m] << 16, wu[m] & 0xFFFF0000u);
+#pragma unroll
+                    for (int a = 0; a < TT; a++) {
+                        const float h = k == 0 ? hv[a].x : k == 1 ? hv[a].y : k == 2 ? hv[a].z : hv[a].w;
+                        const uint64_t hh = pair64(__float_as_uint(h), __float_as_uint(h));
+#pragma unroll
+                        for (int m = 0; m < 4; m++) fma2(acc[a][m], wv[m], hh);
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[s]);
+        }
+        if (live) {
+            const int e0 = (g0 + (warp >> 1)) * 16 + (warp & 1) * 8, b0 = tok0 + tg * TT;
+#pragma unroll
+            for (int a = 0; a < TT; a++) {
+                float l[8];
+#pragma unroll
+                for (int m = 0; m < 4; m++) { l[2 * m] = __uint_as_float((uint32_t)acc[a][m]); l[2 * m + 1] = __uint_as_float((uint32_t)(acc[a][m] >> 32)); }
+                float p = 0.0f;                                            // every lane gets all eight sums and stores that of expert j
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    l[c] = __fadd_rn(l[c], __shfl_xor_sync(0xffffffffu, l[c], 4));
+                    l[c] = __fadd_rn(l[c], __shfl_xor_sync(0xffffffffu, l[c], 1));
+                    l[c] = __fadd_rn(l[c], __shfl_xor_sync(0xffffffffu, l[c], 2));
+                    if (j == c) p = l[c];
+                }
+                if (b0 + a < nb) logits[(size_t)(b0 + a) * NEXP + e0 + j] = bias ? __fadd_rn(p, bias[e0 + j]) : p;
+            }
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && abort_flag) *(volatile int *)err = 31;      // a wait ran out: the host reports it and the logits are not to be used
+}
+static int mid_ctas(int nb, int tt) { return NEXP / 32 * ((nb + 4 * tt - 1) / (4 * tt)); }
+template <int TT>
+static void launch_mid(cudaStream_t st, const void *router_t, const void *hS, const float *bias, float *logits, int nb, int *err) {
+    static bool attr_done = false;
+    const int smem = RM_STAGES * (4 * TT * RM_ROW + RM_WB);
+    if (!attr_done) { cudaFuncSetAttribute(router_mid_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr_done = true; }
+    const dim3 grid(NEXP / 32, (nb + 4 * TT - 1) / (4 * TT));
+    // plainly: placed early, several CTAs end up on the SMs that the norm leaves first (400 tokens: 105.2 against 103.6 us per layer)
+    launch_k(router_mid_kernel<TT>, grid, 160, smem, st, (const uint8_t *)router_t, (const uint8_t *)hS, bias, logits, nb, err);
+}
 extern "C" void k_router_pack_small(cudaStream_t st, const uint16_t *router, void *router_s) {
     router_pack_w_small_kernel<<<NEXP * HID / 4 / 256, 256, 0, st>>>(router, (uint2 *)router_s);
     k_count_add(1);
@@ -277,7 +403,7 @@ extern "C" void k_router_pack_small(cudaStream_t st, const uint16_t *router, voi
 static int g_step_order = 0;
 // single-token calls compute their logits in the order of the reference's `step` (bf_row) instead of `step_batch` (gmoe_set_step_order)
 extern "C" void k_router_step_order(int on) { g_step_order = on != 0; }
-extern "C" void k_router_logits_small(cudaStream_t st, const void *router_s, const float *hn, void *hS, int relaid, const float *bias, float *logits, int nb, int *err) {
+extern "C" void k_router_logits_small(cudaStream_t st, const void *router_s, const void *router_t, const float *hn, void *hS, int relaid, const float *bias, float *logits, int nb, int *err) {
     if (nb <= 0) return;
     static bool attr_done = false;
     if (!attr_done) {
@@ -285,6 +411,15 @@ extern "C" void k_router_logits_small(cudaStream_t st, const void *router_s, con
         cudaFuncSetAttribute(router_small_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_HB + RS_WB); attr_done = true;
     }
     if (!relaid) launch_k(router_pack_h_small_kernel, nb * 2, 256, 0, st, hn, (float4 *)hS, nb);
+    static int sms = 0;
+    if (!sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); if (sms < 1) sms = 148; }
+    if (nb > 2 * 2 * sms / (NEXP / RS_EXP) * RS_TOK) {             // past two waves of the small kernel (148 tokens)
+        // 12 tokens per CTA (10.5 us as one CTA per SM, 16.1 as two), or 16 where that is one CTA per SM and 12 would be two (13.8: 217 to 288 tokens)
+        if (mid_ctas(nb, 4) <= sms && mid_ctas(nb, 3) > sms) launch_mid<4>(st, router_t, hS, bias, logits, nb, err);
+        else launch_mid<3>(st, router_t, hS, bias, logits, nb, err);
+        k_count_add(relaid ? 1 : 2);
+        return;
+    }
     const dim3 grid(NEXP / RS_EXP, (nb + RS_TOK - 1) / RS_TOK);
     if (g_step_order && nb == 1) launch_pdl(router_small_kernel<true>, grid, 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err);
     else launch_pdl(router_small_kernel<false>, grid, 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err);

@@ -61,10 +61,10 @@ void k_norm_prep_relaid(cudaStream_t st, const float *x, const uint16_t *w, floa
 /* prefill-sized batches: router_t = the layer's router rows re-laid by k_router_pack (NEXP*HID*2 bytes), hT = scratch of
  * ceil(nb/16)*16*HID*8 bytes; err receives 31 if a bounded wait inside the kernel ran out */
 void k_router_pack(cudaStream_t st, const uint16_t *router, void *router_t);
-/* decode batches: router_s = the rows re-laid by k_router_pack_small (NEXP*HID*2 bytes), hS = scratch of nb*HID*4 bytes */
+/* up to a few hundred tokens: router_s = the rows re-laid by k_router_pack_small (NEXP*HID*2 bytes), router_t by k_router_pack, hS = scratch of nb*HID*4 bytes */
 void k_router_pack_small(cudaStream_t st, const uint16_t *router, void *router_s);
 void k_router_step_order(int on);   /* nb == 1: the order of maple.c's bf_row (two chains per lane) instead of job_route_small's */
-void k_router_logits_small(cudaStream_t st, const void *router_s, const float *hn, void *hS, int relaid, const float *bias, float *logits, int nb, int *err);
+void k_router_logits_small(cudaStream_t st, const void *router_s, const void *router_t, const float *hn, void *hS, int relaid, const float *bias, float *logits, int nb, int *err);
 void k_router_logits_tile(cudaStream_t st, const void *router_t, const float *hn, void *hT, const float *bias, float *logits, int nb, int *err);
 void k_topk(cudaStream_t st, const float *logits, int *top, float *topw, int nb);
 /* norm + int8 as k_norm_prep, and the normalised rows once more as two fp16 terms per value (hA: [nb][4096] fp16, hi then lo) with the

@@ -1,0 +1,23 @@
+"""The router of a few hundred tokens (csrc/k_router_tile.cu: router_mid_kernel) against the oracle, where its choice of 12 or 16 tokens per CTA changes and
+where the last CTA holds one token or all of them."""
+import numpy as np
+import pytest
+
+from conftest import SEED
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nb", [145, 156, 157, 216, 217, 272, 288, 289, 301, 416])
+def test_mid_router_equals_oracle(nb, gpu, oracle, weights):
+    gpu.synth_layer(SEED, 2)
+    router, _, _ = weights.layer(2)
+    hn = weights.hidden(700, nb)
+    bias = np.linspace(-1.0, 1.0, 256).astype(np.float32)
+    want = oracle.router_logits(router, hn)
+    gpu.poke("hn", hn)
+    gpu.stage("router", 2, nb)
+    assert np.array_equal(gpu.peek("logits", nb).reshape(nb, 256).view(np.uint32), want.view(np.uint32))
+    gpu.poke("bias", bias)
+    gpu.stage("router_bias", 2, nb)
+    assert np.array_equal(gpu.peek("logits", nb).reshape(nb, 256).view(np.uint32), (want + bias[None, :]).view(np.uint32))
