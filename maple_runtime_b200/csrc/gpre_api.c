@@ -419,8 +419,8 @@ static void run_combine(const float *const *dsp, int nb, const float *init, floa
     else k_combine(S.st, S.down, S.uw, S.tp, init, out, nb);
 }
 /* router logits: large batches take the tiled kernel, small ones the kernels that read the norm's re-laid rows in place (k_router_logits_small chooses).
- * The line: a layer takes 103.6 us with the latter and 112 with the former at 400 tokens, 105.1 and 104.5 at 420, 110 and 108.7 at 511. */
-#define ROUTER_TILE_MIN 417
+ * The line: up to here the latter hold two CTAs per SM; a layer takes 110 us with them and 118.5 with the former at 511 tokens. */
+#define ROUTER_TILE_MIN 593
 static void run_router_relaid(const LayerDev *l, const float *bias, int nb, int relaid) {   /* relaid: the norm kernel already wrote S.hT */
     if (nb >= ROUTER_TILE_MIN) k_router_logits_tile(S.st, l->router_t, S.hn, S.hT, bias, S.logits, nb, S.err);
     else k_router_logits_small(S.st, l->router_s, l->router_t, S.hn, S.hT, relaid, bias, S.logits, nb, S.err);

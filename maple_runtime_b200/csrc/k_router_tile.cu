@@ -414,8 +414,8 @@ extern "C" void k_router_logits_small(cudaStream_t st, const void *router_s, con
     static int sms = 0;
     if (!sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); if (sms < 1) sms = 148; }
     if (nb > 2 * 2 * sms / (NEXP / RS_EXP) * RS_TOK) {             // past two waves of the small kernel (148 tokens)
-        // 12 tokens per CTA (10.5 us as one CTA per SM, 16.1 as two), or 16 where that is one CTA per SM and 12 would be two (13.8: 217 to 288 tokens)
-        if (mid_ctas(nb, 4) <= sms && mid_ctas(nb, 3) > sms) launch_mid<4>(st, router_t, hS, bias, logits, nb, err);
+        // 12 tokens per CTA (10.5 us as one CTA per SM, 16.1 as two), or 16 (13.8, 20.1) where that means fewer CTAs per SM: 217 to 288 and from 445 tokens
+        if ((mid_ctas(nb, 4) + sms - 1) / sms < (mid_ctas(nb, 3) + sms - 1) / sms) launch_mid<4>(st, router_t, hS, bias, logits, nb, err);
         else launch_mid<3>(st, router_t, hS, bias, logits, nb, err);
         k_count_add(relaid ? 1 : 2);
         return;

@@ -8,7 +8,7 @@ from conftest import SEED
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nb", [145, 156, 157, 216, 217, 272, 288, 289, 301, 416])
+@pytest.mark.parametrize("nb", [145, 156, 157, 216, 217, 272, 288, 289, 301, 444, 445, 592])
 def test_mid_router_equals_oracle(nb, gpu, oracle, weights):
     gpu.synth_layer(SEED, 2)
     router, _, _ = weights.layer(2)
