@@ -559,6 +559,21 @@ static void decode_layers(int nb, int l0, int nl, const float *bias) {
         else k_combine(S.st, S.down, S.uw, S.tp, S.x, S.x, nb);
     }
 }
+/* A few hundred tokens on the tcgen05 kernels: the same joint of two layers (to 511 tokens: k_edge_wire). */
+#define EDGE_WIRE_MAX 511      /* < ROUTER_TILE_MIN: the rows are left in the re-laid form */
+static int mid_path(int nb) { return nb <= EDGE_WIRE_MAX && use_umma(nb) && !tensor_router(nb) && !S.keep && !S.prof_mask && !S.ep_on; }
+static void mid_layers(int nb, int l0, int nl, const float *bias) {
+    k_norm_prep_relaid(S.st, S.x, S.ly[l0].post_ln, S.hn, S.hq, S.hqs, S.hqsum, (float *)S.hT, nb);
+    for (int L = l0; L < l0 + nl; L++) {
+        const LayerDev *l = &S.ly[L];
+        run_router_relaid(l, bias, nb, 1);
+        k_topk(S.st, S.logits, S.top, S.topw, nb);
+        run_group(nb);
+        run_experts(l->tab, l->maps, (const float *const *)l->dsp, S.ue, nb, 7);
+        if (L + 1 < l0 + nl) k_edge_wire(S.st, S.wire, S.maxp, (const float *const *)l->dsp, S.uw, S.tp, S.x, S.ly[L + 1].post_ln, S.hn, S.hq, S.hqs, S.hqsum, (float *)S.hT, nb);
+        else run_combine((const float *const *)l->dsp, nb, S.x, S.x);
+    }
+}
 /* one layer on normalised rows, without the residual, from and to S.h_rows */
 static void decode_moe(int nb, int L, const float *bias) {
     k_norm_prep_relaid(S.st, S.h_rows, NULL, S.hn, S.hq, S.hqs, S.hqsum, (float *)S.hT, nb);
@@ -569,6 +584,7 @@ static void decode_moe(int nb, int L, const float *bias) {
 static int layers_run(int nb, int l0, int nl, const float *bd, int ep) {
     if (nl == 0) { decode_moe(nb, l0, bd); return 0; }
     if (!ep && decode_path(nb)) { decode_layers(nb, l0, nl, bd); return 0; }
+    if (!ep && mid_path(nb)) { mid_layers(nb, l0, nl, bd); return 0; }
     for (int L = l0; L < l0 + nl; L++) { if (ep) { if (run_layer_ep(L, nb, bd)) return -1; } else run_layer(L, nb, 1, bd); }
     return 0;
 }

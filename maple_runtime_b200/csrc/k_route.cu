@@ -12,6 +12,7 @@
 #include "dev_math.cuh"
 #include "topk.cuh"
 #include "silu_row.cuh"
+#include "wire.cuh"
 
 static long g_launches = 0;
 extern "C" void k_count_reset(void) { g_launches = 0; }
@@ -557,31 +558,53 @@ extern "C" void k_silu_quant(cudaStream_t st, const float *gate, const float *up
 // Decode batches, between two layers: the combine of the one (maple.c:834, as combine_kernel) and the RMSNorm + int8 of the next (as
 // norm_prep_kernel, its sums in the same order) for one token per CTA: one launch and one trip of the hidden row less.  Thread tid holds float4
 // tid and tid + 256 of the row.
+// WIRE: the pairs' rows are the tensor-core path's compact ones, as combine_wire_kernel reads them.  The experts' scales come from L2 for every pair (12 KB a
+// pair with its row) instead of once per CTA: a layer of the stack 98.9 -> 96.4 us at 301 tokens, 110.2 -> 108.0 at 511, but 123.0 -> 124.5 at 600.
+// (512 threads: 99.1 at 301; launched programmatically 96.7.)
 // ------------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) edge_kernel(const float *down, const float *uw, const int *tp, float *x, const uint16_t *__restrict__ w,
+struct EdgeWire { uint8_t *wire; int np_cap; const float *const *dsp; };
+template <bool WIRE>
+__global__ void __launch_bounds__(256) edge_kernel(const float *down, const EdgeWire ew, const float *uw, const int *tp, float *x, const uint16_t *__restrict__ w,
                                                    float *hn, int8_t *q, float *qs, int *qsum, float *hS) {
+    __shared__ const float *s_dsp[WIRE ? NEXP : 1];
     __shared__ double s_term[16 * 32];
     __shared__ float s_k, s_mx[8]; __shared__ int s_sum[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c = blockIdx.x;
     const uint2 ln[2] = {reinterpret_cast<const uint2 *>(w)[tid], reinterpret_cast<const uint2 *>(w)[tid + 256]};      // weights: read before the wait
+    if (WIRE) { static_assert(NEXP == 256, "one entry per thread"); s_dsp[tid] = ew.dsp[tid]; __syncthreads(); }
     pdl_wait(); pdl_trigger();
     int slot[TOPK]; float uv[TOPK];
 #pragma unroll
     for (int k = 0; k < TOPK; k++) slot[k] = tp[c * TOPK + k];
 #pragma unroll
     for (int k = 0; k < TOPK; k++) uv[k] = uw[slot[k]];
+    int4 rec[WIRE ? TOPK : 1];                                          // {scale of the pair's int8 row, expert, escape bits}
+    if (WIRE) {
+#pragma unroll
+        for (int k = 0; k < TOPK; k++) rec[k] = __ldcg(reinterpret_cast<const int4 *>(ew.wire + (size_t)ew.np_cap * WIRE_PITCH + (size_t)slot[k] * WIRE_REC));
+    }
     float4 v[2];
 #pragma unroll
     for (int k = 0; k < 2; k++) {
         const int i = tid + 256 * k;
-        float4 d[TOPK];
+        float4 d[TOPK];                                                 // WIRE: the scales
         v[k] = __ldcg(reinterpret_cast<const float4 *>(x) + (size_t)c * 512 + i);
+        if (WIRE) {
+            uint2 raw[TOPK];
 #pragma unroll
-        for (int t = 0; t < TOPK; t++) d[t] = __ldcg(reinterpret_cast<const float4 *>(down) + (size_t)slot[t] * 512 + i);
+            for (int t = 0; t < TOPK; t++) raw[t] = __ldcg(reinterpret_cast<const uint2 *>(ew.wire + (size_t)slot[t] * WIRE_PITCH) + i);
 #pragma unroll
-        for (int t = 0; t < TOPK; t++) {
-            v[k].x = __fmaf_rn(uv[t], d[t].x, v[k].x); v[k].y = __fmaf_rn(uv[t], d[t].y, v[k].y);
-            v[k].z = __fmaf_rn(uv[t], d[t].z, v[k].z); v[k].w = __fmaf_rn(uv[t], d[t].w, v[k].w);
+            for (int t = 0; t < TOPK; t++) { const float *p = s_dsp[rec[t].y & 0xFF]; d[t] = p ? reinterpret_cast<const float4 *>(p)[i] : make_float4(0.f, 0.f, 0.f, 0.f); }
+#pragma unroll
+            for (int t = 0; t < TOPK; t++) wire_add(v[k], raw[t], uv[t], __int_as_float(rec[t].x), d[t], rec[t].z, warp + 8 * k, lane, ew.wire, ew.np_cap, slot[t]);
+        } else {
+#pragma unroll
+            for (int t = 0; t < TOPK; t++) d[t] = __ldcg(reinterpret_cast<const float4 *>(down) + (size_t)slot[t] * 512 + i);
+#pragma unroll
+            for (int t = 0; t < TOPK; t++) {
+                v[k].x = __fmaf_rn(uv[t], d[t].x, v[k].x); v[k].y = __fmaf_rn(uv[t], d[t].y, v[k].y);
+                v[k].z = __fmaf_rn(uv[t], d[t].z, v[k].z); v[k].w = __fmaf_rn(uv[t], d[t].w, v[k].w);
+            }
         }
         reinterpret_cast<float4 *>(x)[(size_t)c * 512 + i] = v[k];
         s_term[(warp + 8 * k) * 32 + lane] = ((double)v[k].x * (double)v[k].x + (double)v[k].y * (double)v[k].y) + ((double)v[k].z * (double)v[k].z + (double)v[k].w * (double)v[k].w);
@@ -632,7 +655,11 @@ __global__ void __launch_bounds__(256) edge_kernel(const float *down, const floa
 }
 extern "C" void k_edge(cudaStream_t st, const float *down, const float *uw, const int *tp, float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb) {
     if (nb <= 0) return;
-    launch_pdl(edge_kernel, nb, 256, 0, st, down, uw, tp, x, w, hn, q, qs, qsum, hS); g_launches++;
+    launch_pdl(edge_kernel<false>, nb, 256, 0, st, down, EdgeWire{NULL, 0, NULL}, uw, tp, x, w, hn, q, qs, qsum, hS); g_launches++;
+}
+extern "C" void k_edge_wire(cudaStream_t st, uint8_t *wire, int np_cap, const float *const *dsp, const float *uw, const int *tp, float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb) {
+    if (nb <= 0) return;
+    launch_k(edge_kernel<true>, nb, 256, 0, st, (const float *)NULL, EdgeWire{wire, np_cap, dsp}, uw, tp, x, w, hn, q, qs, qsum, hS); g_launches++;
 }
 
 // ------------------------------------------------------------------------------------------------------------

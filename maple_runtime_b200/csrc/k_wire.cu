@@ -9,6 +9,7 @@
 #include <stdint.h>
 #include "kernels.h"
 #include "launch.cuh"
+#include "wire.cuh"
 
 extern "C" void k_count_add(long n);
 #define HID 2048
@@ -16,10 +17,6 @@ extern "C" void k_count_add(long n);
 #define CW_ROWS 128                 /* rows per CTA */
 #define CW_WARPS 32
 #define CW_EX 256                   /* entries of the down-scale pointer table */
-
-// escape code (2 bits) -> bits 16.. of (dot + 32768): 0, +1 or -1
-__device__ __forceinline__ int wire_hi(uint32_t code) { return ((int)(code ^ 2u) - 2) << 16; }
-__device__ __forceinline__ float wire_scale(int dot, float qs, float s) { return __fmul_rn(__fmul_rn((float)dot, qs), s); }
 
 // Grid (16 row blocks, token groups).  The CTA first copies into shared memory its 128-row slice of every expert's down scales
 // (128 KB) and, for every pair of its tokens, {slot, weight, scale of the pair's int8 row, expert | escape bits << 8}: after that
@@ -68,19 +65,7 @@ __global__ void __launch_bounds__(CW_WARPS * 32, 1) combine_wire_kernel(uint8_t 
             const int4 m = mt[k];
             const float w = __int_as_float(m.y), qs = __int_as_float(m.z);
             const int ex = m.w & 0xFF, escbits = m.w >> 8;
-            int d[4] = {(int)(raw[k].x & 0xFFFFu) - 32768, (int)(raw[k].x >> 16) - 32768, (int)(raw[k].y & 0xFFFFu) - 32768, (int)(raw[k].y >> 16) - 32768};
-            if ((escbits >> rb) & 1) {                                    // rare: some value of this row block did not fit 16 bits
-                uint32_t *pw = reinterpret_cast<uint32_t *>(wire + (size_t)m.x * WIRE_PITCH + 4096) + ((rb * CW_ROWS + 4 * lane) >> 4);
-                const uint32_t bits = (*pw >> ((lane & 3) * 8)) & 0xFFu;
-#pragma unroll
-                for (int i = 0; i < 4; i++) d[i] += wire_hi((bits >> (2 * i)) & 3u);
-                __syncwarp();
-                if ((lane & 3) == 0) *pw = 0u;                            // the plane is clean again for the next layer
-                if (lane == 0) atomicAnd(reinterpret_cast<int *>(wire + (size_t)np_cap * WIRE_PITCH + (size_t)m.x * WIRE_REC + 8), ~(1 << rb));
-            }
-            const float4 s = *reinterpret_cast<const float4 *>(sds + ex * CW_ROWS + 4 * lane);
-            acc.x = __fmaf_rn(w, wire_scale(d[0], qs, s.x), acc.x); acc.y = __fmaf_rn(w, wire_scale(d[1], qs, s.y), acc.y);
-            acc.z = __fmaf_rn(w, wire_scale(d[2], qs, s.z), acc.z); acc.w = __fmaf_rn(w, wire_scale(d[3], qs, s.w), acc.w);
+            wire_add(acc, raw[k], w, qs, *reinterpret_cast<const float4 *>(sds + ex * CW_ROWS + 4 * lane), escbits, rb, lane, wire, np_cap, m.x);
         }
         *reinterpret_cast<float4 *>(out + o) = acc;
     }
