@@ -24,7 +24,7 @@ void k_count_add(long n);
 #define FFN 512
 #define MAXREG 256         /* gpu_pre.m:21 has 64; synthetic layers that are generated again take new ids */
 #define MAXSYNTH 64
-#define MAP_CACHE 16384
+#define MAP_SLOTS 16384     /* more than the experts of 24 layers; a full table starts over */
 /* Up to so many tokens (0.8 MB) kernels read and write a caller's page-locked rows in place: 0.5 MB takes 11 us like this and 9 us by a copy, but a
  * copy is a link of its own in the chain of a call (submit, wait for the event, move to its place), 25 us and more with its neighbours. */
 #define INPLACE_MAXTOK 96
@@ -63,8 +63,9 @@ static struct {
     unsigned *mask; int *err, *h_err;      /* the kernels' error word, in page-locked host memory: the device's and the host's pointer to it */
     MoeTile *tiles_a, *tiles_b;
     ExpertPtrs *tab_call;      /* the used experts of one gpre_moe call */
-    ExpertMaps *maps_call, *h_maps; int8_t *hq_sorted; TMap4 bmap_hq, bmap_aq;
-    struct { const void *key; ExpertMaps m; } *map_cache;   /* tensor maps of experts seen by gpre_moe, by code pointer */
+    ExpertMaps *maps_seen, *h_maps; int8_t *hq_sorted; TMap4 bmap_hq, bmap_aq;
+    /* tensor maps of the experts seen by gpre_moe: on the card (maps_seen), the code pointers of slot i in map_key[i], slots found through map_hash */
+    struct MapKey { const uint8_t *gc, *uc, *dc; } *map_key; int *map_hash, map_n, map_sent, map_fresh;
     ExpertPtrs *h_tab;         /* host staging of a layer's pointer table */
     double t_experts;          /* GPU seconds in gfull_moe, reported by gfull_report */
     float *ring; int ring_nb, ring_n;
@@ -137,6 +138,17 @@ static int expert_maps(const char *who, const ExpertPtrs *e, ExpertMaps *m) {
     return 0;
 }
 
+/* the slot of an expert's maps on the card; a new one (S.map_n grows) is for the caller to fill */
+static void maps_forget(void) { S.map_n = S.map_sent = 0; for (int i = 0; i < 2 * MAP_SLOTS; i++) S.map_hash[i] = -1; }
+static int map_slot(const ExpertPtrs *e) {
+    /* experts lie at a fixed distance: the multiplication spreads them (their addresses modulo a power of two take few values) */
+    for (size_t h = ((uintptr_t)e->gc >> 4) * 0x9E3779B97F4A7C15u >> 40;; h++) {
+        int *s = &S.map_hash[h % (2 * MAP_SLOTS)];
+        if (*s < 0) { *s = S.map_n; S.map_key[S.map_n] = (struct MapKey){e->gc, e->uc, e->dc}; return S.map_n++; }
+        if (S.map_key[*s].gc == e->gc && S.map_key[*s].uc == e->uc && S.map_key[*s].dc == e->dc) return *s;
+    }
+}
+
 /* the B operands of the tcgen05 kernels (int8 rows in pair order), one map per box height 32, 64, 96, 128 */
 static int bmaps(const char *who, size_t pairs);
 static int init_common(const char *who, int maxtok, int topk) {
@@ -162,7 +174,7 @@ static int init_common(const char *who, int maxtok, int topk) {
     ALLOC(tiles_a, (P / 8 + NEXP) * sizeof(MoeTile)); ALLOC(tiles_b, (P / 8 + NEXP) * sizeof(MoeTile));
     ALLOC(ntiles_a, 16); ALLOC(ntiles_b, 16);
     ALLOC(act, P * FFN * 4); ALLOC(gate, P * FFN * 4); ALLOC(up, P * FFN * 4); ALLOC(aq, P * FFN); ALLOC(aqs, P * 4); ALLOC(aqsum, P * 4); ALLOC(down, P * HID * 4);
-    ALLOC(tab_call, NEXP * sizeof(ExpertPtrs)); ALLOC(maps_call, NEXP * sizeof(ExpertMaps)); ALLOC(hq_sorted, P * HID);
+    ALLOC(tab_call, NEXP * sizeof(ExpertPtrs)); ALLOC(maps_seen, MAP_SLOTS * sizeof(ExpertMaps)); ALLOC(hq_sorted, P * HID);
     ALLOC(wire, WIRE_BYTES(P)); CU(who, cudaMemset(S.wire, 0, WIRE_BYTES(P))); ALLOC(dsp_call, NEXP * sizeof(void *));
     ALLOC(hA, T * HID * 4); ALLOC(hnorm, T * 4); ALLOC(rpart, (size_t)8 * T * NEXP * 4); ALLOC(flagged, T * 4); ALLOC(nflagged, 16); ALLOC(rdone, T * 4); CU(who, cudaMemset(S.rdone, 0, T * 4));
     CU(who, cudaMemset(S.hA, 0, T * HID * 4)); CU(who, cudaMemset(S.nflagged, 0, 16));
@@ -175,9 +187,9 @@ static int init_common(const char *who, int maxtok, int topk) {
     CU(who, cudaHostAlloc((void **)&CT.h, CT.cap, cudaHostAllocMapped)); CU(who, cudaEventCreateWithFlags(&CT.taken, cudaEventDisableTiming));
     CU(who, cudaHostAlloc((void **)&S.h_rows, (size_t)2 * INPLACE_MAXTOK * INPLACE_WIDE * 4, cudaHostAllocMapped));
     S.h_tab = malloc(NEXP * sizeof(ExpertPtrs));
-    S.h_maps = aligned_alloc(64, NEXP * sizeof(ExpertMaps)); S.map_cache = aligned_alloc(64, MAP_CACHE * sizeof *S.map_cache);
-    if (!S.h_tab || !S.h_maps || !S.map_cache) return fail(who, "out of host memory");
-    memset(S.map_cache, 0, MAP_CACHE * sizeof *S.map_cache);
+    S.h_maps = aligned_alloc(64, NEXP * sizeof(ExpertMaps)); S.map_key = malloc(MAP_SLOTS * sizeof *S.map_key); S.map_hash = malloc(2 * MAP_SLOTS * sizeof(int));
+    if (!S.h_tab || !S.h_maps || !S.map_key || !S.map_hash) return fail(who, "out of host memory");
+    maps_forget();
     S.ready = 1;
     fprintf(stderr, "%s: %s, chunks up to %d tokens, %.0f MB of device workspace, weights resident in HBM\n", who, pr.name, maxtok,
             (double)(T * HID * 13 + P * (FFN * 5 + HID * 4 + 40)) / 1e6);
@@ -366,7 +378,7 @@ static int tile_tn(int nb) { return nb <= 256 ? 8 : 32; }
 static int use_umma(int nb) { return S.path == 2 || (S.path == 0 && nb > 256); }
 static void fill_expert_args(ExpertArgs *a, const ExpertPtrs *tab, const ExpertMaps *maps, const int *ue, int nb) {
     memset(a, 0, sizeof *a);
-    a->call_maps = maps == S.maps_call; a->tab = tab; a->maps = maps; a->ue = ue; a->ptok = S.utok; a->err = S.err;
+    a->call_maps = maps == S.maps_seen; a->fresh_maps = a->call_maps && S.map_fresh; a->tab = tab; a->maps = maps; a->ue = ue; a->ptok = S.utok; a->err = S.err;
     if (use_umma(nb)) { a->tiles = S.tiles_b; a->ntiles = S.ntiles_b; a->max_tiles = nb * TOPK / UMMA_TN + NEXP; }
     else { a->tiles = S.tiles_a; a->ntiles = S.ntiles_a; a->max_tiles = nb * TOPK / tile_tn(nb) + NEXP; if (a->max_tiles > nb * TOPK) a->max_tiles = nb * TOPK; }
     a->hq = S.hq; a->hqs = S.hqs; a->hqsum = S.hqsum; a->act = S.act;
@@ -855,20 +867,21 @@ static int stage_grouping(const char *who, int nb, int nu, const uint32_t *loc, 
     if (ustart[0] != 0) return fail(who, "ustart[0] = %d", ustart[0]);
     const float **dsp = tables_add(S.dsp_call, NEXP * sizeof(void *));
     ExpertPtrs *tab = tables_add(S.tab_call, (size_t)nu * sizeof(ExpertPtrs));
-    ExpertMaps *maps = um ? tables_add(S.maps_call, (size_t)nu * sizeof(ExpertMaps)) : NULL;
+    int mslot[NEXP];
+    S.map_fresh = 0;
+    if (S.map_n != S.map_sent || S.map_n + nu > MAP_SLOTS) maps_forget();      /* a call failed after it took slots, or the table is full */
+    const int first = S.map_n;
     for (int u = 0; u < nu; u++) {
         if (ustart[u + 1] <= ustart[u]) return fail(who, "used expert %d has no pairs", u);
         if (resolve(who, loc + u * 12, regs, &tab[u])) return -1;
         dsp[u] = tab[u].ds;
         if (!um) continue;
-        /* tensor maps of this expert: encoded the first time its codes are seen */
-        size_t hsh = ((uintptr_t)tab[u].gc >> 8) % MAP_CACHE;
-        if (S.map_cache[hsh].key != (const void *)tab[u].gc) {
-            if (expert_maps(who, &tab[u], &S.map_cache[hsh].m)) return -1;
-            S.map_cache[hsh].key = tab[u].gc;
-        }
-        memcpy(&maps[u], &S.map_cache[hsh].m, sizeof(ExpertMaps));
+        /* tensor maps of this expert: encoded and sent the first time its codes are seen */
+        const int n = S.map_n;
+        mslot[u] = map_slot(&tab[u]);
+        if (S.map_n > n && expert_maps(who, &tab[u], &S.h_maps[S.map_fresh++])) return -1;
     }
+    if (S.map_fresh) memcpy(tables_add(S.maps_seen + first, (size_t)S.map_fresh * sizeof(ExpertMaps)), S.h_maps, (size_t)S.map_fresh * sizeof(ExpertMaps));
     for (int u = nu; u < NEXP; u++) dsp[u] = NULL;
     int bad = 0, nt = 0;
     for (int a = 0; a < np; a++) bad |= (unsigned)ptok[a] >= (unsigned)nb;
@@ -878,7 +891,7 @@ static int stage_grouping(const char *who, int nb, int nu, const uint32_t *loc, 
     for (int u = 0; u < nu; u++) nt += (ustart[u + 1] - ustart[u] + tn - 1) / tn;
     MoeTile *t = tables_add(um ? S.tiles_b : S.tiles_a, (size_t)nt * sizeof(MoeTile));
     for (int u = 0; u < nu; u++) for (int p = ustart[u]; p < ustart[u + 1]; p += tn) {   /* gpu_pre.m:329-333 */
-        const MoeTile m = {u, p, ustart[u + 1] - p < tn ? ustart[u + 1] - p : tn, u}; *t++ = m;
+        const MoeTile m = {um ? mslot[u] : u, p, ustart[u + 1] - p < tn ? ustart[u + 1] - p : tn, u}; *t++ = m;
     }
     *(int *)tables_add(um ? S.ntiles_b : S.ntiles_a, 4) = nt; *(int *)tables_add(S.nu, 4) = nu;
     memcpy(tables_add(S.ustart, (size_t)(nu + 1) * 4), ustart, (size_t)(nu + 1) * 4);
@@ -892,6 +905,7 @@ static int tables_send(const char *who) {
     CU(who, cudaEventRecord(CT.taken, S.st)); CT.pending = 1;
     return 0;
 }
+static int grouping_send(const char *who) { const int r = tables_send(who); if (!r) S.map_sent = S.map_n; return r; }
 static int grouping_args(const char *who, int nb, int nu) {
     if (!S.ready) return fail(who, "not initialised");
     if (S.ep_on) return fail(who, "expert parallelism is set up: use the gmoe_ep_* entry points");
@@ -901,7 +915,7 @@ static int grouping_args(const char *who, int nb, int nu) {
 }
 static void run_call_experts(int nb, const float *init, float *out) {
     if (use_umma(nb)) k_gather_rows(S.st, S.hq, S.utok, S.hq_sorted, nb * TOPK);
-    run_experts(S.tab_call, S.maps_call, (const float *const *)S.dsp_call, NULL, nb, 7);
+    run_experts(S.tab_call, S.maps_seen, (const float *const *)S.dsp_call, NULL, nb, 7);
     run_combine((const float *const *)S.dsp_call, nb, init, out);
 }
 /* The experts only see the rows' int8 form, so that is what crosses to the card: a quarter of the bytes, made by the host threads that would
@@ -926,7 +940,7 @@ double gpre_moe(const float *x, int nb, int nu, const uint32_t *loc, const int *
     if (c.bad) return -1.0;
     if (e != cudaSuccess) { fail("gpre", "copy of %d rows to the card: %s", nb, cudaGetErrorString(e)); return -1.0; }
     cudaEventRecord(S.e0, S.st);
-    if (tables_send("gpre")) return -1.0;
+    if (grouping_send("gpre")) return -1.0;
     run_call_experts(nb, NULL, S.y);
     cudaEventRecord(S.e1, S.st);
     if (rows_out("gpre", y, S.y, nb)) return -1.0;
@@ -941,7 +955,7 @@ void gfull_begin(const float *x, int nb, int pos0) {
 }
 void gfull_moe(int nu, const uint32_t *loc, const int *regs, const int *ustart, const int *ptok, const float *pw, const int *tp) {
     int nb = S.nb_cur;
-    if (grouping_args("gfull", nb, nu) || tables_begin("gfull") || stage_grouping("gfull", nb, nu, loc, regs, ustart, ptok, pw, tp) || tables_send("gfull")) return;
+    if (grouping_args("gfull", nb, nu) || tables_begin("gfull") || stage_grouping("gfull", nb, nu, loc, regs, ustart, ptok, pw, tp) || grouping_send("gfull")) return;
     cudaEventRecord(S.e0, S.st);
     run_call_experts(nb, S.x, S.x);            /* hq/hqs/hqsum were left by gmoe_post_norm */
     cudaEventRecord(S.e1, S.st);

@@ -158,11 +158,11 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
                 const MoeTile tile = tnext;
                 if (item + (int)gridDim.x < nitems) {
                     tnext = tile_at((item + gridDim.x) / MB);
-                    const ExpertMaps *en = a.maps + tnext.ex;              // the next item's expert: its maps are in the descriptor cache when its copies start
+                    const ExpertMaps *en = a.maps + (a.call_maps ? tnext.u : tnext.ex);              // the next item's expert: its maps are in the descriptor cache when its copies start
                     if (GATEUP) { tma_prefetch_map(&en->gate); tma_prefetch_map(&en->up); } else tma_prefetch_map(&en->down);
                 }
                 const int mb = item % MB;
-                const ExpertMaps *em = a.maps + tile.ex;
+                const ExpertMaps *em = a.maps + (a.call_maps ? tile.u : tile.ex);
                 for (int sb = 0; sb < NSB && live; sb++, wcnt++) {
                     const int ws = wcnt % UM_WSTAGES;
                     if (!mbar_wait(&sh->w_empty[ws], ((wcnt / UM_WSTAGES) & 1) ^ 1, abortp)) { live = false; break; }
@@ -449,7 +449,7 @@ static void launch(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) {
         int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaFuncSetAttribute(expert_umma_kernel<KB, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     }
-    if (a->call_maps || MODE == 2) launch_k(expert_umma_kernel<KB, MODE>, sms, 640, smem, st, *a, *bmap);
+    if (a->fresh_maps || MODE == 2) launch_k(expert_umma_kernel<KB, MODE>, sms, 640, smem, st, *a, *bmap);
     else launch_pdl(expert_umma_kernel<KB, MODE>, sms, 640, smem, st, *a, *bmap);
     k_count_add(1);
 }

@@ -14,7 +14,7 @@ typedef struct { const uint8_t *gc, *uc, *dc; const float *gs, *us, *ds; } Exper
 typedef struct __attribute__((aligned(64))) { unsigned char b[128]; } TMap;
 typedef struct { TMap gate, up, down; } ExpertMaps;
 /* one unit of grouped-GEMM work: used expert u, first pair p0, cnt pairs (gpu_pre.m:329-333 uses the same triple) */
-typedef struct { int u, p0, cnt, ex; } MoeTile;   /* ex: index of the expert in ExpertArgs.tab / .maps */
+typedef struct { int u, p0, cnt, ex; } MoeTile;   /* ex: index of the expert in ExpertArgs.tab / .maps; with call_maps u is its index in .maps */
 
 typedef struct {
     const ExpertPtrs *tab;   /* indexed by ue[u] when ue != NULL, else by u */
@@ -41,7 +41,8 @@ typedef struct {
     /* the tcgen05 down kernel stores compact rows (see WIRE_* below) instead of fp32 ones: wire [np] rows, or in expert parallel
      * peer_wire[rank] = that rank's buffer */
     uint8_t *wire; uint8_t *const *peer_wire; int wire_cap;   /* wire_cap: pairs each such buffer is laid out for */
-    int call_maps;           /* 1: maps were written by a kernel of the same call: nothing is read through them before that kernel is complete */
+    int call_maps;           /* 1: the tiles index maps by u */
+    int fresh_maps;          /* 1: some maps were written by a kernel of the same call: nothing is read through them before that kernel is complete */
     int *err;                /* set to 1 by a kernel whose bounded wait ran out */
 } ExpertArgs;
 
