@@ -373,9 +373,9 @@ int gmoe_profile_read(double *secs, long *launches) {
 /* ---- the stages ------------------------------------------------------------------------------------------------ */
 static int tile_tn(int nb) { return nb <= 256 ? 8 : 32; }
 
-/* Which expert kernels: up to 256 tokens the mma.sync kernels on tiles of 8, above that the tcgen05 kernels.  At 301 tokens gate+up, SiLU and down
- * take 123 us per layer on the mma.sync kernels' tiles of 32 and 76 us on the tcgen05 kernels; at 256 the two are level. */
-static int use_umma(int nb) { return S.path == 2 || (S.path == 0 && nb > 256); }
+/* Which expert kernels: up to 192 tokens the mma.sync kernels on tiles of 8, above that the tcgen05 kernels, whose time hardly grows while an expert
+ * has few pairs.  A layer of the stack on either: 160 tokens 80.6 and 84.4 us, 200 87.8 and 86.3, 256 100.6 and 91.0. */
+static int use_umma(int nb) { return S.path == 2 || (S.path == 0 && nb > 192); }
 static void fill_expert_args(ExpertArgs *a, const ExpertPtrs *tab, const ExpertMaps *maps, const int *ue, int nb) {
     memset(a, 0, sizeof *a);
     a->call_maps = maps == S.maps_seen; a->fresh_maps = a->call_maps && S.map_fresh; a->tab = tab; a->maps = maps; a->ue = ue; a->ptok = S.utok; a->err = S.err;
@@ -554,7 +554,7 @@ static int graphs_on(void) {
 }
 int gmoe_set_graph(int on) { g_graph_on = on != 0; return 0; }
 static int run_layer_ep(int L, int nb, const float *bias);
-/* Layers of a decode batch (nb <= 256) without the per-stage hooks of run_layer: the combine of a layer and the norm of the next are one kernel, and
+/* Layers of a decode batch without the per-stage hooks of run_layer: the combine of a layer and the norm of the next are one kernel, and
  * so are top-8 and grouping of up to TOPK_IN_MAX tokens. */
 static int decode_path(int nb) { return nb <= 256 && !use_umma(nb) && !tensor_router(nb) && !S.keep && !S.prof_mask; }
 static void decode_body(const LayerDev *l, int nb, const float *bias) {

@@ -239,30 +239,27 @@ __global__ void __launch_bounds__(NEXP) group_place_kernel(const unsigned *__res
 #pragma unroll
     for (int k = 0; k < TOPK; k++) tp[tok * TOPK + k] = sl[k];
 }
-// Decode batches (up to 256 tokens = 2048 pairs): the whole grouping in one CTA, so that the step costs one launch instead of five, and without a
-// serial walk: every pair sets its token's bit in its expert's row of a shared-memory bit table; an expert's
-// count is the population of its row, a pair's place inside its expert the population below its token's bit, which is the
+// Up to 32 tokens: the whole grouping in one CTA, so that the step costs one launch instead of five, and without a
+// serial walk: every pair sets its token's bit in its expert's word of a shared-memory table; an expert's
+// count is the population of its word, a pair's place inside its expert the population below its token's bit, which is the
 // reference's order (pairs of an expert in token order).  The scan over experts and the per-token sort of the eight pair slots
-// follow in the same CTA.
-// MAXTOK tokens at most, NT threads (the first 256 own one expert each).  Used up to 256 tokens; a 2048-token instance (160 KB of
-// shared memory, 1024 threads) works but one SM takes longer over 16,384 pairs than the three kernels of the general path below.
-#define GS_MAXTOK 256
-// TOPK_IN (up to TOPK_IN_MAX tokens): the softmax and top-8 of token w by warp w come first, which saves their kernel.
-template <int MAXTOK, int NT, bool TOPK_IN>
-__global__ void __launch_bounds__(NT) group_cta_kernel(GroupArgs g) {
-    constexpr int WORDS = MAXTOK / 32;
-    extern __shared__ __align__(16) unsigned gs_smem[];
-    unsigned (*s_mask)[WORDS] = reinterpret_cast<unsigned (*)[WORDS]>(gs_smem);                         // [NEXP][WORDS]
-    int *s_slot = reinterpret_cast<int *>(gs_smem + NEXP * WORDS);                                        // [MAXTOK * TOPK]
-    unsigned short (*s_wpre)[WORDS] = reinterpret_cast<unsigned short (*)[WORDS]>(s_slot + MAXTOK * TOPK); // [NEXP][WORDS] pairs before word w
+// follow in the same CTA.  (With more words per expert it also took 256 tokens, 7 us longer than the cluster below.)
+// TOPK_IN (up to eight tokens): the softmax and top-8 of token w by warp w come first, which saves their kernel.
+#define GS_MAXTOK 32
+#define GS_TOPK 8
+template <bool TOPK_IN>
+__global__ void __launch_bounds__(NEXP) group_cta_kernel(GroupArgs g) {
+    constexpr int NT = NEXP;
+    __shared__ unsigned s_mask[NEXP];
+    __shared__ int s_slot[GS_MAXTOK * TOPK];
     __shared__ int s_start[NEXP];
     __shared__ int w_cnt[8], w_used[8], w_ta[8], w_tb[8];
-    __shared__ int s_top[TOPK_IN ? TOPK_IN_MAX * TOPK : 1]; __shared__ float s_topw[TOPK_IN ? TOPK_IN_MAX * TOPK : 1];
+    __shared__ int s_top[TOPK_IN ? GS_TOPK * TOPK : 1]; __shared__ float s_topw[TOPK_IN ? GS_TOPK * TOPK : 1];
     __shared__ __align__(16) float s_row[TOPK_IN ? 8 : 1][NEXP];
     __shared__ unsigned long long tab[TOPK_IN ? 32 : 1];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nb = g.nb, np = nb * TOPK;
     if (TOPK_IN && tid < 32) tab[tid] = DEV_EXP_TAB[tid];
-    for (int i = tid; i < NEXP * WORDS; i += NT) gs_smem[i] = 0u;
+    s_mask[tid] = 0u;
     __syncthreads();
     pdl_wait(); pdl_trigger();
     if (TOPK_IN) {
@@ -282,13 +279,10 @@ __global__ void __launch_bounds__(NT) group_cta_kernel(GroupArgs g) {
         __syncthreads();
     }
     auto expert = [&](const int i) { return TOPK_IN ? s_top[i] : g.top[i]; };
-    for (int i = tid; i < np; i += NT) { const int t = i >> 3; atomicOr(&s_mask[expert(i)][t >> 5], 1u << (t & 31)); }
+    for (int i = tid; i < np; i += NT) { const int t = i >> 3; atomicOr(&s_mask[expert(i)], 1u << t); }
     __syncthreads();
-    if (tid < NEXP) {
-        const int e = tid;
-        int cnt = 0;
-#pragma unroll 8
-        for (int w = 0; w < WORDS; w++) { s_wpre[e][w] = (unsigned short)cnt; cnt += __popc(s_mask[e][w]); }
+    {
+        const int e = tid, cnt = __popc(s_mask[e]);
         const int used = cnt > 0, na = (cnt + g.tn_a - 1) / g.tn_a, nb_ = (cnt + g.tn_b - 1) / g.tn_b;
         int c = cnt, u = used, a = na, b = nb_;
 #pragma unroll
@@ -298,7 +292,7 @@ __global__ void __launch_bounds__(NT) group_cta_kernel(GroupArgs g) {
             if (lane >= o) { c += tc; u += tu; a += t1; b += t2; }
         }
         if (lane == 31) { w_cnt[wid] = c; w_used[wid] = u; w_ta[wid] = a; w_tb[wid] = b; }
-        asm volatile("bar.sync 1, 256;" ::: "memory");                   // the eight warps that own experts
+        __syncthreads();
         int oc = 0, ou = 0, oa = 0, ob = 0;
         for (int w = 0; w < wid; w++) { oc += w_cnt[w]; ou += w_used[w]; oa += w_ta[w]; ob += w_tb[w]; }
         const int start = oc + c - cnt, uidx = ou + u - used, ta0 = oa + a - na, tb0 = ob + b - nb_;
@@ -314,8 +308,7 @@ __global__ void __launch_bounds__(NT) group_cta_kernel(GroupArgs g) {
     }
     __syncthreads();
     for (int i = tid; i < np; i += NT) {                             // every pair finds its place
-        const int x = expert(i), t = i >> 3, w = t >> 5;
-        const int r = s_start[x] + s_wpre[x][w] + __popc(s_mask[x][w] & ((1u << (t & 31)) - 1u));
+        const int x = expert(i), t = i >> 3, r = s_start[x] + __popc(s_mask[x] & ((1u << t) - 1u));
         s_slot[i] = r;
         g.utok[r] = t; g.uw[r] = TOPK_IN ? s_topw[i] : g.topw[i]; if (g.uexp) g.uexp[r] = x;
     }
@@ -332,35 +325,53 @@ __global__ void __launch_bounds__(NT) group_cta_kernel(GroupArgs g) {
         for (int k = 0; k < TOPK; k++) g.tp[t * TOPK + k] = sl[k];
     }
 }
-template <int MAXTOK, int NT, bool TOPK_IN>
-static void launch_group_cta(cudaStream_t st, const GroupArgs *g) {
-    const int smem = NEXP * (MAXTOK / 32) * 4 + MAXTOK * TOPK * 4 + NEXP * (MAXTOK / 32) * 2;
-    static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(group_cta_kernel<MAXTOK, NT, TOPK_IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr_done = true; }
-    launch_pdl(group_cta_kernel<MAXTOK, NT, TOPK_IN>, 1, NT, smem, st, *g);
-}
-// 257 to GROUP_CLUSTER_MAX tokens: one launch of one cluster of CTAS CTAs.  CTA r owns its share of the tokens (in whole
+// Up to GROUP_CLUSTER_MAX tokens: one launch of one cluster of CTAS CTAs.  CTA r owns its share of the tokens (in whole
 // words of 32) and keeps their bits in its shared memory; the counts are exchanged through distributed shared memory, after which every CTA
 // scans the experts for itself and its threads place one token each.  Bound by latency: what counts is the number of launches (a launch costs
 // the host 3.9 us; clearing, marking and placing as three kernels took 16.4 us per call at 1000 tokens, 10.2 us like this) and of trips through
 // global memory (inside a layer of 2048 tokens, against the router setting the bits and the place kernel reading them: 4 us less).  Eight
 // CTAs are what every GPU has to allow; from 513 tokens on sixteen share the scattered stores (2048 tokens: 14.4 -> 11.9 us).
+// Against one CTA for up to 256 tokens, a layer of the stack: 96 tokens 70.8 -> 70.0 us, 128 77.7 -> 75.9, 256 106.1 -> 100.7.
+// TOPK_IN (9 to TOPK_IN_MAX tokens): the softmax and top-8 come first, a warp per token (20 tokens 41.8 -> 41.3 us, 64 61.2 -> 60.7).
 #define GC_WORDS 8
-template <int GC_CTAS>
+template <int GC_CTAS, bool TOPK_IN>
 __global__ void __launch_bounds__(NEXP) group_cluster_kernel(GroupArgs g) {
     __shared__ unsigned s_mask[NEXP][GC_WORDS + 1];           // + 1: a warp's 32 experts of one word lie in 32 banks
     __shared__ unsigned short s_pre[NEXP][GC_WORDS + 1];      // the pairs of the CTA's expert in front of word w
     __shared__ int s_cnt[NEXP], s_start[NEXP];
     __shared__ int w_cnt[8], w_used[8], w_ta[8], w_tb[8];
     const int e = threadIdx.x, lane = e & 31, wid = e >> 5, nb = g.nb;
-    const int per = (((nb + 31) / 32 + GC_CTAS - 1) / GC_CTAS) * 32, tok = blockIdx.x * per + e;      // per <= 32 GC_WORDS = one token per thread
+    const int per = TOPK_IN ? (nb + GC_CTAS - 1) / GC_CTAS : (((nb + 31) / 32 + GC_CTAS - 1) / GC_CTAS) * 32, tok = blockIdx.x * per + e;      // per <= 32 GC_WORDS = one token per thread
     const bool mine = e < per && tok < nb;
+    constexpr int TT = TOPK_IN ? TOPK_IN_MAX / GC_CTAS : 1;
+    __shared__ __align__(16) int s_top[TT * TOPK]; __shared__ __align__(16) float s_topw[TT * TOPK];
+    __shared__ __align__(16) float s_row[TOPK_IN ? 8 : 1][NEXP];
+    __shared__ unsigned long long tab[TOPK_IN ? 32 : 1];
+    if (TOPK_IN && e < 32) tab[e] = DEV_EXP_TAB[e];
+    if (TOPK_IN) __syncthreads();
     pdl_wait(); pdl_trigger();
+    if (TOPK_IN) {                                              // a warp per token
+        for (int i = wid; i < per && (int)blockIdx.x * per + i < nb; i += 8) {
+            const int t = blockIdx.x * per + i;
+            const float4 *lr = reinterpret_cast<const float4 *>(g.logits + (size_t)t * NEXP + lane * 8);
+            const float4 v0 = __ldcg(lr), v1 = __ldcg(lr + 1);
+            float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+            int isel; float wsel, tsum;
+            exact_topk_warp(p, lane, tab, s_row[wid], isel, wsel, tsum);
+            if (lane < TOPK) {
+                const float tw = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));
+                s_top[i * TOPK + lane] = isel; s_topw[i * TOPK + lane] = tw;
+                g.top_out[t * TOPK + lane] = isel; g.topw_out[t * TOPK + lane] = tw;
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+    }
     const bool wide = (((uintptr_t)g.top | (uintptr_t)g.topw | (uintptr_t)g.tp | (uintptr_t)g.slot) & 15) == 0;      // the caller's arrays may lie anywhere
     int x[TOPK]; float w[TOPK];
     if (mine) {
-        const int *tr = g.top + (size_t)tok * TOPK; const float *wr = g.topw + (size_t)tok * TOPK;
-        if (wide) {
+        const int *tr = TOPK_IN ? s_top + e * TOPK : g.top + (size_t)tok * TOPK; const float *wr = TOPK_IN ? s_topw + e * TOPK : g.topw + (size_t)tok * TOPK;
+        if (TOPK_IN || wide) {
             const int4 a = reinterpret_cast<const int4 *>(tr)[0], b = reinterpret_cast<const int4 *>(tr)[1];
             const float4 c = reinterpret_cast<const float4 *>(wr)[0], d = reinterpret_cast<const float4 *>(wr)[1];
             x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
@@ -442,17 +453,18 @@ __global__ void __launch_bounds__(NEXP) group_cluster_kernel(GroupArgs g) {
 }
 extern "C" void k_group(cudaStream_t st, const GroupArgs *g) {
     if (g->nb <= 0) return;
-    if (g->nb <= 256) {
-        if (g->logits) launch_group_cta<32, 256, true>(st, g); else if (g->nb <= 32) launch_group_cta<32, 256, false>(st, g); else launch_group_cta<256, 256, false>(st, g);
+    if (g->nb <= (g->logits ? GS_TOPK : GS_MAXTOK)) {
+        if (g->logits) launch_pdl(group_cta_kernel<true>, 1, NEXP, 0, st, *g); else launch_pdl(group_cta_kernel<false>, 1, NEXP, 0, st, *g);
         g_launches++; return;
     }
     const int np = g->nb * TOPK;
     if (g->nb <= GROUP_CLUSTER_MAX) {
-        if (g->nb <= 512) launch_cluster(group_cluster_kernel<8>, 8, NEXP, st, *g);
+        if (g->logits) launch_cluster(group_cluster_kernel<8, true>, 8, NEXP, st, *g);
+        else if (g->nb <= 512) launch_cluster(group_cluster_kernel<8, false>, 8, NEXP, st, *g);
         else {
             static bool attr_done = false;
-            if (!attr_done) { cudaFuncSetAttribute(group_cluster_kernel<16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); attr_done = true; }
-            launch_cluster(group_cluster_kernel<16>, 16, NEXP, st, *g);
+            if (!attr_done) { cudaFuncSetAttribute(group_cluster_kernel<16, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); attr_done = true; }
+            launch_cluster(group_cluster_kernel<16, false>, 16, NEXP, st, *g);
         }
         g_launches++; return;
     }

@@ -66,7 +66,7 @@ extern "C" int gmoe_group_noalloc(const int *top, const float *topw, int nb, int
     g.mask = s->mask; g.mask_words = (nb + 31) / 32;
     g.nu = nu; g.ue = ue; g.estart = s->estart; g.ustart = ustart; g.utok = utok; g.slot = s->slot; g.tp = tp; g.uw = uw;
     g.tiles_a = s->tiles_a; g.tiles_b = s->tiles_b; g.ntiles_a = s->ntiles_a; g.ntiles_b = s->ntiles_b; g.tn_a = 8; g.tn_b = UMMA_TN;
-    k_group(static_cast<cudaStream_t>(stream), &g);   // one kernel with its masks in shared memory (up to 256 tokens one CTA, above that a cluster of eight)
+    k_group(static_cast<cudaStream_t>(stream), &g);   // one kernel with its masks in shared memory (up to 32 tokens one CTA, above that a cluster of eight or more)
     e = cudaGetLastError();
     if (e != cudaSuccess) { fprintf(stderr, "gmoe: gmoe_group_noalloc: launch failed: %s\n", cudaGetErrorString(e)); return -3; }
     return 0;

@@ -1,4 +1,4 @@
-"""The grouping of 257 and more tokens as one cluster of CTAs (csrc/k_route.cu: group_cluster_kernel) against the oracle, at the sizes where its
+"""The grouping of 33 and more tokens as one cluster of CTAs (csrc/k_route.cu: group_cluster_kernel) against the oracle, at the sizes where its
 split changes: one token past a word, eight and sixteen CTAs, CTAs without tokens, skewed and identical rows, arrays that are not 16-byte aligned."""
 import numpy as np
 import pytest
@@ -9,7 +9,7 @@ from test_zz_no_alloc import routing
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nb,kind", [(257, "even"), (288, "skew"), (511, "even"), (512, "same"), (513, "even"), (777, "skew"), (2047, "even"), (2048, "same")])
+@pytest.mark.parametrize("nb,kind", [(33, "even"), (64, "same"), (97, "skew"), (256, "even"), (257, "even"), (288, "skew"), (511, "even"), (512, "same"), (513, "even"), (777, "skew"), (2047, "even"), (2048, "same")])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_cluster_grouping_equals_oracle(nb, kind, shift, gpu, clib, oracle):
     torch = pytest.importorskip("torch")   # only to own device buffers for the caller's side of the call

@@ -18,8 +18,8 @@ def g(gpu):
     gpu.keep_stages(True)
 
 
-# 3/4: all weights in flight at once or not; 8/9: top-8 inside the grouping; 32/33: its bit table; 96/97: rows in place or copied
-@pytest.mark.parametrize("nb", [1, 2, 3, 4, 8, 9, 32, 33, 96, 97, 256])
+# 3/4: all weights in flight at once or not; 8/9, 64/65: top-8 inside the grouping, one CTA or eight; 32/33: its bit table; 192: the last on mma.sync; 96/97: rows in place or copied
+@pytest.mark.parametrize("nb", [1, 2, 3, 4, 8, 9, 17, 32, 33, 64, 65, 96, 97, 192, 256])
 def test_fused_decode_layers_equal_stages(nb, g, weights, clib):
     from maple_runtime_b200 import lib as ml
     x = weights.hidden(2100 + nb, nb)
