@@ -26,6 +26,7 @@
 
 extern "C" void k_count_add(long n);
 
+
 __device__ __forceinline__ void mma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
@@ -44,9 +45,9 @@ __device__ __forceinline__ MoeTile ldcg_tile(const MoeTile *t) {
 // KCH: K-chunks of 256 columns (8 for gate/up K=2048, 2 for down K=512).  NBLK: 8-token blocks per tile.
 // GATEUP: rows block A = gate rows, block B = up rows of the same index, epilogue = SiLU*up;
 // otherwise A and B are two consecutive 16-row blocks of the down matrix, epilogue = scale only.
-// PF: chunks of weights in flight per thread.
-template <int KCH, int NBLK, bool GATEUP, int PF>
-__global__ void __launch_bounds__(128) expert_mma_kernel(ExpertArgs a) {
+// PF: chunks of weights in flight per thread.  NW: warps per CTA.
+template <int KCH, int NBLK, bool GATEUP, int PF, int NW>
+__global__ void __launch_bounds__(NW * 32) expert_mma_kernel(ExpertArgs a) {
     constexpr int TN = NBLK * 8, KB = KCH * 256;            // tokens per tile, bytes of one int8 activation vector
     extern __shared__ __align__(16) uint8_t smem[];          // [KCH][4][TN][4][16]
     const int tile_i = blockIdx.y;
@@ -59,7 +60,7 @@ __global__ void __launch_bounds__(128) expert_mma_kernel(ExpertArgs a) {
     const ExpertPtrs ep = a.tab[tile.ex];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
 
-    const int rows_per_cta = GATEUP ? 64 : 128;
+    const int rows_per_cta = NW * (GATEUP ? 16 : 32);
     const int r0 = blockIdx.x * rows_per_cta + warp * (GATEUP ? 16 : 32);
     const uint8_t *wa = (GATEUP ? ep.gc : ep.dc) + (size_t)(r0 + g) * (KB / 4) + t * 16;
     const uint8_t *wb = GATEUP ? ep.uc + (size_t)(r0 + g) * (KB / 4) + t * 16 : wa + 16 * (KB / 4);
@@ -75,7 +76,7 @@ __global__ void __launch_bounds__(128) expert_mma_kernel(ExpertArgs a) {
     // stage the tile's activation vectors (16-byte pieces) in fragment order
     if (GATEUP || !a.act_for_down) {
         const int8_t *src = GATEUP ? a.hq : a.aq;
-        for (int i = tid; i < tile.cnt * (KB / 16); i += 128) {
+        for (int i = tid; i < tile.cnt * (KB / 16); i += NW * 32) {
             int n = i / (KB / 16), q = i % (KB / 16);            // piece q covers columns 16q..16q+15
             int row = (GATEUP && a.ptok) ? a.ptok[tile.p0 + n] : tile.p0 + n;
             uint4 v = *reinterpret_cast<const uint4 *>(src + (size_t)row * KB + q * 16);
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(128) expert_mma_kernel(ExpertArgs a) {
         // down, decode path: the SiLU outputs arrive as fp32 and are quantised here (the prep of maple.c:831), one warp per pair;
         // every row-block CTA of the tile repeats this for the tile's few pairs, the first one also stores the result
         float *s_qs = reinterpret_cast<float *>(smem + KCH * 4 * TN * 64); int *s_qsum = reinterpret_cast<int *>(s_qs + TN);
-        for (int n = warp; n < tile.cnt; n += 4) {
+        for (int n = warp; n < tile.cnt; n += NW) {
             const int pair = tile.p0 + n;
             const float4 *r = reinterpret_cast<const float4 *>(a.act_for_down + (size_t)pair * 512) + lane * 4;
             float v[16];
@@ -179,26 +180,30 @@ __global__ void __launch_bounds__(128) expert_mma_kernel(ExpertArgs a) {
         }
 }
 
-template <int KCH, int NBLK, bool GATEUP, int PF>
+template <int KCH, int NBLK, bool GATEUP, int PF, int NW>
 static void launch(cudaStream_t st, const ExpertArgs *a) {
     const size_t smem = (size_t)KCH * 4 * NBLK * 8 * 64 + (GATEUP ? 0 : NBLK * 8 * 8);   // + scale and code sum per pair when down quantises itself
     static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<KCH, NBLK, GATEUP, PF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
-    dim3 grid(GATEUP ? 8 : 16, a->max_tiles);
-    launch_pdl(expert_mma_kernel<KCH, NBLK, GATEUP, PF>, grid, 128, smem, st, *a);
+    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<KCH, NBLK, GATEUP, PF, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
+    dim3 grid((GATEUP ? 32 : 64) / NW, a->max_tiles);
+    launch_pdl(expert_mma_kernel<KCH, NBLK, GATEUP, PF, NW>, grid, NW * 32, smem, st, *a);
     k_count_add(1);
 }
 // Two chunks in flight leave room for six CTAs per SM, which is what a long list of tiles wants (four chunks: 64 tokens 34.5 instead of 31 us).
 // Where the whole list is resident at once at one or two CTAs per SM, all eight chunks go out together: one trip to memory instead of four
 // (1 token 22.1 -> 20.9 us per layer; from 4 tokens on the two are level).
 #define PF8_TILES 24
+// Eight warps per CTA share a tile's staged rows once an expert has several pairs: 192 tokens 86.2 -> 82.5 us per layer, 160 80.6 -> 79.0, 128 the same, but
+// 64 tokens 60.8 -> 61.8.  max_tiles is 256 + the tokens, as many tiles as there could be.
+#define NW8_TILES 384
 extern "C" void k_gateup_mma(cudaStream_t st, const ExpertArgs *a, int tn) {
     if (a->max_tiles <= 0) return;
-    if (tn != 8) launch<8, 4, true, 2>(st, a); else if (a->max_tiles <= PF8_TILES) launch<8, 1, true, 8>(st, a); else launch<8, 1, true, 2>(st, a);
+    if (tn != 8) launch<8, 4, true, 2, 4>(st, a); else if (a->max_tiles <= PF8_TILES) launch<8, 1, true, 8, 4>(st, a);
+    else if (a->max_tiles <= NW8_TILES) launch<8, 1, true, 2, 4>(st, a); else launch<8, 1, true, 2, 8>(st, a);
 }
 extern "C" void k_down_mma(cudaStream_t st, const ExpertArgs *a, int tn) {
     if (a->max_tiles <= 0) return;
-    if (tn == 8) launch<2, 1, false, 2>(st, a); else launch<2, 4, false, 2>(st, a);
+    if (tn != 8) launch<2, 4, false, 2, 4>(st, a); else if (a->max_tiles <= NW8_TILES) launch<2, 1, false, 2, 4>(st, a); else launch<2, 1, false, 2, 8>(st, a);
 }
 
 // The attention projections (gpu_pre.m:200-256 gpre_dense*): the same int8 x 2-bit product with one matrix instead of 256
@@ -209,8 +214,8 @@ template <int NBLK, int PF>
 static void launch_dense(cudaStream_t st, const ExpertArgs *a, int rows) {
     const size_t smem = (size_t)8 * 4 * NBLK * 8 * 64 + NBLK * 8 * 8;
     static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<8, NBLK, false, PF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
-    launch_pdl(expert_mma_kernel<8, NBLK, false, PF>, dim3(rows / 128, (a->dense_n + NBLK * 8 - 1) / (NBLK * 8)), 128, smem, st, *a);
+    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<8, NBLK, false, PF, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
+    launch_pdl(expert_mma_kernel<8, NBLK, false, PF, 4>, dim3(rows / 128, (a->dense_n + NBLK * 8 - 1) / (NBLK * 8)), 128, smem, st, *a);
     k_count_add(1);
 }
 extern "C" void k_dense_mma(cudaStream_t st, const ExpertArgs *a, int rows) {

@@ -8,7 +8,7 @@ from conftest import same_bits
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nb", [193, 600])
+@pytest.mark.parametrize("nb", [209, 600])
 def test_maps_of_host_supplied_groupings(nb, gpu, oracle, weights):
     from maple_runtime_b200 import lib as ml
     g = gpu

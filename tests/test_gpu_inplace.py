@@ -10,16 +10,20 @@ from conftest import SEED, same_bits
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture()
-def g(gpu):
+@pytest.fixture(scope="module")
+def synth(gpu):
     for L in (3, 4):
         gpu.synth_layer(SEED, L)
+
+
+@pytest.fixture()
+def g(gpu, synth):
     yield gpu
     gpu.keep_stages(True)
 
 
-# 3/4: all weights in flight at once or not; 8/9, 64/65: top-8 inside the grouping, one CTA or eight; 32/33: its bit table; 192: the last on mma.sync; 96/97: rows in place or copied
-@pytest.mark.parametrize("nb", [1, 2, 3, 4, 8, 9, 17, 32, 33, 64, 65, 96, 97, 192, 256])
+# 3/4: all weights in flight at once or not; 8/9, 64/65: top-8 inside the grouping, one CTA or eight; 32/33: its bit table; 128/129: four warps per CTA or eight; 208: the last on mma.sync; 96/97: rows in place or copied
+@pytest.mark.parametrize("nb", [1, 2, 3, 4, 8, 9, 17, 32, 33, 64, 65, 96, 97, 128, 129, 208, 256])
 def test_fused_decode_layers_equal_stages(nb, g, weights, clib):
     from maple_runtime_b200 import lib as ml
     x = weights.hidden(2100 + nb, nb)

@@ -8,9 +8,13 @@ from conftest import SEED
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nb", [145, 156, 157, 216, 217, 272, 288, 289, 301, 444, 445, 592])
-def test_mid_router_equals_oracle(nb, gpu, oracle, weights):
+@pytest.fixture(scope="module")
+def layer(gpu):
     gpu.synth_layer(SEED, 2)
+
+
+@pytest.mark.parametrize("nb", [145, 156, 157, 216, 217, 272, 288, 289, 301, 444, 445, 592])
+def test_mid_router_equals_oracle(nb, layer, gpu, oracle, weights):
     router, _, _ = weights.layer(2)
     hn = weights.hidden(700, nb)
     bias = np.linspace(-1.0, 1.0, 256).astype(np.float32)
