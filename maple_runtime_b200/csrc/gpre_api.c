@@ -30,6 +30,7 @@ void k_count_add(long n);
 #define INPLACE_MAXTOK 96
 #define INPLACE_WIDE 3072
 #define H_ROWS_OUT (S.h_rows + (size_t)INPLACE_MAXTOK * INPLACE_WIDE)
+#define H_BIAS (S.h_rows + (size_t)2 * INPLACE_MAXTOK * INPLACE_WIDE)      /* a call's bias, behind the rows */
 
 static char g_err[512];
 static int fail(const char *who, const char *fmt, ...) {
@@ -185,7 +186,7 @@ static int init_common(const char *who, int maxtok, int topk) {
     CU(who, cudaHostGetDevicePointer((void **)&S.err, S.h_err, 0));
     CT.cap = (size_t)INPLACE_MAXTOK * (HID + 8) + P * 12 + (P / 8 + NEXP) * sizeof(MoeTile) + T * 8 + NEXP * (sizeof(ExpertMaps) + sizeof(ExpertPtrs) + 16) + 4096;
     CU(who, cudaHostAlloc((void **)&CT.h, CT.cap, cudaHostAllocMapped)); CU(who, cudaEventCreateWithFlags(&CT.taken, cudaEventDisableTiming));
-    CU(who, cudaHostAlloc((void **)&S.h_rows, (size_t)2 * INPLACE_MAXTOK * INPLACE_WIDE * 4, cudaHostAllocMapped));
+    CU(who, cudaHostAlloc((void **)&S.h_rows, ((size_t)2 * INPLACE_MAXTOK * INPLACE_WIDE + NEXP) * 4, cudaHostAllocMapped));
     S.h_tab = malloc(NEXP * sizeof(ExpertPtrs));
     S.h_maps = aligned_alloc(64, NEXP * sizeof(ExpertMaps)); S.map_key = malloc(MAP_SLOTS * sizeof *S.map_key); S.map_hash = malloc(2 * MAP_SLOTS * sizeof(int));
     if (!S.h_tab || !S.h_maps || !S.map_key || !S.map_hash) return fail(who, "out of host memory");
@@ -588,7 +589,7 @@ static void mid_layers(int nb, int l0, int nl, const float *bias) {
 }
 /* one layer on normalised rows, without the residual, from and to S.h_rows */
 static void decode_moe(int nb, int L, const float *bias) {
-    k_norm_prep_relaid(S.st, S.h_rows, NULL, S.hn, S.hq, S.hqs, S.hqsum, (float *)S.hT, nb);
+    k_norm_prep_call(S.st, S.h_rows, S.hn, S.hq, S.hqs, S.hqsum, (float *)S.hT, nb, bias ? H_BIAS : NULL, S.bias);
     decode_body(&S.ly[L], nb, bias);
     k_combine(S.st, S.down, S.uw, S.tp, NULL, H_ROWS_OUT, nb);
 }
@@ -640,10 +641,10 @@ double gmoe_moe(int L, const float *x, int nb, float *y, const float *bias) {
     if (check_call("gmoe", L, nb)) return -1.0;
     if (nb <= INPLACE_MAXTOK && decode_path(nb)) {
         const size_t n = (size_t)nb * HID;
-        const float *bias_d = bias_dev(bias);
+        if (bias) memcpy(H_BIAS, bias, NEXP * 4);
         hio_copy_shared(S.h_rows, x, n * 4);
         cudaEventRecord(S.e0, S.st);
-        if (layers_enqueue(nb, L, 0, bias_d)) return -1.0;
+        if (layers_enqueue(nb, L, 0, bias ? S.bias : NULL)) return -1.0;      /* the first kernel brings the bias */
         cudaEventRecord(S.e1, S.st);
         S.nb_cur = nb;
         const double t = finish("gmoe");

@@ -59,6 +59,8 @@ void k_rows(cudaStream_t st, void *dst, const void *src, size_t bytes);
 void k_norm_prep(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, int nb);
 /* the same, and the normalised rows once more in the decode router's layout (hS, nb*HID*4 bytes): k_router_logits_small then takes relaid = 1 */
 void k_norm_prep_relaid(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb);
+/* as k_norm_prep_relaid of rows that are normalised already, up to 256; bias_src != NULL: the 256 values there (page-locked host memory) go to bias */
+void k_norm_prep_call(cudaStream_t st, const float *x, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb, const float *bias_src, float *bias);
 /* prefill-sized batches: router_t = the layer's router rows re-laid by k_router_pack (NEXP*HID*2 bytes), hT = scratch of
  * ceil(nb/16)*16*HID*8 bytes; err receives 31 if a bounded wait inside the kernel ran out */
 void k_router_pack(cudaStream_t st, const uint16_t *router, void *router_t);
