@@ -558,18 +558,28 @@ static int run_layer_ep(int L, int nb, const float *bias);
 /* Layers of a decode batch without the per-stage hooks of run_layer: the combine of a layer and the norm of the next are one kernel, and
  * so are top-8 and grouping of up to TOPK_IN_MAX tokens. */
 static int decode_path(int nb) { return nb <= 256 && !use_umma(nb) && !tensor_router(nb) && !S.keep && !S.prof_mask; }
-static void decode_body(const LayerDev *l, int nb, const float *bias) {
-    k_router_logits_small(S.st, l->router_s, l->router_t, S.hn, S.hT, 1, bias, S.logits, nb, S.err);
+static void decode_routed(const LayerDev *l, int nb) {      /* from the logits to the down rows */
     if (nb > TOPK_IN_MAX) k_topk(S.st, S.logits, S.top, S.topw, nb);
     run_group_l(nb, 0, nb > TOPK_IN_MAX ? NULL : S.logits);
     run_experts(l->tab, l->maps, (const float *const *)l->dsp, S.ue, nb, 7);
 }
+static void decode_body(const LayerDev *l, int nb, const float *bias) {
+    k_router_logits_small(S.st, l->router_s, l->router_t, S.hn, S.hT, 1, bias, S.logits, nb, S.err);
+    decode_routed(l, nb);
+}
 static void decode_layers(int nb, int l0, int nl, const float *bias) {
     k_norm_prep_relaid(S.st, S.x, S.ly[l0].post_ln, S.hn, S.hq, S.hqs, S.hqsum, (float *)S.hT, nb);
+    const int joint = nb == 1;            /* with the next router too; x then alternates between two buffers */
+    float *x = S.x, *other = S.y;
     for (int L = l0; L < l0 + nl; L++) {
-        decode_body(&S.ly[L], nb, bias);
-        if (L + 1 < l0 + nl) k_edge(S.st, S.down, S.uw, S.tp, S.x, S.ly[L + 1].post_ln, S.hn, S.hq, S.hqs, S.hqsum, (float *)S.hT, nb);
-        else k_combine(S.st, S.down, S.uw, S.tp, S.x, S.x, nb);
+        const LayerDev *l = &S.ly[L], *n = l + 1;
+        if (L > l0 && joint) decode_routed(l, nb); else decode_body(l, nb, bias);
+        if (L + 1 == l0 + nl) k_combine(S.st, S.down, S.uw, S.tp, x, S.x, nb);
+        else if (!joint) k_edge(S.st, S.down, S.uw, S.tp, S.x, n->post_ln, S.hn, S.hq, S.hqs, S.hqsum, (float *)S.hT, nb);
+        else {
+            k_router_edge(S.st, n->router_s, S.down, S.uw, S.tp, x, other, n->post_ln, S.hn, S.hq, S.hqs, S.hqsum, bias, S.logits, S.err);
+            float *t = x; x = other; other = t;
+        }
     }
 }
 /* A few hundred tokens on the tcgen05 kernels: the same joint of two layers (to 511 tokens: k_edge_wire). */

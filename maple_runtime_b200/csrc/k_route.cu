@@ -13,6 +13,7 @@
 #include "topk.cuh"
 #include "silu_row.cuh"
 #include "wire.cuh"
+#include "edge.cuh"
 
 static long g_launches = 0;
 extern "C" void k_count_reset(void) { g_launches = 0; }
@@ -587,96 +588,15 @@ extern "C" void k_silu_quant(cudaStream_t st, const float *gate, const float *up
 // pair with its row) instead of once per CTA: a layer of the stack 98.9 -> 96.4 us at 301 tokens, 110.2 -> 108.0 at 511, but 123.0 -> 124.5 at 600.
 // (512 threads: 99.1 at 301; launched programmatically 96.7.)
 // ------------------------------------------------------------------------------------------------------------
-struct EdgeWire { uint8_t *wire; int np_cap; const float *const *dsp; };
 template <bool WIRE>
 __global__ void __launch_bounds__(256) edge_kernel(const float *down, const EdgeWire ew, const float *uw, const int *tp, float *x, const uint16_t *__restrict__ w,
                                                    float *hn, int8_t *q, float *qs, int *qsum, float *hS) {
     __shared__ const float *s_dsp[WIRE ? NEXP : 1];
-    __shared__ double s_term[16 * 32];
-    __shared__ float s_k, s_mx[8]; __shared__ int s_sum[8];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c = blockIdx.x;
+    const int tid = threadIdx.x, c = blockIdx.x;
     const uint2 ln[2] = {reinterpret_cast<const uint2 *>(w)[tid], reinterpret_cast<const uint2 *>(w)[tid + 256]};      // weights: read before the wait
     if (WIRE) { static_assert(NEXP == 256, "one entry per thread"); s_dsp[tid] = ew.dsp[tid]; __syncthreads(); }
     pdl_wait(); pdl_trigger();
-    int slot[TOPK]; float uv[TOPK];
-#pragma unroll
-    for (int k = 0; k < TOPK; k++) slot[k] = tp[c * TOPK + k];
-#pragma unroll
-    for (int k = 0; k < TOPK; k++) uv[k] = uw[slot[k]];
-    int4 rec[WIRE ? TOPK : 1];                                          // {scale of the pair's int8 row, expert, escape bits}
-    if (WIRE) {
-#pragma unroll
-        for (int k = 0; k < TOPK; k++) rec[k] = __ldcg(reinterpret_cast<const int4 *>(ew.wire + (size_t)ew.np_cap * WIRE_PITCH + (size_t)slot[k] * WIRE_REC));
-    }
-    float4 v[2];
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const int i = tid + 256 * k;
-        float4 d[TOPK];                                                 // WIRE: the scales
-        v[k] = __ldcg(reinterpret_cast<const float4 *>(x) + (size_t)c * 512 + i);
-        if (WIRE) {
-            uint2 raw[TOPK];
-#pragma unroll
-            for (int t = 0; t < TOPK; t++) raw[t] = __ldcg(reinterpret_cast<const uint2 *>(ew.wire + (size_t)slot[t] * WIRE_PITCH) + i);
-#pragma unroll
-            for (int t = 0; t < TOPK; t++) { const float *p = s_dsp[rec[t].y & 0xFF]; d[t] = p ? reinterpret_cast<const float4 *>(p)[i] : make_float4(0.f, 0.f, 0.f, 0.f); }
-#pragma unroll
-            for (int t = 0; t < TOPK; t++) wire_add(v[k], raw[t], uv[t], __int_as_float(rec[t].x), d[t], rec[t].z, warp + 8 * k, lane, ew.wire, ew.np_cap, slot[t]);
-        } else {
-#pragma unroll
-            for (int t = 0; t < TOPK; t++) d[t] = __ldcg(reinterpret_cast<const float4 *>(down) + (size_t)slot[t] * 512 + i);
-#pragma unroll
-            for (int t = 0; t < TOPK; t++) {
-                v[k].x = __fmaf_rn(uv[t], d[t].x, v[k].x); v[k].y = __fmaf_rn(uv[t], d[t].y, v[k].y);
-                v[k].z = __fmaf_rn(uv[t], d[t].z, v[k].z); v[k].w = __fmaf_rn(uv[t], d[t].w, v[k].w);
-            }
-        }
-        reinterpret_cast<float4 *>(x)[(size_t)c * 512 + i] = v[k];
-        s_term[(warp + 8 * k) * 32 + lane] = ((double)v[k].x * (double)v[k].x + (double)v[k].y * (double)v[k].y) + ((double)v[k].z * (double)v[k].z + (double)v[k].w * (double)v[k].w);
-    }
-    __syncthreads();
-    if (warp == 0) {
-        double ss = 0.0;
-#pragma unroll
-        for (int i = 0; i < 16; i++) ss += s_term[i * 32 + lane];
-#pragma unroll
-        for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (lane == 0) s_k = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn((float)(ss / (double)HID), 1e-6f)));
-    }
-    __syncthreads();
-    const float kk = s_k;
-    float mx = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const int i = tid + 256 * k, col = 4 * i;
-        v[k].x = __fmul_rn(__fmul_rn(v[k].x, kk), __uint_as_float(ln[k].x << 16)); v[k].y = __fmul_rn(__fmul_rn(v[k].y, kk), __uint_as_float(ln[k].x & 0xFFFF0000u));
-        v[k].z = __fmul_rn(__fmul_rn(v[k].z, kk), __uint_as_float(ln[k].y << 16)); v[k].w = __fmul_rn(__fmul_rn(v[k].w, kk), __uint_as_float(ln[k].y & 0xFFFF0000u));
-        mx = fmaxf(fmaxf(mx, fmaxf(fabsf(v[k].x), fabsf(v[k].y))), fmaxf(fabsf(v[k].z), fabsf(v[k].w)));
-        reinterpret_cast<float4 *>(hn)[(size_t)c * 512 + i] = v[k];
-        float *p = hS + (size_t)c * HID + (col >> 5) * 32 + (col & 7) * 4 + ((col >> 3) & 3);
-        p[0] = v[k].x; p[4] = v[k].y; p[8] = v[k].z; p[12] = v[k].w;
-    }
-    mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));      // >= 0: the bits order like the values
-    if (lane == 0) s_mx[warp] = mx;
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 8; k++) mx = fmaxf(mx, s_mx[k]);
-    const float s = mx > 0.0f ? __fdiv_rn(mx, 127.0f) : 1.0f, inv = __fdiv_rn(1.0f, s);
-    int tot = 0;
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const int q0 = __float2int_rn(__fmul_rn(v[k].x, inv)), q1 = __float2int_rn(__fmul_rn(v[k].y, inv)), q2 = __float2int_rn(__fmul_rn(v[k].z, inv)), q3 = __float2int_rn(__fmul_rn(v[k].w, inv));
-        tot += (q0 + q1) + (q2 + q3);
-        reinterpret_cast<uint32_t *>(q)[(size_t)c * 512 + tid + 256 * k] = (uint32_t)(q0 & 0xFF) | ((uint32_t)(q1 & 0xFF) << 8) | ((uint32_t)(q2 & 0xFF) << 16) | ((uint32_t)(q3 & 0xFF) << 24);
-    }
-    tot = __reduce_add_sync(0xffffffffu, tot);
-    if (lane == 0) s_sum[warp] = tot;
-    __syncthreads();
-    if (tid == 0) {
-        int t = 0;
-        for (int k = 0; k < 8; k++) t += s_sum[k];
-        qs[c] = s; qsum[c] = t;
-    }
+    edge_token<WIRE>(c, down, ew, s_dsp, uw, tp, x, x, ln, hn, q, qs, qsum, hS + (size_t)c * HID, true);
 }
 extern "C" void k_edge(cudaStream_t st, const float *down, const float *uw, const int *tp, float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb) {
     if (nb <= 0) return;

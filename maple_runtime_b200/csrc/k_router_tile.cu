@@ -16,6 +16,7 @@
 #include "kernels.h"
 #include "launch.cuh"
 #include "umma.cuh"
+#include "edge.cuh"
 
 #define HID 2048
 #define NEXP 256
@@ -224,9 +225,13 @@ __global__ void __launch_bounds__(256) router_pack_h_small_kernel(const float *_
 }
 // STEP: the order of the reference's single-token decode (bf_row, maple.c:146-157, called at maple.c:609): per lane two chains, one over
 // columns 16m + j and one over 16m + 8 + j, added before the lanes are; otherwise one chain per lane (job_route_small/multi).
-template <bool STEP>
+// EDGE (one token, between layers): every CTA first does the joint of the two layers for itself (edge.cuh; 64 KB of down rows out of L2), the first one
+// also stores what it gives; the row goes into shared memory.  One kernel less in the chain: 24 layers 500 -> 459 us.  From two tokens on repeating the joint in
+// every CTA costs more than the launch (2: 548 -> 561, 4: 600 -> 715).
+struct RouterEdge { const float *down, *uw; const int *tp; const float *x; float *xo; const uint16_t *w; float *hn; int8_t *q; float *qs; int *qsum; };
+template <bool STEP, bool EDGE>
 __global__ void __launch_bounds__(256, 2) router_small_kernel(const uint8_t *__restrict__ WS, const uint8_t *__restrict__ hS, const float *__restrict__ bias,
-                                                             float *__restrict__ logits, int nb, int *err) {
+                                                             float *__restrict__ logits, int nb, int *err, const RouterEdge ed) {
     extern __shared__ __align__(128) uint8_t rs_sm[];                  // hidden 64 KB, then weights 32 KB
     __shared__ uint64_t bar; __shared__ int abort_flag;
     const int tid = threadIdx.x, j = tid & 7, pos = tid >> 3, tok = pos & 7, ep = pos >> 3;
@@ -234,12 +239,19 @@ __global__ void __launch_bounds__(256, 2) router_small_kernel(const uint8_t *__r
     if (tid == 0) { mbar_init(&bar, 1); abort_flag = 0; mbar_init_fence(); }
     __syncthreads();
     if (tid == 0) {
-        mbar_expect_tx(&bar, (uint32_t)(ntok * HID * 4 + RS_WB));
+        mbar_expect_tx(&bar, (uint32_t)((EDGE ? 0 : ntok * HID * 4) + RS_WB));
         bulk_load(smem_u32(rs_sm + RS_HB), WS + (size_t)e0 * HID * 2, RS_WB, &bar);      // the layer's weights: no kernel of the layer loop writes them
-        pdl_wait();
-        bulk_load(smem_u32(rs_sm), hS + (size_t)b0 * HID * 4, (uint32_t)(ntok * HID * 4), &bar);
+        if (!EDGE) {
+            pdl_wait();
+            bulk_load(smem_u32(rs_sm), hS + (size_t)b0 * HID * 4, (uint32_t)(ntok * HID * 4), &bar);
+        }
     }
-    pdl_wait(); pdl_trigger();
+    if (EDGE) {
+        const uint2 ln[2] = {reinterpret_cast<const uint2 *>(ed.w)[tid], reinterpret_cast<const uint2 *>(ed.w)[tid + 256]};
+        pdl_wait(); pdl_trigger();
+        edge_token<false>(0, ed.down, EdgeWire{}, nullptr, ed.uw, ed.tp, ed.x, ed.xo, ln, ed.hn, ed.q, ed.qs, ed.qsum, reinterpret_cast<float *>(rs_sm), blockIdx.x == 0);
+        __syncthreads();
+    } else { pdl_wait(); pdl_trigger(); }
     const bool ok = mbar_wait(&bar, 0, &abort_flag);
     float acc0 = 0.0f, acc1 = 0.0f, odd0 = 0.0f, odd1 = 0.0f;       // odd0/odd1: the second chain of the step order (columns 16m + 8 + j)
     if (ok && tok < ntok) {
@@ -407,8 +419,8 @@ extern "C" void k_router_logits_small(cudaStream_t st, const void *router_s, con
     if (nb <= 0) return;
     static bool attr_done = false;
     if (!attr_done) {
-        cudaFuncSetAttribute(router_small_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_HB + RS_WB);
-        cudaFuncSetAttribute(router_small_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_HB + RS_WB); attr_done = true;
+        cudaFuncSetAttribute(router_small_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_HB + RS_WB);
+        cudaFuncSetAttribute(router_small_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_HB + RS_WB); attr_done = true;
     }
     if (!relaid) launch_k(router_pack_h_small_kernel, nb * 2, 256, 0, st, hn, (float4 *)hS, nb);
     static int sms = 0;
@@ -421,7 +433,20 @@ extern "C" void k_router_logits_small(cudaStream_t st, const void *router_s, con
         return;
     }
     const dim3 grid(NEXP / RS_EXP, (nb + RS_TOK - 1) / RS_TOK);
-    if (g_step_order && nb == 1) launch_pdl(router_small_kernel<true>, grid, 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err);
-    else launch_pdl(router_small_kernel<false>, grid, 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err);
+    if (g_step_order && nb == 1) launch_pdl(router_small_kernel<true, false>, grid, 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err, RouterEdge{});
+    else launch_pdl(router_small_kernel<false, false>, grid, 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err, RouterEdge{});
     k_count_add(relaid ? 1 : 2);
+}
+// the joint of two layers and the router of the next, for one token; x and xo are different buffers (the CTAs read x while the first writes xo)
+extern "C" void k_router_edge(cudaStream_t st, const void *router_s, const float *down, const float *uw, const int *tp, const float *x, float *xo, const uint16_t *w,
+                              float *hn, int8_t *q, float *qs, int *qsum, const float *bias, float *logits, int *err) {
+    static bool attr_done = false;
+    if (!attr_done) {
+        cudaFuncSetAttribute(router_small_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_HB + RS_WB);
+        cudaFuncSetAttribute(router_small_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_HB + RS_WB); attr_done = true;
+    }
+    const RouterEdge ed = {down, uw, tp, x, xo, w, hn, q, qs, qsum};
+    if (g_step_order) launch_pdl(router_small_kernel<true, true>, dim3(NEXP / RS_EXP), 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)NULL, bias, logits, 1, err, ed);
+    else launch_pdl(router_small_kernel<false, true>, dim3(NEXP / RS_EXP), 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)NULL, bias, logits, 1, err, ed);
+    k_count_add(1);
 }

@@ -93,6 +93,9 @@ void k_actq(cudaStream_t st, const float *act, int8_t *aq, float *aqs, int *aqsu
 void k_silu_quant(cudaStream_t st, const float *gate, const float *up, float *act, int8_t *aq, float *aqs, int *aqsum, int np, const int *np_dev);
 /* decode batches, between two layers: x += the pairs' weighted rows, then norm + int8 of x as k_norm_prep_relaid */
 void k_edge(cudaStream_t st, const float *down, const float *uw, const int *tp, float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb);
+/* one token: k_edge and the next layer's k_router_logits_small in one kernel; x -> xo, which is another buffer */
+void k_router_edge(cudaStream_t st, const void *router_s, const float *down, const float *uw, const int *tp, const float *x, float *xo, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum,
+                   const float *bias, float *logits, int *err);
 /* the same from the tcgen05 down kernel's compact rows */
 void k_edge_wire(cudaStream_t st, uint8_t *wire, int np_cap, const float *const *dsp, const float *uw, const int *tp, float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb);
 void k_combine(cudaStream_t st, const float *down, const float *uw, const int *tp, const float *init, float *out, int nb);

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(scope="module")
 def synth(gpu):
-    for L in (3, 4):
+    for L in (3, 4, 5, 6):
         gpu.synth_layer(SEED, L)
 
 
@@ -37,6 +37,25 @@ def test_fused_decode_layers_equal_stages(nb, g, weights, clib):
             assert same_bits(y, want), f"stack, call {call}"
             y, _ = g.moe(3, x, bias)
             assert same_bits(y, want_y), f"layer, call {call}"
+
+
+@pytest.mark.parametrize("nl", [2, 3, 4])
+@pytest.mark.parametrize("step", [0, 1])
+def test_one_token_through_several_layers(nl, step, g, weights, clib):
+    """The joint of two layers inside the next router's kernel: the hidden row alternates between two buffers."""
+    from maple_runtime_b200 import lib as ml
+    x = weights.hidden(2300, 1)
+    clib.gmoe_set_step_order(step)
+    try:
+        for bias in (None, ml.synth_zipf_bias(clib, 7)):
+            g.keep_stages(True)
+            want = x.copy(); g.forward(want, 3, nl, bias)
+            g.keep_stages(False)
+            for call in range(3):
+                y = x.copy(); g.forward(y, 3, nl, bias)
+                assert same_bits(y, want), f"call {call}"
+    finally:
+        clib.gmoe_set_step_order(0)
 
 
 @pytest.mark.parametrize("shift", [0, 1])
