@@ -6,6 +6,7 @@
 #include <stdint.h>
 #include "kernels.h"
 #include "launch.cuh"
+#include "umma.cuh"
 
 extern "C" void k_count_add(long n);
 
@@ -18,6 +19,7 @@ __global__ void __launch_bounds__(256) tables_kernel(const __grid_constant__ Tab
     const unsigned vecs = wide ? words / 4 : 0;
     for (unsigned i = blockIdx.x * 256 + threadIdx.x; i < vecs; i += step) reinterpret_cast<uint4 *>(dst)[i] = reinterpret_cast<const uint4 *>(src)[i];
     for (unsigned i = vecs * 4 + blockIdx.x * 256 + threadIdx.x; i < words; i += step) dst[i] = src[i];
+    tma_release_maps();                                                  // some segments are tensor maps
 }
 extern "C" void k_tables(cudaStream_t st, const TableSegs *t) {
     if (t->n <= 0) return;

@@ -140,6 +140,13 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const void *tmap,
                  ::"r"(dst_smem), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
 }
 
+// Tensor maps in global memory are read through a proxy of their own.  Whoever wrote one with ordinary stores releases it to that proxy; a CTA
+// acquires each map before its first use of it, prefetches included: without that it may see what was at the address before.  gpu: written
+// by a kernel on this GPU; sys: by a copy from the host.
+__device__ __forceinline__ void tma_release_maps() { asm volatile("fence.proxy.tensormap::generic.release.gpu;" ::: "memory"); }
+__device__ __forceinline__ void tma_acquire_map_gpu(const void *tmap) { asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tmap) : "memory"); }
+__device__ __forceinline__ void tma_acquire_map_sys(const void *tmap) { asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(tmap) : "memory"); }
+
 // pulls a tensor map into the descriptor cache ahead of its first use: a copy through a map that is not there waits for it, and the copies
 // queued behind it wait too
 __device__ __forceinline__ void tma_prefetch_map(const void *tmap) { asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory"); }
