@@ -462,7 +462,7 @@ def main():
         ones = np.ones(128, np.float32)
         ts = sorted(g.qk_rope(qkv, pos, 0, ones, ones)[3] for _ in range(7))
         ah_bytes = NB * (3072 * 4 + 2048 * 4 + 2 * 512 * 2)
-        out["attention_head"] = {"what": "gmoe_qk_rope on one 2048-token chunk: q/k RMS norm, half-rotary embedding, fp16 key and value rows (kernel only, median of 7)",
+        out["attention_head"] = {"what": "gmoe_qk_rope on one 2048-token chunk: q/k RMS norm, half-rotary embedding, fp16 key and value rows (the sum of its kernels over the chunks that the call is cut into, median of 7)",
                                  "us": ts[3] * 1e6, "algorithmic_bytes": ah_bytes, "achieved_gbs": ah_bytes / ts[3] / 1e9, "frac_of_measured_hbm": ah_bytes / ts[3] / 1e9 / pk["hbm_gbs"]}
     if not args.no_decode and rank == 0 and world == 1:
         out["decode"] = decode_leg(g, clib, ml, nl, pk, warm, args.steps)
@@ -475,8 +475,8 @@ def main():
 
 def dense_leg(g, ml, pk, warm, steps):
     """The attention projections of one layer on the 2048-token chunk (gpre_dense, gpu_pre.m:235-256): q,k,v as one group of 3072
-    rows and o (2048 rows), synthetic ternary matrices; GPU seconds of the call (per-token int8 + the grouped kernel), host copies
-    outside.  Reported beside the headline, not part of it."""
+    rows and o (2048 rows), synthetic ternary matrices; GPU seconds of the call: the sum of the product's kernels over the chunks that
+    it is cut into; the rows' int8 form (made by the host) and the copies are outside.  Reported beside the headline, not part of it."""
     rng = np.random.default_rng(SEED & 0xFFFFFFFF)
 
     def matrix(rows):   # codes 0..2 in every 2-bit field (never 3), scales as for the experts

@@ -75,7 +75,8 @@ int gpre_pin_policy(int on);
  * (i, i + 32), maple.c:403-411) with cos and sin from the table the host builds for gfull_init (maple.c:1151-1153:
  * cs[position][32][2] = (cos, sin), handed over once with gmoe_rope_table), queries out in fp32, keys and values out in fp16 (the rows
  * the KV cache receives, maple.c:716-717).  qkv [nb][3072] = q 2048 | k 512 | v 512 (the q,k,v projections' output, gpre_dense group 2L);
- * pos [nb]; q [nb][2048]; kc, vc [nb][512] fp16.  Host pointers, synchronous; returns the kernel's seconds or a negative value.  Results
+ * pos [nb]; q [nb][2048]; kc, vc [nb][512] fp16.  Host pointers, synchronous; returns the kernel's seconds (a call of more than 96 tokens
+ * is cut into chunks: the sum of their kernels' seconds; the host's and the copies' time is not in it) or a negative value.  Results
  * are the compiled reference's bits.  This is the first piece of the attention half; attention itself, the cache and the output head
  * are not on the card (gfull_init answers "unavailable"). */
 int gmoe_rope_table(const float *cs, int positions);

@@ -75,7 +75,8 @@ void gpre_dense_add(int g, const uint8_t *codes, const float *scales, int rows, 
  * the projections on the CPU, as the reference does when its buffers do not fit). */
 int gpre_dense_done(int maxtok);
 /* gpu_pre.m:235-256 / maple.c:266: y[nb][rows of the group] = the group's matrices times prep(x[nb][2048]) (tdot_multi of
- * maple.c:459-470: per-token absmax int8, int32 dot, (float)(tot - qsum) * qs * s[r]).  Returns GPU seconds, -1.0 on error. */
+ * maple.c:459-470: per-token absmax int8, int32 dot, (float)(tot - qsum) * qs * s[r]).  Returns GPU seconds, -1.0 on
+ * error: up to 96 tokens from the first kernel to the end of the last (they also move the rows), above that the sum of the product's kernels. */
 double gpre_dense(int g, const float *x, int nb, float *y);
 
 /* ---- present so the reference links; not part of the MoE path; each reports "unavailable" ---- */

@@ -29,6 +29,7 @@ void k_count_add(long n);
  * copy is a link of its own in the chain of a call (submit, wait for the event, move to its place), 25 us and more with its neighbours. */
 #define INPLACE_MAXTOK 96
 #define INPLACE_WIDE 3072
+#define SPANS 256           /* chunks of a call whose kernels are timed one by one: 16384 tokens make 64 */
 #define H_ROWS_OUT (S.h_rows + (size_t)INPLACE_MAXTOK * INPLACE_WIDE)
 #define H_BIAS (S.h_rows + (size_t)2 * INPLACE_MAXTOK * INPLACE_WIDE)      /* a call's bias, behind the rows */
 
@@ -61,6 +62,7 @@ static struct {
     int8_t *hq, *aq;
     float *h_rows;             /* page-locked: a decode batch's rows in, and behind them its rows out (INPLACE_WIDE values per token each) */
     int *ecnt, *uexp, *hqsum, *top, *nu, *ue, *estart, *ustart, *utok, *slot, *tp, *aqsum, *ntiles_a, *ntiles_b, *gu_dots, *dn_dots;
+    unsigned long long *span, *ns, *h_ns; int spans, span_bad;      /* start and end of each chunk's kernel (span.cuh); their sum, device's and host's pointer */
     unsigned *mask; int *err, *h_err;      /* the kernels' error word, in page-locked host memory: the device's and the host's pointer to it */
     MoeTile *tiles_a, *tiles_b;
     ExpertPtrs *tab_call;      /* the used experts of one gpre_moe call */
@@ -184,6 +186,7 @@ static int init_common(const char *who, int maxtok, int topk) {
     if (bmaps(who, P)) return -1;
     CU(who, cudaHostAlloc((void **)&S.h_err, 16, cudaHostAllocMapped)); *S.h_err = 0;
     CU(who, cudaHostGetDevicePointer((void **)&S.err, S.h_err, 0));
+    S.h_ns = (unsigned long long *)S.h_err + 1; S.ns = (unsigned long long *)S.err + 1; ALLOC(span, SPANS * 16); S.span_bad = 1;
     CT.cap = (size_t)INPLACE_MAXTOK * (HID + 8) + P * 12 + (P / 8 + NEXP) * sizeof(MoeTile) + T * 8 + NEXP * (sizeof(ExpertMaps) + sizeof(ExpertPtrs) + 16) + 4096;
     CU(who, cudaHostAlloc((void **)&CT.h, CT.cap, cudaHostAllocMapped)); CU(who, cudaEventCreateWithFlags(&CT.taken, cudaEventDisableTiming));
     CU(who, cudaHostAlloc((void **)&S.h_rows, ((size_t)2 * INPLACE_MAXTOK * INPLACE_WIDE + NEXP) * 4, cudaHostAllocMapped));
@@ -518,6 +521,16 @@ static double finish(const char *who) {      /* and the seconds between the call
     float ms = 0; cudaEventElapsedTime(&ms, S.e0, S.e1);
     return ms * 1e-3;
 }
+
+/* The seconds of a call whose kernels follow the chunks of its rows: what the kernels themselves took.  span_open before the first chunk, span_next
+ * for each, span_close behind the last one's kernel, span_secs once the stream has been waited for. */
+static void span_open(void) {
+    if (S.span_bad) cudaMemsetAsync(S.span, 0, SPANS * 16, S.st);      /* a call that failed left them open */
+    S.span_bad = 1; S.spans = 0;
+}
+static unsigned long long *span_next(void) { const int i = S.spans < SPANS ? S.spans++ : SPANS - 1; return S.span + 2 * i; }
+static void span_close(void) { k_span_sum(S.st, S.span, S.spans, S.ns); S.span_bad = 0; }
+static double span_secs(void) { return (double)*(volatile unsigned long long *)S.h_ns * 1e-9; }
 
 /* hidden rows between a caller's host array and the card (hostflow.h) */
 static int rows_in(const char *who, float *dev, const float *x, int nb) {
@@ -1079,8 +1092,11 @@ int gmoe_rope_table(const float *cs, int positions) {
     CU("gmoe", cudaMemcpyAsync(AT.cs, cs, (size_t)positions * 64 * 4, cudaMemcpyHostToDevice, S.st)); CU("gmoe", cudaStreamSynchronize(S.st));
     AT.positions = positions; return 0;
 }
+typedef struct { int glob, nb; } RopeCall;
 static int rope_rows(void *ctx, int r, int n) {
-    k_qk_rope(S.st, AT.qkv + (size_t)r * 3072, AT.pos + r, n, *(int *)ctx, AT.norms, AT.norms + 128, AT.cs, AT.positions, AT.q + (size_t)r * 2048, (uint16_t *)AT.kc + (size_t)r * 512, (uint16_t *)AT.vc + (size_t)r * 512, S.err);
+    const RopeCall *c = ctx;
+    k_qk_rope(S.st, AT.qkv + (size_t)r * 3072, AT.pos + r, n, c->glob, AT.norms, AT.norms + 128, AT.cs, AT.positions, AT.q + (size_t)r * 2048, (uint16_t *)AT.kc + (size_t)r * 512, (uint16_t *)AT.vc + (size_t)r * 512, S.err, span_next());
+    if (r + n == c->nb) span_close();
     return 0;
 }
 double gmoe_qk_rope(const float *qkv, const int *pos, int nb, int glob, const float *qn, const float *kn, float *q, uint16_t *kc, uint16_t *vc) {
@@ -1114,12 +1130,14 @@ double gmoe_qk_rope(const float *qkv, const int *pos, int nb, int glob, const fl
     memcpy(tables_add(AT.pos, (size_t)nb * 4), pos, (size_t)nb * 4);
     float *nn = tables_add(AT.norms, 256 * 4); memcpy(nn, qn, 128 * 4); memcpy(nn + 128, kn, 128 * 4);
     if (tables_send("gmoe")) return -1.0;
+    RopeCall rc = {glob, nb};
+    span_open();
     Flow f; memset(&f, 0, sizeof f);
-    f.rows = nb; f.src = qkv; f.row = 3072 * 4; f.dst = AT.qkv; f.compute = rope_rows; f.ctx = &glob; f.timed = 1;
+    f.rows = nb; f.src = qkv; f.row = 3072 * 4; f.dst = AT.qkv; f.compute = rope_rows; f.ctx = &rc;
     f.nout = 3; f.osrc[0] = AT.q; f.odst[0] = q; f.orow[0] = 2048 * 4; f.osrc[1] = AT.kc; f.odst[1] = kc; f.orow[1] = 512 * 2; f.osrc[2] = AT.vc; f.odst[2] = vc; f.orow[2] = 512 * 2;
     const cudaError_t e = flow_run(&f, S.st);
     if (e != cudaSuccess) { fail("gmoe", "gmoe_qk_rope of %d tokens: %s", nb, cudaGetErrorString(e)); return -1.0; }
-    return check_done("gmoe") ? -1.0 : f.secs;
+    return check_done("gmoe") ? -1.0 : span_secs();
 }
 
 /* ---- the attention projections (gpu_pre.m:200-256): every layer's q,k,v (group 2L) and o (group 2L+1) resident on the card.
@@ -1189,14 +1207,16 @@ int gpre_dense_done(int maxtok) {
 /* A call is cut into chunks of 256 tokens, whose rows cross the link in both directions while other chunks are multiplied: 14 us of kernel
  * against 57 us for the 3.1 MB of q,k,v results, so a chunk need not fill the card. */
 #define DENSE_CHUNK 256
-typedef struct { int g, nb; } DenseCall;
+typedef struct { int g, nb, spans; } DenseCall;
 static int dense_rows(void *ctx, int r, int n) {
     const DenseCall *c = ctx;
     const int ys = DG[c->g].rows, um = n > 128 && ys % 256 == 0;
     ExpertArgs a; memset(&a, 0, sizeof a);
     a.tab = DG[c->g].tab; a.maps = DG[c->g].maps; a.err = S.err; a.dense_p0 = r; a.dense_n = n;
     a.aq = S.hq; a.aqs = S.hqs; a.aqsum = S.hqsum; a.down = DY; a.down_stride = ys; a.dense_mblocks = ys / 256;
+    if (c->spans) a.span = span_next();
     if (um) k_dense_umma(S.st, &a, &bmap_tok); else k_dense_mma(S.st, &a, ys);
+    if (c->spans && r + n == c->nb) span_close();
     return 0;
 }
 #define QUANT_ROWS 3              /* rows per piece of work: 24 KB */
@@ -1211,7 +1231,7 @@ double gpre_dense(int g, const float *x, int nb, float *y) {
     if (g < 0 || g >= DGRP || !DG[g].codes) { fail("gpre", "gpre_dense: group %d has no matrices on the card", g); return -1.0; }
     if (nb < 1 || nb > DY_tok) { fail("gpre", "gpre_dense: %d tokens outside 1..%d", nb, DY_tok); return -1.0; }
     if (S.keep && rows_in("gpre", S.hn, x, nb)) return -1.0;
-    DenseCall d = {g, nb};
+    DenseCall d = {g, nb, 0};
     if (nb <= INPLACE_MAXTOK && DG[g].rows <= INPLACE_WIDE) {      /* three kernels in a row: int8 rows in, the product, its rows out */
         if (tables_begin("gpre")) return -1.0;
         QuantJob j = {x, nb, tables_add(S.hq, (size_t)nb * HID), tables_add(S.hqs, (size_t)nb * 4), tables_add(S.hqsum, (size_t)nb * 4)};
@@ -1230,12 +1250,12 @@ double gpre_dense(int g, const float *x, int nb, float *y) {
     }
     Flow f; memset(&f, 0, sizeof f);
     f.rows = nb; f.chunk = DENSE_CHUNK; f.src = x; f.row = HID * 4; f.dst = S.hq; f.quant = 1; f.hqs = DH_qs; f.hqsum = DH_qsum; f.dst_qs = S.hqs; f.qs_pitch = (size_t)S.maxtok;
-    f.compute = dense_rows; f.ctx = &d; f.timed = 1;
+    f.compute = dense_rows; f.ctx = &d; d.spans = 1; span_open();
     f.nout = 1; f.osrc[0] = DY; f.odst[0] = y; f.orow[0] = (size_t)DG[g].rows * 4;
     const cudaError_t e = flow_run(&f, S.st);
     if (e != cudaSuccess) { fail("gpre", "gpre_dense of %d tokens: %s", nb, cudaGetErrorString(e)); return -1.0; }
     S.nb_cur = nb;
-    return check_done("gpre") ? -1.0 : f.secs;
+    return check_done("gpre") ? -1.0 : span_secs();
 }
 int gpu_head_init(const uint16_t *w, int rows, int cols) { (void)w; (void)rows; (void)cols; return -1; }
 int gpu_head_init_i8(const int8_t *w, const float *scale, int rows, int cols) { (void)w; (void)scale; (void)rows; (void)cols; return -1; }

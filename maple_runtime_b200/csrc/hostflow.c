@@ -13,7 +13,6 @@
 #define SLOT_BYTES (3u << 20)             /* 256 tokens of the widest row (12 KB) */
 #define CHUNK_MIN (1024u << 10)           /* a chunk costs about 10 us of calls into the driver; 300 tokens through the plug-in call 589 us at 512 KB, 566 at 1 MB */
 #define STREAM_BYTES (8u << 20)           /* results larger than this are stored past the caches */
-#define MAXCHUNKS 256
 
 typedef struct { Flow *f; int slot, row0, n, per; } Part;
 static struct {
@@ -22,7 +21,6 @@ static struct {
     cudaStream_t sin, sout;
     cudaEvent_t begun, in_done[SLOTS], ran[SLOTS], out_done[SLOTS];
     int in_used[SLOTS];                   /* in_done[] has been recorded and not yet seen complete */
-    cudaEvent_t t0[MAXCHUNKS], t1[MAXCHUNKS]; int nt;
     Part fill[SLOTS], drain[SLOTS];
 } FL;
 
@@ -97,16 +95,6 @@ static cudaError_t copy_out(Flow *f, int direct, int slot, int row0, int n, cuda
     }
     return e;
 }
-static cudaError_t timed_compute(Flow *f, int chunk, int row0, int n, cudaStream_t st) {
-    if (!f->compute) return cudaSuccess;
-    const int t = f->timed && chunk < MAXCHUNKS;
-    cudaError_t e = cudaSuccess;
-    for (; t && FL.nt <= chunk && !e; FL.nt++) { e = cudaEventCreate(&FL.t0[FL.nt]); if (!e) e = cudaEventCreate(&FL.t1[FL.nt]); }
-    if (!e && t) e = cudaEventRecord(FL.t0[chunk], st);
-    if (!e && f->compute(f->ctx, row0, n)) e = cudaErrorUnknown;
-    if (!e && t) e = cudaEventRecord(FL.t1[chunk], st);
-    return e;
-}
 static cudaError_t slot_free(int s, int wait) {       /* cudaSuccess: the slot's last copy to the card has been made */
     if (!FL.in_used[s]) return cudaSuccess;
     const cudaError_t e = wait ? cudaEventSynchronize(FL.in_done[s]) : cudaEventQuery(FL.in_done[s]);
@@ -156,7 +144,7 @@ cudaError_t flow_run(Flow *f, cudaStream_t st) {
                 e = copy_in(f, din, s, row0, n, sin);
                 if (!e && (nch > 1 || !f->nout) ) { e = cudaEventRecord(FL.in_done[s], sin); FL.in_used[s] = !din; if (!e && sin != st) e = cudaStreamWaitEvent(st, FL.in_done[s], 0); }
             }
-            if (!e) e = timed_compute(f, issued, row0, n, st);
+            if (!e && f->compute && f->compute(f->ctx, row0, n)) e = cudaErrorUnknown;
             if (!e && f->nout) {
                 if (sout != st) { e = cudaEventRecord(FL.ran[s], st); if (!e) e = cudaStreamWaitEvent(sout, FL.ran[s], 0); }
                 if (!e) e = copy_out(f, dout, s, row0, n, sout);
@@ -180,10 +168,6 @@ cudaError_t flow_run(Flow *f, cudaStream_t st) {
     for (int s = 0; s < SLOTS; s++) {                          /* only after an error: the parts and the caller's rows are still in use */
         if (jin[s]) hio_wait(tin[s]);
         if (jout[s]) hio_wait(tout[s]);
-    }
-    if (!e && f->timed && f->nout) {
-        f->secs = 0;
-        for (int c = 0; c < nch && c < MAXCHUNKS; c++) { float ms = 0; cudaEventElapsedTime(&ms, FL.t0[c], FL.t1[c]); f->secs += ms * 1e-3; }
     }
     return e;
 }

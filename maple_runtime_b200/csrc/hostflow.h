@@ -16,7 +16,6 @@ typedef struct {
     float *hqs; int *hqsum; float *dst_qs; size_t qs_pitch;
     int (*compute)(void *ctx, int row0, int n); void *ctx;      /* queues the chunk's kernels on the library's stream; 0 = queued */
     int (*meanwhile)(void *mctx); void *mctx;                     /* the calling thread's own work while the rows are being read; non-zero = give up */
-    int timed; double secs;                                       /* timed: secs = device time of the computations (waits included only inside one chunk's) */
     /* out: `nout` arrays of `orow` bytes per row on the card, to host arrays */
     int nout; const void *osrc[FLOW_OUTS]; void *odst[FLOW_OUTS]; size_t orow[FLOW_OUTS];
 } Flow;

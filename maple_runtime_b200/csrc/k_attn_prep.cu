@@ -10,6 +10,7 @@
 #include <stdint.h>
 #include "kernels.h"
 #include "launch.cuh"
+#include "span.cuh"
 
 extern "C" void k_count_add(long n);
 
@@ -24,7 +25,8 @@ extern "C" void k_count_add(long n);
 template <bool SMALL>
 __global__ void __launch_bounds__(256) qk_rope_kernel(const float *__restrict__ qkv, const int *__restrict__ pos, int nb, int glob,
                                                       const float *__restrict__ qn, const float *__restrict__ kn, const float *__restrict__ cs, int cs_positions,
-                                                      float *__restrict__ q, __half *__restrict__ kc, __half *__restrict__ vc, int *err, const __grid_constant__ RopeArgs prm) {
+                                                      float *__restrict__ q, __half *__restrict__ kc, __half *__restrict__ vc, int *err, unsigned long long *span, const __grid_constant__ RopeArgs prm) {
+    if (!SMALL && threadIdx.x == 0) span_begin(span);
     __shared__ __align__(16) float s_norm[SMALL ? 2 * AP_HD : 4];
     if (SMALL) { s_norm[threadIdx.x] = threadIdx.x < AP_HD ? prm.qn[threadIdx.x] : prm.kn[threadIdx.x - AP_HD]; __syncthreads(); }
     const int lane = threadIdx.x & 31, item = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -40,6 +42,7 @@ __global__ void __launch_bounds__(256) qk_rope_kernel(const float *__restrict__ 
         for (int i = 0; i < 4; i++) {
             o[i * (AP_HD / 2)] = __halves2half2(__float2half_rn(v[i].x), __float2half_rn(v[i].y)); o[i * (AP_HD / 2) + 1] = __halves2half2(__float2half_rn(v[i].z), __float2half_rn(v[i].w));
         }
+        if (!SMALL && threadIdx.x == 0) span_end(span);
         return;
     }
     const float4 w = SMALL ? reinterpret_cast<const float4 *>(s_norm + (grp < 4 ? 0 : AP_HD))[lane] : reinterpret_cast<const float4 *>(grp < 4 ? qn : kn)[lane];
@@ -73,17 +76,18 @@ __global__ void __launch_bounds__(256) qk_rope_kernel(const float *__restrict__ 
             o2[0] = __halves2half2(__float2half_rn(x.x), __float2half_rn(x.y)); o2[1] = __halves2half2(__float2half_rn(x.z), __float2half_rn(x.w));
         }
     }
+    if (!SMALL && threadIdx.x == 0) span_end(span);      // the CTA's warps do the same amount of work each
 }
 extern "C" void k_qk_rope(cudaStream_t st, const float *qkv, const int *pos, int nb, int glob, const float *qn, const float *kn, const float *cs, int cs_positions,
-                          float *q, void *kc, void *vc, int *err) {
+                          float *q, void *kc, void *vc, int *err, unsigned long long *span) {
     if (nb <= 0) return;
     const int items = nb * 6;
     static const RopeArgs none = {};
-    launch_k(qk_rope_kernel<false>, (items + 7) / 8, 256, 0, st, qkv, pos, nb, glob, qn, kn, cs, cs_positions, q, (__half *)kc, (__half *)vc, err, none);
+    launch_k(qk_rope_kernel<false>, (items + 7) / 8, 256, 0, st, qkv, pos, nb, glob, qn, kn, cs, cs_positions, q, (__half *)kc, (__half *)vc, err, span, none);
     k_count_add(1);
 }
 extern "C" void k_qk_rope_small(cudaStream_t st, const float *qkv, const RopeArgs *prm, int nb, int glob, const float *cs, int cs_positions, float *q, void *kc, void *vc, int *err) {
     if (nb <= 0) return;
-    launch_k(qk_rope_kernel<true>, (nb * 6 + 7) / 8, 256, 0, st, qkv, (const int *)NULL, nb, glob, (const float *)NULL, (const float *)NULL, cs, cs_positions, q, (__half *)kc, (__half *)vc, err, *prm);
+    launch_k(qk_rope_kernel<true>, (nb * 6 + 7) / 8, 256, 0, st, qkv, (const int *)NULL, nb, glob, (const float *)NULL, (const float *)NULL, cs, cs_positions, q, (__half *)kc, (__half *)vc, err, (unsigned long long *)NULL, *prm);
     k_count_add(1);
 }

@@ -23,6 +23,7 @@
 #include "kernels.h"
 #include "launch.cuh"
 #include "dev_math.cuh"
+#include "span.cuh"
 
 extern "C" void k_count_add(long n);
 
@@ -52,7 +53,7 @@ __global__ void __launch_bounds__(NW * 32) expert_mma_kernel(ExpertArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];          // [KCH][4][TN][4][16]
     const int tile_i = blockIdx.y;
     if (GATEUP) { pdl_wait(); pdl_trigger(); }       // the tiles are its predecessor's; the down kernel's are two kernels old, so that its weights come in before its wait
-    const bool dense = !GATEUP && KCH == 8;
+    constexpr bool dense = !GATEUP && KCH == 8;
     const int ntiles = dense ? gridDim.y : __ldcg(a.ntiles);
     const MoeTile tile = dense ? MoeTile{0, a.dense_p0 + tile_i * TN, min(TN, a.dense_n - tile_i * TN), 0}
                                : ldcg_tile(a.tiles + (tile_i < a.max_tiles ? tile_i : 0));      // read beside the count, not after it
@@ -73,6 +74,7 @@ __global__ void __launch_bounds__(NW * 32) expert_mma_kernel(ExpertArgs a) {
     }
 
     if (!GATEUP) { pdl_wait(); pdl_trigger(); }
+    if (dense && tid == 0) span_begin(a.span);
     // stage the tile's activation vectors (16-byte pieces) in fragment order
     if (GATEUP || !a.act_for_down) {
         const int8_t *src = GATEUP ? a.hq : a.aq;
@@ -178,6 +180,7 @@ __global__ void __launch_bounds__(NW * 32) expert_mma_kernel(ExpertArgs a) {
                 if (a.dn_dots) { a.dn_dots[(size_t)pair * 2048 + rr] = da; a.dn_dots[(size_t)pair * 2048 + rr + 16] = db; }
             }
         }
+    if (dense && tid == 0) span_end(a.span);
 }
 
 template <int KCH, int NBLK, bool GATEUP, int PF, int NW>

@@ -41,6 +41,7 @@
 #include "launch.cuh"
 #include "dev_math.cuh"
 #include "umma.cuh"
+#include "span.cuh"
 
 extern "C" void k_count_add(long n);
 
@@ -118,6 +119,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
     // launched programmatically: the weights start to come in before the wait (the tile list is two kernels old), everything else after it
     if (warp != 8) pdl_wait();
     pdl_trigger();
+    if (DENSE && tid == 0) span_begin(a.span);
 
     if (warp < 8) {
         // ---------------- decode: this warp's 32 rows of both halves, every second block, from the shared-memory ring ----------------
@@ -445,6 +447,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
     }
     tc_fence_before();
     __syncthreads();
+    if (DENSE && tid == 0) span_end(a.span);
     if (warp == 10) {
         __syncwarp();
         tc_fence_after();

@@ -43,3 +43,19 @@ extern "C" void k_rows(cudaStream_t st, void *dst, const void *src, size_t bytes
     launch_pdl(rows_kernel, (n + 255) / 256, 256, 0, st, static_cast<uint4 *>(dst), static_cast<const uint4 *>(src), n);
     k_count_add(1);
 }
+
+__global__ void __launch_bounds__(32) span_sum_kernel(unsigned long long *span, int n, unsigned long long *ns) {
+    unsigned long long sum = 0;
+    for (int i = threadIdx.x; i < n; i += 32) {
+        const unsigned long long start = ~span[2 * i], end = span[2 * i + 1];
+        if (end > start) sum += end - start;
+        span[2 * i] = span[2 * i + 1] = 0;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (threadIdx.x == 0) *ns = sum;
+}
+extern "C" void k_span_sum(cudaStream_t st, unsigned long long *span, int n, unsigned long long *ns) {
+    launch_k(span_sum_kernel, 1, 32, 0, st, span, n, ns);
+    k_count_add(1);
+}

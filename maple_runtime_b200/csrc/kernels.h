@@ -30,6 +30,7 @@ typedef struct {
     float *down;             /* [np][2048], or [np][down_stride] when down_stride != 0 (the dense projections: several matrices side by side) */
     int down_stride;
     int dense_mblocks;       /* k_dense_umma: 256-row blocks of the matrix */
+    unsigned long long *span;   /* k_dense_*: two words that receive the kernel's start and end (span.cuh); NULL = off */
     int dense_p0, dense_n;   /* k_dense_*: the first token and the token count; there is no tile list, tile t is tokens dense_p0 + t * (tile size) .. */
     /* decode path: the down kernel quantises the fp32 SiLU outputs itself (no separate pass): act_for_down [np][512] in, and the
      * int8 rows, scales and sums it computed are also stored here for later inspection */
@@ -55,6 +56,9 @@ void k_tables(cudaStream_t st, const TableSegs *t);
 
 /* bytes (a multiple of 16) from src to dst, either of which may be page-locked host memory */
 void k_rows(cudaStream_t st, void *dst, const void *src, size_t bytes);
+
+/* n spans (span.cuh): the sum of their lengths in nanoseconds to *ns, and the spans zeroed for the next call */
+void k_span_sum(cudaStream_t st, unsigned long long *span, int n, unsigned long long *ns);
 
 void k_norm_prep(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, int nb);
 /* the same, and the normalised rows once more in the decode router's layout (hS, nb*HID*4 bytes): k_router_logits_small then takes relaid = 1 */
@@ -123,7 +127,7 @@ void k_gather_rows(cudaStream_t st, const int8_t *src, const int *rows, int8_t *
 /* ---- the head of the attention half (k_attn_prep.cu): q/k RMS norm, half-rotary embedding, fp16 keys and values.  qkv [nb][3072]
  * = q 2048 | k 512 | v 512; pos [nb]; qn, kn [128] fp32; cs [cs_positions][32][2] (cos, sin); q [nb][2048] fp32; kc, vc [nb][512] fp16 */
 void k_qk_rope(cudaStream_t st, const float *qkv, const int *pos, int nb, int glob, const float *qn, const float *kn, const float *cs, int cs_positions,
-               float *q, void *kc, void *vc, int *err);
+               float *q, void *kc, void *vc, int *err, unsigned long long *span);
 /* the same for up to ROPE_SMALL tokens, norms and positions by value; qkv, q, kc, vc may be page-locked host memory */
 #define ROPE_SMALL 96
 typedef struct { float qn[128], kn[128]; int pos[ROPE_SMALL]; } RopeArgs;
