@@ -15,6 +15,7 @@
 #include "synth.h"
 #include "hostflow.h"
 #include "hostio.h"
+#include "replay.h"
 
 void k_count_add(long n);
 
@@ -550,17 +551,16 @@ static int rows_out(const char *who, float *y, const float *dev, int nb) {
  * Every kernel takes its sizes from device memory, so the sequence for (nb, l0, nl, bias?, path) is the same every time and can
  * be replayed.  The second call with a key captures it (the first runs plainly, so that one-time set-up calls made by the
  * launchers happen outside a capture).  Per-stage events are captured as event-record nodes, so gmoe_profile_read then reports the
- * last replay.  Not used while stages are kept or when GMOE_GRAPH=0 is set.  Under expert parallelism the ranks make the same calls
+ * last replay.  Which loops are kept: replay.c.  Not used while stages are kept or when GMOE_GRAPH=0 is set.  Under expert parallelism the ranks make the same calls
  * in the same order, so they capture and replay together; nothing on that path calls NCCL. */
-#define NGRAPH 256          /* a host that comes back for every layer has 24 per batch size */
-static struct { int nb, l0, nl, bias, path, prof, ep, seen; long launches; cudaGraphExec_t exec; } GR[NGRAPH];
 static int g_graph_on = -1;
 static long g_graph_launches;
 long gmoe_graph_launches(void) { return g_graph_launches; }
 /* forget every captured layer loop: the weights or the work buffers a replay names have changed */
+static void exec_destroy(void *exec) { cudaGraphExecDestroy((cudaGraphExec_t)exec); }
 static void graphs_drop(void) {
     if (S.st) cudaStreamSynchronize(S.st);
-    for (int i = 0; i < NGRAPH; i++) { if (GR[i].exec) cudaGraphExecDestroy(GR[i].exec); memset(&GR[i], 0, sizeof GR[i]); }
+    replay_clear(exec_destroy);
 }
 static int graphs_on(void) {
     if (g_graph_on < 0) { const char *e = getenv("GMOE_GRAPH"); g_graph_on = !(e && e[0] == '0'); }
@@ -626,35 +626,30 @@ static int layers_run(int nb, int l0, int nl, const float *bd, int ep) {
 }
 static int layers_enqueue_ep(int nb, int l0, int nl, const float *bd, int ep) {
     if (!graphs_on()) return layers_run(nb, l0, nl, bd, ep);
-    int k = -1, free_k = -1;
-    for (int i = 0; i < NGRAPH; i++) {
-        if (GR[i].seen && GR[i].nb == nb && GR[i].l0 == l0 && GR[i].nl == nl && GR[i].bias == (bd != NULL) && GR[i].path == S.path + 8 * S.router_mode && GR[i].prof == (int)S.prof_mask && GR[i].ep == ep) { k = i; break; }
-        if (!GR[i].seen && free_k < 0) free_k = i;
-    }
-    if (k < 0) {   /* first sight: run plainly and remember the key */
+    const ReplayKey key = {nb, l0, nl, bd != NULL, S.path + 8 * S.router_mode, (int)S.prof_mask, ep};
+    ReplaySlot *r = replay_find(&key);
+    if (!r) {      /* first sight: run plainly and remember the key */
         if (layers_run(nb, l0, nl, bd, ep)) return -1;
-        if (free_k < 0) {   /* table full: the slots are reused in turn */
-            static int victim;
-            free_k = victim; victim = (victim + 1) % NGRAPH;
-            cudaStreamSynchronize(S.st);
-            if (GR[free_k].exec) cudaGraphExecDestroy(GR[free_k].exec);
-            memset(&GR[free_k], 0, sizeof GR[free_k]);
-        }
-        if (free_k >= 0) { GR[free_k].nb = nb; GR[free_k].l0 = l0; GR[free_k].nl = nl; GR[free_k].bias = bd != NULL; GR[free_k].path = S.path + 8 * S.router_mode; GR[free_k].prof = (int)S.prof_mask; GR[free_k].ep = ep; GR[free_k].seen = 1; GR[free_k].exec = NULL; }
+        void *gone;
+        replay_admit(&key, &gone);
+        if (gone) { cudaStreamSynchronize(S.st); exec_destroy(gone); }
         return 0;
     }
-    if (!GR[k].exec) {
-        cudaGraph_t g = NULL; long before = k_count();
+    if (!r->exec) {
+        if (r->tried) return layers_run(nb, l0, nl, bd, ep);
+        r->tried = 1;
+        cudaGraph_t g = NULL; cudaGraphExec_t exec = NULL; long before = k_count();
         if (cudaStreamBeginCapture(S.st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return layers_run(nb, l0, nl, bd, ep);
         int bad = layers_run(nb, l0, nl, bd, ep);
         cudaError_t e = cudaStreamEndCapture(S.st, &g);
-        GR[k].launches = k_count() - before;
-        if (e == cudaSuccess && !bad) e = cudaGraphInstantiate(&GR[k].exec, g, 0);
+        r->launches = k_count() - before;
+        if (e == cudaSuccess && !bad) e = cudaGraphInstantiate(&exec, g, 0);
         if (g) cudaGraphDestroy(g);
-        if (bad) { GR[k].exec = NULL; GR[k].seen = 2; return -1; }
-        if (e != cudaSuccess) { GR[k].exec = NULL; GR[k].seen = 2; cudaGetLastError(); return fail("gmoe", "graph capture of the layer loop: %s", cudaGetErrorString(e)); }
-    } else k_count_add(GR[k].launches);
-    CU("gmoe", cudaGraphLaunch(GR[k].exec, S.st));
+        if (bad) return -1;
+        if (e != cudaSuccess) { cudaGetLastError(); return fail("gmoe", "graph capture of the layer loop: %s", cudaGetErrorString(e)); }      /* the next call runs plainly */
+        r->exec = exec;
+    } else k_count_add(r->launches);
+    CU("gmoe", cudaGraphLaunch((cudaGraphExec_t)r->exec, S.st));
     g_graph_launches++;
     return 0;
 }
