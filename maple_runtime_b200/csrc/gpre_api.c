@@ -655,7 +655,7 @@ static int layers_enqueue_ep(int nb, int l0, int nl, const float *bd, int ep) {
 }
 static int layers_enqueue(int nb, int l0, int nl, const float *bd) { return layers_enqueue_ep(nb, l0, nl, bd, 0); }
 
-double gmoe_moe(int L, const float *x, int nb, float *y, const float *bias) {
+static double moe_call(int L, const float *x, int nb, float *y, const float *bias) {
     if (check_call("gmoe", L, nb)) return -1.0;
     if (nb <= INPLACE_MAXTOK && decode_path(nb)) {
         const size_t n = (size_t)nb * HID;
@@ -678,6 +678,7 @@ double gmoe_moe(int L, const float *x, int nb, float *y, const float *bias) {
     S.nb_cur = nb;
     return finish("gmoe");
 }
+double gmoe_moe(int L, const float *x, int nb, float *y, const float *bias) { hio_begin(HIO_LAYER); const double t = moe_call(L, x, nb, y, bias); hio_end(); return t; }
 int gmoe_forward_dev(int nb, int l0, int nl, const float *bias) {
     for (int L = l0; L < l0 + nl; L++) if (check_call("gmoe", L, nb)) return -1;
     const float *bd = bias_dev(bias);
@@ -944,7 +945,7 @@ static int stage_call(void *p) {
     CallTables *c = p;
     return c->bad = stage_grouping("gpre", c->nb, c->nu, c->loc, c->regs, c->ustart, c->ptok, c->pw, c->tp);
 }
-double gpre_moe(const float *x, int nb, int nu, const uint32_t *loc, const int *regs, const int *next,
+static double pre_moe_call(const float *x, int nb, int nu, const uint32_t *loc, const int *regs, const int *next,
                 const int *ustart, const int *ptok, const float *pw, const int *tp, float *y) {
     (void)next;
     if (grouping_args("gpre", nb, nu) || tables_begin("gpre")) return -1.0;
@@ -965,6 +966,11 @@ double gpre_moe(const float *x, int nb, int nu, const uint32_t *loc, const int *
     if (rows_out("gpre", y, S.y, nb)) return -1.0;
     S.nb_cur = nb;
     return finish("gpre");
+}
+double gpre_moe(const float *x, int nb, int nu, const uint32_t *loc, const int *regs, const int *next,
+                const int *ustart, const int *ptok, const float *pw, const int *tp, float *y) {
+    hio_begin(HIO_PLUGIN); const double t = pre_moe_call(x, nb, nu, loc, regs, next, ustart, ptok, pw, tp, y); hio_end();
+    return t;
 }
 void gfull_begin(const float *x, int nb, int pos0) {
     (void)pos0;
@@ -1094,7 +1100,7 @@ static int rope_rows(void *ctx, int r, int n) {
     if (r + n == c->nb) span_close();
     return 0;
 }
-double gmoe_qk_rope(const float *qkv, const int *pos, int nb, int glob, const float *qn, const float *kn, float *q, uint16_t *kc, uint16_t *vc) {
+static double qk_rope_call(const float *qkv, const int *pos, int nb, int glob, const float *qn, const float *kn, float *q, uint16_t *kc, uint16_t *vc) {
     if (!S.ready) { fail("gmoe", "not initialised"); return -1.0; }
     if (nb < 1 || nb > S.maxtok) { fail("gmoe", "gmoe_qk_rope: %d tokens outside 1..%d", nb, S.maxtok); return -1.0; }
     if (!qkv || !pos || !qn || !kn || !q || !kc || !vc) { fail("gmoe", "gmoe_qk_rope: null argument"); return -1.0; }
@@ -1134,6 +1140,7 @@ double gmoe_qk_rope(const float *qkv, const int *pos, int nb, int glob, const fl
     if (e != cudaSuccess) { fail("gmoe", "gmoe_qk_rope of %d tokens: %s", nb, cudaGetErrorString(e)); return -1.0; }
     return check_done("gmoe") ? -1.0 : span_secs();
 }
+double gmoe_qk_rope(const float *qkv, const int *pos, int nb, int glob, const float *qn, const float *kn, float *q, uint16_t *kc, uint16_t *vc) { hio_begin(HIO_ROPE); const double t = qk_rope_call(qkv, pos, nb, glob, qn, kn, q, kc, vc); hio_end(); return t; }
 
 /* ---- the attention projections (gpu_pre.m:200-256): every layer's q,k,v (group 2L) and o (group 2L+1) resident on the card.
  * y[nb][rows of the group] = the group's matrices times prep(x[nb][2048]): the expert product with one matrix and all tokens.
@@ -1221,7 +1228,7 @@ static void quant_piece(void *p, int i) {
     const int r = i * QUANT_ROWS, n = j->nb - r < QUANT_ROWS ? j->nb - r : QUANT_ROWS;
     hio_quant_rows(j->x + (size_t)r * HID, n, j->q + (size_t)r * HID, j->qs + r, j->qsum + r);
 }
-double gpre_dense(int g, const float *x, int nb, float *y) {
+static double dense_call(int g, const float *x, int nb, float *y) {
     if (!S.ready || !DY) { fail("gpre", "gpre_dense before gpre_dense_done"); return -1.0; }
     if (g < 0 || g >= DGRP || !DG[g].codes) { fail("gpre", "gpre_dense: group %d has no matrices on the card", g); return -1.0; }
     if (nb < 1 || nb > DY_tok) { fail("gpre", "gpre_dense: %d tokens outside 1..%d", nb, DY_tok); return -1.0; }
@@ -1252,6 +1259,7 @@ double gpre_dense(int g, const float *x, int nb, float *y) {
     S.nb_cur = nb;
     return check_done("gpre") ? -1.0 : span_secs();
 }
+double gpre_dense(int g, const float *x, int nb, float *y) { hio_begin(g & 1 ? HIO_O : HIO_QKV); const double t = dense_call(g, x, nb, y); hio_end(); return t; }
 int gpu_head_init(const uint16_t *w, int rows, int cols) { (void)w; (void)rows; (void)cols; return -1; }
 int gpu_head_init_i8(const int8_t *w, const float *scale, int rows, int cols) { (void)w; (void)scale; (void)rows; (void)cols; return -1; }
 void gpu_head_run(const float *x, float *y) { (void)x; (void)y; }

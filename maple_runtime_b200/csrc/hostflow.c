@@ -102,7 +102,7 @@ static cudaError_t slot_free(int s, int wait) {       /* cudaSuccess: the slot's
     return e;
 }
 
-cudaError_t flow_run(Flow *f, cudaStream_t st) {
+static cudaError_t run(Flow *f, cudaStream_t st) {
     cudaError_t e = setup();
     if (e) return e;
     size_t widest = f->src ? in_row(f) : 1, orow = 0;
@@ -171,3 +171,4 @@ cudaError_t flow_run(Flow *f, cudaStream_t st) {
     }
     return e;
 }
+cudaError_t flow_run(Flow *f, cudaStream_t st) { hio_begin(HIO_ROWS); const cudaError_t e = run(f, st); hio_end(); return e; }

@@ -7,6 +7,11 @@
 /* A job is fn(arg, piece) for piece = 0..pieces-1, in any order, on any of the pool's threads and on the caller's (hio_help).  One
  * thread submits; jobs are started in the order of their submission.  arg must live until hio_done. */
 typedef void (*hio_fn)(void *arg, int piece);
+/* around a call that uses the pool (they nest; the outermost one's kind counts): its threads, once it has woken them, stay awake to its end, and for
+ * a moment longer where a call of that kind is usually followed by another at once */
+enum { HIO_ROWS, HIO_LAYER, HIO_PLUGIN, HIO_ROPE, HIO_QKV, HIO_O, HIO_KINDS };
+void hio_begin(int kind);
+void hio_end(void);
 unsigned hio_submit(hio_fn fn, void *arg, int pieces);
 int hio_done(unsigned ticket);
 int hio_help(void);                       /* runs one unclaimed piece; 0 = there is none */
