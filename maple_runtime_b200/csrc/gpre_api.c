@@ -733,7 +733,7 @@ double gmoe_forward(float *x, int nb, int l0, int nl, const float *bias) {   /* 
 static struct {
     cudaStream_t in, out; int ready, seq, done;          /* seq: chunks submitted, done: chunks waited for */
     float *xin[2], *xout[2]; size_t cap;                /* staging slots on the card, cap floats each */
-    cudaEvent_t mark, start[2], loaded[2], taken[2], ran[2], stored[2];
+    cudaEvent_t mark, loaded[2], taken[2], ran[2], stored[2];
     int bad;                                             /* chunks still to be reported as invalid after a kernel's error */
 } PIPE;
 static int pipe_setup(int nb) {
@@ -741,7 +741,7 @@ static int pipe_setup(int nb) {
         CU("gmoe", cudaStreamCreateWithFlags(&PIPE.in, cudaStreamNonBlocking)); CU("gmoe", cudaStreamCreateWithFlags(&PIPE.out, cudaStreamNonBlocking));
         CU("gmoe", cudaEventCreate(&PIPE.mark));
         for (int k = 0; k < 2; k++) {
-            CU("gmoe", cudaEventCreate(&PIPE.start[k])); CU("gmoe", cudaEventCreate(&PIPE.stored[k]));
+            CU("gmoe", cudaEventCreate(&PIPE.stored[k]));
             CU("gmoe", cudaEventCreateWithFlags(&PIPE.loaded[k], cudaEventDisableTiming)); CU("gmoe", cudaEventCreateWithFlags(&PIPE.taken[k], cudaEventDisableTiming));
             CU("gmoe", cudaEventCreateWithFlags(&PIPE.ran[k], cudaEventDisableTiming));
         }
@@ -778,7 +778,6 @@ int gmoe_forward_submit(const float *x_in, float *x_out, int nb, int l0, int nl,
     if (nb <= INPLACE_MAXTOK) {
         const float *dx = host_mapped(x_in, bytes); float *dy = (float *)host_mapped(x_out, bytes);
         if (dx && dy) {
-            CU("gmoe", cudaEventRecord(PIPE.start[k], S.st));
             k_rows(S.st, S.x, dx, bytes);
             CU("gmoe", cudaEventRecord(PIPE.taken[k], S.st));
             if (layers_enqueue_ep(nb, l0, nl, bd, S.ep_on)) return -1;
@@ -789,7 +788,6 @@ int gmoe_forward_submit(const float *x_in, float *x_out, int nb, int l0, int nl,
         }
     }
     if (PIPE.seq >= 2) CU("gmoe", cudaStreamWaitEvent(PIPE.in, PIPE.taken[k], 0));           /* the slot's previous chunk has been moved into x */
-    CU("gmoe", cudaEventRecord(PIPE.start[k], PIPE.in));
     CU("gmoe", cudaMemcpyAsync(PIPE.xin[k], x_in, bytes, cudaMemcpyHostToDevice, PIPE.in));
     CU("gmoe", cudaEventRecord(PIPE.loaded[k], PIPE.in));
     CU("gmoe", cudaStreamWaitEvent(S.st, PIPE.loaded[k], 0));
