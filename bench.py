@@ -13,7 +13,7 @@ bandwidth (the roof that binds at 64 pairs per expert), and its integer operatio
 this GPU in the same run (`roofline.tensor`).  `e2e_gpre_moe` is the same chunk through 24 calls of the reference-signature gpre_moe (host
 grouping tables, host buffers: the call an unmodified maple.c makes).  `parity_check` compares two layers of the chunk with
 the reference (oracle/_ref) before anything is timed.  `cpu_baseline` times the reference's own CPU code on a bounded sample
-on this host; `--impl reference` runs that code over the whole 24-layer stack.  `decode` repeats the measurement for the
+on this host; `--impl reference` runs that code over the whole 24-layer stack, and says `unavailable` where the reference is not built.  `decode` repeats the measurement for the
 64-conversation decode shape (HBM-bound).  Prints ONE JSON line on rank 0.
 """
 import argparse
@@ -168,6 +168,10 @@ def cpu_reference_arm(steps, warmup, nlay, budget_s=None):
 
 def reference_main(args, rank, world):
     if rank != 0:
+        return
+    from oracle import oracle as orc
+    if not orc.Reference.available(fast=True):
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref is not built: the reference's sources are not on this machine"}))
         return
     value, per_step, done, cb = cpu_reference_arm(args.steps, args.warmup, LAYERS)
     print(json.dumps({
