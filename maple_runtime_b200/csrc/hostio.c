@@ -39,7 +39,8 @@ static struct { _Atomic uint64_t state; atomic_int left; hio_fn fn; void *arg; }
 static atomic_uint head, tail;            /* jobs head..tail-1 may have unclaimed pieces */
 static pthread_t th[MAXHELP];
 static int nth = -1;                      /* -1: not started yet */
-static atomic_int stop, sleepers, in_call, tail_on;
+static atomic_int stop, sleepers;
+static struct { atomic_int in_call, tail_on; } now __attribute__((aligned(64)));      /* written by the caller only, polled by the helpers */
 static pthread_mutex_t mu = PTHREAD_MUTEX_INITIALIZER;
 static pthread_cond_t cv = PTHREAD_COND_INITIALIZER;
 
@@ -61,9 +62,9 @@ static void *helper(void *p) {
     uint64_t t0 = __rdtsc(); unsigned polls = 0; int was = 0;
     while (!atomic_load_explicit(&stop, memory_order_relaxed)) {
         if (hio_help()) { t0 = __rdtsc(); continue; }
-        const int busy = atomic_load_explicit(&in_call, memory_order_relaxed);
+        const int busy = atomic_load_explicit(&now.in_call, memory_order_relaxed);
         if (busy != was) { was = busy; t0 = __rdtsc(); }
-        if (__rdtsc() - t0 < (busy ? CALL_CYCLES : atomic_load_explicit(&tail_on, memory_order_relaxed) ? TAIL_CYCLES : 0)) {
+        if (__rdtsc() - t0 < (busy ? CALL_CYCLES : atomic_load_explicit(&now.tail_on, memory_order_relaxed) ? TAIL_CYCLES : 0)) {
             if (++polls % YIELD_EVERY) _mm_pause(); else sched_yield();
             continue;
         }
@@ -92,15 +93,18 @@ __attribute__((destructor)) static void finish_threads(void) {
     for (int i = 0; i < nth; i++) pthread_join(th[i], NULL);
     nth = 0;
 }
-static int kind_of_last, followed[HIO_KINDS];      /* by kind of call: another one began within TAIL_CYCLES of its end */
+static int depth, kind_of_last, followed[HIO_KINDS];      /* followed: by kind of call, another one began within TAIL_CYCLES of its end */
 static uint64_t ended;
 void hio_begin(int kind) {
-    if (atomic_load(&in_call) == 0) { followed[kind_of_last] = __rdtsc() - ended < TAIL_CYCLES; kind_of_last = kind; }
-    atomic_fetch_add(&in_call, 1);
+    if (depth++) return;
+    followed[kind_of_last] = __rdtsc() - ended < TAIL_CYCLES; kind_of_last = kind;
+    atomic_store_explicit(&now.in_call, 1, memory_order_release);
 }
 void hio_end(void) {
-    if (atomic_load(&in_call) == 1) { ended = __rdtsc(); atomic_store(&tail_on, followed[kind_of_last]); }
-    atomic_fetch_sub(&in_call, 1);
+    if (--depth) return;
+    ended = __rdtsc();
+    if (atomic_load_explicit(&now.tail_on, memory_order_relaxed) != followed[kind_of_last]) atomic_store_explicit(&now.tail_on, followed[kind_of_last], memory_order_release);
+    atomic_store_explicit(&now.in_call, 0, memory_order_release);
 }
 unsigned hio_submit(hio_fn fn, void *arg, int pieces) {
     if (nth < 0) start();
