@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(CW_WARPS * 32, 1) combine_wire_kernel(uint8_t 
 #pragma unroll
         for (int it = 0; it < CW_EX / CW_WARPS; it++)
             v[it] = p[it] ? reinterpret_cast<const float4 *>(p[it] + rb * CW_ROWS)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-        pdl_wait(); pdl_trigger();                                     // the scales are weights: read while the down kernel still runs elsewhere
+        pdl_trigger();                                                 // launched plainly (launch.cuh): the down kernel has ended
         int slot[(CW_MAXTOK * TOPK + CW_WARPS * 32 - 1) / (CW_WARPS * 32)];
 #pragma unroll
         for (int it = 0; it < (int)(sizeof slot / sizeof slot[0]); it++) { const int i = tid + it * CW_WARPS * 32; slot[it] = i < npair ? tp[b_begin * TOPK + i] : -1; }
