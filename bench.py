@@ -267,7 +267,7 @@ def main():
     ap.add_argument("--no-decode", action="store_true")
     ap.add_argument("--capture", choices=["prefill", "decode", "attn"], help="a short run for a profiler, no timing and no JSON line: 2 layers, 3 passes of "
                     "one chunk (2048 tokens, or 64 for decode) with plain launches (no graph replay), so that a capture of a few launches of one kernel stays small")
-    ap.add_argument("--zipf", action="store_true", help="skewed routing: a per-expert logit bias from a Zipf(s=1.2) ranking (BASELINE config 4); not the headline line")
+    ap.add_argument("--zipf", action="store_true", help="skewed routing: a per-expert logit bias from a Zipf(s=1.2) ranking; not the headline line")
     args = ap.parse_args()
     rank, local, world = dist_env()
     if args.impl == "reference":

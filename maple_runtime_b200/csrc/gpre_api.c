@@ -841,7 +841,8 @@ int gmoe_post_norm(int L, int nb, float *logits) {
 
 /* ---- page-locking the host's own buffers ---------------------------------------------------------------------------
  * The reference's card path reads and writes the host's hidden-state arrays in place (unified memory, gpu_pre.m:318-385); here they cross
- * PCIe, and from pageable memory that runs at a quarter of the link's rate.  maple.c holds those arrays for the life of the process
+ * PCIe, and pageable ones go through page-locked slots that helper threads fill and empty (hostflow.c); a host with few cores has no helpers, and
+ * one copying thread keeps a third of the link busy.  maple.c holds those arrays for the life of the process
  * (HNB, YB: static).  With the policy on (gpre_pin_policy(1), or GPRE_PIN_HOST=1 in the environment when the library initialises: no
  * change to the host's source), a buffer of 1 MB or more that a reference-shaped call sees a second time at the same address and length
  * is page-locked where it lies (cudaHostRegister) and stays so; the copies then run at the rate of pinned memory.  A registration that

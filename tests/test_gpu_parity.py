@@ -282,7 +282,7 @@ def test_zipf_bias_skewed_load(layers, clib, oracle, weights):
 
 
 def test_full_chunk_2048_properties(layers, oracle, weights):
-    """BASELINE config 3's chunk size on one layer: oracle comparison of the integer stages plus size-independent
+    """A chunk of 2048 tokens on one layer: oracle comparison of the integer stages plus size-independent
     properties (each token in exactly 8 groups, permutation is a bijection, the layer is a function of each token
     alone)."""
     g = layers
