@@ -646,7 +646,10 @@ static int layers_enqueue_ep(int nb, int l0, int nl, const float *bd, int ep) {
         if (e == cudaSuccess && !bad) e = cudaGraphInstantiate(&exec, g, 0);
         if (g) cudaGraphDestroy(g);
         if (bad) return -1;
-        if (e != cudaSuccess) { cudaGetLastError(); return fail("gmoe", "graph capture of the layer loop: %s", cudaGetErrorString(e)); }      /* the next call runs plainly */
+        if (e != cudaSuccess) {      /* no memory for the graph, say: nothing of the capture has run, so this call and later ones run plainly */
+            cudaGetLastError(); k_count_add(-r->launches);
+            return layers_run(nb, l0, nl, bd, ep);
+        }
         r->exec = exec;
     } else k_count_add(r->launches);
     CU("gmoe", cudaGraphLaunch((cudaGraphExec_t)r->exec, S.st));
