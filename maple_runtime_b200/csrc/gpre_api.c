@@ -67,7 +67,7 @@ static struct {
     unsigned *mask; int *err, *h_err;      /* the kernels' error word, in page-locked host memory: the device's and the host's pointer to it */
     MoeTile *tiles_a, *tiles_b;
     ExpertPtrs *tab_call;      /* the used experts of one gpre_moe call */
-    ExpertMaps *maps_seen, *h_maps; int8_t *hq_sorted; TMap4 bmap_hq, bmap_aq;
+    ExpertMaps *maps_seen, *h_maps; int8_t *hq_sorted; float *hqs_sorted; int *hqsum_sorted; TMap4 bmap_hq, bmap_aq;
     /* tensor maps of the experts seen by gpre_moe: on the card (maps_seen), the code pointers of slot i in map_key[i], slots found through map_hash */
     struct MapKey { const uint8_t *gc, *uc, *dc; } *map_key; int *map_hash, map_n, map_sent, map_fresh;
     ExpertPtrs *h_tab;         /* host staging of a layer's pointer table */
@@ -178,7 +178,7 @@ static int init_common(const char *who, int maxtok, int topk) {
     ALLOC(tiles_a, (P / 8 + NEXP) * sizeof(MoeTile)); ALLOC(tiles_b, (P / 8 + NEXP) * sizeof(MoeTile));
     ALLOC(ntiles_a, 16); ALLOC(ntiles_b, 16);
     ALLOC(act, P * FFN * 4); ALLOC(gate, P * FFN * 4); ALLOC(up, P * FFN * 4); ALLOC(aq, P * FFN); ALLOC(aqs, P * 4); ALLOC(aqsum, P * 4); ALLOC(down, P * HID * 4);
-    ALLOC(tab_call, NEXP * sizeof(ExpertPtrs)); ALLOC(maps_seen, MAP_SLOTS * sizeof(ExpertMaps)); ALLOC(hq_sorted, P * HID);
+    ALLOC(tab_call, NEXP * sizeof(ExpertPtrs)); ALLOC(maps_seen, MAP_SLOTS * sizeof(ExpertMaps)); ALLOC(hq_sorted, P * HID); ALLOC(hqs_sorted, P * 8); S.hqsum_sorted = (int *)S.hqs_sorted + P;
     ALLOC(wire, WIRE_BYTES(P)); CU(who, cudaMemset(S.wire, 0, WIRE_BYTES(P))); ALLOC(dsp_call, NEXP * sizeof(void *));
     ALLOC(hA, T * HID * 4); ALLOC(hnorm, T * 4); ALLOC(rpart, (size_t)8 * T * NEXP * 4); ALLOC(flagged, T * 4); ALLOC(nflagged, 16); ALLOC(rdone, T * 4); CU(who, cudaMemset(S.rdone, 0, T * 4));
     CU(who, cudaMemset(S.hA, 0, T * HID * 4)); CU(who, cudaMemset(S.nflagged, 0, 16));
@@ -387,10 +387,13 @@ static void fill_expert_args(ExpertArgs *a, const ExpertPtrs *tab, const ExpertM
     if (use_umma(nb)) { a->tiles = S.tiles_b; a->ntiles = S.ntiles_b; a->max_tiles = nb * TOPK / UMMA_TN + NEXP; }
     else { a->tiles = S.tiles_a; a->ntiles = S.ntiles_a; a->max_tiles = nb * TOPK / tile_tn(nb) + NEXP; if (a->max_tiles > nb * TOPK) a->max_tiles = nb * TOPK; }
     a->hq = S.hq; a->hqs = S.hqs; a->hqsum = S.hqsum; a->act = S.act;
+    if (use_umma(nb)) { a->hqs = S.hqs_sorted; a->hqsum = S.hqsum_sorted; }
     a->aq = S.aq; a->aqs = S.aqs; a->aqsum = S.aqsum; a->down = S.down; a->wire = S.wire; a->wire_cap = S.maxp;
     if (S.keep || use_umma(nb)) { a->gate = S.gate; a->up = S.up; }          /* the tensor-core GEMM always stores gate and up */
     if (S.keep) { a->gu_dots = S.gu_dots; a->dn_dots = S.dn_dots; }
 }
+/* the permute: int8 rows into pair order for the TMA, their scales and code sums with them */
+static void run_gather(int nb) { k_gather_rows(S.st, S.hq, S.hqs, S.hqsum, S.utok, S.hq_sorted, S.hqs_sorted, S.hqsum_sorted, nb * TOPK); }
 static void run_group_l(int nb, int marked, const float *logits);
 static void run_group_m(int nb, int marked) { run_group_l(nb, marked, NULL); }
 /* logits: up to TOPK_IN_MAX tokens, the top-8 comes from them in the same kernel */
@@ -402,7 +405,7 @@ static void run_group_l(int nb, int marked, const float *logits) {
     g.ustart = S.ustart; g.utok = S.utok; g.slot = S.slot; g.tp = S.tp; g.uw = S.uw; g.ecnt = S.ecnt; g.uexp = S.uexp;
     g.tiles_a = S.tiles_a; g.tiles_b = S.tiles_b; g.ntiles_a = S.ntiles_a; g.ntiles_b = S.ntiles_b; g.tn_a = tile_tn(nb); g.tn_b = UMMA_TN;
     k_group(S.st, &g);
-    if (use_umma(nb) && !S.ep_on) k_gather_rows(S.st, S.hq, S.utok, S.hq_sorted, nb * TOPK);   /* the permute: int8 rows into pair order for the TMA */
+    if (use_umma(nb) && !S.ep_on) run_gather(nb);
 }
 static void run_group(int nb) { run_group_m(nb, 0); }
 /* which: 1 gateup, 2 actq, 4 down; dsp: the down-scale pointers the tiles' expert indices name (the combine needs the same) */
@@ -936,7 +939,7 @@ static int grouping_args(const char *who, int nb, int nu) {
     return 0;
 }
 static void run_call_experts(int nb, const float *init, float *out) {
-    if (use_umma(nb)) k_gather_rows(S.st, S.hq, S.utok, S.hq_sorted, nb * TOPK);
+    if (use_umma(nb)) run_gather(nb);
     run_experts(S.tab_call, S.maps_seen, (const float *const *)S.dsp_call, NULL, nb, 7);
     run_combine((const float *const *)S.dsp_call, nb, init, out);
 }
@@ -1046,7 +1049,7 @@ int gmoe_stage(const char *name, int L, int nb) {
     }
     else if (!strcmp(name, "topk")) k_topk(S.st, S.logits, S.top, S.topw, nb);
     else if (!strcmp(name, "group")) run_group(nb);
-    else if (!strcmp(name, "gateup")) { if (use_umma(nb)) k_gather_rows(S.st, S.hq, S.utok, S.hq_sorted, nb * TOPK); run_experts(l->tab, l->maps, (const float *const *)l->dsp, S.ue, nb, 1); }
+    else if (!strcmp(name, "gateup")) { if (use_umma(nb)) run_gather(nb); run_experts(l->tab, l->maps, (const float *const *)l->dsp, S.ue, nb, 1); }
     else if (!strcmp(name, "actq")) run_experts(l->tab, l->maps, (const float *const *)l->dsp, S.ue, nb, 2);
     else if (!strcmp(name, "down")) { if (use_umma(nb)) cudaMemsetAsync(S.wire, 0, WIRE_BYTES((size_t)S.maxp), S.st);   /* a repeated stage must not find the previous run's escape bits */
         run_experts(l->tab, l->maps, (const float *const *)l->dsp, S.ue, nb, 4); }

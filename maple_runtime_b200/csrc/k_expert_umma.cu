@@ -24,18 +24,19 @@
 //
 // Warps (640 threads): 0-7 decode (warp w: tensor-memory lanes 32 (w % 4).., blocks of parity w / 4), 8 weight TMA, 9 B TMA,
 // 10 and 11 MMA issue (one per accumulator half), 12-19 epilogue.
-// What the tensor pipe needs from the issuing warp (measured with one-off probes): a kind::i8 MMA with A in tensor memory issues
-// in ~11 cycles from an elected lane of warp-uniform code (45 from inside a `lane == 0` branch) and executes in N/2 cycles, but a
-// loop iteration that waits on an mbarrier costs the issuing thread ~135 cycles more, whatever it waits for.  So the MMA warp runs
-// its loop with all lanes and elects a lane per instruction; a block (8 MMAs) per wait is enough, because the MMAs themselves run at
-// ~45 cycles each here: at N ~ 72 they are bound by shared-memory bandwidth (both halves read the B tile, the TMA writes it).  The producer side
-// (commit -> decode warps wake -> tcgen05.st -> arrive -> MMA warp wakes) is a chain of several hundred cycles, so the A operand
-// needs more than two stages to keep the pipe fed; tensor memory decides how many:
-// two accumulator pairs (4 x 96 columns), so that an item's epilogue runs under the next item's MMAs, + 2 A stages of 64 columns (one
-// 128-column block of both halves each); more A stages at the price of one accumulator pair measured the same.
-// What bounds it: the hand-overs between these roles, not a unit (2048 tokens, gate+up 49.7 us: DRAM 53%, L2 32%, shared memory 36%, issue 50%, tensor pipe 45% of
-// their peaks).  With all copies, MMAs, decoding and the epilogue taken out the barriers alone take 26.5 us for 7 items of 16 blocks, at 301 tokens as at 2048; any one
-// part taken out saves at most a tenth.  Down: 20 of 39 us for 14 items of 4 blocks, and at 2048 tokens 11 us of epilogue that four blocks do not hide.
+// An MMA is issued by one elected lane of warp-uniform code; a kind::i8 MMA with A in tensor memory executes in N/2 cycles.
+// Instructions in the SM's cache bound these kernels as much as any unit: five roles run side by side on every scheduler, each in code of its own, and what does not fit the
+// instruction cache is fetched again from the L2 side in every round.  The kernels were 72 to 78 KB of code (spin loops unrolled four times at every wait, the
+// copying warps' loops unrolled whole, stage outputs and expert parallelism beside the lean path); they are 26 to 31 KB now, and with nothing else changed a layer of 301 / 843 /
+// 2048 tokens took 93.2 / 116.3 / 163.4 us instead of 97.5 / 119.9 / 168.0.  So: loops over blocks, stages and items stay rolled, one copy of an epilogue piece, a
+// predicated block of MMAs instead of a branch per MMA, and FULL = the variant with stage outputs and expert parallelism.  With the three points below: 92.4 / 114.0 / 162.2.
+// One barrier pair per 128-column block (k_full: the four decode warps that wrote the A stage, and the bytes of the B stage; k_empty: both MMA warps) instead of one per
+// ring: a wait that succeeds at once still costs a warp 100 to 180 cycles here.  A look at the next barrier ahead of time (test_wait) made it slower (92.9 / 114.8 / 163.1): more
+// instructions.  One MMA warp for both halves: 93.2 / 115.3 / 163.5.  Sixteen decode warps, one half each: 96.9 / 121.6 / 173.9, at 72 registers a thread.
+// Tensor memory: three A stages of 64 columns (two: 94.2 / 116.7 / 163.1), and 320 columns which the accumulators of two items share, even items from the low end and odd
+// ones from the high end, 2 N columns each: neighbours of up to 160 pairs (rounded up to 16s) fit beside each other, so that an item's epilogue runs under the next
+// one's MMAs; larger ones wait for each other (acc_place).
+// An item's scales come in pair order (gather_rows_kernel puts them there): through the token index they were a second global read in front of every item.
 // Every mbarrier wait is bounded (umma.cuh): on a timeout the CTA raises args.err, frees tensor memory and returns.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -50,16 +51,15 @@ extern "C" void k_count_add(long n);
 
 #define UM_TN UMMA_TN                /* 96 */
 #define UM_WSTAGES 3                 /* four 128-column blocks each */
-#ifndef UM_NACC
-#define UM_NACC 2                    /* accumulator pairs (2 x 96 columns each): 2 = an item's epilogue runs under the next item's MMAs */
-#endif
-#define UM_NA ((512 - UM_NACC * 2 * UM_TN) / 64)   /* A stages in what is left of tensor memory: one 128-column block of both halves (64 columns) each */
+#define UM_NACC 2                    /* items whose accumulators are in use at a time: an item's epilogue runs under the next item's MMAs */
+#define UM_NA 3                      /* A stages: one 128-column block of both halves (64 columns) each */
+#define UM_ACC (512 - 64 * UM_NA)    /* columns the accumulators share */
 #define UM_BSTAGES 8                 /* B stages in shared memory: one 128-column block each */
 #define UM_WBYTES (256 * 128)
 #define UM_BBYTES (UM_TN * 128)
 
 struct __align__(16) UmShared {
-    uint64_t w_full[UM_WSTAGES], w_empty[UM_WSTAGES], s_full[UM_NA], s_empty[UM_NA], b_full[UM_BSTAGES], b_empty[UM_BSTAGES], acc_full[UM_NACC], acc_empty[UM_NACC];
+    uint64_t w_full[UM_WSTAGES], w_empty[UM_WSTAGES], k_full[UM_BSTAGES], k_empty[UM_BSTAGES], acc_full[UM_NACC], acc_empty[UM_NACC];
     uint32_t tmem_base; int abort_flag;
     __align__(16) float m_qs[8][UM_TN]; __align__(16) int m_qsum[8][UM_TN];      // per epilogue warp: scale and code-sum correction of the tile's tokens
     __align__(16) unsigned long long m_dst[8][UM_TN];                             // expert parallel, down: where each token's compact row lives (a peer's memory)
@@ -69,7 +69,7 @@ __device__ __forceinline__ MoeTile ldcg_tile(const MoeTile *t) {
     const int4 v = __ldcg(reinterpret_cast<const int4 *>(t)); return MoeTile{v.x, v.y, v.z, v.w};
 }
 
-template <int KB, int MODE>
+template <int KB, int MODE, bool FULL>
 __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const __grid_constant__ TMap4 bmap) {
     extern __shared__ __align__(1024) uint8_t um_smem_raw[];
     uint8_t *base = (uint8_t *)(((uintptr_t)um_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -81,8 +81,8 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
     constexpr bool GATEUP = MODE == 0, DENSE = MODE == 2, DOWN = MODE == 1;
     constexpr int NA = UM_NA;
     constexpr int NACC = UM_NACC;
-    constexpr uint32_t ACOL = NACC * 2 * UM_TN;                     // first A column (behind the accumulators)
-    static_assert(ACOL + NA * 64 <= 512, "tensor memory");
+    constexpr uint32_t ACOL = UM_ACC;                               // first A column (behind the accumulators)
+    static_assert(UM_ACC >= 2 * UM_TN && NACC == 2 && NA < UM_BSTAGES, "tensor memory");
     static_assert(KB % 4 == 0, "blocks");
     const int MB = GATEUP ? 4 : (DENSE ? a.dense_mblocks : 8);      // 256-row blocks of the matrix (gate+up: 128 + 128)
     constexpr int NSB = KB / 4;
@@ -92,8 +92,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
         for (int s = 0; s < UM_WSTAGES; s++) { mbar_init(&sh->w_full[s], 1); mbar_init(&sh->w_empty[s], 8); }
         // an A stage is full when its four decode warps have stored it, a B stage when its bytes have landed; both are empty again
         // when both issuing warps' MMAs on them have completed
-        for (int s = 0; s < UM_NA; s++) { mbar_init(&sh->s_full[s], 4); mbar_init(&sh->s_empty[s], 2); }
-        for (int s = 0; s < UM_BSTAGES; s++) { mbar_init(&sh->b_full[s], 1); mbar_init(&sh->b_empty[s], 2); }
+        for (int s = 0; s < UM_BSTAGES; s++) { mbar_init(&sh->k_full[s], 5); mbar_init(&sh->k_empty[s], 2); }
         for (int b = 0; b < NACC; b++) { mbar_init(&sh->acc_full[b], 2); mbar_init(&sh->acc_empty[b], 8); }
         sh->abort_flag = 0; mbar_init_fence();
     }
@@ -107,6 +106,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
     auto maps_of = [&](const MoeTile &t) { return a.maps + (a.call_maps ? t.u : t.ex); };
     auto acquire = [&](const TMap *m) { if (a.call_maps) tma_acquire_map_gpu(m); else tma_acquire_map_sys(m); };
     if (warp < 8) {
+#pragma unroll 1
         for (int i = blockIdx.x + (lane * 8 + warp) * gridDim.x; i < nitems; i += 256 * gridDim.x) {
             const ExpertMaps *e = maps_of(tile_at(i / MB));
             if (GATEUP) { acquire(&e->gate); acquire(&e->up); } else acquire(&e->down);
@@ -124,11 +124,19 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
     pdl_trigger();
     if (DENSE && tid == 0) span_begin(a.span);
 
+    // where item number i of this CTA keeps its accumulators (half 0, then half 1, n2 columns in all); over: they cover columns of the item before it
+    uint32_t acc_prev = 0;
+    auto acc_place = [&](const uint32_t i, const uint32_t n2, bool &over) {
+        over = n2 + acc_prev > (uint32_t)UM_ACC; acc_prev = n2;
+        return i & 1 ? (uint32_t)UM_ACC - n2 : 0u;
+    };
+
     if (warp < 8) {
         // ---------------- decode: this warp's 32 rows of both halves, every second block, from the shared-memory ring ----------------
         const int q4 = warp & 3, par = warp >> 2, R = q4 * 32 + lane;       // R: row inside a half = tensor-memory lane
         const uint32_t a_lane = tb + ((uint32_t)(q4 * 32) << 16) + ACOL;
-        uint32_t wcnt = 0, blk = 0;                                    // blk: blocks handed to the A ring so far (all warps count alike)
+        uint32_t wcnt = 0, blk = 0;                                     // blk: blocks handed to the A ring so far (all warps count alike)
+#pragma unroll 1
         for (int item = blockIdx.x; item < nitems && live; item += gridDim.x) {
 #pragma unroll 1
             for (int sb = 0; sb < NSB && live; sb++, wcnt++, blk += 4) {
@@ -138,7 +146,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
 #pragma unroll
                 for (int qq = 0; qq < 2; qq++) {                         // this warp's two blocks of the weight stage
                     const int q = 2 * qq + par;
-                    const uint32_t b = blk + q, as = b % NA, ap = ((b / NA) & 1) ^ 1;
+                    const uint32_t b = blk + q, as = b % NA, bo = b - NA;      // bo: the block that had the stage before
                     uint32_t r0[32], r1[32];
                     // gate+up and dense: left shifts, which the multiply pipe can take beside the masks; the operand is 64 x code and the epilogue shifts the
                     // sums back, exactly (at most 192 * 127 * 2048 = 5e7).  2048 tokens: gate+up 51.0 -> 49.5 us between events, 4096: 80.7 -> 79.1.  The down
@@ -153,14 +161,14 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
                             for (int j = 0; j < 8; j++) o[sft * 8 + j] = DOWN ? (w[j] >> (2 * sft)) & 0x03030303u : (w[j] << (6 - 2 * sft)) & 0xC0C0C0C0u;
                     };
                     decode(wr0, r0); decode(wr1, r1);                     // both halves are ready before the stage is asked for
-                    if (!mbar_wait(&sh->s_empty[as], ap, abortp)) { live = false; break; }
+                    if (b >= NA && !mbar_wait(&sh->k_empty[bo % UM_BSTAGES], (bo / UM_BSTAGES) & 1, abortp)) { live = false; break; }
                     tc_fence_after();
                     tmem_st32(a_lane + as * 64, r0);
                     tmem_st32(a_lane + as * 64 + 32, r1);
                     tmem_st_wait();
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&sh->s_full[as]);
+                    if (lane == 0) mbar_arrive(&sh->k_full[b % UM_BSTAGES]);
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sh->w_empty[ws]);
@@ -171,6 +179,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
         if (lane == 0) {
             uint32_t wcnt = 0;
             MoeTile tnext = blockIdx.x < nitems ? tile_at(blockIdx.x / MB) : MoeTile{0, 0, 0, 0};      // one item ahead: no load latency at an item's start
+#pragma unroll 1
             for (int item = blockIdx.x; item < nitems && live; item += gridDim.x) {
                 const MoeTile tile = tnext;
                 if (item + (int)gridDim.x < nitems) {
@@ -180,6 +189,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
                 }
                 const int mb = item % MB;
                 const ExpertMaps *em = maps_of(tile);
+#pragma unroll 1
                 for (int sb = 0; sb < NSB && live; sb++, wcnt++) {
                     const int ws = wcnt % UM_WSTAGES;
                     if (!mbar_wait(&sh->w_empty[ws], ((wcnt / UM_WSTAGES) & 1) ^ 1, abortp)) { live = false; break; }
@@ -200,16 +210,18 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
         if (lane == 0) {
             uint32_t bcnt = 0;
             MoeTile tnext = blockIdx.x < nitems ? tile_at(blockIdx.x / MB) : MoeTile{0, 0, 0, 0};
+#pragma unroll 1
             for (int item = blockIdx.x; item < nitems && live; item += gridDim.x) {
                 const MoeTile tile = tnext;
                 if (item + (int)gridDim.x < nitems) tnext = tile_at((item + gridDim.x) / MB);
                 // only as many rows as the tile has pairs, in steps of 32 (the MMA reads (cnt + 15) & ~15 <= that many)
                 const int bi = tile.cnt > 0 ? (tile.cnt - 1) >> 5 : 0;
+#pragma unroll 1
                 for (int kb = 0; kb < KB && live; kb++, bcnt++) {
                     const int s = bcnt % UM_BSTAGES;
-                    if (!mbar_wait(&sh->b_empty[s], ((bcnt / UM_BSTAGES) & 1) ^ 1, abortp)) { live = false; break; }
-                    mbar_expect_tx(&sh->b_full[s], 128 * 32 * (bi + 1));
-                    tma_load_2d(smem_u32(bsm + s * UM_BBYTES), &bmap.m[bi], kb * 128, tile.p0, &sh->b_full[s]);
+                    if (!mbar_wait(&sh->k_empty[s], ((bcnt / UM_BSTAGES) & 1) ^ 1, abortp)) { live = false; break; }
+                    mbar_expect_tx(&sh->k_full[s], 128 * 32 * (bi + 1));
+                    tma_load_2d(smem_u32(bsm + s * UM_BBYTES), &bmap.m[bi], kb * 128, tile.p0, &sh->k_full[s]);
                 }
             }
         }
@@ -218,32 +230,28 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
         // MMAs keep the tensor pipe busy.  The whole warp walks the loop and waits; one elected lane issues and commits ----------------
         const uint32_t h = warp - 10;
         const uint64_t bdesc0 = smem_desc_k128(__shfl_sync(0xffffffffu, smem_u32(bsm), 0), 0);
-        const uint32_t sfull0 = smem_u32(&sh->s_full[0]), sempty0 = smem_u32(&sh->s_empty[0]);
-        const uint32_t bfull0 = smem_u32(&sh->b_full[0]), bempty0 = smem_u32(&sh->b_empty[0]);
-        uint32_t as = 0, ap = 0, bs = 0, bp = 0, icnt = 0;
+        const uint32_t kfull0 = smem_u32(&sh->k_full[0]), kempty0 = smem_u32(&sh->k_empty[0]);
+        uint32_t as = 0, bs = 0, bp = 0, icnt = 0;
         int cnt_next = blockIdx.x < nitems ? tile_at(blockIdx.x / MB).cnt : 0;
+#pragma unroll 1
         for (int item = blockIdx.x; item < nitems && live; item += gridDim.x, icnt++) {
             const int cnt = __shfl_sync(0xffffffffu, cnt_next, 0);
             if (item + (int)gridDim.x < nitems) cnt_next = tile_at((item + gridDim.x) / MB).cnt;
-            const uint32_t idesc = idesc_i8_u8s8((uint32_t)((cnt + 15) & ~15));
-            const uint32_t buf = icnt % NACC, d = tb + buf * (2 * UM_TN) + h * UM_TN;
+            const uint32_t N = (uint32_t)((cnt + 15) & ~15), idesc = idesc_i8_u8s8(N);
+            bool over;
+            const uint32_t buf = icnt % NACC, d = tb + acc_place(icnt, 2 * N, over) + h * N;
             if (!mbar_wait(&sh->acc_empty[buf], ((icnt / NACC) & 1) ^ 1, abortp)) { live = false; break; }
+            if (over && icnt && !mbar_wait(&sh->acc_empty[buf ^ 1], ((icnt - 1) / NACC) & 1, abortp)) { live = false; break; }
             tc_fence_after();
 #pragma unroll 1
             for (int kb = 0; kb < KB; kb++) {
-                if (!mbar_wait_addr(bfull0 + bs * 8, bp, abortp) || !mbar_wait_addr(sfull0 + as * 8, ap, abortp)) { live = false; break; }
+                if (!mbar_wait_addr(kfull0 + bs * 8, bp, abortp)) { live = false; break; }
                 tc_fence_after();
-                const uint32_t acol = tb + ACOL + as * 64 + h * 32;
+                const uint32_t acol = tb + ACOL + as * 64 + h * 32, kb_empty = kempty0 + bs * 8;
                 const uint64_t bd = bdesc0 + (uint64_t)(bs * (UM_BBYTES >> 4));
-                // one election per instruction: a single predicated MMA stays in warp-uniform code
-                if (elect_one()) umma_i8_ts(d, acol, bd, idesc, kb != 0);
-                if (elect_one()) umma_i8_ts(d, acol + 8, bd + 2, idesc, 1);
-                if (elect_one()) umma_i8_ts(d, acol + 16, bd + 4, idesc, 1);
-                if (elect_one()) umma_i8_ts(d, acol + 24, bd + 6, idesc, 1);
-                if (elect_one()) umma_commit_addr(sempty0 + as * 8);
-                if (elect_one()) umma_commit_addr(bempty0 + bs * 8);
-                if (++as == NA) { as = 0; ap ^= 1; }
+                if (++as == NA) as = 0;
                 if (++bs == UM_BSTAGES) { bs = 0; bp ^= 1; }
+                umma_i8_block(d, acol, bd, idesc, kb != 0, kb_empty);
             }
             if (live && elect_one()) umma_commit(&sh->acc_full[buf]);
             __syncwarp();
@@ -252,7 +260,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
         // ---------------- epilogue: lane = weight row, columns = tokens; warps 12-15 take the even 16-column pieces, 16-19 the odd ----------------
         const int ew = warp - 12, q4 = warp & 3, half = ew >> 2, row = q4 * 32 + lane;   // a warp reaches the tensor-memory lanes 32 (warp % 4) ..
         uint32_t icnt = 0;
-        // An item's header is a chain tile -> (token of the pair ->) scale and code sum of its tokens, and tile -> pointer table -> row
+        // An item's header is a chain tile -> scale and code sum of its tokens, and tile -> pointer table -> row
         // scales: the tile is read two items ahead, the pointer table and the tokens' values one item ahead (into registers; they go
         // to shared memory when the item starts), so that an item starts without a dependent global read in front of it.
         const int stride = gridDim.x;
@@ -264,10 +272,10 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
         auto header_load = [&](const MoeTile &t) {      // the values of tokens lane, lane + 32, lane + 64 of tile t (clamped to its pairs)
 #pragma unroll
             for (int i = 0; i < HN; i++) {
-                const int n = lane + 32 * i, pair = t.p0 + (n < t.cnt ? n : 0), tk = (GATEUP && a.ptok) ? a.ptok[pair] : pair;
-                h_qs[i] = GATEUP ? a.hqs[tk] : a.aqs[tk];
-                h_qsum[i] = GATEUP ? a.hqsum[tk] : (DENSE ? a.aqsum[tk] : 32768 - a.aqsum[tk]);
-                if (DOWN && a.rx_src) { const int2 sp = a.rx_src[pair]; h_dst[i] = (unsigned long long)(uintptr_t)(a.peer_wire[sp.x] + (size_t)sp.y * WIRE_PITCH); }
+                const int n = lane + 32 * i, pair = t.p0 + (n < t.cnt ? n : 0);
+                h_qs[i] = GATEUP ? a.hqs[pair] : a.aqs[pair];
+                h_qsum[i] = GATEUP ? a.hqsum[pair] : (DENSE ? a.aqsum[pair] : 32768 - a.aqsum[pair]);
+                if (DOWN && FULL && a.rx_src) { const int2 sp = a.rx_src[pair]; h_dst[i] = (unsigned long long)(uintptr_t)(a.peer_wire[sp.x] + (size_t)sp.y * WIRE_PITCH); }
             }
         };
         if (blockIdx.x < nitems) header_load(t1);
@@ -278,6 +286,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
             s0n = GATEUP ? e.gs[r] : (DENSE ? e.ds[r] : 0.0f); s1n = GATEUP ? e.us[r] : (DENSE ? e.ds[r + 1] : 0.0f);
         };
         if (blockIdx.x < nitems) scales_load(ep1, blockIdx.x);
+#pragma unroll 1
         for (int item = blockIdx.x; item < nitems && live; item += stride, icnt++) {
             const MoeTile tile = t1;
             const int mb = item % MB, cnt = tile.cnt, N = (cnt + 15) & ~15;
@@ -288,7 +297,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
 #pragma unroll
             for (int i = 0; i < HN; i++) {
                 sh->m_qs[ew][lane + 32 * i] = h_qs[i]; sh->m_qsum[ew][lane + 32 * i] = h_qsum[i];
-                if (DOWN && a.rx_src) sh->m_dst[ew][lane + 32 * i] = h_dst[i];
+                if (DOWN && FULL && a.rx_src) sh->m_dst[ew][lane + 32 * i] = h_dst[i];
             }
             __syncwarp();
             t1 = t2; ep1 = a.tab[t1.ex];
@@ -296,7 +305,8 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
             if (item + stride < nitems) header_load(t1);                     // in flight while this item's pieces are worked on
             if (!mbar_wait(&sh->acc_full[buf], (icnt / NACC) & 1, abortp)) { live = false; break; }
             tc_fence_after();
-            const uint32_t d_lane = tb + ((uint32_t)(q4 * 32) << 16) + buf * (2 * UM_TN);
+            bool over;
+            const uint32_t d_lane = tb + ((uint32_t)(q4 * 32) << 16) + acc_place(icnt, 2 * (uint32_t)N, over);
             auto release = [&]() { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(&sh->acc_empty[buf]); };
             auto piece = [&](const int c0, uint32_t (&v0)[16], uint32_t (&v1)[16]) {
                 const int lim = cnt - c0;                                 // tokens of this piece that exist
@@ -327,7 +337,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
                     float *gp = a.gate + (size_t)(tile.p0 + c0) * 512 + r0, *up_ = a.up + (size_t)(tile.p0 + c0) * 512 + r0;
 #pragma unroll
                     for (int j = 0; j < 16; j++) if (j < lim) { gp[j * 512] = o0[j]; up_[j * 512] = o1[j]; }
-                    if (a.gu_dots) {
+                    if (FULL && a.gu_dots) {
                         int *dp = a.gu_dots + (size_t)(tile.p0 + c0) * 1024 + r0;
 #pragma unroll
                         for (int j = 0; j < 16; j++) if (j < lim) { dp[j * 1024] = (int)v0[j]; dp[j * 1024 + 512] = (int)v1[j]; }
@@ -336,19 +346,26 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
             };
             // down: (dot + 32768) of this thread's two rows in one 32-bit word per token (the scales are applied where the rows are
             // combined); cd = two more bits per value, nonzero only when a value needs more than 16 bits (|dot| >= 32768)
-            auto pack = [&](const int c0, const uint32_t (&v0)[16], const uint32_t (&v1)[16], uint32_t (&pk)[16], unsigned long long &cd) {
+            auto pack = [&](const int c0, uint32_t (&v0)[16], uint32_t (&v1)[16], uint32_t (&pk)[16], unsigned long long &cd) {
                 const int4 *qsv = reinterpret_cast<const int4 *>(&sh->m_qsum[ew][c0]);
-                cd = 0ull;
+                uint32_t high = 0u;
 #pragma unroll
                 for (int g4 = 0; g4 < 4; g4++) {
                     const int4 qs4 = qsv[g4]; const int bq[4] = {qs4.x, qs4.y, qs4.z, qs4.w};       // 32768 - qsum
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
                         const int j = g4 * 4 + k;
-                        const uint32_t x0 = v0[j] + (uint32_t)bq[k], x1 = v1[j] + (uint32_t)bq[k];
-                        pk[j] = __byte_perm(x0, x1, 0x5410);
-                        cd |= (unsigned long long)(((x0 >> 16) & 3u) | (((x1 >> 16) & 3u) << 2)) << (4 * j);
+                        v0[j] += (uint32_t)bq[k]; v1[j] += (uint32_t)bq[k];
+                        pk[j] = __byte_perm(v0[j], v1[j], 0x5410);
+                        high |= v0[j] | v1[j];
                     }
+                }
+                // the two more bits are looked at only where the warp has one that is set (or a stage comparison wants the sums): per token and thread that is
+                // four instructions instead of thirteen
+                cd = 0ull;
+                if (__any_sync(0xffffffffu, high >> 16) || (FULL && a.dn_dots)) {
+#pragma unroll
+                    for (int j = 0; j < 16; j++) cd |= (unsigned long long)(((v0[j] >> 16) & 3u) | (((v1[j] >> 16) & 3u) << 2)) << (4 * j);
                 }
             };
             auto store = [&](const int c0, const uint32_t (&pk)[16], const unsigned long long cd) {
@@ -356,7 +373,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
                 const bool esc = __any_sync(0xffffffffu, cd != 0ull);
                 const size_t rec0 = (size_t)a.wire_cap * WIRE_PITCH;            // the records sit behind the rows
                 const bool recw = mb == 0 && q4 == 0 && lane < 16 && lane < lim; // one warp per piece writes the tokens' records
-                if (!a.rx_src) {
+                if (!FULL || !a.rx_src) {
                     uint8_t *rowp = a.wire + (size_t)(tile.p0 + c0) * WIRE_PITCH;
                     uint32_t *dp = reinterpret_cast<uint32_t *>(rowp) + (r0 >> 1);
 #pragma unroll
@@ -398,7 +415,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
                         }
                     }
                 }
-                if (a.dn_dots) {      // (dot + 32768) again from the 16 stored bits and the two escape bits: 0, +65536 or -65536 on top
+                if (FULL && a.dn_dots) {      // (dot + 32768) again from the 16 stored bits and the two escape bits: 0, +65536 or -65536 on top
                     int *ip = a.dn_dots + (size_t)(tile.p0 + c0) * 2048 + r0;
 #pragma unroll
                     for (int j = 0; j < 16; j++) if (j < lim) {
@@ -418,28 +435,19 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
                 for (int k = 0; k < np; k++) {
                     uint32_t v0[16], v1[16], pk[16]; unsigned long long cd;
                     const int c0 = half * 16 + 32 * k;
-                    tmem_ld16(d_lane + c0, v0); tmem_ld16(d_lane + UM_TN + c0, v1);
+                    tmem_ld16(d_lane + c0, v0); tmem_ld16(d_lane + N + c0, v1);
                     tmem_ld_wait();
                     if (k == np - 1) release();
                     pack(c0, v0, v1, pk, cd);
                     store(c0, pk, cd);
                 }
             } else {
-                // the last two pieces are copied out together and the accumulators handed back before their arithmetic (all of them
-                // when there are at most two)
                 if (np == 0) release();
                 int c0 = half * 16;
+#pragma unroll 1
                 for (int k = 0; k < np; k++, c0 += 32) {
                     uint32_t v0[16], v1[16];
-                    tmem_ld16(d_lane + c0, v0); tmem_ld16(d_lane + UM_TN + c0, v1);
-                    if (np - k == 2) {
-                        uint32_t w0[16], w1[16];
-                        tmem_ld16(d_lane + c0 + 32, w0); tmem_ld16(d_lane + UM_TN + c0 + 32, w1);
-                        tmem_ld_wait();
-                        release();
-                        piece(c0, v0, v1); piece(c0 + 32, w0, w1);
-                        break;
-                    }
+                    tmem_ld16(d_lane + c0, v0); tmem_ld16(d_lane + N + c0, v1);
                     tmem_ld_wait();
                     if (np - k == 1) release();
                     piece(c0, v0, v1);
@@ -459,25 +467,26 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
     }
 }
 
-template <int KB, int MODE>
+template <int KB, int MODE, bool FULL>
 static void launch(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) {
     const size_t smem = (size_t)UM_WSTAGES * UM_WBYTES + UM_BSTAGES * UM_BBYTES + 1024;
     static int sms = 0;
     if (!sms) {
         int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(expert_umma_kernel<KB, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(expert_umma_kernel<KB, MODE, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     }
-    if (a->fresh_maps || MODE == 2) launch_k(expert_umma_kernel<KB, MODE>, sms, 640, smem, st, *a, *bmap);
-    else launch_pdl(expert_umma_kernel<KB, MODE>, sms, 640, smem, st, *a, *bmap);
+    if (a->fresh_maps || MODE == 2) launch_k(expert_umma_kernel<KB, MODE, FULL>, sms, 640, smem, st, *a, *bmap);
+    else launch_pdl(expert_umma_kernel<KB, MODE, FULL>, sms, 640, smem, st, *a, *bmap);
     k_count_add(1);
 }
-extern "C" void k_gateup_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->max_tiles > 0) launch<16, 0>(st, a, bmap); }
-extern "C" void k_down_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->max_tiles > 0) launch<4, 1>(st, a, bmap); }
+extern "C" void k_gateup_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->max_tiles > 0) { if (a->gu_dots) launch<16, 0, true>(st, a, bmap); else launch<16, 0, false>(st, a, bmap); } }
+extern "C" void k_down_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->max_tiles > 0) { if (a->dn_dots || a->rx_src) launch<4, 1, true>(st, a, bmap); else launch<4, 1, false>(st, a, bmap); } }
 /* dense projections: tab[ex].ds / maps[ex].down of a matrix of 256 * a->dense_mblocks rows x 2048 columns, B rows = the tokens' int8 rows */
-extern "C" void k_dense_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->dense_n > 0) launch<16, 2>(st, a, bmap); }
+extern "C" void k_dense_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->dense_n > 0) launch<16, 2, false>(st, a, bmap); }
 
 // ---- rows of the per-token int8 matrix copied into pair (expert-grouped) order: the B operand the TMA can tile ----
-__global__ void __launch_bounds__(256) gather_rows_kernel(const int8_t *__restrict__ src, const int *__restrict__ rows, int8_t *__restrict__ dst, int np) {
+__global__ void __launch_bounds__(256) gather_rows_kernel(const int8_t *__restrict__ src, const float *__restrict__ qs, const int *__restrict__ qsum, const int *__restrict__ rows,
+                                                          int8_t *__restrict__ dst, float *__restrict__ dqs, int *__restrict__ dqsum, int np) {
     pdl_wait(); pdl_trigger();
     // 8 pairs per CTA: each thread moves one 16-byte piece of four rows, all four loads in flight together
     const int p0 = blockIdx.x * 8 + (threadIdx.x >> 7) * 4, c = threadIdx.x & 127;
@@ -488,9 +497,11 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const int8_t *__restri
     for (int k = 0; k < 4; k++) v[k] = reinterpret_cast<const uint4 *>(src + (size_t)r[k] * 2048)[c];
 #pragma unroll
     for (int k = 0; k < 4; k++) if (p0 + k < np) reinterpret_cast<uint4 *>(dst + (size_t)(p0 + k) * 2048)[c] = v[k];
+#pragma unroll
+    for (int k = 0; k < 4; k++) if (c == 32 * k && p0 + k < np) { dqs[p0 + k] = qs[r[k]]; dqsum[p0 + k] = qsum[r[k]]; }
 }
-extern "C" void k_gather_rows(cudaStream_t st, const int8_t *src, const int *rows, int8_t *dst, int np) {
+extern "C" void k_gather_rows(cudaStream_t st, const int8_t *src, const float *qs, const int *qsum, const int *rows, int8_t *dst, float *dqs, int *dqsum, int np) {
     if (np <= 0) return;
-    launch_pdl(gather_rows_kernel, (np + 7) / 8, 256, 0, st, src, rows, dst, np);
+    launch_pdl(gather_rows_kernel, (np + 7) / 8, 256, 0, st, src, qs, qsum, rows, dst, dqs, dqsum, np);
     k_count_add(1);
 }

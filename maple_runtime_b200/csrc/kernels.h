@@ -21,9 +21,9 @@ typedef struct {
     const ExpertMaps *maps;  /* same indexing; only the tcgen05 kernels read it */
     const int *ue;
     const MoeTile *tiles; const int *ntiles; int max_tiles;
-    const int *ptok;         /* [np] token of each pair; NULL = the per-token arrays below are already in pair order (expert parallel) */
+    const int *ptok;         /* [np] token of each pair; NULL = the per-token arrays below are already in pair order (as the tcgen05 kernels take them) */
     /* gate+up inputs */
-    const int8_t *hq; const float *hqs; const int *hqsum;          /* per token */
+    const int8_t *hq; const float *hqs; const int *hqsum;          /* per token; k_gateup_umma: in pair order */
     float *act;              /* [np][512] */
     /* down inputs */
     const int8_t *aq; const float *aqs; const int *aqsum;          /* per pair */
@@ -121,8 +121,8 @@ void k_down_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap);
 /* a dense matrix (rows a multiple of 256, 2048 columns) on the same kernel: maps[ex].down = its 3-D map (even / odd rows), tab[ex].ds = row
  * scales, bmap over the tokens' int8 rows, tiles of up to UMMA_TN tokens; fp32 results to down[token * down_stride + row] */
 void k_dense_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap);
-/* dst[pair] = src[rows[pair]]: 2048-byte int8 rows put into pair (expert-grouped) order */
-void k_gather_rows(cudaStream_t st, const int8_t *src, const int *rows, int8_t *dst, int np);
+/* dst[pair] = src[rows[pair]]: 2048-byte int8 rows put into pair (expert-grouped) order; their scales and code sums likewise */
+void k_gather_rows(cudaStream_t st, const int8_t *src, const float *qs, const int *qsum, const int *rows, int8_t *dst, float *dqs, int *dqsum, int np);
 
 /* ---- the head of the attention half (k_attn_prep.cu): q/k RMS norm, half-rotary embedding, fp16 keys and values.  qkv [nb][3072]
  * = q 2048 | k 512 | v 512; pos [nb]; qn, kn [128] fp32; cs [cs_positions][32][2] (cos, sin); q [nb][2048] fp32; kc, vc [nb][512] fp16 */
