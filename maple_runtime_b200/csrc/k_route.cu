@@ -526,57 +526,63 @@ extern "C" void k_actq(cudaStream_t st, const float *act, int8_t *aq, float *aqs
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// SiLU*up + int8 in one pass (maple.c:825-832) for the tensor-core path, whose GEMM stores gate and up: one warp per pair.  EXACT evaluates
-// every element with the libm-equal expf in double (dev_math.cuh) and can also store the fp32 activations (act, optional) for stage
-// comparisons; the other variant is silu_row.cuh.  The results are the reference's bits in both.
+// SiLU*up + int8 in one pass (maple.c:825-832) for the tensor-core path, whose GEMM stores gate and up: one warp per pair (silu_row.cuh).  The results are
+// the reference's bits, as those of the kernel below that evaluates every element exactly.
+// Bound by instruction issue (800 per pair at first, 60% of the slots used) beside 75 MB per 2048 tokens: the bytes of a row are cut out of the rounding sums with
+// byte permutes and added with dp4a, and the distance to a rounding boundary is one running maximum per lane that is taken apart only where it is near.  CTAs of two warps
+// instead of eight, so that an SM takes new rows as each pair of warps ends: between events 22.1 -> 20.1 us at 2048 tokens, 14.3 -> 12.5 at 843.
+// (Two rows per warp, whose exact evaluations share a pass, at 122 registers: 24.6.  Rows brought ahead into shared memory by resident warps, 24 per SM: 21.3.)
 // ------------------------------------------------------------------------------------------------------------
-template <bool EXACT>
-__global__ void __launch_bounds__(256, 4) silu_quant_kernel(const float *__restrict__ gate, const float *__restrict__ up, float *__restrict__ act,
+__global__ void __launch_bounds__(64, 16) silu_quant_kernel(const float *__restrict__ gate, const float *__restrict__ up,
                                                          int8_t *__restrict__ aq, float *__restrict__ aqs, int *__restrict__ aqsum, int np, const int *__restrict__ np_dev) {
     __shared__ unsigned long long tab[32];
     if (threadIdx.x < 32) tab[threadIdx.x] = DEV_EXP_TAB[threadIdx.x];
     __syncthreads();
     pdl_wait(); pdl_trigger();
     if (np_dev) np = min(np, *np_dev);
+    const int lane = threadIdx.x & 31, a = blockIdx.x * 2 + (threadIdx.x >> 5);
+    if (a >= np) return;
+    float s; int tot; uint32_t pk[4];
+    silu_quant_row(gate + (size_t)a * FFN, up + (size_t)a * FFN, tab, lane, pk, s, tot);
+#pragma unroll
+    for (int i = 0; i < 4; i++) reinterpret_cast<uint32_t *>(aq + (size_t)a * FFN)[32 * i + lane] = pk[i];
+    if (lane == 0) { aqs[a] = s; aqsum[a] = tot; }
+}
+// Every element evaluated exactly with the libm-equal expf in double (dev_math.cuh), and the fp32 activations stored (stage comparisons).
+__global__ void __launch_bounds__(256, 4) silu_quant_exact_kernel(const float *__restrict__ gate, const float *__restrict__ up, float *__restrict__ act,
+                                                         int8_t *__restrict__ aq, float *__restrict__ aqs, int *__restrict__ aqsum, int np, const int *__restrict__ np_dev) {
+    __shared__ unsigned long long tab[32];
+    if (threadIdx.x < 32) tab[threadIdx.x] = DEV_EXP_TAB[threadIdx.x];
+    __syncthreads();
+    if (np_dev) np = min(np, *np_dev);
     const int lane = threadIdx.x & 31, a = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (a >= np) return;
-    const float4 *gr = reinterpret_cast<const float4 *>(gate + (size_t)a * FFN) + lane;
-    const float4 *ur = reinterpret_cast<const float4 *>(up + (size_t)a * FFN) + lane;
-    float4 g4[4], u4[4]; float s; int tot; uint32_t pk[4] = {0, 0, 0, 0};
+    const float4 *gr = reinterpret_cast<const float4 *>(gate + (size_t)a * FFN) + lane, *ur = reinterpret_cast<const float4 *>(up + (size_t)a * FFN) + lane;
+    float4 *o = reinterpret_cast<float4 *>(act + (size_t)a * FFN) + lane;
+    float v[16], mx = 0.0f; int tot = 0; uint32_t pk[4] = {0, 0, 0, 0};
 #pragma unroll
-    for (int i = 0; i < 4; i++) { g4[i] = gr[32 * i]; u4[i] = ur[32 * i]; }
-    if (EXACT) {
-        float gv[16], uv[16], v[16], mx = 0.0f;
+    for (int i = 0; i < 4; i++) {
+        const float4 g = gr[32 * i], u = ur[32 * i];
+        v[4 * i] = dev_silu_mul_tab(g.x, u.x, tab); v[4 * i + 1] = dev_silu_mul_tab(g.y, u.y, tab); v[4 * i + 2] = dev_silu_mul_tab(g.z, u.z, tab); v[4 * i + 3] = dev_silu_mul_tab(g.w, u.w, tab);
+        o[32 * i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    }
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            gv[4 * i] = g4[i].x; gv[4 * i + 1] = g4[i].y; gv[4 * i + 2] = g4[i].z; gv[4 * i + 3] = g4[i].w;
-            uv[4 * i] = u4[i].x; uv[4 * i + 1] = u4[i].y; uv[4 * i + 2] = u4[i].z; uv[4 * i + 3] = u4[i].w;
-        }
+    for (int i = 0; i < 16; i++) mx = fmaxf(mx, fabsf(v[i]));
 #pragma unroll
-        for (int i = 0; i < 16; i++) { v[i] = dev_silu_mul_tab(gv[i], uv[i], tab); mx = fmaxf(mx, fabsf(v[i])); }
-        if (act) {
-            float4 *o = reinterpret_cast<float4 *>(act + (size_t)a * FFN) + lane;
+    for (int i = 16; i; i >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, i));
+    const float s = mx > 0.0f ? __fdiv_rn(mx, 127.0f) : 1.0f, inv = __fdiv_rn(1.0f, s);
 #pragma unroll
-            for (int i = 0; i < 4; i++) o[32 * i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-        }
+    for (int i = 0; i < 16; i++) { const int qi = __float2int_rn(__fmul_rn(v[i], inv)); tot += qi; pk[i >> 2] |= (uint32_t)(qi & 0xFF) << (8 * (i & 3)); }
 #pragma unroll
-        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        s = mx > 0.0f ? __fdiv_rn(mx, 127.0f) : 1.0f;
-        const float inv = __fdiv_rn(1.0f, s);
-        tot = 0;
-#pragma unroll
-        for (int i = 0; i < 16; i++) { int qi = __float2int_rn(__fmul_rn(v[i], inv)); tot += qi; pk[i >> 2] |= (uint32_t)(qi & 0xFF) << (8 * (i & 3)); }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    } else silu_quant_row(g4, u4, gate + (size_t)a * FFN, up + (size_t)a * FFN, tab, lane, pk, s, tot);
+    for (int i = 16; i; i >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, i);
 #pragma unroll
     for (int i = 0; i < 4; i++) reinterpret_cast<uint32_t *>(aq + (size_t)a * FFN)[32 * i + lane] = pk[i];
     if (lane == 0) { aqs[a] = s; aqsum[a] = tot; }
 }
 extern "C" void k_silu_quant(cudaStream_t st, const float *gate, const float *up, float *act, int8_t *aq, float *aqs, int *aqsum, int np, const int *np_dev) {
     if (np <= 0) return;
-    if (act) launch_k(silu_quant_kernel<true>, (np + 7) / 8, 256, 0, st, gate, up, act, aq, aqs, aqsum, np, np_dev);
-    else launch_k(silu_quant_kernel<false>, (np + 7) / 8, 256, 0, st, gate, up, (float *)NULL, aq, aqs, aqsum, np, np_dev);
+    if (act) launch_k(silu_quant_exact_kernel, (np + 7) / 8, 256, 0, st, gate, up, act, aq, aqs, aqsum, np, np_dev);
+    else launch_k(silu_quant_kernel, (np + 1) / 2, 64, 0, st, gate, up, aq, aqs, aqsum, np, np_dev);
     g_launches++;
 }
 
