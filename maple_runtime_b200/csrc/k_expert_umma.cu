@@ -36,6 +36,8 @@
 // Tensor memory: three A stages of 64 columns (two: 94.2 / 116.7 / 163.1), and 320 columns which the accumulators of two items share, even items from the low end and odd
 // ones from the high end, 2 N columns each: neighbours of up to 160 pairs (rounded up to 16s) fit beside each other, so that an item's epilogue runs under the next
 // one's MMAs; larger ones wait for each other (acc_place).
+// The codes are read once per tile: their copies say so to the L2 (evict_first), which then still holds the rows that come in, the results and what the next kernels read
+// when they are asked for: a layer of 301 / 511 / 843 / 2048 tokens 92.1 / 104.4 / 113.8 / 159.8 -> 88.1 / 99.6 / 111.0 / 157.4 us.
 // An item's scales come in pair order (gather_rows_kernel puts them there): through the token index they were a second global read in front of every item.
 // Every mbarrier wait is bounded (umma.cuh): on a timeout the CTA raises args.err, frees tensor memory and returns.
 #include <cuda_runtime.h>
@@ -177,7 +179,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
     } else if (warp == 8) {
         // ---------------- weight TMA (one lane): per stage the 128 rows of half 0 and the 128 of half 1, 512 columns ----------------
         if (lane == 0) {
-            uint32_t wcnt = 0;
+            uint32_t wcnt = 0; const uint64_t once = l2_evict_first();
             MoeTile tnext = blockIdx.x < nitems ? tile_at(blockIdx.x / MB) : MoeTile{0, 0, 0, 0};      // one item ahead: no load latency at an item's start
 #pragma unroll 1
             for (int item = blockIdx.x; item < nitems && live; item += gridDim.x) {
@@ -196,11 +198,11 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
                     const uint32_t dst = smem_u32(wsm + ws * UM_WBYTES);
                     mbar_expect_tx(&sh->w_full[ws], UM_WBYTES);
                     if (GATEUP) {
-                        tma_load_2d(dst, &em->gate, sb * 128, mb * 128, &sh->w_full[ws]);
-                        tma_load_2d(dst + 128 * 128, &em->up, sb * 128, mb * 128, &sh->w_full[ws]);
+                        tma_load_2d_once(dst, &em->gate, sb * 128, mb * 128, &sh->w_full[ws], once);
+                        tma_load_2d_once(dst + 128 * 128, &em->up, sb * 128, mb * 128, &sh->w_full[ws], once);
                     } else {
-                        tma_load_3d(dst, &em->down, sb * 128, 0, mb * 128, &sh->w_full[ws]);             // the even rows of the 256-row block
-                        tma_load_3d(dst + 128 * 128, &em->down, sb * 128, 1, mb * 128, &sh->w_full[ws]);   // the odd rows
+                        tma_load_3d_once(dst, &em->down, sb * 128, 0, mb * 128, &sh->w_full[ws], once);             // the even rows of the 256-row block
+                        tma_load_3d_once(dst + 128 * 128, &em->down, sb * 128, 1, mb * 128, &sh->w_full[ws], once);   // the odd rows
                     }
                 }
             }
