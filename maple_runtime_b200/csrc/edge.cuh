@@ -52,6 +52,7 @@ __device__ __forceinline__ void edge_token(const int c, const float *down, const
         s_term[(warp + 8 * k) * 32 + lane] = ((double)v[k].x * (double)v[k].x + (double)v[k].y * (double)v[k].y) + ((double)v[k].z * (double)v[k].z + (double)v[k].w * (double)v[k].w);
     }
     __syncthreads();
+    if (WIRE) l2_discard(ew.wire + (size_t)tp[c * TOPK + warp] * WIRE_PITCH + lane * 128);      // the row of pair `warp`: 32 lines, all read (not its escape plane)
     if (warp == 0) {
         double ss = 0.0;
 #pragma unroll

@@ -422,7 +422,7 @@ static void run_experts(const ExpertPtrs *tab, const ExpertMaps *maps, const flo
     if (fuse_q) { a.act_for_down = S.act; a.aq_out = S.aq; a.aqs_out = S.aqs; a.aqsum_out = S.aqsum; }
     if ((which & 2) && !fuse_q) {
         prof_begin(5);
-        if (um) k_silu_quant(S.st, S.gate, S.up, S.keep ? S.act : NULL, S.aq, S.aqs, S.aqsum, nb * TOPK, NULL);
+        if (um) k_silu_quant(S.st, S.gate, S.up, S.keep ? S.act : NULL, S.aq, S.aqs, S.aqsum, nb * TOPK, NULL, which == 7 && !S.keep);
         else k_actq(S.st, S.act, S.aq, S.aqs, S.aqsum, NULL, nb * TOPK);
         prof_end(5);
     }
@@ -433,9 +433,9 @@ static void run_experts(const ExpertPtrs *tab, const ExpertMaps *maps, const flo
         prof_end(6);
     }
 }
-/* weighted combine of the pairs' down rows into out (init + sum): compact rows after the tcgen05 kernel, fp32 rows otherwise */
-static void run_combine(const float *const *dsp, int nb, const float *init, float *out) {
-    if (use_umma(nb)) k_combine_wire(S.st, S.wire, S.maxp, dsp, S.uw, S.tp, init, out, nb);
+/* weighted combine of the pairs' down rows into out (init + sum): compact rows after the tcgen05 kernel (drop: not needed afterwards), fp32 rows otherwise */
+static void run_combine(const float *const *dsp, int nb, const float *init, float *out, int drop) {
+    if (use_umma(nb)) k_combine_wire(S.st, S.wire, S.maxp, dsp, S.uw, S.tp, init, out, nb, drop);
     else k_combine(S.st, S.down, S.uw, S.tp, init, out, nb);
 }
 /* router logits: large batches take the tiled kernel, small ones the kernels that read the norm's re-laid rows in place (k_router_logits_small chooses).
@@ -480,7 +480,7 @@ static void run_layer(int L, int nb, int norm, const float *bias) {
     prof_begin(3); run_group_m(nb, tr); prof_end(3);
     run_experts(l->tab, l->maps, (const float *const *)l->dsp, S.ue, nb, 7);
     prof_begin(7);
-    if (norm) run_combine((const float *const *)l->dsp, nb, S.x, S.x); else run_combine((const float *const *)l->dsp, nb, NULL, S.y);
+    if (norm) run_combine((const float *const *)l->dsp, nb, S.x, S.x, !S.keep); else run_combine((const float *const *)l->dsp, nb, NULL, S.y, !S.keep);
     prof_end(7);
 }
 static int g_ep_call;      /* set while an expert-parallel entry point runs its checks */
@@ -610,7 +610,7 @@ static void mid_layers(int nb, int l0, int nl, const float *bias) {
         run_group(nb);
         run_experts(l->tab, l->maps, (const float *const *)l->dsp, S.ue, nb, 7);
         if (L + 1 < l0 + nl) k_edge_wire(S.st, S.wire, S.maxp, (const float *const *)l->dsp, S.uw, S.tp, S.x, S.ly[L + 1].post_ln, S.hn, S.hq, S.hqs, S.hqsum, (float *)S.hT, nb);
-        else run_combine((const float *const *)l->dsp, nb, S.x, S.x);
+        else run_combine((const float *const *)l->dsp, nb, S.x, S.x, 1);
     }
 }
 /* one layer on normalised rows, without the residual, from and to S.h_rows */
@@ -941,7 +941,7 @@ static int grouping_args(const char *who, int nb, int nu) {
 static void run_call_experts(int nb, const float *init, float *out) {
     if (use_umma(nb)) run_gather(nb);
     run_experts(S.tab_call, S.maps_seen, (const float *const *)S.dsp_call, NULL, nb, 7);
-    run_combine((const float *const *)S.dsp_call, nb, init, out);
+    run_combine((const float *const *)S.dsp_call, nb, init, out, !S.keep);
 }
 /* The experts only see the rows' int8 form, so that is what crosses to the card: a quarter of the bytes, made by the host threads that would
  * otherwise copy the rows into page-locked memory (same bits as the device's prep, hostio.c). */
@@ -1053,8 +1053,8 @@ int gmoe_stage(const char *name, int L, int nb) {
     else if (!strcmp(name, "actq")) run_experts(l->tab, l->maps, (const float *const *)l->dsp, S.ue, nb, 2);
     else if (!strcmp(name, "down")) { if (use_umma(nb)) cudaMemsetAsync(S.wire, 0, WIRE_BYTES((size_t)S.maxp), S.st);   /* a repeated stage must not find the previous run's escape bits */
         run_experts(l->tab, l->maps, (const float *const *)l->dsp, S.ue, nb, 4); }
-    else if (!strcmp(name, "combine_y")) run_combine((const float *const *)l->dsp, nb, NULL, S.y);
-    else if (!strcmp(name, "combine_x")) run_combine((const float *const *)l->dsp, nb, S.x, S.x);
+    else if (!strcmp(name, "combine_y")) run_combine((const float *const *)l->dsp, nb, NULL, S.y, 0);
+    else if (!strcmp(name, "combine_x")) run_combine((const float *const *)l->dsp, nb, S.x, S.x, 0);
     else return fail("gmoe", "no stage named %s", name);
     cudaEventRecord(S.e1, S.st);
     return finish("gmoe") < 0 ? -1 : 0;
@@ -1433,14 +1433,14 @@ static int run_layer_ep(int L, int nb, const float *bias) {
     if (S.keep) { a.gu_dots = S.gu_dots; a.dn_dots = S.dn_dots; }
     prof_begin(4); if (um) k_gateup_umma(S.st, &a, &S.bmap_hq); else k_gateup_mma(S.st, &a, tn); prof_end(4);
     prof_begin(5);
-    if (um) k_silu_quant(S.st, S.gate, S.up, S.keep ? S.act : NULL, S.aq, S.aqs, S.aqsum, (int)EP.rcap, EP.total);
+    if (um) k_silu_quant(S.st, S.gate, S.up, S.keep ? S.act : NULL, S.aq, S.aqs, S.aqsum, (int)EP.rcap, EP.total, 0);
     else k_actq(S.st, S.act, S.aq, S.aqs, S.aqsum, EP.total, (int)EP.rcap);
     prof_end(5);
     prof_begin(6); if (um) k_down_umma(S.st, &a, &S.bmap_aq); else k_down_mma(S.st, &a, tn); prof_end(6);
     prof_begin(7);
     if (ep_barrier(NULL)) return -1;
     if (um && S.keep) k_wire_decode(S.st, S.wire, S.maxp, (const float *const *)EP.dsp[L], S.down, nb * TOPK);
-    run_combine((const float *const *)EP.dsp[L], nb, S.x, S.x);
+    run_combine((const float *const *)EP.dsp[L], nb, S.x, S.x, 0);
     prof_end(7);
     return 0;
 }

@@ -534,7 +534,7 @@ extern "C" void k_actq(cudaStream_t st, const float *act, int8_t *aq, float *aqs
 // (Two rows per warp, whose exact evaluations share a pass, at 122 registers: 24.6.  Rows brought ahead into shared memory by resident warps, 24 per SM: 21.3.)
 // ------------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(64, 16) silu_quant_kernel(const float *__restrict__ gate, const float *__restrict__ up,
-                                                         int8_t *__restrict__ aq, float *__restrict__ aqs, int *__restrict__ aqsum, int np, const int *__restrict__ np_dev) {
+                                                         int8_t *__restrict__ aq, float *__restrict__ aqs, int *__restrict__ aqsum, int np, const int *__restrict__ np_dev, int drop) {
     __shared__ unsigned long long tab[32];
     if (threadIdx.x < 32) tab[threadIdx.x] = DEV_EXP_TAB[threadIdx.x];
     __syncthreads();
@@ -547,6 +547,7 @@ __global__ void __launch_bounds__(64, 16) silu_quant_kernel(const float *__restr
 #pragma unroll
     for (int i = 0; i < 4; i++) reinterpret_cast<uint32_t *>(aq + (size_t)a * FFN)[32 * i + lane] = pk[i];
     if (lane == 0) { aqs[a] = s; aqsum[a] = tot; }
+    if (drop) { __syncwarp(); l2_discard((lane < 16 ? gate : up) + (size_t)a * FFN + (lane & 15) * 32); }
 }
 // Every element evaluated exactly with the libm-equal expf in double (dev_math.cuh), and the fp32 activations stored (stage comparisons).
 __global__ void __launch_bounds__(256, 4) silu_quant_exact_kernel(const float *__restrict__ gate, const float *__restrict__ up, float *__restrict__ act,
@@ -579,10 +580,10 @@ __global__ void __launch_bounds__(256, 4) silu_quant_exact_kernel(const float *_
     for (int i = 0; i < 4; i++) reinterpret_cast<uint32_t *>(aq + (size_t)a * FFN)[32 * i + lane] = pk[i];
     if (lane == 0) { aqs[a] = s; aqsum[a] = tot; }
 }
-extern "C" void k_silu_quant(cudaStream_t st, const float *gate, const float *up, float *act, int8_t *aq, float *aqs, int *aqsum, int np, const int *np_dev) {
+extern "C" void k_silu_quant(cudaStream_t st, const float *gate, const float *up, float *act, int8_t *aq, float *aqs, int *aqsum, int np, const int *np_dev, int drop) {
     if (np <= 0) return;
     if (act) launch_k(silu_quant_exact_kernel, (np + 7) / 8, 256, 0, st, gate, up, act, aq, aqs, aqsum, np, np_dev);
-    else launch_k(silu_quant_kernel, (np + 1) / 2, 64, 0, st, gate, up, aq, aqs, aqsum, np, np_dev);
+    else launch_k(silu_quant_kernel, (np + 1) / 2, 64, 0, st, gate, up, aq, aqs, aqsum, np, np_dev, drop);
     g_launches++;
 }
 

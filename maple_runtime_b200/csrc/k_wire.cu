@@ -25,7 +25,7 @@ extern "C" void k_count_add(long n);
 #define CW_MAXTOK 288               /* tokens per CTA the pair table is sized for */
 __global__ void __launch_bounds__(CW_WARPS * 32, 1) combine_wire_kernel(uint8_t *__restrict__ wire, int np_cap, const float *const *__restrict__ dsp,
                                                                        const float *__restrict__ uw, const int *__restrict__ tp,
-                                                                       const float *__restrict__ init, float *__restrict__ out, int nb, int tok_per_cta) {
+                                                                       const float *__restrict__ init, float *__restrict__ out, int nb, int tok_per_cta, int drop) {
     extern __shared__ __align__(16) float sds[];                       // [CW_EX][CW_ROWS] scales, then [tok_per_cta * 8] pair records
     int4 *smeta = reinterpret_cast<int4 *>(sds + CW_EX * CW_ROWS);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rb = blockIdx.x;
@@ -68,10 +68,14 @@ __global__ void __launch_bounds__(CW_WARPS * 32, 1) combine_wire_kernel(uint8_t 
             wire_add(acc, raw[k], w, qs, *reinterpret_cast<const float4 *>(sds + ex * CW_ROWS + 4 * lane), escbits, rb, lane, wire, np_cap, m.x);
         }
         *reinterpret_cast<float4 *>(out + o) = acc;
+        if (drop) {                                                    // the two lines of each of the eight rows that this warp alone has read
+            __syncwarp();
+            if (lane < 2 * TOPK) l2_discard(wire + (size_t)mt[lane >> 1].x * WIRE_PITCH + rb * CW_ROWS * 2 + (lane & 1) * 128);
+        }
     }
 }
 extern "C" void k_combine_wire(cudaStream_t st, uint8_t *wire, int np_cap, const float *const *dsp, const float *uw, const int *tp,
-                               const float *init, float *out, int nb) {
+                               const float *init, float *out, int nb, int drop) {
     if (nb <= 0) return;
     static int sms = 0; const int smem = CW_EX * CW_ROWS * 4 + CW_MAXTOK * TOPK * 16;
     if (!sms) {
@@ -85,7 +89,7 @@ extern "C" void k_combine_wire(cudaStream_t st, uint8_t *wire, int np_cap, const
     int per = (nb + groups - 1) / groups; if (per < CW_WARPS) per = CW_WARPS;
     if (per > CW_MAXTOK) per = CW_MAXTOK;
     groups = (nb + per - 1) / per;
-    launch_k(combine_wire_kernel, dim3(HID / CW_ROWS, groups), CW_WARPS * 32, smem, st, wire, np_cap, dsp, uw, tp, init, out, nb, per);
+    launch_k(combine_wire_kernel, dim3(HID / CW_ROWS, groups), CW_WARPS * 32, smem, st, wire, np_cap, dsp, uw, tp, init, out, nb, per, drop);
     k_count_add(1);
 }
 

@@ -93,14 +93,15 @@ typedef struct {
 void k_group(cudaStream_t st, const GroupArgs *g);
 /* np_dev (optional, device): the pair count when only a capacity np_max is known on the host */
 void k_actq(cudaStream_t st, const float *act, int8_t *aq, float *aqs, int *aqsum, const int *np_dev, int np_max);
-/* SiLU*up then per-pair int8 from stored gate and up (the tensor-core path); act may be NULL */
-void k_silu_quant(cudaStream_t st, const float *gate, const float *up, float *act, int8_t *aq, float *aqs, int *aqsum, int np, const int *np_dev);
+/* SiLU*up then per-pair int8 from stored gate and up (the tensor-core path); act may be NULL.  drop = 1: gate and up are read for the last time and their
+ * contents are given up (launch.cuh: l2_discard); not with act */
+void k_silu_quant(cudaStream_t st, const float *gate, const float *up, float *act, int8_t *aq, float *aqs, int *aqsum, int np, const int *np_dev, int drop);
 /* decode batches, between two layers: x += the pairs' weighted rows, then norm + int8 of x as k_norm_prep_relaid */
 void k_edge(cudaStream_t st, const float *down, const float *uw, const int *tp, float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb);
 /* one token: k_edge and the next layer's k_router_logits_small in one kernel; x -> xo, which is another buffer */
 void k_router_edge(cudaStream_t st, const void *router_s, const float *down, const float *uw, const int *tp, const float *x, float *xo, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum,
                    const float *bias, float *logits, int *err);
-/* the same from the tcgen05 down kernel's compact rows */
+/* the same from the tcgen05 down kernel's compact rows, whose contents it gives up */
 void k_edge_wire(cudaStream_t st, uint8_t *wire, int np_cap, const float *const *dsp, const float *uw, const int *tp, float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb);
 void k_combine(cudaStream_t st, const float *down, const float *uw, const int *tp, const float *init, float *out, int nb);
 
@@ -163,9 +164,10 @@ void k_router_tensor(cudaStream_t st, const RouterTensorArgs *r);
 #define WIRE_REC 16
 #define WIRE_BYTES(np_cap) ((size_t)(np_cap) * (WIRE_PITCH + WIRE_REC))
 /* out[b] = init[b] (or 0) + sum over the token's pairs, in the order of tp, of uw * ((float)dot * scale * ds[expert][row]): the
- * same operations in the same order as the fp32 form (k_combine after a down kernel that scaled).  dsp[ex] = 2048 down scales. */
+ * same operations in the same order as the fp32 form (k_combine after a down kernel that scaled).  dsp[ex] = 2048 down scales.  drop = 1: the rows (not their
+ * escape planes and records) are read for the last time and their contents are given up. */
 void k_combine_wire(cudaStream_t st, uint8_t *wire, int np_cap, const float *const *dsp, const float *uw, const int *tp,
-                    const float *init, float *out, int nb);
+                    const float *init, float *out, int nb, int drop);
 /* fp32 rows [np][2048] from compact ones (stage comparisons); leaves the escape planes as they are */
 void k_wire_decode(cudaStream_t st, const uint8_t *wire, int np_cap, const float *const *dsp, float *down, int np);
 

@@ -30,6 +30,12 @@ static inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 b
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #endif
+#ifdef __CUDACC__
+// Scratch that has been read for the last time: its 128-byte line at p (aligned) leaves the L2 without being written to memory.  What lies there afterwards is
+// undefined until it is written again.  For gate and up rows and compact down rows (143 MB per layer of 2048 tokens, more than the L2): a layer of 511 / 843 / 2048 tokens
+// 99.6 / 110.7 / 157.8 -> 97.5 / 107.3 / 156.4 us.  The pair-ordered int8 rows and the router's partial sums too: no further change.
+__device__ __forceinline__ void l2_discard(const void *p) { asm volatile("discard.global.L2 [%0], 128;" ::"l"(p) : "memory"); }
+#endif
 // the same, programmatically too, as one cluster of `ctas` CTAs
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_cluster(void (*kernel)(KArgs...), unsigned ctas, dim3 block, cudaStream_t st, Args... args) {
