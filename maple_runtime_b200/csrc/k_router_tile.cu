@@ -208,6 +208,7 @@ extern "C" void k_router_logits_tile(cudaStream_t st, const void *router_t, cons
 #define RS_EXP 8
 #define RS_HB (RS_TOK * HID * 4)
 #define RS_WB (RS_EXP * HID * 2)
+#define RS_ALONE (120 << 10)              /* shared memory that leaves no room for a second CTA on the SM */
 // router rows (bf16 [256][2048]) -> [expert][i4 = column / 32][lane j][4 steps]; once per layer
 __global__ void __launch_bounds__(256) router_pack_w_small_kernel(const uint16_t *__restrict__ W, uint2 *__restrict__ WS) {
     const int o = blockIdx.x * 256 + threadIdx.x, j = o & 7, i4 = (o >> 3) & 63, e = o >> 9;
@@ -286,15 +287,17 @@ __global__ void __launch_bounds__(256, 2) router_small_kernel(const uint8_t *__r
 // A few hundred tokens.  The kernel above runs one wave per 74 of them (a multiply-add costs it three quarters of a shared-memory read and an unpacking);
 // the prefill kernel's CTAs are too few to fill the SMs, its one warp per scheduler issues every 2.5 cycles, and it wants its rows copied once more.  Here a
 // warp is 8 lanes x 4 positions of TT tokens x 8 experts, small enough for two warps per scheduler at 300 tokens; a CTA is four of them on the same 4 TT
-// tokens and 32 experts, and a fifth that fills a ring of three stages of 256 columns.  Rows and weights are read as they lie: rows in the decode layout that
-// the norm left, weights in the tile layout.  Kernel above -> here, per layer of the stack: 160 tokens 84.8 -> 83.1, 256 108.2 -> 105.6, 301 103.3 -> 98.7,
-// 416 112.5 -> 104.9 us.  (TT = 4 with 16 experts per position, two warps per CTA: 103 at 301, 107 at 400.)
+// tokens and 32 experts, and a fifth that fills a ring of two stages of 256 columns (three: 0.4 to 0.9 us slower, 511 tokens 1.2).  Rows and weights are read as they
+// lie: rows in the decode layout that the norm left, weights in the tile layout.  Kernel above -> here, per layer of the stack: 160 tokens 84.8 -> 83.1, 256 108.2 -> 105.6,
+// 301 103.3 -> 98.7, 416 112.5 -> 104.9 us.  With the tokens per CTA chosen by the SMs they fill (below), 12 or 16 before: 230 tokens 82.8 -> 79.5, 296 84.8 -> 80.4,
+// 301 87.5 -> 86.9, 400 92.2 -> 88.8, 511 97.6 -> 96.4.  (TT = 4 with 16 experts per position, two warps per CTA: 103 at 301, 107 at 400.  CTAs of 16 experts: 85 to 86 at 230
+// to 256 with TT = 4, 83 with 3, level with 32 experts for TT = 2.)
 // ---------------------------------------------------------------------------------------------------------------------
 #define RM_COLS 256
 #define RM_NCH (HID / RM_COLS)
 #define RM_ROW (RM_COLS * 4)
 #define RM_WB (2 * 2 * RP_GRP)            /* two chunks of the tile layout x two groups of 16 experts */
-#define RM_STAGES 3
+#define RM_STAGES 2
 template <int TT>
 __global__ void __launch_bounds__(160) router_mid_kernel(const uint8_t *__restrict__ WT, const uint8_t *__restrict__ hS, const float *__restrict__ bias,
                                                          float *__restrict__ logits, int nb, int *err) {
@@ -398,15 +401,19 @@ __global__ void __launch_bounds__(160) router_mid_kernel(const uint8_t *__restri
     __syncthreads();
     if (tid == 0 && abort_flag) *(volatile int *)err = 31;      // a wait ran out: the host reports it and the logits are not to be used
 }
-static int mid_ctas(int nb, int tt) { return NEXP / 32 * ((nb + 4 * tt - 1) / (4 * tt)); }
+// Launched plainly (programmatically: 301 tokens 87.0 -> 88.3 us per layer, 400 88.8 -> 92.2) and with so much shared memory that per_sm CTAs fit an SM and no more.
+// Without the preference for shared memory the driver leaves room for fewer than two CTAs at some sizes (400 tokens 92.0 -> 89.3).
+#define RM_ALONE (116 << 10)
+#define RM_PAIR (78 << 10)
 template <int TT>
-static void launch_mid(cudaStream_t st, const void *router_t, const void *hS, const float *bias, float *logits, int nb, int *err) {
+static void launch_mid(cudaStream_t st, const void *router_t, const void *hS, const float *bias, float *logits, int nb, int *err, int per_sm) {
     static bool attr_done = false;
-    const int smem = RM_STAGES * (4 * TT * RM_ROW + RM_WB);
-    if (!attr_done) { cudaFuncSetAttribute(router_mid_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); attr_done = true; }
-    const dim3 grid(NEXP / 32, (nb + 4 * TT - 1) / (4 * TT));
-    // plainly: placed early, several CTAs end up on the SMs that the norm leaves first (400 tokens: 105.2 against 103.6 us per layer)
-    launch_k(router_mid_kernel<TT>, grid, 160, smem, st, (const uint8_t *)router_t, (const uint8_t *)hS, bias, logits, nb, err);
+    if (!attr_done) {
+        cudaFuncSetAttribute(router_mid_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, RM_ALONE);
+        cudaFuncSetAttribute(router_mid_kernel<TT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared); attr_done = true;
+    }
+    static_assert(RM_STAGES * (4 * TT * RM_ROW + RM_WB) <= RM_PAIR, "ring");
+    launch_k(router_mid_kernel<TT>, dim3(NEXP / 32, (nb + 4 * TT - 1) / (4 * TT)), 160, per_sm == 1 ? RM_ALONE : RM_PAIR, st, (const uint8_t *)router_t, (const uint8_t *)hS, bias, logits, nb, err);
 }
 extern "C" void k_router_pack_small(cudaStream_t st, const uint16_t *router, void *router_s) {
     router_pack_w_small_kernel<<<NEXP * HID / 4 / 256, 256, 0, st>>>(router, (uint2 *)router_s);
@@ -419,22 +426,29 @@ extern "C" void k_router_logits_small(cudaStream_t st, const void *router_s, con
     if (nb <= 0) return;
     static bool attr_done = false;
     if (!attr_done) {
-        cudaFuncSetAttribute(router_small_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_HB + RS_WB);
-        cudaFuncSetAttribute(router_small_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_HB + RS_WB); attr_done = true;
+        cudaFuncSetAttribute(router_small_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_ALONE);
+        cudaFuncSetAttribute(router_small_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_ALONE); attr_done = true;
     }
     if (!relaid) launch_k(router_pack_h_small_kernel, nb * 2, 256, 0, st, hn, (float4 *)hS, nb);
     static int sms = 0;
     if (!sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); if (sms < 1) sms = 148; }
     if (nb > 2 * 2 * sms / (NEXP / RS_EXP) * RS_TOK) {             // past two waves of the small kernel (148 tokens)
-        // 12 tokens per CTA (10.5 us as one CTA per SM, 16.1 as two), or 16 (13.8, 20.1) where that means fewer CTAs per SM: 217 to 288 and from 445 tokens
-        if ((mid_ctas(nb, 4) + sms - 1) / sms < (mid_ctas(nb, 3) + sms - 1) / sms) launch_mid<4>(st, router_t, hS, bias, logits, nb, err);
-        else launch_mid<3>(st, router_t, hS, bias, logits, nb, err);
+        // tokens per CTA (8 CTAs of 32 experts cover them): the fewest CTA-times of work per SM.  One CTA of 12 on each SM is the cheapest (to 216 tokens); two of 8 take
+        // 0.5 us more (to 296), two of 12 another 3.5 (to 444), two of 16 another 6 (to 592); three of 8 take 1 us more than two of 12, three of 12 1.5 more than two of 16.
+        const int one = sms / (NEXP / 32), two = 2 * sms / (NEXP / 32);
+        if (nb <= 12 * one) launch_mid<3>(st, router_t, hS, bias, logits, nb, err, 1);
+        else if (nb <= 8 * two) launch_mid<2>(st, router_t, hS, bias, logits, nb, err, 2);
+        else if (nb <= 12 * two) launch_mid<3>(st, router_t, hS, bias, logits, nb, err, 2);
+        else launch_mid<4>(st, router_t, hS, bias, logits, nb, err, 2);
         k_count_add(relaid ? 1 : 2);
         return;
     }
     const dim3 grid(NEXP / RS_EXP, (nb + RS_TOK - 1) / RS_TOK);
-    if (g_step_order && nb == 1) launch_pdl(router_small_kernel<true, false>, grid, 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err, RouterEdge{});
-    else launch_pdl(router_small_kernel<false, false>, grid, 256, RS_HB + RS_WB, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err, RouterEdge{});
+    // CTAs that are no more than the SMs get one each: placed while the kernel before them ends, they would pair up on the SMs that are free first (32 tokens, 128 CTAs:
+    // 50.5 -> 48.3 us per layer; no change up to 24 tokens, whose CTAs are fewer)
+    const int rsm = (int)(grid.x * grid.y) <= sms ? RS_ALONE : RS_HB + RS_WB;
+    if (g_step_order && nb == 1) launch_pdl(router_small_kernel<true, false>, grid, 256, rsm, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err, RouterEdge{});
+    else launch_pdl(router_small_kernel<false, false>, grid, 256, rsm, st, (const uint8_t *)router_s, (const uint8_t *)hS, bias, logits, nb, err, RouterEdge{});
     k_count_add(relaid ? 1 : 2);
 }
 // the joint of two layers and the router of the next, for one token; x and xo are different buffers (the CTAs read x while the first writes xo)

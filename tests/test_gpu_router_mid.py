@@ -25,3 +25,12 @@ def test_mid_router_equals_oracle(nb, layer, gpu, oracle, weights):
     gpu.poke("bias", bias)
     gpu.stage("router_bias", 2, nb)
     assert np.array_equal(gpu.peek("logits", nb).reshape(nb, 256).view(np.uint32), (want + bias[None, :]).view(np.uint32))
+
+
+@pytest.mark.parametrize("nb", [217, 296, 297])
+def test_where_eight_tokens_per_cta_begin_and_end(nb, layer, gpu, oracle, weights):
+    router, _, _ = weights.layer(2)
+    hn = weights.hidden(701, nb)
+    gpu.poke("hn", hn)
+    gpu.stage("router", 2, nb)
+    assert np.array_equal(gpu.peek("logits", nb).reshape(nb, 256).view(np.uint32), oracle.router_logits(router, hn).view(np.uint32))
