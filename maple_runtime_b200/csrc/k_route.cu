@@ -594,9 +594,12 @@ extern "C" void k_silu_quant(cudaStream_t st, const float *gate, const float *up
 // WIRE: the pairs' rows are the tensor-core path's compact ones, as combine_wire_kernel reads them.  The experts' scales come from L2 for every pair (12 KB a
 // pair with its row) instead of once per CTA: a layer of the stack 98.9 -> 96.4 us at 301 tokens, 110.2 -> 108.0 at 511, but 123.0 -> 124.5 at 600.
 // (512 threads: 99.1 at 301; launched programmatically 96.7.)
+// PER_SM (WIRE): two CTAs fit an SM at 128 registers, three at 80 with a few spilled.  The latter where it saves the second wave, 297 to 444 tokens: 301 tokens
+// 86.9 -> 85.6 us per layer, 400 88.8 -> 87.0; elsewhere it costs 0.8 to 1.7.
+// (fp32 rows): told that one CTA per SM is enough, the compiler keeps all loads of the joint in flight: 13 tokens 35.2 -> 33.9 us per layer, 64 60.6 -> 59.2.
 // ------------------------------------------------------------------------------------------------------------
-template <bool WIRE>
-__global__ void __launch_bounds__(256) edge_kernel(const float *down, const EdgeWire ew, const float *uw, const int *tp, float *x, const uint16_t *__restrict__ w,
+template <bool WIRE, int PER_SM>
+__global__ void __launch_bounds__(256, PER_SM) edge_kernel(const float *down, const EdgeWire ew, const float *uw, const int *tp, float *x, const uint16_t *__restrict__ w,
                                                    float *hn, int8_t *q, float *qs, int *qsum, float *hS) {
     __shared__ const float *s_dsp[WIRE ? NEXP : 1];
     const int tid = threadIdx.x, c = blockIdx.x;
@@ -607,11 +610,15 @@ __global__ void __launch_bounds__(256) edge_kernel(const float *down, const Edge
 }
 extern "C" void k_edge(cudaStream_t st, const float *down, const float *uw, const int *tp, float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb) {
     if (nb <= 0) return;
-    launch_pdl(edge_kernel<false>, nb, 256, 0, st, down, EdgeWire{NULL, 0, NULL}, uw, tp, x, w, hn, q, qs, qsum, hS); g_launches++;
+    launch_pdl(edge_kernel<false, 1>, nb, 256, 0, st, down, EdgeWire{NULL, 0, NULL}, uw, tp, x, w, hn, q, qs, qsum, hS); g_launches++;
 }
 extern "C" void k_edge_wire(cudaStream_t st, uint8_t *wire, int np_cap, const float *const *dsp, const float *uw, const int *tp, float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb) {
     if (nb <= 0) return;
-    launch_k(edge_kernel<true>, nb, 256, 0, st, (const float *)NULL, EdgeWire{wire, np_cap, dsp}, uw, tp, x, w, hn, q, qs, qsum, hS); g_launches++;
+    static int sms = 0;
+    if (!sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
+    if (nb > 2 * sms && nb <= 3 * sms) launch_k(edge_kernel<true, 3>, nb, 256, 0, st, (const float *)NULL, EdgeWire{wire, np_cap, dsp}, uw, tp, x, w, hn, q, qs, qsum, hS);
+    else launch_k(edge_kernel<true, 2>, nb, 256, 0, st, (const float *)NULL, EdgeWire{wire, np_cap, dsp}, uw, tp, x, w, hn, q, qs, qsum, hS);
+    g_launches++;
 }
 
 // ------------------------------------------------------------------------------------------------------------
