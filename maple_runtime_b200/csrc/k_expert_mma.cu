@@ -47,7 +47,7 @@ __device__ __forceinline__ MoeTile ldcg_tile(const MoeTile *t) {
 // GATEUP: rows block A = gate rows, block B = up rows of the same index, epilogue = SiLU*up;
 // otherwise A and B are two consecutive 16-row blocks of the down matrix, epilogue = scale only.
 // PF: chunks of weights in flight per thread.  NW: warps per CTA.
-template <int KCH, int NBLK, bool GATEUP, int PF, int NW>
+template <int KCH, int NBLK, bool GATEUP, int PF, int NW, bool FULL>
 __global__ void __launch_bounds__(NW * 32) expert_mma_kernel(ExpertArgs a) {
     constexpr int TN = NBLK * 8, KB = KCH * 256;            // tokens per tile, bytes of one int8 activation vector
     extern __shared__ __align__(16) uint8_t smem[];          // [KCH][4][TN][4][16]
@@ -166,31 +166,37 @@ __global__ void __launch_bounds__(NW * 32) expert_mma_kernel(ExpertArgs a) {
                 float qs = a.hqs[tok];
                 float gv = __fmul_rn(__fmul_rn((float)da, qs), sca[k >> 1]), uv = __fmul_rn(__fmul_rn((float)db, qs), scb[k >> 1]);
                 a.act[(size_t)pair * 512 + rr] = dev_silu_mul(gv, uv);
-                if (a.gate) { a.gate[(size_t)pair * 512 + rr] = gv; a.up[(size_t)pair * 512 + rr] = uv; }
-                if (a.gu_dots) { a.gu_dots[(size_t)pair * 1024 + rr] = da; a.gu_dots[(size_t)pair * 1024 + 512 + rr] = db; }
+                if (FULL && a.gate) { a.gate[(size_t)pair * 512 + rr] = gv; a.up[(size_t)pair * 512 + rr] = uv; }
+                if (FULL && a.gu_dots) { a.gu_dots[(size_t)pair * 1024 + rr] = da; a.gu_dots[(size_t)pair * 1024 + 512 + rr] = db; }
             } else {
                 int qsum_p; float qs;
                 if (a.act_for_down) { const float *s_qs = reinterpret_cast<const float *>(smem + KCH * 4 * TN * 64); qs = s_qs[n]; qsum_p = reinterpret_cast<const int *>(s_qs + TN)[n]; }
                 else { qs = a.aqs[pair]; qsum_p = a.aqsum[pair]; }
                 int da = acc_a[j][k] - qsum_p, db = acc_b[j][k] - qsum_p;
                 float *drow = a.down + (size_t)pair * (a.down_stride ? a.down_stride : 2048);
-                if (a.rx_src) { const int2 sp = a.rx_src[pair]; drow = a.peer_down[sp.x] + (size_t)sp.y * 2048; }   // the row goes to the token's rank
+                if (FULL && a.rx_src) { const int2 sp = a.rx_src[pair]; drow = a.peer_down[sp.x] + (size_t)sp.y * 2048; }   // the row goes to the token's rank
                 drow[rr] = __fmul_rn(__fmul_rn((float)da, qs), sca[k >> 1]);
                 drow[rr + 16] = __fmul_rn(__fmul_rn((float)db, qs), scb[k >> 1]);
-                if (a.dn_dots) { a.dn_dots[(size_t)pair * 2048 + rr] = da; a.dn_dots[(size_t)pair * 2048 + rr + 16] = db; }
+                if (FULL && a.dn_dots) { a.dn_dots[(size_t)pair * 2048 + rr] = da; a.dn_dots[(size_t)pair * 2048 + rr + 16] = db; }
             }
         }
     if (dense && tid == 0) span_end(a.span);
 }
 
-template <int KCH, int NBLK, bool GATEUP, int PF, int NW>
-static void launch(cudaStream_t st, const ExpertArgs *a) {
+template <int KCH, int NBLK, bool GATEUP, int PF, int NW, bool FULL>
+static void launch_as(cudaStream_t st, const ExpertArgs *a) {
     const size_t smem = (size_t)KCH * 4 * NBLK * 8 * 64 + (GATEUP ? 0 : NBLK * 8 * 8);   // + scale and code sum per pair when down quantises itself
     static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<KCH, NBLK, GATEUP, PF, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
+    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<KCH, NBLK, GATEUP, PF, NW, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
     dim3 grid((GATEUP ? 32 : 64) / NW, a->max_tiles);
-    launch_pdl(expert_mma_kernel<KCH, NBLK, GATEUP, PF, NW>, grid, NW * 32, smem, st, *a);
+    launch_pdl(expert_mma_kernel<KCH, NBLK, GATEUP, PF, NW, FULL>, grid, NW * 32, smem, st, *a);
     k_count_add(1);
+}
+// FULL: the stage outputs and the rows that go to other ranks, which the lean kernels have no code for (13 tokens 35.1 -> 34.8 us per layer, 64 60.6 -> 60.1)
+template <int KCH, int NBLK, bool GATEUP, int PF, int NW>
+static void launch(cudaStream_t st, const ExpertArgs *a) {
+    if (GATEUP ? a->gate != NULL || a->gu_dots != NULL : a->dn_dots != NULL || a->rx_src != NULL) launch_as<KCH, NBLK, GATEUP, PF, NW, true>(st, a);
+    else launch_as<KCH, NBLK, GATEUP, PF, NW, false>(st, a);
 }
 // Two chunks in flight leave room for six CTAs per SM, which is what a long list of tiles wants (four chunks: 64 tokens 34.5 instead of 31 us).
 // Where the whole list is resident at once at one or two CTAs per SM, all eight chunks go out together: one trip to memory instead of four
@@ -217,8 +223,8 @@ template <int NBLK, int PF>
 static void launch_dense(cudaStream_t st, const ExpertArgs *a, int rows) {
     const size_t smem = (size_t)8 * 4 * NBLK * 8 * 64 + NBLK * 8 * 8;
     static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<8, NBLK, false, PF, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
-    launch_pdl(expert_mma_kernel<8, NBLK, false, PF, 4>, dim3(rows / 128, (a->dense_n + NBLK * 8 - 1) / (NBLK * 8)), 128, smem, st, *a);
+    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<8, NBLK, false, PF, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
+    launch_pdl(expert_mma_kernel<8, NBLK, false, PF, 4, false>, dim3(rows / 128, (a->dense_n + NBLK * 8 - 1) / (NBLK * 8)), 128, smem, st, *a);
     k_count_add(1);
 }
 extern "C" void k_dense_mma(cudaStream_t st, const ExpertArgs *a, int rows) {

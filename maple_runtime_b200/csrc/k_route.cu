@@ -147,7 +147,7 @@ extern "C" void k_norm_prep_split(cudaStream_t st, const float *x, const uint16_
 // p = expf(l - max); the sum runs over experts in index order (a chain through the lanes); p /= sum; eight rounds
 // of "first strict maximum" (lowest index wins a tie); weights divided by (their sum in selection order + 1e-20f).
 // ------------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) topk_kernel(const float *__restrict__ logits, int *__restrict__ top, float *__restrict__ topw, int nb) {
+__global__ void __launch_bounds__(256, 1) topk_kernel(const float *__restrict__ logits, int *__restrict__ top, float *__restrict__ topw, int nb) {
     __shared__ unsigned long long tab[32];                  // the expf table beside the arithmetic (lane-varying index)
     __shared__ __align__(16) float s_row[8][NEXP];
     if (threadIdx.x < 32) tab[threadIdx.x] = DEV_EXP_TAB[threadIdx.x];
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(NEXP) group_place_kernel(const unsigned *__res
 #define GS_MAXTOK 32
 #define GS_TOPK 8
 template <bool TOPK_IN>
-__global__ void __launch_bounds__(NEXP) group_cta_kernel(GroupArgs g) {
+__global__ void __launch_bounds__(NEXP, 1) group_cta_kernel(GroupArgs g) {
     constexpr int NT = NEXP;
     __shared__ unsigned s_mask[NEXP];
     __shared__ int s_slot[GS_MAXTOK * TOPK];
@@ -346,10 +346,11 @@ __global__ void __launch_bounds__(NEXP) group_cta_kernel(GroupArgs g) {
 // global memory (inside a layer of 2048 tokens, against the router setting the bits and the place kernel reading them: 4 us less).  Eight
 // CTAs are what every GPU has to allow; from 513 tokens on sixteen share the scattered stores (2048 tokens: 14.4 -> 11.9 us).
 // Against one CTA for up to 256 tokens, a layer of the stack: 96 tokens 70.8 -> 70.0 us, 128 77.7 -> 75.9, 256 106.1 -> 100.7.
+// (One CTA per SM in the launch bounds of the grouping kernels: registers instead of reloads, 0.1 us.)
 // TOPK_IN (9 to TOPK_IN_MAX tokens): the softmax and top-8 come first, a warp per token (20 tokens 41.8 -> 41.3 us, 64 61.2 -> 60.7).
 #define GC_WORDS 8
 template <int GC_CTAS, bool TOPK_IN>
-__global__ void __launch_bounds__(NEXP) group_cluster_kernel(GroupArgs g) {
+__global__ void __launch_bounds__(NEXP, 1) group_cluster_kernel(GroupArgs g) {
     __shared__ unsigned s_mask[NEXP][GC_WORDS + 1];           // + 1: a warp's 32 experts of one word lie in 32 banks
     __shared__ unsigned short s_pre[NEXP][GC_WORDS + 1];      // the pairs of the CTA's expert in front of word w
     __shared__ int s_cnt[NEXP], s_start[NEXP];
@@ -625,7 +626,7 @@ extern "C" void k_edge_wire(cudaStream_t st, uint8_t *wire, int np_cap, const fl
 // Combine (maple.c:834): out[b] = init[b] (or 0) then, for the token's pairs in ascending pair order,
 // out = fma(w, down, out) -- the order and the fused rounding of the reference's compiled loop.
 // ------------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) combine_kernel(const float *__restrict__ down, const float *__restrict__ uw, const int *__restrict__ tp,
+__global__ void __launch_bounds__(256, 1) combine_kernel(const float *__restrict__ down, const float *__restrict__ uw, const int *__restrict__ tp,
                                                       const float *__restrict__ init, float *__restrict__ out, int nb) {
     const int i = blockIdx.x * 256 + threadIdx.x, b = i >> 9, c = (i & 511) * 4;
     pdl_wait(); pdl_trigger();
