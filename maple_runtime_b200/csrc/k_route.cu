@@ -532,8 +532,10 @@ extern "C" void k_actq(cudaStream_t st, const float *act, int8_t *aq, float *aqs
 // Bound by instruction issue (800 per pair at first, 60% of the slots used) beside 75 MB per 2048 tokens: the bytes of a row are cut out of the rounding sums with
 // byte permutes and added with dp4a, and the distance to a rounding boundary is one running maximum per lane that is taken apart only where it is near.  CTAs of two warps
 // instead of eight, so that an SM takes new rows as each pair of warps ends: between events 22.1 -> 20.1 us at 2048 tokens, 14.3 -> 12.5 at 843.
+// Launched programmatically up to 1536 tokens: 511 tokens 96.4 -> 96.0 us per layer, 843 106.3 -> 105.7, 1300 125.8 -> 125.1, 2048 the same, 3000 222.2 -> 224.7.
 // (Two rows per warp, whose exact evaluations share a pass, at 122 registers: 24.6.  Rows brought ahead into shared memory by resident warps, 24 per SM: 21.3.)
 // ------------------------------------------------------------------------------------------------------------
+#define SQ_EARLY (1536 * TOPK)
 __global__ void __launch_bounds__(64, 16) silu_quant_kernel(const float *__restrict__ gate, const float *__restrict__ up,
                                                          int8_t *__restrict__ aq, float *__restrict__ aqs, int *__restrict__ aqsum, int np, const int *__restrict__ np_dev, int drop) {
     __shared__ unsigned long long tab[32];
@@ -584,6 +586,7 @@ __global__ void __launch_bounds__(256, 4) silu_quant_exact_kernel(const float *_
 extern "C" void k_silu_quant(cudaStream_t st, const float *gate, const float *up, float *act, int8_t *aq, float *aqs, int *aqsum, int np, const int *np_dev, int drop) {
     if (np <= 0) return;
     if (act) launch_k(silu_quant_exact_kernel, (np + 7) / 8, 256, 0, st, gate, up, act, aq, aqs, aqsum, np, np_dev);
+    else if (np <= SQ_EARLY) launch_pdl(silu_quant_kernel, (np + 1) / 2, 64, 0, st, gate, up, aq, aqs, aqsum, np, np_dev, drop);
     else launch_k(silu_quant_kernel, (np + 1) / 2, 64, 0, st, gate, up, aq, aqs, aqsum, np, np_dev, drop);
     g_launches++;
 }
