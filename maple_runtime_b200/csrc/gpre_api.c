@@ -378,9 +378,10 @@ int gmoe_profile_read(double *secs, long *launches) {
 /* ---- the stages ------------------------------------------------------------------------------------------------ */
 static int tile_tn(int nb) { return nb <= 256 ? 8 : 32; }
 
-/* Which expert kernels: up to 208 tokens the mma.sync kernels on tiles of 8, above that the tcgen05 kernels, whose time hardly grows while an expert
- * has few pairs.  A layer of the stack on either: 160 tokens 79.0 and 84.0 us, 208 86.2 and 86.5, 256 96.1 and 90.2. */
-static int use_umma(int nb) { return S.path == 2 || (S.path == 0 && nb > 208); }
+/* Which expert kernels: up to 160 tokens the mma.sync kernels on tiles of 8, above that the tcgen05 kernels, whose time hardly grows while an expert
+ * has few pairs.  A layer of the stack on either: 128 tokens 73.6 and 75.6 us, 144 76.0 and 77.2, 160 76.5 and 76.5, 176 78.0 and 76.8, 208 84.0 and 78.4; a layer
+ * call's kernels 85.0 and 86.0 at 160, 87.0 and 86.0 at 176, a plug-in call's 69.6 and 69.6, 73.7 and 69.6 at 192. */
+static int use_umma(int nb) { return S.path == 2 || (S.path == 0 && nb > 160); }
 static void fill_expert_args(ExpertArgs *a, const ExpertPtrs *tab, const ExpertMaps *maps, const int *ue, int nb) {
     memset(a, 0, sizeof *a);
     a->call_maps = maps == S.maps_seen; a->fresh_maps = a->call_maps && S.map_fresh; a->tab = tab; a->maps = maps; a->ue = ue; a->ptok = S.utok; a->err = S.err;

@@ -49,3 +49,21 @@ def test_layers_in_one_call_equal_layers_one_by_one(nb, l0, stacks, gpu, weights
             assert same_bits(got, want)
     finally:
         g.keep_stages(True)
+
+
+@pytest.mark.parametrize("nb", [160, 161, 208])
+def test_where_the_tensor_cores_take_over(nb, stacks, gpu, weights):
+    """160 tokens are the last on the mma.sync kernels, 161 the first on the tcgen05 ones: both like the mma.sync kernels, bit for bit."""
+    g = gpu
+    x = weights.hidden(950 + nb, nb)
+    out = {}
+    g.keep_stages(False)
+    try:
+        for path in (1, 0):
+            g.set_path(path)
+            out[path] = x.copy()
+            g.forward(out[path], 0, 3)
+    finally:
+        g.set_path(0)
+        g.keep_stages(True)
+    assert same_bits(out[0], out[1])
