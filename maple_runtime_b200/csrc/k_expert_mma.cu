@@ -221,6 +221,9 @@ static void launch(cudaStream_t st, const ExpertArgs *a) {
 // Eight warps per CTA share a tile's staged rows once an expert has several pairs: 192 tokens 86.2 -> 82.5 us per layer, 160 80.6 -> 79.0, 128 the same, but
 // 64 tokens 60.8 -> 61.8.  max_tiles is 256 + the tokens, as many tiles as there could be.
 #define NW8_TILES 384
+// The down kernel, whose CTAs each quantise the tile's activations for themselves, from 96 tokens: 96 66.9 -> 66.7 us per layer, 112 71.1 -> 70.5, 128 73.6 -> 72.4, but 72 tokens
+// 62.3 -> 62.8 and 32 45.2 -> 46.0.
+#define DOWN8_TILES 351
 extern "C" void k_gateup_mma(cudaStream_t st, const ExpertArgs *a, int tn) {
     if (a->max_tiles <= 0) return;
     if (tn != 8) launch<8, 4, true, 2, 4>(st, a); else if (a->max_tiles <= PF8_TILES) launch<8, 1, true, 8, 4>(st, a);
@@ -228,7 +231,7 @@ extern "C" void k_gateup_mma(cudaStream_t st, const ExpertArgs *a, int tn) {
 }
 extern "C" void k_down_mma(cudaStream_t st, const ExpertArgs *a, int tn) {
     if (a->max_tiles <= 0) return;
-    if (tn != 8) launch<2, 4, false, 2, 4>(st, a); else if (a->max_tiles <= NW8_TILES) launch<2, 1, false, 2, 4>(st, a); else launch<2, 1, false, 2, 8>(st, a);
+    if (tn != 8) launch<2, 4, false, 2, 4>(st, a); else if (a->max_tiles <= DOWN8_TILES) launch<2, 1, false, 2, 4>(st, a); else launch<2, 1, false, 2, 8>(st, a);
 }
 
 // The attention projections (gpu_pre.m:200-256 gpre_dense*): the same int8 x 2-bit product with one matrix instead of 256
