@@ -270,19 +270,40 @@ __device__ __forceinline__ int2 group_scan(int2 v, const int lane) {
     }
     return v;
 }
-// One token: softmax, top-8 and grouping by one warp.  A pair's place is its expert's rank among the eight: no scan over the experts and no barrier.  24 layers of one
-// token 17.5 -> 16.7 us each; as a branch of the kernel below it cost that kernel 0.15 us.
-__global__ void __launch_bounds__(32, 1) group_one_kernel(GroupArgs g) {
-    __shared__ __align__(16) float s_row[NEXP];
+// One token: softmax, top-8 and grouping by one warp, beside which a second one adds up the softmax's sum.  A pair's place is its expert's rank among the eight: no scan
+// over the experts.  24 layers of one token 17.25 -> 16.35 us each, and with the sum beside the selection 16.1; as a branch of the kernel below it cost that one 0.15 us.
+__global__ void __launch_bounds__(64, 1) group_one_kernel(GroupArgs g) {
+    __shared__ __align__(16) float s_row[NEXP], s_run;
     __shared__ unsigned long long tab[32];
-    const int lane = threadIdx.x;
-    tab[lane] = DEV_EXP_TAB[lane];
-    __syncwarp();
+    const int lane = threadIdx.x & 31, sum_warp = threadIdx.x >> 5;
+    if (threadIdx.x < 32) tab[lane] = DEV_EXP_TAB[lane];
+    __syncthreads();
     pdl_wait(); pdl_trigger();
     const float4 v0 = __ldcg(reinterpret_cast<const float4 *>(g.logits) + 2 * lane), v1 = __ldcg(reinterpret_cast<const float4 *>(g.logits) + 2 * lane + 1);
     float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-    int isel; float wsel, tsum;
-    exact_topk_warp(p, lane, tab, s_row, isel, wsel, tsum);
+    // warp 1 adds the exponentials in the reference's order (256 dependent additions) while warp 0 selects by them
+    exact_exp_warp(p, lane, tab);
+    if (sum_warp) {
+        reinterpret_cast<float4 *>(s_row)[2 * lane] = make_float4(p[0], p[1], p[2], p[3]); reinterpret_cast<float4 *>(s_row)[2 * lane + 1] = make_float4(p[4], p[5], p[6], p[7]);
+        __syncwarp();
+        const float run = exact_sum_row(s_row);
+        if (lane == 0) s_run = run;
+        __syncthreads();
+        return;
+    }
+    int isel; float psel, tsum;                                          // lane k < 9: the k-th largest
+    top_select_warp<TOPK + 1>(p, lane, isel, psel, tsum);
+    __syncthreads();
+    const float run = s_run;
+    float wsel = __fdiv_rn(psel, run);
+    // the reference selects by the quotients: another order only where unequal exponentials have equal quotients (or are not numbers)
+    const float pn = __shfl_down_sync(0xffffffffu, psel, 1), wn = __shfl_down_sync(0xffffffffu, wsel, 1);
+    if (__any_sync(0xffffffffu, lane < TOPK && !(wsel > wn || psel == pn))) exact_topk_warp_from(p, lane, run, isel, wsel, tsum);
+    else {
+        tsum = 0.0f;
+#pragma unroll
+        for (int k = 0; k < TOPK; k++) tsum = __fadd_rn(tsum, __shfl_sync(0xffffffffu, wsel, k));
+    }
     const float w = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));          // lane k < 8: the k-th selected expert
     int r = 0, st[8] = {-1, -1, -1, -1, -1, -1, -1, -1};                // st: where the pairs of experts 8 lane .. + 7 start
 #pragma unroll
@@ -498,7 +519,7 @@ __global__ void __launch_bounds__(NEXP, 1) group_cluster_kernel(GroupArgs g) {
 extern "C" void k_group(cudaStream_t st, const GroupArgs *g) {
     if (g->nb <= 0) return;
     if (g->nb <= (g->logits ? GS_TOPK : GS_MAXTOK)) {
-        if (g->logits && g->nb == 1) launch_pdl(group_one_kernel, 1, 32, 0, st, *g);
+        if (g->logits && g->nb == 1) launch_pdl(group_one_kernel, 1, 64, 0, st, *g);
         else if (g->logits) launch_pdl(group_cta_kernel<true>, 1, NEXP, 0, st, *g); else launch_pdl(group_cta_kernel<false>, 1, NEXP, 0, st, *g);
         g_launches++; return;
     }

@@ -7,8 +7,9 @@
 #pragma once
 #include "dev_math.cuh"
 
+// exponentials of the logits over their maximum
 template <typename TabT>
-__device__ __forceinline__ void exact_topk_warp(float (&p)[8], const int lane, const TabT *tab, float *row, int &isel, float &wsel, float &tsum) {
+__device__ __forceinline__ void exact_exp_warp(float (&p)[8], const int lane, const TabT *tab) {
     float mx = -1e30f;
 #pragma unroll
     for (int i = 0; i < 8; i++) mx = p[i] > mx ? p[i] : mx;
@@ -16,26 +17,26 @@ __device__ __forceinline__ void exact_topk_warp(float (&p)[8], const int lane, c
     for (int o = 16; o; o >>= 1) { float t = __shfl_xor_sync(0xffffffffu, mx, o); mx = t > mx ? t : mx; }
 #pragma unroll
     for (int i = 0; i < 8; i++) p[i] = dev_expf_tab(__fsub_rn(p[i], mx), tab);
-    __syncwarp();
-    reinterpret_cast<float4 *>(row)[2 * lane] = make_float4(p[0], p[1], p[2], p[3]);
-    reinterpret_cast<float4 *>(row)[2 * lane + 1] = make_float4(p[4], p[5], p[6], p[7]);
-    __syncwarp();
+}
+__device__ __forceinline__ float exact_sum_row(const float *row) {
     float run = 0.0f;
 #pragma unroll 8
     for (int i = 0; i < 64; i++) {
         const float4 v = reinterpret_cast<const float4 *>(row)[i];
         run = __fadd_rn(run, v.x); run = __fadd_rn(run, v.y); run = __fadd_rn(run, v.z); run = __fadd_rn(run, v.w);
     }
-#pragma unroll
-    for (int i = 0; i < 8; i++) p[i] = __fdiv_rn(p[i], run);
-    // Eight rounds of "first strict maximum" (maple.c:917-921).  Probabilities are >= +0, so their bit patterns order like the
-    // values: key = bits + 1, a taken entry becomes 0.  One redux.sync gives the warp's maximum, the lowest lane holding it (and
-    // the lowest of its eight entries) is the first maximum in expert order.
+    return run;
+}
+// N rounds of "first strict maximum" (maple.c:917-921).  Probabilities are >= +0, so their bit patterns order like the
+// values: key = bits + 1, a taken entry becomes 0.  One redux.sync gives the warp's maximum, the lowest lane holding it (and
+// the lowest of its eight entries) is the first maximum in expert order.  Lane k < N returns the k-th, every lane the sum of all in that order.
+template <int N>
+__device__ __forceinline__ void top_select_warp(const float (&p)[8], const int lane, int &isel, float &wsel, float &tsum) {
     unsigned key[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) key[i] = __float_as_uint(p[i]) + 1u;
-    tsum = 0.0f; wsel = 0.0f; isel = 0;
-    for (int k = 0; k < 8; k++) {
+    wsel = 0.0f; isel = 0; tsum = 0.0f;
+    for (int k = 0; k < N; k++) {
         unsigned lk = key[0];
 #pragma unroll
         for (int i = 1; i < 8; i++) lk = max(lk, key[i]);
@@ -51,4 +52,19 @@ __device__ __forceinline__ void exact_topk_warp(float (&p)[8], const int lane, c
         tsum = __fadd_rn(tsum, bv);
         if (lane == k) { wsel = bv; isel = be; }
     }
+}
+// from the exponentials p and their sum
+__device__ __forceinline__ void exact_topk_warp_from(float (&p)[8], const int lane, const float run, int &isel, float &wsel, float &tsum) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) p[i] = __fdiv_rn(p[i], run);
+    top_select_warp<8>(p, lane, isel, wsel, tsum);
+}
+template <typename TabT>
+__device__ __forceinline__ void exact_topk_warp(float (&p)[8], const int lane, const TabT *tab, float *row, int &isel, float &wsel, float &tsum) {
+    exact_exp_warp(p, lane, tab);
+    __syncwarp();
+    reinterpret_cast<float4 *>(row)[2 * lane] = make_float4(p[0], p[1], p[2], p[3]);
+    reinterpret_cast<float4 *>(row)[2 * lane + 1] = make_float4(p[4], p[5], p[6], p[7]);
+    __syncwarp();
+    exact_topk_warp_from(p, lane, exact_sum_row(row), isel, wsel, tsum);
 }
