@@ -100,14 +100,12 @@ __global__ void __launch_bounds__(NW * 32) expert_mma_kernel(ExpertArgs a) {
             float mx = 0.0f;
 #pragma unroll
             for (int i = 0; i < 16; i++) mx = fmaxf(mx, fabsf(v[i]));
-#pragma unroll
-            for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));      // >= 0: the bits order like the values
             const float sc = mx > 0.0f ? __fdiv_rn(mx, 127.0f) : 1.0f, inv = __fdiv_rn(1.0f, sc);
             int tot = 0; uint32_t pk[4] = {0, 0, 0, 0};
 #pragma unroll
             for (int i = 0; i < 16; i++) { int qi = __float2int_rn(__fmul_rn(v[i], inv)); tot += qi; pk[i >> 2] |= (uint32_t)(qi & 0xFF) << (8 * (i & 3)); }
-#pragma unroll
-            for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+            tot = __reduce_add_sync(0xffffffffu, tot);
             // lane holds columns 16 lane .. 16 lane + 15 = piece q = lane
             const int q = lane, G = q >> 3, s = (q & 7) >> 1, h = q & 1, c = G >> 1, tt = (G & 1) * 2 + h;
             *reinterpret_cast<uint4 *>(smem + ((((c * 4 + s) * TN + n) * 4 + tt) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);

@@ -13,8 +13,9 @@ __device__ __forceinline__ void exact_exp_warp(float (&p)[8], const int lane, co
     float mx = -1e30f;
 #pragma unroll
     for (int i = 0; i < 8; i++) mx = p[i] > mx ? p[i] : mx;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) { float t = __shfl_xor_sync(0xffffffffu, mx, o); mx = t > mx ? t : mx; }
+    // (not a NaN) one integer maximum over the warp: the bits of a float order like it once those of the negative ones are turned over
+    const int mb = __reduce_max_sync(0xffffffffu, __float_as_int(mx) ^ (__float_as_int(mx) >> 31 & 0x7FFFFFFF));
+    mx = __int_as_float(mb ^ (mb >> 31 & 0x7FFFFFFF));
 #pragma unroll
     for (int i = 0; i < 8; i++) p[i] = dev_expf_tab(__fsub_rn(p[i], mx), tab);
 }
