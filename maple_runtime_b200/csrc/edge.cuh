@@ -1,15 +1,30 @@
 // edge.cuh -- the joint of two layers for one token and 256 threads: the combine of the one (maple.c:834, as combine_kernel) and the RMSNorm + int8 of the next
 // (as norm_prep_kernel, its sums in the same order).  Thread tid holds float4 tid and tid + 256 of the row.  The row x of token c goes to xo, hn, q, qs and
 // qsum (all with the token's index) unless store is off, and always, in the decode router's layout, to hS (token 0's place there is hS itself).
-// WIRE: the pairs' rows are the tensor-core path's compact ones, as combine_wire_kernel reads them; s_dsp: the experts' down scales in shared memory.
+// pre: edge_pre (not WIRE).  WIRE: the pairs' rows are the tensor-core path's compact ones, as combine_wire_kernel reads them; s_dsp: the experts' down scales in shared memory.
 #pragma once
 #include <stdint.h>
 #include "launch.cuh"
 #include "wire.cuh"
 
 struct EdgeWire { uint8_t *wire; int np_cap; const float *const *dsp; };
+// What the joint reads that is older than the kernel before it (the grouping's tables; the row x, which the joint before this one wrote): read before the wait for
+// that kernel, past L1: 1 token 15.85 -> 15.6 us per layer, 7 26.5 -> 26.05, 13 32.65 -> 32.2, 64 56.7 -> 56.3.  ONE: a single token, whose pairs are 0..7 in order.
+// (The joint on compact rows reads them with the rest: the registers they would hold cost it 0.3 to 0.7 us.)
+struct EdgePre { int slot[8]; float uv[8]; float4 x[2]; };
+template <bool ONE>
+__device__ __forceinline__ EdgePre edge_pre(const int c, const float *uw, const int *tp, const float *x) {
+    EdgePre e;
+#pragma unroll
+    for (int k = 0; k < 8; k++) e.slot[k] = ONE ? k : __ldcg(tp + c * 8 + k);
+#pragma unroll
+    for (int k = 0; k < 8; k++) e.uv[k] = __ldcg(uw + e.slot[k]);
+#pragma unroll
+    for (int k = 0; k < 2; k++) e.x[k] = __ldcg(reinterpret_cast<const float4 *>(x) + (size_t)c * 512 + threadIdx.x + 256 * k);
+    return e;
+}
 template <bool WIRE>
-__device__ __forceinline__ void edge_token(const int c, const float *down, const EdgeWire ew, const float *const *s_dsp, const float *uw, const int *tp, const float *x, float *xo,
+__device__ __forceinline__ void edge_token(const int c, const float *down, const EdgeWire ew, const float *const *s_dsp, const EdgePre &pre, const float *uw, const int *tp, const float *x, float *xo,
                                            const uint2 (&ln)[2], float *hn, int8_t *q, float *qs, int *qsum, float *hS, const bool store) {
     constexpr int HID = 2048, TOPK = 8;
     __shared__ double s_term[16 * 32];
@@ -17,9 +32,9 @@ __device__ __forceinline__ void edge_token(const int c, const float *down, const
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int slot[TOPK]; float uv[TOPK];
 #pragma unroll
-    for (int k = 0; k < TOPK; k++) slot[k] = tp[c * TOPK + k];
+    for (int k = 0; k < TOPK; k++) slot[k] = WIRE ? tp[c * TOPK + k] : pre.slot[k];
 #pragma unroll
-    for (int k = 0; k < TOPK; k++) uv[k] = uw[slot[k]];
+    for (int k = 0; k < TOPK; k++) uv[k] = WIRE ? uw[slot[k]] : pre.uv[k];
     int4 rec[WIRE ? TOPK : 1];                                          // {scale of the pair's int8 row, expert, escape bits}
     if (WIRE) {
 #pragma unroll
@@ -30,7 +45,7 @@ __device__ __forceinline__ void edge_token(const int c, const float *down, const
     for (int k = 0; k < 2; k++) {
         const int i = tid + 256 * k;
         float4 d[TOPK];                                                 // WIRE: the scales
-        v[k] = __ldcg(reinterpret_cast<const float4 *>(x) + (size_t)c * 512 + i);
+        v[k] = WIRE ? __ldcg(reinterpret_cast<const float4 *>(x) + (size_t)c * 512 + i) : pre.x[k];
         if (WIRE) {
             uint2 raw[TOPK];
 #pragma unroll

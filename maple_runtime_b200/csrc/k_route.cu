@@ -660,8 +660,10 @@ __global__ void __launch_bounds__(256, PER_SM) edge_kernel(const float *down, co
     const int tid = threadIdx.x, c = blockIdx.x;
     const uint2 ln[2] = {reinterpret_cast<const uint2 *>(w)[tid], reinterpret_cast<const uint2 *>(w)[tid + 256]};      // weights: read before the wait
     if (WIRE) { static_assert(NEXP == 256, "one entry per thread"); s_dsp[tid] = ew.dsp[tid]; __syncthreads(); }
+    EdgePre pre;
+    if (!WIRE) pre = edge_pre<false>(c, uw, tp, x);
     pdl_wait(); pdl_trigger();
-    edge_token<WIRE>(c, down, ew, s_dsp, uw, tp, x, x, ln, hn, q, qs, qsum, hS + (size_t)c * HID, true);
+    edge_token<WIRE>(c, down, ew, s_dsp, pre, uw, tp, x, x, ln, hn, q, qs, qsum, hS + (size_t)c * HID, true);
 }
 extern "C" void k_edge(cudaStream_t st, const float *down, const float *uw, const int *tp, float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb) {
     if (nb <= 0) return;
@@ -683,14 +685,23 @@ extern "C" void k_edge_wire(cudaStream_t st, uint8_t *wire, int np_cap, const fl
 __global__ void __launch_bounds__(256, 1) combine_kernel(const float *__restrict__ down, const float *__restrict__ uw, const int *__restrict__ tp,
                                                       const float *__restrict__ init, float *__restrict__ out, int nb) {
     const int i = blockIdx.x * 256 + threadIdx.x, b = i >> 9, c = (i & 511) * 4;
+    // the tables and the rows to add to are older than the down kernel: read before the wait for it, past L1
+    int a[TOPK]; float w[TOPK]; float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (b < nb) {
+#pragma unroll
+        for (int k = 0; k < TOPK; k++) a[k] = __ldcg(tp + b * TOPK + k);
+#pragma unroll
+        for (int k = 0; k < TOPK; k++) w[k] = __ldcg(uw + a[k]);
+        if (init) acc = __ldcg(reinterpret_cast<const float4 *>(init + (size_t)b * HID + c));
+    }
     pdl_wait(); pdl_trigger();
     if (b >= nb) return;
-    float4 acc = init ? *reinterpret_cast<const float4 *>(init + (size_t)b * HID + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 d[TOPK];
+#pragma unroll
+    for (int k = 0; k < TOPK; k++) d[k] = *reinterpret_cast<const float4 *>(down + (size_t)a[k] * HID + c);
 #pragma unroll
     for (int k = 0; k < TOPK; k++) {
-        int a = tp[b * TOPK + k]; float w = uw[a];
-        float4 d = *reinterpret_cast<const float4 *>(down + (size_t)a * HID + c);
-        acc.x = __fmaf_rn(w, d.x, acc.x); acc.y = __fmaf_rn(w, d.y, acc.y); acc.z = __fmaf_rn(w, d.z, acc.z); acc.w = __fmaf_rn(w, d.w, acc.w);
+        acc.x = __fmaf_rn(w[k], d[k].x, acc.x); acc.y = __fmaf_rn(w[k], d[k].y, acc.y); acc.z = __fmaf_rn(w[k], d[k].z, acc.z); acc.w = __fmaf_rn(w[k], d[k].w, acc.w);
     }
     *reinterpret_cast<float4 *>(out + (size_t)b * HID + c) = acc;
 }

@@ -249,8 +249,9 @@ __global__ void __launch_bounds__(256, 2) router_small_kernel(const uint8_t *__r
     }
     if (EDGE) {
         const uint2 ln[2] = {reinterpret_cast<const uint2 *>(ed.w)[tid], reinterpret_cast<const uint2 *>(ed.w)[tid + 256]};
+        const EdgePre pre = edge_pre<true>(0, ed.uw, nullptr, ed.x);
         pdl_wait(); pdl_trigger();
-        edge_token<false>(0, ed.down, EdgeWire{}, nullptr, ed.uw, ed.tp, ed.x, ed.xo, ln, ed.hn, ed.q, ed.qs, ed.qsum, reinterpret_cast<float *>(rs_sm), blockIdx.x == 0);
+        edge_token<false>(0, ed.down, EdgeWire{}, nullptr, pre, ed.uw, ed.tp, ed.x, ed.xo, ln, ed.hn, ed.q, ed.qs, ed.qsum, reinterpret_cast<float *>(rs_sm), blockIdx.x == 0);
         __syncthreads();
     } else { pdl_wait(); pdl_trigger(); }
     const bool ok = mbar_wait(&bar, 0, &abort_flag);
