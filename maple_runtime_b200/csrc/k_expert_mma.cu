@@ -46,8 +46,8 @@ __device__ __forceinline__ MoeTile ldcg_tile(const MoeTile *t) {
 // KCH: K-chunks of 256 columns (8 for gate/up K=2048, 2 for down K=512).  NBLK: 8-token blocks per tile.
 // GATEUP: rows block A = gate rows, block B = up rows of the same index, epilogue = SiLU*up;
 // otherwise A and B are two consecutive 16-row blocks of the down matrix, epilogue = scale only.
-// PF: chunks of weights in flight per thread.  NW: warps per CTA.
-template <int KCH, int NBLK, bool GATEUP, int PF, int NW, bool FULL>
+// PF: chunks of weights in flight per thread.  NW: warps per CTA.  ITER: row blocks that a CTA takes in turn (down).
+template <int KCH, int NBLK, bool GATEUP, int PF, int NW, bool FULL, int ITER>
 __global__ void __launch_bounds__(NW * 32) expert_mma_kernel(ExpertArgs a) {
     constexpr bool STAGED = GATEUP && PF == 8;               // gate+up: the tokens' scales come with their rows, not behind the products (one tile deep 17.4 -> 17.2 us per layer, longer lists lose)
     constexpr int TN = NBLK * 8, KB = KCH * 256;            // tokens per tile, bytes of one int8 activation vector
@@ -63,7 +63,8 @@ __global__ void __launch_bounds__(NW * 32) expert_mma_kernel(ExpertArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
 
     const int rows_per_cta = NW * (GATEUP ? 16 : 32);
-    const int r0 = blockIdx.x * rows_per_cta + warp * (GATEUP ? 16 : 32);
+    int r0 = blockIdx.x * (rows_per_cta * ITER) + warp * (GATEUP ? 16 : 32);
+    static_assert(ITER == 1 || (PF == KCH && !GATEUP), "all weights of a round at once");
     const uint8_t *wa = (GATEUP ? ep.gc : ep.dc) + (size_t)(r0 + g) * (KB / 4) + t * 16;
     const uint8_t *wb = GATEUP ? ep.uc + (size_t)(r0 + g) * (KB / 4) + t * 16 : wa + 16 * (KB / 4);
     // the weight stream starts before anything else: the first PF chunks are on their way while the activations are staged
@@ -118,99 +119,110 @@ __global__ void __launch_bounds__(NW * 32) expert_mma_kernel(ExpertArgs a) {
     }
     __syncthreads();
 
-    int acc_a[NBLK][4], acc_b[NBLK][4];
-#pragma unroll
-    for (int j = 0; j < NBLK; j++)
-#pragma unroll
-        for (int k = 0; k < 4; k++) { acc_a[j][k] = 0; acc_b[j][k] = 0; }
-
-#pragma unroll
-    for (int c = 0; c < KCH; c++) {
-        const uint4 wa0 = wq[c % PF][0], wa1 = wq[c % PF][1], wb0 = wq[c % PF][2], wb1 = wq[c % PF][3];
-        if (c + PF < KCH) {   // PF chunks in flight while this one is multiplied
-            wq[c % PF][0] = ldg_stream(wa + (c + PF) * 64); wq[c % PF][1] = ldg_stream(wa + 8 * (KB / 4) + (c + PF) * 64);
-            wq[c % PF][2] = ldg_stream(wb + (c + PF) * 64); wq[c % PF][3] = ldg_stream(wb + 8 * (KB / 4) + (c + PF) * 64);
-        }
-#pragma unroll
-        for (int s = 0; s < 4; s++) {
-            const uint32_t m = 0x03030303u;
-            uint32_t ax0 = (wa0.x >> (2 * s)) & m, ay0 = (wa0.y >> (2 * s)) & m, az0 = (wa0.z >> (2 * s)) & m, aw0 = (wa0.w >> (2 * s)) & m;
-            uint32_t ax1 = (wa1.x >> (2 * s)) & m, ay1 = (wa1.y >> (2 * s)) & m, az1 = (wa1.z >> (2 * s)) & m, aw1 = (wa1.w >> (2 * s)) & m;
-            uint32_t bx0 = (wb0.x >> (2 * s)) & m, by0 = (wb0.y >> (2 * s)) & m, bz0 = (wb0.z >> (2 * s)) & m, bw0 = (wb0.w >> (2 * s)) & m;
-            uint32_t bx1 = (wb1.x >> (2 * s)) & m, by1 = (wb1.y >> (2 * s)) & m, bz1 = (wb1.z >> (2 * s)) & m, bw1 = (wb1.w >> (2 * s)) & m;
-            const uint8_t *bs = smem + ((((c * 4 + s) * TN + g) * 4 + t) << 4);
-#pragma unroll
-            for (int j = 0; j < NBLK; j++) {
-                uint4 q = *reinterpret_cast<const uint4 *>(bs + j * 8 * 64);
-                mma_u8s8(acc_a[j], ax0, ax1, ay0, ay1, q.x, q.y);
-                mma_u8s8(acc_a[j], az0, az1, aw0, aw1, q.z, q.w);
-                mma_u8s8(acc_b[j], bx0, bx1, by0, by1, q.x, q.y);
-                mma_u8s8(acc_b[j], bz0, bz1, bw0, bw1, q.z, q.w);
-            }
-        }
-    }
-
-    // epilogue: acc[j][0..3] = (row g, token 2t), (row g, token 2t+1), (row g+8, token 2t), (row g+8, token 2t+1)
-    if (GATEUP) {
-        // Two tokens at a time: their 32 values lie four to a lane in the eight lanes of one t and go one to a lane, so that the SiLU (a hundred and fifty
-        // instructions, part of them in double) runs once for them and not four times, and not at all for tokens that do not exist: 1 token 17.8 -> 17.2 us per layer,
-        // 4 22.6 -> 22.3, 13 33.4 -> 33.1, 32 46.5 -> 45.3, 64 58.6 -> 57.9, 128 73.9 -> 73.6
-        const int k = lane & 3, rr = r0 + g + (k >> 1) * 8;
-        const float s_a = ep.gs[rr], s_b = ep.us[rr];
-#pragma unroll
-        for (int j = 0; j < NBLK; j++)
 #pragma unroll 1
-            for (int tt = 0; tt < 4 && j * 8 + 2 * tt < tile.cnt; tt++) {
-                const int src = (lane & ~3) | tt, n = j * 8 + 2 * tt + (k & 1), pair = tile.p0 + n;
-                int va[4], vb[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) { va[i] = __shfl_sync(0xffffffffu, acc_a[j][i], src); vb[i] = __shfl_sync(0xffffffffu, acc_b[j][i], src); }
-                if (n >= tile.cnt) continue;
-                const int tok = STAGED ? 0 : a.ptok ? a.ptok[pair] : pair, qsum = STAGED ? t_qsum[n] : a.hqsum[tok];
-                const float qs = STAGED ? t_qs[n] : a.hqs[tok];
-                const int da = (k & 2 ? (k & 1 ? va[3] : va[2]) : (k & 1 ? va[1] : va[0])) - qsum, db = (k & 2 ? (k & 1 ? vb[3] : vb[2]) : (k & 1 ? vb[1] : vb[0])) - qsum;
-                const float gv = __fmul_rn(__fmul_rn((float)da, qs), s_a), uv = __fmul_rn(__fmul_rn((float)db, qs), s_b);
-                a.act[(size_t)pair * 512 + rr] = dev_silu_mul(gv, uv);
-                if (FULL && a.gate) { a.gate[(size_t)pair * 512 + rr] = gv; a.up[(size_t)pair * 512 + rr] = uv; }
-                if (FULL && a.gu_dots) { a.gu_dots[(size_t)pair * 1024 + rr] = da; a.gu_dots[(size_t)pair * 1024 + 512 + rr] = db; }
-            }
-    } else {
-        const float sca[2] = {ep.ds[r0 + g], ep.ds[r0 + g + 8]}, scb[2] = {ep.ds[r0 + g + 16], ep.ds[r0 + g + 24]};
+    for (int it = 0; it < ITER; it++, r0 += rows_per_cta) {
+        int acc_a[NBLK][4], acc_b[NBLK][4];
 #pragma unroll
         for (int j = 0; j < NBLK; j++)
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int n = j * 8 + 2 * t + (k & 1), rr = r0 + g + (k >> 1) * 8;
-                if (n >= tile.cnt) continue;
-                const int pair = tile.p0 + n;
-                int qsum_p; float qs;
-                if (a.act_for_down) { qs = t_qs[n]; qsum_p = t_qsum[n]; }
-                else { qs = a.aqs[pair]; qsum_p = a.aqsum[pair]; }
-                const int da = acc_a[j][k] - qsum_p, db = acc_b[j][k] - qsum_p;
-                float *drow = a.down + (size_t)pair * (a.down_stride ? a.down_stride : 2048);
-                if (FULL && a.rx_src) { const int2 sp = a.rx_src[pair]; drow = a.peer_down[sp.x] + (size_t)sp.y * 2048; }   // the row goes to the token's rank
-                drow[rr] = __fmul_rn(__fmul_rn((float)da, qs), sca[k >> 1]);
-                drow[rr + 16] = __fmul_rn(__fmul_rn((float)db, qs), scb[k >> 1]);
-                if (FULL && a.dn_dots) { a.dn_dots[(size_t)pair * 2048 + rr] = da; a.dn_dots[(size_t)pair * 2048 + rr + 16] = db; }
+            for (int k = 0; k < 4; k++) { acc_a[j][k] = 0; acc_b[j][k] = 0; }
+
+#pragma unroll
+        for (int c = 0; c < KCH; c++) {
+            const uint4 wa0 = wq[c % PF][0], wa1 = wq[c % PF][1], wb0 = wq[c % PF][2], wb1 = wq[c % PF][3];
+            if (c + PF < KCH) {   // PF chunks in flight while this one is multiplied
+                wq[c % PF][0] = ldg_stream(wa + (c + PF) * 64); wq[c % PF][1] = ldg_stream(wa + 8 * (KB / 4) + (c + PF) * 64);
+                wq[c % PF][2] = ldg_stream(wb + (c + PF) * 64); wq[c % PF][3] = ldg_stream(wb + 8 * (KB / 4) + (c + PF) * 64);
             }
+#pragma unroll
+            for (int s = 0; s < 4; s++) {
+                const uint32_t m = 0x03030303u;
+                uint32_t ax0 = (wa0.x >> (2 * s)) & m, ay0 = (wa0.y >> (2 * s)) & m, az0 = (wa0.z >> (2 * s)) & m, aw0 = (wa0.w >> (2 * s)) & m;
+                uint32_t ax1 = (wa1.x >> (2 * s)) & m, ay1 = (wa1.y >> (2 * s)) & m, az1 = (wa1.z >> (2 * s)) & m, aw1 = (wa1.w >> (2 * s)) & m;
+                uint32_t bx0 = (wb0.x >> (2 * s)) & m, by0 = (wb0.y >> (2 * s)) & m, bz0 = (wb0.z >> (2 * s)) & m, bw0 = (wb0.w >> (2 * s)) & m;
+                uint32_t bx1 = (wb1.x >> (2 * s)) & m, by1 = (wb1.y >> (2 * s)) & m, bz1 = (wb1.z >> (2 * s)) & m, bw1 = (wb1.w >> (2 * s)) & m;
+                const uint8_t *bs = smem + ((((c * 4 + s) * TN + g) * 4 + t) << 4);
+#pragma unroll
+                for (int j = 0; j < NBLK; j++) {
+                    uint4 q = *reinterpret_cast<const uint4 *>(bs + j * 8 * 64);
+                    mma_u8s8(acc_a[j], ax0, ax1, ay0, ay1, q.x, q.y);
+                    mma_u8s8(acc_a[j], az0, az1, aw0, aw1, q.z, q.w);
+                    mma_u8s8(acc_b[j], bx0, bx1, by0, by1, q.x, q.y);
+                    mma_u8s8(acc_b[j], bz0, bz1, bw0, bw1, q.z, q.w);
+                }
+            }
+        }
+
+        if (ITER > 1 && it + 1 < ITER) {                         // the next round's weights: on their way while this one's results are stored
+            wa += (size_t)rows_per_cta * (KB / 4); wb += (size_t)rows_per_cta * (KB / 4);
+#pragma unroll
+            for (int p = 0; p < PF; p++) {
+                wq[p][0] = ldg_stream(wa + p * 64); wq[p][1] = ldg_stream(wa + 8 * (KB / 4) + p * 64);
+                wq[p][2] = ldg_stream(wb + p * 64); wq[p][3] = ldg_stream(wb + 8 * (KB / 4) + p * 64);
+            }
+        }
+        // epilogue: acc[j][0..3] = (row g, token 2t), (row g, token 2t+1), (row g+8, token 2t), (row g+8, token 2t+1)
+        if (GATEUP) {
+            // Two tokens at a time: their 32 values lie four to a lane in the eight lanes of one t and go one to a lane, so that the SiLU (a hundred and fifty
+            // instructions, part of them in double) runs once for them and not four times, and not at all for tokens that do not exist: 1 token 17.8 -> 17.2 us per layer,
+            // 4 22.6 -> 22.3, 13 33.4 -> 33.1, 32 46.5 -> 45.3, 64 58.6 -> 57.9, 128 73.9 -> 73.6
+            const int k = lane & 3, rr = r0 + g + (k >> 1) * 8;
+            const float s_a = ep.gs[rr], s_b = ep.us[rr];
+#pragma unroll
+            for (int j = 0; j < NBLK; j++)
+#pragma unroll 1
+                for (int tt = 0; tt < 4 && j * 8 + 2 * tt < tile.cnt; tt++) {
+                    const int src = (lane & ~3) | tt, n = j * 8 + 2 * tt + (k & 1), pair = tile.p0 + n;
+                    int va[4], vb[4];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) { va[i] = __shfl_sync(0xffffffffu, acc_a[j][i], src); vb[i] = __shfl_sync(0xffffffffu, acc_b[j][i], src); }
+                    if (n >= tile.cnt) continue;
+                    const int tok = STAGED ? 0 : a.ptok ? a.ptok[pair] : pair, qsum = STAGED ? t_qsum[n] : a.hqsum[tok];
+                    const float qs = STAGED ? t_qs[n] : a.hqs[tok];
+                    const int da = (k & 2 ? (k & 1 ? va[3] : va[2]) : (k & 1 ? va[1] : va[0])) - qsum, db = (k & 2 ? (k & 1 ? vb[3] : vb[2]) : (k & 1 ? vb[1] : vb[0])) - qsum;
+                    const float gv = __fmul_rn(__fmul_rn((float)da, qs), s_a), uv = __fmul_rn(__fmul_rn((float)db, qs), s_b);
+                    a.act[(size_t)pair * 512 + rr] = dev_silu_mul(gv, uv);
+                    if (FULL && a.gate) { a.gate[(size_t)pair * 512 + rr] = gv; a.up[(size_t)pair * 512 + rr] = uv; }
+                    if (FULL && a.gu_dots) { a.gu_dots[(size_t)pair * 1024 + rr] = da; a.gu_dots[(size_t)pair * 1024 + 512 + rr] = db; }
+                }
+        } else {
+            const float sca[2] = {ep.ds[r0 + g], ep.ds[r0 + g + 8]}, scb[2] = {ep.ds[r0 + g + 16], ep.ds[r0 + g + 24]};
+#pragma unroll
+            for (int j = 0; j < NBLK; j++)
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int n = j * 8 + 2 * t + (k & 1), rr = r0 + g + (k >> 1) * 8;
+                    if (n >= tile.cnt) continue;
+                    const int pair = tile.p0 + n;
+                    int qsum_p; float qs;
+                    if (a.act_for_down) { qs = t_qs[n]; qsum_p = t_qsum[n]; }
+                    else { qs = a.aqs[pair]; qsum_p = a.aqsum[pair]; }
+                    const int da = acc_a[j][k] - qsum_p, db = acc_b[j][k] - qsum_p;
+                    float *drow = a.down + (size_t)pair * (a.down_stride ? a.down_stride : 2048);
+                    if (FULL && a.rx_src) { const int2 sp = a.rx_src[pair]; drow = a.peer_down[sp.x] + (size_t)sp.y * 2048; }   // the row goes to the token's rank
+                    drow[rr] = __fmul_rn(__fmul_rn((float)da, qs), sca[k >> 1]);
+                    drow[rr + 16] = __fmul_rn(__fmul_rn((float)db, qs), scb[k >> 1]);
+                    if (FULL && a.dn_dots) { a.dn_dots[(size_t)pair * 2048 + rr] = da; a.dn_dots[(size_t)pair * 2048 + rr + 16] = db; }
+                }
+        }
     }
     if (dense && tid == 0) span_end(a.span);
 }
 
-template <int KCH, int NBLK, bool GATEUP, int PF, int NW, bool FULL>
+template <int KCH, int NBLK, bool GATEUP, int PF, int NW, bool FULL, int ITER>
 static void launch_as(cudaStream_t st, const ExpertArgs *a) {
     const size_t smem = (size_t)KCH * 4 * NBLK * 8 * 64 + NBLK * 8 * 8;   // + scale and code sum per token
     static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<KCH, NBLK, GATEUP, PF, NW, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
-    dim3 grid((GATEUP ? 32 : 64) / NW, a->max_tiles);
-    launch_pdl(expert_mma_kernel<KCH, NBLK, GATEUP, PF, NW, FULL>, grid, NW * 32, smem, st, *a);
+    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<KCH, NBLK, GATEUP, PF, NW, FULL, ITER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
+    dim3 grid((GATEUP ? 32 : 64) / (NW * ITER), a->max_tiles);
+    launch_pdl(expert_mma_kernel<KCH, NBLK, GATEUP, PF, NW, FULL, ITER>, grid, NW * 32, smem, st, *a);
     k_count_add(1);
 }
 // FULL: the stage outputs and the rows that go to other ranks, which the lean kernels have no code for (13 tokens 35.1 -> 34.8 us per layer, 64 60.6 -> 60.1)
-template <int KCH, int NBLK, bool GATEUP, int PF, int NW>
+template <int KCH, int NBLK, bool GATEUP, int PF, int NW, int ITER = 1>
 static void launch(cudaStream_t st, const ExpertArgs *a) {
-    if (GATEUP ? a->gate != NULL || a->gu_dots != NULL : a->dn_dots != NULL || a->rx_src != NULL) launch_as<KCH, NBLK, GATEUP, PF, NW, true>(st, a);
-    else launch_as<KCH, NBLK, GATEUP, PF, NW, false>(st, a);
+    if (GATEUP ? a->gate != NULL || a->gu_dots != NULL : a->dn_dots != NULL || a->rx_src != NULL) launch_as<KCH, NBLK, GATEUP, PF, NW, true, ITER>(st, a);
+    else launch_as<KCH, NBLK, GATEUP, PF, NW, false, ITER>(st, a);
 }
 // Two chunks in flight leave room for six CTAs per SM, which is what a long list of tiles wants (four chunks: 64 tokens 34.5 instead of 31 us).
 // Where the whole list is resident at once at one or two CTAs per SM, all eight chunks go out together: one trip to memory instead of four
@@ -219,9 +231,11 @@ static void launch(cudaStream_t st, const ExpertArgs *a) {
 // Eight warps per CTA share a tile's staged rows once an expert has several pairs: 192 tokens 86.2 -> 82.5 us per layer, 160 80.6 -> 79.0, 128 the same, but
 // 64 tokens 60.8 -> 61.8.  max_tiles is 256 + the tokens, as many tiles as there could be.
 #define NW8_TILES 384
-// The down kernel, whose CTAs each quantise the tile's activations for themselves, from 96 tokens: 96 66.9 -> 66.7 us per layer, 112 71.1 -> 70.5, 128 73.6 -> 72.4, but 72 tokens
-// 62.3 -> 62.8 and 32 45.2 -> 46.0.
-#define DOWN8_TILES 351
+// The down kernel's CTAs each quantise the tile's activations for themselves and wait for its tile and its pointers: with more tiles than CTAs fit at once they take two
+// or four blocks of 128 rows in turn, the next one's codes on their way while the results of this one are stored.  Rounds 1 / 2 / 4: 32 tokens 44.2 / 44.2 / 47.9 us per layer,
+// 52 53.3 / 53.2 / 55.5, 64 56.4 / 55.9 / 57.8, 96 66.8 / 64.5 / 64.9, 112 71.1 / 68.4 / 68.1, 128 73.6 / 70.4 / 69.5.
+#define DOWN2_TILES 304
+#define DOWN4_TILES 360
 extern "C" void k_gateup_mma(cudaStream_t st, const ExpertArgs *a, int tn) {
     if (a->max_tiles <= 0) return;
     if (tn != 8) launch<8, 4, true, 2, 4>(st, a); else if (a->max_tiles <= PF8_TILES) launch<8, 1, true, 8, 4>(st, a);
@@ -229,7 +243,8 @@ extern "C" void k_gateup_mma(cudaStream_t st, const ExpertArgs *a, int tn) {
 }
 extern "C" void k_down_mma(cudaStream_t st, const ExpertArgs *a, int tn) {
     if (a->max_tiles <= 0) return;
-    if (tn != 8) launch<2, 4, false, 2, 4>(st, a); else if (a->max_tiles <= DOWN8_TILES) launch<2, 1, false, 2, 4>(st, a); else launch<2, 1, false, 2, 8>(st, a);
+    if (tn != 8) launch<2, 4, false, 2, 4>(st, a); else if (a->max_tiles <= DOWN2_TILES) launch<2, 1, false, 2, 4>(st, a);
+    else if (a->max_tiles <= DOWN4_TILES) launch<2, 1, false, 2, 4, 2>(st, a); else launch<2, 1, false, 2, 4, 4>(st, a);
 }
 
 // The attention projections (gpu_pre.m:200-256 gpre_dense*): the same int8 x 2-bit product with one matrix instead of 256
@@ -240,8 +255,8 @@ template <int NBLK, int PF>
 static void launch_dense(cudaStream_t st, const ExpertArgs *a, int rows) {
     const size_t smem = (size_t)8 * 4 * NBLK * 8 * 64 + NBLK * 8 * 8;
     static bool attr_done = false;
-    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<8, NBLK, false, PF, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
-    launch_pdl(expert_mma_kernel<8, NBLK, false, PF, 4, false>, dim3(rows / 128, (a->dense_n + NBLK * 8 - 1) / (NBLK * 8)), 128, smem, st, *a);
+    if (!attr_done) { cudaFuncSetAttribute(expert_mma_kernel<8, NBLK, false, PF, 4, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); attr_done = true; }
+    launch_pdl(expert_mma_kernel<8, NBLK, false, PF, 4, false, 1>, dim3(rows / 128, (a->dense_n + NBLK * 8 - 1) / (NBLK * 8)), 128, smem, st, *a);
     k_count_add(1);
 }
 extern "C" void k_dense_mma(cudaStream_t st, const ExpertArgs *a, int rows) {

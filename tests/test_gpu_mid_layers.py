@@ -51,19 +51,20 @@ def test_layers_in_one_call_equal_layers_one_by_one(nb, l0, stacks, gpu, weights
         g.keep_stages(True)
 
 
-@pytest.mark.parametrize("nb", [160, 161, 208])
-def test_where_the_tensor_cores_take_over(nb, stacks, gpu, weights):
-    """160 tokens are the last on the mma.sync kernels, 161 the first on the tcgen05 ones: both like the mma.sync kernels, bit for bit."""
+@pytest.mark.parametrize("nb", [48, 49, 104, 105, 160, 161, 208])
+def test_where_the_expert_kernels_change(nb, stacks, gpu, weights):
+    """Up to 48, 104 and 160 tokens the mma.sync down kernel takes one, two and four blocks of rows per CTA; from 161 the tcgen05 kernels run.  Either path alone
+    and the one that the size chooses: the same bits."""
     g = gpu
     x = weights.hidden(950 + nb, nb)
     out = {}
     g.keep_stages(False)
     try:
-        for path in (1, 0):
+        for path in (1, 2, 0):
             g.set_path(path)
             out[path] = x.copy()
             g.forward(out[path], 0, 3)
     finally:
         g.set_path(0)
         g.keep_stages(True)
-    assert same_bits(out[0], out[1])
+    assert same_bits(out[0], out[1]) and same_bits(out[0], out[2])
