@@ -177,6 +177,12 @@ __device__ __forceinline__ void tma_acquire_map_sys(const void *tmap) { asm vola
 // queued behind it wait too
 __device__ __forceinline__ void tma_prefetch_map(const void *tmap) { asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory"); }
 
+// ---- bulk copies shared -> global: 16-byte aligned, a multiple of 16 bytes; a thread's own copies have left shared memory when its wait returns ----
+__device__ __forceinline__ void bulk_store(void *dst, uint32_t src_smem, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src_smem), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_store_wait() { asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // ---- asynchronous 16-byte copies global -> shared (gathered activation rows) -------------------------------------
 __device__ __forceinline__ void cp_async16(uint32_t dst_smem, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_smem), "l"(src) : "memory");
