@@ -28,7 +28,8 @@ extern "C" void k_count_add(long n) { g_launches += n; }
 // ------------------------------------------------------------------------------------------------------------
 // RMSNorm (maple.c:398-402) + prep (maple.c:184-194), one warp per token: lane l holds columns 128 i + 4 l .. + 3 for i = 0..15 (every
 // load and store instruction of the warp covers one contiguous run of the row, all sixteen loads are in flight together, and the three
-// reductions are shuffles: no block-wide barrier).  WPC warps (tokens) per CTA: 8 for chunks, 1 for decode batches (more CTAs).
+// reductions are shuffles: no block-wide barrier).  CTAs of one warp spread evenly over the SMs at every size (eight per CTA before: 512 tokens 93.8 -> 92.7 us per layer,
+// 843 103.7 -> 103.2, 1300 123.3 -> 121.4, 2048 153.8 -> 153.4; launched programmatically 512 tokens take 96.2).
 // w == NULL: x is already normalised (hn = x, not rewritten when hn == x).
 // The sum of squares is accumulated in double like the reference; the tree order differs from its left-to-right
 // order only below double precision, which the conversion to float absorbs.
@@ -36,16 +37,15 @@ extern "C" void k_count_add(long n) { g_launches += n; }
 // hS != NULL: the normalised row is also stored as the decode router wants it, [column / 32][lane j][4 steps] (k_router_tile.cu).
 // hA != NULL: the normalised row is also stored as two fp16 terms, hi = fp16(h) in columns 0..2047 and lo = fp16(h - hi) in columns
 // 2048..4095 of a 4096-column row (the tensor-core router's A operand, k_router_umma.cu), and its Euclidean norm goes to hnorm.
-template <int WPC>
-__global__ void __launch_bounds__(WPC * 32) norm_prep_kernel(const float *__restrict__ x, const uint16_t *__restrict__ w,
+__global__ void __launch_bounds__(32) norm_prep_kernel(const float *__restrict__ x, const uint16_t *__restrict__ w,
                                                              float *__restrict__ hn, int8_t *__restrict__ q,
                                                              float *__restrict__ qs, int *__restrict__ qsum, float *__restrict__ hS,
                                                              __half *__restrict__ hA, float *__restrict__ hnorm, int nb,
                                                              const float *__restrict__ bias_src, float *__restrict__ bias) {
-    const int lane = threadIdx.x & 31, b = blockIdx.x * WPC + (threadIdx.x >> 5);
+    const int lane = threadIdx.x, b = blockIdx.x;
     pdl_wait(); pdl_trigger();
     if (b >= nb) {
-        if (WPC == 1 && bias_src) {
+        if (bias_src) {
             const float4 *s = reinterpret_cast<const float4 *>(bias_src) + lane; float4 *d = reinterpret_cast<float4 *>(bias) + lane;
             const float4 u = s[0], v = s[32];
             d[0] = u; d[32] = v;
@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(WPC * 32) norm_prep_kernel(const float *__rest
 }
 static void norm_launch(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, float *hS, __half *hA, float *hnorm, int nb) {
     if (nb <= 0) return;
-    if (nb > 256) launch_k(norm_prep_kernel<8>, (nb + 7) / 8, 256, 0, st, x, w, hn, q, qs, qsum, hS, hA, hnorm, nb, (const float *)NULL, (float *)NULL);
-    else launch_pdl(norm_prep_kernel<1>, nb, 32, 0, st, x, w, hn, q, qs, qsum, hS, hA, hnorm, nb, (const float *)NULL, (float *)NULL);
+    if (nb > 256) launch_k(norm_prep_kernel, nb, 32, 0, st, x, w, hn, q, qs, qsum, hS, hA, hnorm, nb, (const float *)NULL, (float *)NULL);
+    else launch_pdl(norm_prep_kernel, nb, 32, 0, st, x, w, hn, q, qs, qsum, hS, hA, hnorm, nb, (const float *)NULL, (float *)NULL);
     g_launches++;
 }
 extern "C" void k_norm_prep(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, int nb) {
@@ -133,7 +133,7 @@ extern "C" void k_norm_prep_relaid(cudaStream_t st, const float *x, const uint16
 }
 // One more CTA brings the call's bias from the host's page-locked memory: no pageable copy in front of the kernels (24 calls of 1 token 1182 -> 1113 us, 7 1502 -> 1464).
 extern "C" void k_norm_prep_call(cudaStream_t st, const float *x, float *hn, int8_t *q, float *qs, int *qsum, float *hS, int nb, const float *bias_src, float *bias) {
-    launch_pdl(norm_prep_kernel<1>, nb + (bias_src != NULL), 32, 0, st, x, (const uint16_t *)NULL, hn, q, qs, qsum, hS, (__half *)NULL, (float *)NULL, nb, bias_src, bias);
+    launch_pdl(norm_prep_kernel, nb + (bias_src != NULL), 32, 0, st, x, (const uint16_t *)NULL, hn, q, qs, qsum, hS, (__half *)NULL, (float *)NULL, nb, bias_src, bias);
     g_launches++;
 }
 extern "C" void k_norm_prep_split(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, void *hA, float *hnorm, int nb) {
