@@ -393,7 +393,8 @@ static void fill_expert_args(ExpertArgs *a, const ExpertPtrs *tab, const ExpertM
     if (S.keep || use_umma(nb)) { a->gate = S.gate; a->up = S.up; }          /* the tensor-core GEMM always stores gate and up */
     if (S.keep) { a->gu_dots = S.gu_dots; a->dn_dots = S.dn_dots; }
 }
-/* the permute: int8 rows into pair order for the TMA, their scales and code sums with them */
+/* the permute: int8 rows into pair order for the TMA, their scales and code sums with them; by pair for a host's tables, by token for those made here */
+static void run_scatter(int nb) { k_scatter_rows(S.st, S.hq, S.hqs, S.hqsum, S.tp, S.hq_sorted, S.hqs_sorted, S.hqsum_sorted, nb); }
 static void run_gather(int nb) { k_gather_rows(S.st, S.hq, S.hqs, S.hqsum, S.utok, S.hq_sorted, S.hqs_sorted, S.hqsum_sorted, nb * TOPK); }
 static void run_group_l(int nb, int marked, const float *logits);
 static void run_group_m(int nb, int marked) { run_group_l(nb, marked, NULL); }
@@ -406,7 +407,7 @@ static void run_group_l(int nb, int marked, const float *logits) {
     g.ustart = S.ustart; g.utok = S.utok; g.slot = S.slot; g.tp = S.tp; g.uw = S.uw; g.ecnt = S.ecnt; g.uexp = S.uexp;
     g.tiles_a = S.tiles_a; g.tiles_b = S.tiles_b; g.ntiles_a = S.ntiles_a; g.ntiles_b = S.ntiles_b; g.tn_a = tile_tn(nb); g.tn_b = UMMA_TN;
     k_group(S.st, &g);
-    if (use_umma(nb) && !S.ep_on) run_gather(nb);
+    if (use_umma(nb) && !S.ep_on) run_scatter(nb);
 }
 static void run_group(int nb) { run_group_m(nb, 0); }
 /* which: 1 gateup, 2 actq, 4 down; dsp: the down-scale pointers the tiles' expert indices name (the combine needs the same) */

@@ -124,6 +124,8 @@ void k_down_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap);
 void k_dense_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap);
 /* dst[pair] = src[rows[pair]]: 2048-byte int8 rows put into pair (expert-grouped) order; their scales and code sums likewise */
 void k_gather_rows(cudaStream_t st, const int8_t *src, const float *qs, const int *qsum, const int *rows, int8_t *dst, float *dqs, int *dqsum, int np);
+/* the same by token: its eight slots are tp[8 b ..] (16-byte aligned) */
+void k_scatter_rows(cudaStream_t st, const int8_t *src, const float *qs, const int *qsum, const int *tp, int8_t *dst, float *dqs, int *dqsum, int nb);
 
 /* ---- the head of the attention half (k_attn_prep.cu): q/k RMS norm, half-rotary embedding, fp16 keys and values.  qkv [nb][3072]
  * = q 2048 | k 512 | v 512; pos [nb]; qn, kn [128] fp32; cs [cs_positions][32][2] (cos, sin); q [nb][2048] fp32; kc, vc [nb][512] fp16 */
