@@ -1216,13 +1216,13 @@ int gpre_dense_done(int maxtok) {
 /* A call is cut into chunks of 256 tokens, whose rows cross the link in both directions while other chunks are multiplied: 14 us of kernel
  * against 57 us for the 3.1 MB of q,k,v results, so a chunk need not fill the card. */
 #define DENSE_CHUNK 256
-typedef struct { int g, nb, spans; } DenseCall;
+typedef struct { int g, nb, spans; float *y; } DenseCall;
 static int dense_rows(void *ctx, int r, int n) {
     const DenseCall *c = ctx;
     const int ys = DG[c->g].rows, um = n > 128 && ys % 256 == 0;
     ExpertArgs a; memset(&a, 0, sizeof a);
     a.tab = DG[c->g].tab; a.maps = DG[c->g].maps; a.err = S.err; a.dense_p0 = r; a.dense_n = n;
-    a.aq = S.hq; a.aqs = S.hqs; a.aqsum = S.hqsum; a.down = DY; a.down_stride = ys; a.dense_mblocks = ys / 256;
+    a.aq = S.hq; a.aqs = S.hqs; a.aqsum = S.hqsum; a.down = c->y; a.down_stride = ys; a.dense_mblocks = ys / 256;
     if (c->spans) a.span = span_next();
     if (um) k_dense_umma(S.st, &a, &bmap_tok); else k_dense_mma(S.st, &a, ys);
     if (c->spans && r + n == c->nb) span_close();
@@ -1240,8 +1240,8 @@ static double dense_call(int g, const float *x, int nb, float *y) {
     if (g < 0 || g >= DGRP || !DG[g].codes) { fail("gpre", "gpre_dense: group %d has no matrices on the card", g); return -1.0; }
     if (nb < 1 || nb > DY_tok) { fail("gpre", "gpre_dense: %d tokens outside 1..%d", nb, DY_tok); return -1.0; }
     if (S.keep && rows_in("gpre", S.hn, x, nb)) return -1.0;
-    DenseCall d = {g, nb, 0};
-    if (nb <= INPLACE_MAXTOK && DG[g].rows <= INPLACE_WIDE) {      /* three kernels in a row: int8 rows in, the product, its rows out */
+    DenseCall d = {g, nb, 0, DY};
+    if (nb <= INPLACE_MAXTOK && DG[g].rows <= INPLACE_WIDE) {      /* two kernels in a row: int8 rows in, the product with its rows straight out (copied out by a kernel of its own: 64 tokens 73.9 and 66.5 us a call for q,k,v and o, like this 69.5 and 63) */
         if (tables_begin("gpre")) return -1.0;
         QuantJob j = {x, nb, tables_add(S.hq, (size_t)nb * HID), tables_add(S.hqs, (size_t)nb * 4), tables_add(S.hqsum, (size_t)nb * 4)};
         if ((size_t)nb * HID * 4 < HIO_POOL_BYTES) { for (int i = 0; i * QUANT_ROWS < nb; i++) quant_piece(&j, i); }
@@ -1249,8 +1249,8 @@ static double dense_call(int g, const float *x, int nb, float *y) {
         const size_t bytes = (size_t)nb * DG[g].rows * 4;
         cudaEventRecord(S.e0, S.st);
         k_tables(S.st, &CT.seg);             /* no event behind it: the call waits for the stream anyway, and the product is launched programmatically */
+        d.y = H_ROWS_OUT;
         dense_rows(&d, 0, nb);
-        k_rows(S.st, H_ROWS_OUT, DY, bytes);
         cudaEventRecord(S.e1, S.st);
         S.nb_cur = nb;
         const double t = finish("gpre");

@@ -185,6 +185,24 @@ __global__ void __launch_bounds__(NW * 32) expert_mma_kernel(ExpertArgs a) {
                     if (FULL && a.gate) { a.gate[(size_t)pair * 512 + rr] = gv; a.up[(size_t)pair * 512 + rr] = uv; }
                     if (FULL && a.gu_dots) { a.gu_dots[(size_t)pair * 1024 + rr] = da; a.gu_dots[(size_t)pair * 1024 + 512 + rr] = db; }
                 }
+        } else if (dense && NBLK == 1) {
+            // the tile's 8 x 128 results through shared memory, so that a token's 128 leave as one run of 512 bytes: the rows may be page-locked host memory
+            constexpr int PITCH = NW * 32 + 4;                   // the four token pairs of a store eight banks apart
+            const float sca[2] = {ep.ds[r0 + g], ep.ds[r0 + g + 8]}, scb[2] = {ep.ds[r0 + g + 16], ep.ds[r0 + g + 24]};
+            float *const out = reinterpret_cast<float *>(smem);
+            float qs2[2]; int qsum2[2];
+#pragma unroll
+            for (int i = 0; i < 2; i++) { const int pair = tile.p0 + min(2 * t + i, tile.cnt - 1); qs2[i] = a.aqs[pair]; qsum2[i] = a.aqsum[pair]; }
+            __syncthreads();                                     // the activations have been read
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                float *o = out + (2 * t + (k & 1)) * PITCH + warp * 32 + g + (k >> 1) * 8;
+                o[0] = __fmul_rn(__fmul_rn((float)(acc_a[0][k] - qsum2[k & 1]), qs2[k & 1]), sca[k >> 1]);
+                o[16] = __fmul_rn(__fmul_rn((float)(acc_b[0][k] - qsum2[k & 1]), qs2[k & 1]), scb[k >> 1]);
+            }
+            __syncthreads();
+            for (int n = warp; n < tile.cnt; n += NW)
+                reinterpret_cast<float4 *>(a.down + (size_t)(tile.p0 + n) * a.down_stride + blockIdx.x * (NW * 32))[lane] = reinterpret_cast<const float4 *>(out + n * PITCH)[lane];
         } else {
             const float sca[2] = {ep.ds[r0 + g], ep.ds[r0 + g + 8]}, scb[2] = {ep.ds[r0 + g + 16], ep.ds[r0 + g + 24]};
 #pragma unroll
