@@ -12,13 +12,13 @@
 //   weights  HBM -> shared memory, still 2-bit packed: TMA tiled copies (cp.async.bulk.tensor, one tensor map per expert
 //            matrix, box = 128 bytes x 128 rows, 128-byte swizzle), 32 KB stages = 256 rows x 512 columns; the swizzle makes
 //            the later row-per-thread reads free of bank conflicts;
-//   decode   eight warps; a thread owns one row of each accumulator half and every second 128-column block: it reads 32 packed
+//   decode   eight warps; a thread owns one row of each accumulator half and every second block (of 128 or 256 columns): per 128 columns it reads 32 packed
 //            bytes per row, expands every 32-bit word with (w >> 2s) & 0x03030303 (the four codes of columns 32s+4j..32s+4j+3
 //            of the group, in column order; convert.py:29-33) and writes the block with tcgen05.st into the tensor-memory A
 //            operand: lane = row, one 32-bit cell = four consecutive K values.  Decoded weights never touch shared memory;
-//   B        int8 activation rows in pair order (a gather kernel puts the tokens' rows into expert-grouped order first), TMA
+//   B        int8 activation rows in pair order (the tokens' rows are put into expert-grouped order first), TMA
 //            tiled copies (box = 128 bytes x 32, 64 or 96 rows, whichever covers the tile's pairs; 128-byte swizzle = the
-//            K-major layout the MMA descriptor names), one 128-column block per stage.
+//            K-major layout the MMA descriptor names), one block per stage.
 // Arithmetic = maple.c:425-458: out = (float)(sum(code*q) - qsum) * qs * s[r]; integer sums are exact.  gate+up scales here;
 // down stores sum(code*q) - qsum as integers and the combine applies qs and s[r] (same two roundings, same order).
 //
@@ -30,15 +30,16 @@
 // copying warps' loops unrolled whole, stage outputs and expert parallelism beside the lean path); they are 26 to 31 KB now, and with nothing else changed a layer of 301 / 843 /
 // 2048 tokens took 93.2 / 116.3 / 163.4 us instead of 97.5 / 119.9 / 168.0.  So: loops over blocks, stages and items stay rolled, one copy of an epilogue piece, a
 // predicated block of MMAs instead of a branch per MMA, and FULL = the variant with stage outputs and expert parallelism.  With the three points below: 92.4 / 114.0 / 162.2.
-// One barrier pair per 128-column block (k_full: the four decode warps that wrote the A stage, and the bytes of the B stage; k_empty: both MMA warps) instead of one per
+// One barrier pair per block (k_full: the four decode warps that wrote the A stage, and the bytes of the B stage; k_empty: both MMA warps) instead of one per
 // ring: a wait that succeeds at once still costs a warp 100 to 180 cycles here.  A look at the next barrier ahead of time (test_wait) made it slower (92.9 / 114.8 / 163.1): more
 // instructions.  One MMA warp for both halves: 93.2 / 115.3 / 163.5.  Sixteen decode warps, one half each: 96.9 / 121.6 / 173.9, at 72 registers a thread.
-// Tensor memory: three A stages of 64 columns (two: 94.2 / 116.7 / 163.1), and 320 columns which the accumulators of two items share, even items from the low end and odd
-// ones from the high end, 2 N columns each: neighbours of up to 160 pairs (rounded up to 16s) fit beside each other, so that an item's epilogue runs under the next
-// one's MMAs; larger ones wait for each other (acc_place).
+// Tensor memory: A stages for two blocks of 256 or three of 128 columns (UmShape), and the rest, which the accumulators of two items share, even items from the low end
+// and odd ones from the high end, 2 N columns each: those that fit beside each other (pairs rounded up to 16s, 128 or 160 for both) let an item's epilogue run under the next
+// one's MMAs; larger ones wait for each other (acc_place).  Deeper rings are not faster: B stages 3 against 4 of 256 columns 99.3 and 100.1 us at 843 tokens, weight stages 4
+// against 3 83.3 and 82.5 at 301 (2: 86.2); tiles of 32 pairs in the room that leaves: level.
 // The codes are read once per tile: their copies say so to the L2 (evict_first), which then still holds the rows that come in, the results and what the next kernels read
 // when they are asked for: a layer of 301 / 511 / 843 / 2048 tokens 92.1 / 104.4 / 113.8 / 159.8 -> 88.1 / 99.6 / 111.0 / 157.4 us.
-// An item's scales come in pair order (gather_rows_kernel puts them there): through the token index they were a second global read in front of every item.
+// An item's scales come in pair order (the kernels at the end of this file put them there): through the token index they were a second global read in front of every item.
 // Every mbarrier wait is bounded (umma.cuh): on a timeout the CTA raises args.err, frees tensor memory and returns.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -52,13 +53,16 @@
 extern "C" void k_count_add(long n);
 
 #define UM_TN UMMA_TN                /* 96 */
-#define UM_WSTAGES 3                 /* four 128-column blocks each */
 #define UM_NACC 2                    /* items whose accumulators are in use at a time: an item's epilogue runs under the next item's MMAs */
-#define UM_NA 3                      /* A stages: one 128-column block of both halves (64 columns) each */
-#define UM_ACC (512 - 64 * UM_NA)    /* columns the accumulators share */
-#define UM_BSTAGES 8                 /* B stages in shared memory: one 128-column block each */
-#define UM_WBYTES (256 * 128)
-#define UM_BBYTES (UM_TN * 128)
+#define UM_WBYTES (256 * 128)        /* a weight stage: 256 rows x 512 columns */
+#define UM_WSTAGES 3
+#define UM_BSTAGES 8                 /* at most */
+// What is handed over at a time: BW x 128 columns.  NA A stages (64 BW columns of tensor memory each: the block in both halves), the rest of tensor memory for the
+// accumulators; BST stages of the tile's rows, BW sub-tiles of 128 columns each.
+template <int BW> struct UmShape {
+    static constexpr int NA = BW == 2 ? 2 : 3, ACC = 512 - 64 * BW * NA, BST = BW == 2 ? 3 : 8, BBYTES = UM_TN * 128 * BW, KCOLS = 128 * BW;
+    static_assert(ACC >= 2 * UM_TN && NA < BST && BST <= UM_BSTAGES, "stages");
+};
 
 struct __align__(16) UmShared {
     uint64_t w_full[UM_WSTAGES], w_empty[UM_WSTAGES], k_full[UM_BSTAGES], k_empty[UM_BSTAGES], acc_full[UM_NACC], acc_empty[UM_NACC];
@@ -71,36 +75,36 @@ __device__ __forceinline__ MoeTile ldcg_tile(const MoeTile *t) {
     const int4 v = __ldcg(reinterpret_cast<const int4 *>(t)); return MoeTile{v.x, v.y, v.z, v.w};
 }
 
-template <int KB, int MODE, bool FULL>
+template <int K, int MODE, bool FULL, int BW>
 __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const __grid_constant__ TMap4 bmap) {
     extern __shared__ __align__(1024) uint8_t um_smem_raw[];
     uint8_t *base = (uint8_t *)(((uintptr_t)um_smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t *wsm = base;                                              // UM_WSTAGES x 32 KB packed weights
-    uint8_t *bsm = base + UM_WSTAGES * UM_WBYTES;                      // UM_BSTAGES x 12 KB int8 activations
+    uint8_t *wsm = base;                                              // packed weights
+    using SH = UmShape<BW>;
+    uint8_t *bsm = base + UM_WSTAGES * UM_WBYTES;                         // int8 activations
     __shared__ UmShared sh_static;                                    // static, so that the compiler knows these accesses are shared-memory ones
     UmShared *sh = &sh_static;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     constexpr bool GATEUP = MODE == 0, DENSE = MODE == 2, DOWN = MODE == 1;
-    constexpr int NA = UM_NA;
+    constexpr int NA = SH::NA, WST = UM_WSTAGES, BST = SH::BST, KB = K / SH::KCOLS, BPS = 4 / BW, TN = UM_TN;      // KB: blocks of an item, BPS: of a weight stage
     constexpr int NACC = UM_NACC;
-    constexpr uint32_t ACOL = UM_ACC;                               // first A column (behind the accumulators)
-    static_assert(UM_ACC >= 2 * UM_TN && NACC == 2 && NA < UM_BSTAGES, "tensor memory");
-    static_assert(KB % 4 == 0, "blocks");
+    constexpr uint32_t ACOL = SH::ACC;                              // first A column (behind the accumulators)
+    static_assert(NACC == 2 && KB % BPS == 0, "blocks");
     const int MB = GATEUP ? 4 : (DENSE ? a.dense_mblocks : 8);      // 256-row blocks of the matrix (gate+up: 128 + 128)
-    constexpr int NSB = KB / 4;
+    constexpr int NSB = KB / BPS;
     volatile int *abortp = &sh->abort_flag;
 
     if (tid == 0) {
-        for (int s = 0; s < UM_WSTAGES; s++) { mbar_init(&sh->w_full[s], 1); mbar_init(&sh->w_empty[s], 8); }
+        for (int s = 0; s < WST; s++) { mbar_init(&sh->w_full[s], 1); mbar_init(&sh->w_empty[s], 8); }
         // an A stage is full when its four decode warps have stored it, a B stage when its bytes have landed; both are empty again
         // when both issuing warps' MMAs on them have completed
-        for (int s = 0; s < UM_BSTAGES; s++) { mbar_init(&sh->k_full[s], 5); mbar_init(&sh->k_empty[s], 2); }
+        for (int s = 0; s < BST; s++) { mbar_init(&sh->k_full[s], 5); mbar_init(&sh->k_empty[s], 2); }
         for (int b = 0; b < NACC; b++) { mbar_init(&sh->acc_full[b], 2); mbar_init(&sh->acc_empty[b], 8); }
         sh->abort_flag = 0; mbar_init_fence();
     }
-    const int ntiles = DENSE ? (a.dense_n + UM_TN - 1) / UM_TN : __ldcg(a.ntiles), nitems = ntiles * MB;
+    const int ntiles = DENSE ? (a.dense_n + TN - 1) / TN : __ldcg(a.ntiles), nitems = ntiles * MB;
     auto tile_at = [&](const int i) {
-        return DENSE ? MoeTile{0, a.dense_p0 + i * UM_TN, min(UM_TN, a.dense_n - i * UM_TN), 0} : ldcg_tile(a.tiles + i);
+        return DENSE ? MoeTile{0, a.dense_p0 + i * TN, min(TN, a.dense_n - i * TN), 0} : ldcg_tile(a.tiles + i);
     };
     // The CTA acquires the maps that it will read through, all of them before its first copy and each by a thread of its own: that adds 0.5 us to a layer of two
     // such kernels (301 tokens 97.6 -> 98.1 us, 2048 168.2 -> 169.0).  By the weight warp ahead of each item it added 6.5 us, by the decode warps while
@@ -129,51 +133,52 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
     // where item number i of this CTA keeps its accumulators (half 0, then half 1, n2 columns in all); over: they cover columns of the item before it
     uint32_t acc_prev = 0;
     auto acc_place = [&](const uint32_t i, const uint32_t n2, bool &over) {
-        over = n2 + acc_prev > (uint32_t)UM_ACC; acc_prev = n2;
-        return i & 1 ? (uint32_t)UM_ACC - n2 : 0u;
+        over = n2 + acc_prev > (uint32_t)SH::ACC; acc_prev = n2;
+        return i & 1 ? (uint32_t)SH::ACC - n2 : 0u;
     };
 
     if (warp < 8) {
         // ---------------- decode: this warp's 32 rows of both halves, every second block, from the shared-memory ring ----------------
         const int q4 = warp & 3, par = warp >> 2, R = q4 * 32 + lane;       // R: row inside a half = tensor-memory lane
         const uint32_t a_lane = tb + ((uint32_t)(q4 * 32) << 16) + ACOL;
-        uint32_t wcnt = 0, blk = 0;                                     // blk: blocks handed to the A ring so far (all warps count alike)
+        uint32_t wcnt = 0;
 #pragma unroll 1
         for (int item = blockIdx.x; item < nitems && live; item += gridDim.x) {
 #pragma unroll 1
-            for (int sb = 0; sb < NSB && live; sb++, wcnt++, blk += 4) {
-                const int ws = wcnt % UM_WSTAGES;
-                if (!mbar_wait(&sh->w_full[ws], (wcnt / UM_WSTAGES) & 1, abortp)) { live = false; break; }
-                const uint8_t *wr0 = wsm + ws * UM_WBYTES + R * 128, *wr1 = wr0 + 128 * 128;
+            for (int sb = 0; sb < NSB && live; sb++, wcnt++) {
+                const int ws = wcnt % WST;
+                if (!mbar_wait(&sh->w_full[ws], (wcnt / WST) & 1, abortp)) { live = false; break; }
+                const uint8_t *wr = wsm + ws * UM_WBYTES + R * 128;
 #pragma unroll
-                for (int qq = 0; qq < 2; qq++) {                         // this warp's two blocks of the weight stage
-                    const int q = 2 * qq + par;
-                    const uint32_t b = blk + q, as = b % NA, bo = b - NA;      // bo: the block that had the stage before
-                    uint32_t r0[32], r1[32];
-                    // gate+up and dense: left shifts, which the multiply pipe can take beside the masks; the operand is 64 x code and the epilogue shifts the
-                    // sums back, exactly (at most 192 * 127 * 2048 = 5e7).  2048 tokens: gate+up 51.0 -> 49.5 us between events, 4096: 80.7 -> 79.1.  The down
-                    // kernel has four blocks per epilogue instead of sixteen and loses (38.4 -> 39.3): plain codes.
-                    auto decode = [&](const uint8_t *wr, uint32_t (&o)[32]) {
-                        const uint4 v0 = *reinterpret_cast<const uint4 *>(wr + (((2 * q) ^ (R & 7)) << 4));
-                        const uint4 v1 = *reinterpret_cast<const uint4 *>(wr + (((2 * q + 1) ^ (R & 7)) << 4));
+                for (int q = par, qq = 0; qq < BPS / 2 && live; qq++, q += 2) {      // this warp's blocks of the weight stage
+                    const uint32_t b = BPS * wcnt + q, as = b % NA, bo = b - NA;      // bo: the block that had the A stage before
+#pragma unroll
+                    for (int u = 0; u < 2 * BW; u++) {                   // 128 columns of one half at a time
+                        const int sub = u >> 1, half = u & 1, c = 2 * (BW * q + sub);
+                        const uint8_t *w_ = wr + half * (128 * 128);
+                        const uint4 v0 = *reinterpret_cast<const uint4 *>(w_ + ((c ^ (R & 7)) << 4)), v1 = *reinterpret_cast<const uint4 *>(w_ + (((c + 1) ^ (R & 7)) << 4));
                         const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+                        uint32_t o[32];
+                        // gate+up and dense: left shifts, which the multiply pipe can take beside the masks; the operand is 64 x code and the epilogue shifts the
+                        // sums back, exactly (at most 192 * 127 * 2048 = 5e7).  2048 tokens: gate+up 51.0 -> 49.5 us between events, 4096: 80.7 -> 79.1.  The down
+                        // kernel has fewer blocks per epilogue and loses (38.4 -> 39.3): plain codes.
 #pragma unroll
                         for (int sft = 0; sft < 4; sft++)
 #pragma unroll
                             for (int j = 0; j < 8; j++) o[sft * 8 + j] = DOWN ? (w[j] >> (2 * sft)) & 0x03030303u : (w[j] << (6 - 2 * sft)) & 0xC0C0C0C0u;
-                    };
-                    decode(wr0, r0); decode(wr1, r1);                     // both halves are ready before the stage is asked for
-                    if (b >= NA && !mbar_wait(&sh->k_empty[bo % UM_BSTAGES], (bo / UM_BSTAGES) & 1, abortp)) { live = false; break; }
-                    tc_fence_after();
-                    tmem_st32(a_lane + as * 64, r0);
-                    tmem_st32(a_lane + as * 64 + 32, r1);
+                        if (u == 0) {
+                            if (b >= NA && !mbar_wait(&sh->k_empty[bo % BST], (bo / BST) & 1, abortp)) { live = false; break; }
+                            tc_fence_after();
+                        }
+                        tmem_st32(a_lane + as * (64 * BW) + half * (32 * BW) + sub * 32, o);
+                    }
+                    if (!live) break;
                     tmem_st_wait();
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&sh->k_full[b % UM_BSTAGES]);
+                    if (lane == 0) mbar_arrive(&sh->k_full[b % BST]);
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sh->w_empty[ws]);
+                if (live && lane == 0) mbar_arrive(&sh->w_empty[ws]);
             }
         }
     } else if (warp == 8) {
@@ -193,8 +198,8 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
                 const ExpertMaps *em = maps_of(tile);
 #pragma unroll 1
                 for (int sb = 0; sb < NSB && live; sb++, wcnt++) {
-                    const int ws = wcnt % UM_WSTAGES;
-                    if (!mbar_wait(&sh->w_empty[ws], ((wcnt / UM_WSTAGES) & 1) ^ 1, abortp)) { live = false; break; }
+                    const int ws = wcnt % WST;
+                    if (!mbar_wait(&sh->w_empty[ws], ((wcnt / WST) & 1) ^ 1, abortp)) { live = false; break; }
                     const uint32_t dst = smem_u32(wsm + ws * UM_WBYTES);
                     mbar_expect_tx(&sh->w_full[ws], UM_WBYTES);
                     if (GATEUP) {
@@ -220,10 +225,11 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
                 const int bi = tile.cnt > 0 ? (tile.cnt - 1) >> 5 : 0;
 #pragma unroll 1
                 for (int kb = 0; kb < KB && live; kb++, bcnt++) {
-                    const int s = bcnt % UM_BSTAGES;
-                    if (!mbar_wait(&sh->k_empty[s], ((bcnt / UM_BSTAGES) & 1) ^ 1, abortp)) { live = false; break; }
-                    mbar_expect_tx(&sh->k_full[s], 128 * 32 * (bi + 1));
-                    tma_load_2d(smem_u32(bsm + s * UM_BBYTES), &bmap.m[bi], kb * 128, tile.p0, &sh->k_full[s]);
+                    const int s = bcnt % BST;
+                    if (!mbar_wait(&sh->k_empty[s], ((bcnt / BST) & 1) ^ 1, abortp)) { live = false; break; }
+                    mbar_expect_tx(&sh->k_full[s], 128 * BW * 32 * (bi + 1));
+#pragma unroll
+                    for (int i = 0; i < BW; i++) tma_load_2d(smem_u32(bsm + s * SH::BBYTES + i * UM_TN * 128), &bmap.m[bi], kb * SH::KCOLS + i * 128, tile.p0, &sh->k_full[s]);
                 }
             }
         }
@@ -249,11 +255,12 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
             for (int kb = 0; kb < KB; kb++) {
                 if (!mbar_wait_addr(kfull0 + bs * 8, bp, abortp)) { live = false; break; }
                 tc_fence_after();
-                const uint32_t acol = tb + ACOL + as * 64 + h * 32, kb_empty = kempty0 + bs * 8;
-                const uint64_t bd = bdesc0 + (uint64_t)(bs * (UM_BBYTES >> 4));
+                const uint32_t acol = tb + ACOL + as * (64 * BW) + h * (32 * BW), kb_empty = kempty0 + bs * 8;
+                const uint64_t bd = bdesc0 + (uint64_t)(bs * (SH::BBYTES >> 4));
                 if (++as == NA) as = 0;
-                if (++bs == UM_BSTAGES) { bs = 0; bp ^= 1; }
-                umma_i8_block(d, acol, bd, idesc, kb != 0, kb_empty);
+                if (++bs == BST) { bs = 0; bp ^= 1; }
+                if (BW == 2) umma_i8_block<false>(d, acol, bd, idesc, kb != 0, 0);
+                umma_i8_block<true>(d, acol + 32 * (BW - 1), bd + (BW - 1) * (UM_TN * 128 >> 4), idesc, BW == 2 || kb != 0, kb_empty);
             }
             if (live && elect_one()) umma_commit(&sh->acc_full[buf]);
             __syncwarp();
@@ -266,7 +273,7 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
         // scales: the tile is read two items ahead, the pointer table and the tokens' values one item ahead (into registers; they go
         // to shared memory when the item starts), so that an item starts without a dependent global read in front of it.
         const int stride = gridDim.x;
-        constexpr int HN = UM_TN / 32;
+        constexpr int HN = TN / 32;
         MoeTile t1 = blockIdx.x < nitems ? tile_at(blockIdx.x / MB) : MoeTile{0, 0, 0, 0};
         MoeTile t2 = (int)blockIdx.x + stride < nitems ? tile_at((blockIdx.x + stride) / MB) : MoeTile{0, 0, 0, 0};
         ExpertPtrs ep1 = a.tab[t1.ex];
@@ -469,22 +476,35 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
     }
 }
 
-template <int KB, int MODE, bool FULL>
+template <int K, int MODE, bool FULL, int BW>
 static void launch(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) {
-    const size_t smem = (size_t)UM_WSTAGES * UM_WBYTES + UM_BSTAGES * UM_BBYTES + 1024;
+    const size_t smem = (size_t)UM_WSTAGES * UM_WBYTES + UmShape<BW>::BST * UmShape<BW>::BBYTES + 1024;
     static int sms = 0;
     if (!sms) {
         int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaFuncSetAttribute(expert_umma_kernel<KB, MODE, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(expert_umma_kernel<K, MODE, FULL, BW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     }
-    if (a->fresh_maps || MODE == 2) launch_k(expert_umma_kernel<KB, MODE, FULL>, sms, 640, smem, st, *a, *bmap);
-    else launch_pdl(expert_umma_kernel<KB, MODE, FULL>, sms, 640, smem, st, *a, *bmap);
+    if (a->fresh_maps || MODE == 2) launch_k(expert_umma_kernel<K, MODE, FULL, BW>, sms, 640, smem, st, *a, *bmap);
+    else launch_pdl(expert_umma_kernel<K, MODE, FULL, BW>, sms, 640, smem, st, *a, *bmap);
     k_count_add(1);
 }
-extern "C" void k_gateup_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->max_tiles > 0) { if (a->gu_dots) launch<16, 0, true>(st, a, bmap); else launch<16, 0, false>(st, a, bmap); } }
-extern "C" void k_down_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->max_tiles > 0) { if (a->dn_dots || a->rx_src) launch<4, 1, true>(st, a, bmap); else launch<4, 1, false>(st, a, bmap); } }
+// Blocks of 256 columns halve the hand-overs but leave the accumulators 256 columns of tensor memory instead of 320, which two items of more than 64 pairs do not share.
+// A layer with blocks of 128 and of 256: 176 tokens 76.6 and 74.4 us, 301 83.1 and 82.0, 511 94.7 and 93.5, 843 101.2 and 99.8, 1300 119.5 and 119.4, 1500 127.2 and 127.7,
+// 2048 148.9 and 155.0.
+#define UM_WIDE_TILES (1300 * 8 / UMMA_TN + 256)
+template <int K, int MODE, bool FULL>
+static void launch_by_size(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) {
+    if (a->max_tiles <= 0) return;
+    if (a->max_tiles <= UM_WIDE_TILES) launch<K, MODE, FULL, 2>(st, a, bmap); else launch<K, MODE, FULL, 1>(st, a, bmap);
+}
+extern "C" void k_gateup_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) {
+    if (a->gu_dots) launch_by_size<2048, 0, true>(st, a, bmap); else launch_by_size<2048, 0, false>(st, a, bmap);
+}
+extern "C" void k_down_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) {
+    if (a->dn_dots || a->rx_src) launch_by_size<512, 1, true>(st, a, bmap); else launch_by_size<512, 1, false>(st, a, bmap);
+}
 /* dense projections: tab[ex].ds / maps[ex].down of a matrix of 256 * a->dense_mblocks rows x 2048 columns, B rows = the tokens' int8 rows */
-extern "C" void k_dense_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->dense_n > 0) launch<16, 2, false>(st, a, bmap); }
+extern "C" void k_dense_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) { if (a->dense_n > 0) launch<2048, 2, false, 2>(st, a, bmap); }
 
 // ---- rows of the per-token int8 matrix copied into pair (expert-grouped) order: the B operand the TMA can tile ----
 __global__ void __launch_bounds__(256) gather_rows_kernel(const int8_t *__restrict__ src, const float *__restrict__ qs, const int *__restrict__ qsum, const int *__restrict__ rows,

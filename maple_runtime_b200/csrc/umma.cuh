@@ -98,8 +98,9 @@ __device__ __forceinline__ void umma_commit_addr(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// The MMAs of one 128-column block (four K slices of 32; A at a_tmem, 8 columns apart, B 32 bytes apart) and the arrival that frees it on barrier `done`, by
-// one elected lane of a fully active warp.  One election and predicated instructions: no branch.
+// The MMAs of 128 columns (four K slices of 32; A at a_tmem, 8 columns apart, B 32 bytes apart) and, with COMMIT, the arrival that frees the block on barrier
+// `done`, by one elected lane of a fully active warp.  One election and predicated instructions: no branch.
+template <bool COMMIT>
 __device__ __forceinline__ void umma_i8_block(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate, uint32_t done) {
     asm volatile("{\n\t.reg .pred P, Q;\n\telect.sync _|P, 0xffffffff;\n\tsetp.ne.b32 Q, %9, 0;\n\t"
                  "@P tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %5, %10, Q;\n\t"
@@ -107,9 +108,10 @@ __device__ __forceinline__ void umma_i8_block(uint32_t d_tmem, uint32_t a_tmem, 
                  "@P tcgen05.mma.cta_group::1.kind::i8 [%0], [%2], %6, %10, Q;\n\t"
                  "@P tcgen05.mma.cta_group::1.kind::i8 [%0], [%3], %7, %10, Q;\n\t"
                  "@P tcgen05.mma.cta_group::1.kind::i8 [%0], [%4], %8, %10, Q;\n\t"
-                 "@P tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%11];\n\t}"
+                 ".reg .pred C;\n\tsetp.ne.and.b32 C, %12, 0, P;\n\t"
+                 "@C tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%11];\n\t}"
                  ::"r"(d_tmem), "r"(a_tmem), "r"(a_tmem + 8), "r"(a_tmem + 16), "r"(a_tmem + 24), "l"(b_desc), "l"(b_desc + 2), "l"(b_desc + 4), "l"(b_desc + 6),
-                   "r"(accumulate), "r"(idesc), "r"(done) : "memory");
+                   "r"(accumulate), "r"(idesc), "r"(done), "n"(COMMIT ? 1 : 0) : "memory");
 }
 
 // ---- tensor memory <-> registers: thread t of warp w touches lane 32 (w % 4) + t, 32 consecutive columns ------------
