@@ -557,3 +557,40 @@ extern "C" void k_scatter_rows(cudaStream_t st, const int8_t *src, const float *
     launch_pdl(scatter_rows_kernel, (nb + 3) / 4, 128, 0, st, src, qs, qsum, tp, dst, dqs, dqsum, nb);
     k_count_add(1);
 }
+
+// The same behind a grouping that has left the places open (GroupArgs.place_base): pair k of token b goes to the start of its expert's pairs of b's word of 32 tokens
+// plus the number of them in front of b.  The grouping runs in 8 or 16 CTAs, whose scattered stores these are otherwise; here they are spread over nb / 4.
+__global__ void __launch_bounds__(128) place_rows_kernel(const GroupArgs g, const int8_t *__restrict__ src, const float *__restrict__ qs, const int *__restrict__ qsum,
+                                                         int8_t *__restrict__ dst, float *__restrict__ dqs, int *__restrict__ dqsum) {
+    const int lane = threadIdx.x & 31, k = lane & 7, b = blockIdx.x * 4 + (threadIdx.x >> 5);
+    uint4 v[4]; float s = 0.0f, w = 0.0f; int t = 0, x = 0;
+    if (b < g.nb) {                                              // older than the grouping: read before the wait
+        x = __ldcg(g.top + (size_t)b * 8 + k); w = __ldcg(g.topw + (size_t)b * 8 + k);
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] = __ldcg(reinterpret_cast<const uint4 *>(src + (size_t)b * 2048) + 32 * i + lane);
+        s = __ldcg(qs + b); t = __ldcg(qsum + b);
+    }
+    pdl_wait(); pdl_trigger();
+    if (b >= g.nb) return;
+    const size_t at = (size_t)(b >> 5) * 256 + x;
+    const int slot = g.place_base[at] + __popc(g.place_bits[at] & ((1u << (b & 31)) - 1u));      // lanes 8 i + k: the same eight
+    int rank = 0;
+#pragma unroll
+    for (int j = 0; j < 8; j++) rank += __shfl_sync(0xffffffffu, slot, j) < slot;
+    if (lane < 8) {
+        g.utok[slot] = b; g.uw[slot] = w; if (g.uexp) g.uexp[slot] = x;
+        g.slot[(size_t)b * 8 + k] = slot; g.tp[(size_t)b * 8 + rank] = slot;
+        dqs[slot] = s; dqsum[slot] = t;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        uint4 *d = reinterpret_cast<uint4 *>(dst + (size_t)__shfl_sync(0xffffffffu, slot, j) * 2048) + lane;
+#pragma unroll
+        for (int i = 0; i < 4; i++) d[32 * i] = v[i];
+    }
+}
+extern "C" void k_place_rows(cudaStream_t st, const GroupArgs *g, const int8_t *src, const float *qs, const int *qsum, int8_t *dst, float *dqs, int *dqsum) {
+    if (g->nb <= 0) return;
+    launch_pdl(place_rows_kernel, (g->nb + 3) / 4, 128, 0, st, *g, src, qs, qsum, dst, dqs, dqsum);
+    k_count_add(1);
+}

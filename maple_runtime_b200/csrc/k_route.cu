@@ -482,8 +482,13 @@ __global__ void __launch_bounds__(NEXP, 1) group_cluster_kernel(GroupArgs g) {
     for (int k = 0; k < wid; k++) { v.x += w_tot[k].x; v.y += w_tot[k].y; }
     const int start = (v.x & 0xFFFF) - cnt, uidx = (v.x >> 16) - used, ta0 = (v.y & 0xFFFF) - na, tb0 = (v.y >> 16) - nt;
     s_start[e] = start + before;
+    if (!TOPK_IN && g.place_base) {                            // the pairs are placed by the kernel that moves the rows: it gets, for every word, where the experts' pairs of it start
+        const int w0 = blockIdx.x * (per >> 5);
+#pragma unroll
+        for (int k = 0; k < GC_WORDS; k++) if (k < per >> 5 && (w0 + k) * 32 < nb) { g.place_base[(w0 + k) * NEXP + e] = start + before + s_pre[e][k]; g.place_bits[(w0 + k) * NEXP + e] = s_mask[e][k]; }
+    }
     __syncthreads();
-    if (mine) {
+    if (mine && (TOPK_IN || !g.place_base)) {
         int sl[TOPK];
 #pragma unroll
         for (int k = 0; k < TOPK; k++) sl[k] = s_start[x[k]] + s_pre[x[k]][wid] + __popc(s_mask[x[k]][wid] & ((1u << lane) - 1u));

@@ -86,6 +86,7 @@ typedef struct {
     int mask_words;
     int *nu, *ue, *estart, *ustart, *utok, *slot, *tp; float *uw;
     int marked;              /* 1: the routing kernels have already set the bits and counters in mask */
+    int *place_base; unsigned *place_bits;                   /* optional, 33 to GROUP_CLUSTER_MAX tokens and no logits: [mask_words][256] each; utok, uw, uexp, slot and tp are then left to k_place_rows */
     const float *logits; int *top_out; float *topw_out;      /* optional, up to TOPK_IN_MAX tokens: the top-8 is computed first, from the logits, and also stored here */
     int *ecnt, *uexp;        /* optional: pairs per expert [256], expert of every pair [np] (expert parallel) */
     MoeTile *tiles_a, *tiles_b; int *ntiles_a, *ntiles_b; int tn_a, tn_b;   /* two tile lists: sizes tn_a and tn_b */
@@ -126,6 +127,8 @@ void k_dense_umma(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap);
 void k_gather_rows(cudaStream_t st, const int8_t *src, const float *qs, const int *qsum, const int *rows, int8_t *dst, float *dqs, int *dqsum, int np);
 /* the same by token: its eight slots are tp[8 b ..] (16-byte aligned) */
 void k_scatter_rows(cudaStream_t st, const int8_t *src, const float *qs, const int *qsum, const int *tp, int8_t *dst, float *dqs, int *dqsum, int nb);
+/* the same, and the places themselves, behind a k_group with place_base and place_bits */
+void k_place_rows(cudaStream_t st, const GroupArgs *g, const int8_t *src, const float *qs, const int *qsum, int8_t *dst, float *dqs, int *dqsum);
 
 /* ---- the head of the attention half (k_attn_prep.cu): q/k RMS norm, half-rotary embedding, fp16 keys and values.  qkv [nb][3072]
  * = q 2048 | k 512 | v 512; pos [nb]; qn, kn [128] fp32; cs [cs_positions][32][2] (cos, sin); q [nb][2048] fp32; kc, vc [nb][512] fp16 */
