@@ -300,13 +300,13 @@ __global__ void __launch_bounds__(256, 2) router_small_kernel(const uint8_t *__r
 #define RM_WB (2 * 2 * RP_GRP)            /* two chunks of the tile layout x two groups of 16 experts */
 #define RM_STAGES 2
 template <int TT>
-__global__ void __launch_bounds__(160) router_mid_kernel(const uint8_t *__restrict__ WT, const uint8_t *__restrict__ hS, const float *__restrict__ bias,
-                                                         float *__restrict__ logits, int nb, int *err) {
+__device__ __forceinline__ void router_mid_cta(const uint8_t *__restrict__ WT, const uint8_t *__restrict__ hS, const float *__restrict__ bias,
+                                               float *__restrict__ logits, int nb, int *err, const int tok0) {
     extern __shared__ __align__(128) uint8_t rm_ring[];
     __shared__ uint64_t full[RM_STAGES], empty[RM_STAGES]; __shared__ int abort_flag, late;
     constexpr int HB = 4 * TT * RM_ROW, STAGE = HB + RM_WB;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, j = lane & 7, tg = lane >> 3;
-    const int tok0 = blockIdx.y * 4 * TT, g0 = blockIdx.x * 2;            // first token, first group of 16 experts
+    const int g0 = blockIdx.x * 2;                                         // first group of 16 experts
     if (tid == 0) {
         for (int s = 0; s < RM_STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); }
         abort_flag = late = 0; mbar_init_fence();
@@ -402,19 +402,30 @@ __global__ void __launch_bounds__(160) router_mid_kernel(const uint8_t *__restri
     __syncthreads();
     if (tid == 0 && abort_flag) *(volatile int *)err = 31;      // a wait ran out: the host reports it and the logits are not to be used
 }
+// The first nbig rows of the grid take 4 TB tokens each, the others 4 TS: CTAs go to the SMs one each before any gets its second, so an SM that has a big one gets a small
+// one beside it (the small rows first: 301 tokens 82.3 us per layer instead of 80.3).
+template <int TB, int TS>
+__global__ void __launch_bounds__(160) router_mid_kernel(const uint8_t *__restrict__ WT, const uint8_t *__restrict__ hS, const float *__restrict__ bias,
+                                                         float *__restrict__ logits, int nb, int nbig, int *err) {
+    const int y = blockIdx.y;
+    if (TB == TS || y < nbig) router_mid_cta<TB>(WT, hS, bias, logits, nb, err, y * 4 * TB);
+    else if constexpr (TB != TS) router_mid_cta<TS>(WT, hS, bias, logits, nb, err, nbig * 4 * TB + (y - nbig) * 4 * TS);
+}
 // Launched plainly (programmatically: 301 tokens 87.0 -> 88.3 us per layer, 400 88.8 -> 92.2) and with so much shared memory that per_sm CTAs fit an SM and no more.
 // Without the preference for shared memory the driver leaves room for fewer than two CTAs at some sizes (400 tokens 92.0 -> 89.3).
 #define RM_ALONE (116 << 10)
 #define RM_PAIR (78 << 10)
-template <int TT>
-static void launch_mid(cudaStream_t st, const void *router_t, const void *hS, const float *bias, float *logits, int nb, int *err, int per_sm) {
+// nbig = 0: all rows of 4 TB tokens
+template <int TB, int TS>
+static void launch_mid(cudaStream_t st, const void *router_t, const void *hS, const float *bias, float *logits, int nb, int nbig, int *err, int per_sm) {
     static bool attr_done = false;
     if (!attr_done) {
-        cudaFuncSetAttribute(router_mid_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, RM_ALONE);
-        cudaFuncSetAttribute(router_mid_kernel<TT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared); attr_done = true;
+        cudaFuncSetAttribute(router_mid_kernel<TB, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, RM_ALONE);
+        cudaFuncSetAttribute(router_mid_kernel<TB, TS>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared); attr_done = true;
     }
-    static_assert(RM_STAGES * (4 * TT * RM_ROW + RM_WB) <= RM_PAIR, "ring");
-    launch_k(router_mid_kernel<TT>, dim3(NEXP / 32, (nb + 4 * TT - 1) / (4 * TT)), 160, per_sm == 1 ? RM_ALONE : RM_PAIR, st, (const uint8_t *)router_t, (const uint8_t *)hS, bias, logits, nb, err);
+    static_assert(RM_STAGES * (4 * TB * RM_ROW + RM_WB) <= RM_PAIR && TS <= TB, "ring");
+    const int small = nb - nbig * 4 * TB, rows = nbig + (small + 4 * TS - 1) / (4 * TS);
+    launch_k(router_mid_kernel<TB, TS>, dim3(NEXP / 32, rows), 160, per_sm == 1 ? RM_ALONE : RM_PAIR, st, (const uint8_t *)router_t, (const uint8_t *)hS, bias, logits, nb, nbig, err);
 }
 extern "C" void k_router_pack_small(cudaStream_t st, const uint16_t *router, void *router_s) {
     router_pack_w_small_kernel<<<NEXP * HID / 4 / 256, 256, 0, st>>>(router, (uint2 *)router_s);
@@ -437,10 +448,15 @@ extern "C" void k_router_logits_small(cudaStream_t st, const void *router_s, con
         // tokens per CTA (8 CTAs of 32 experts cover them): the fewest CTA-times of work per SM.  One CTA of 12 on each SM is the cheapest (to 216 tokens); two of 8 take
         // 0.5 us more (to 296), two of 12 another 3.5 (to 444), two of 16 another 6 (to 592); three of 8 take 1 us more than two of 12, three of 12 1.5 more than two of 16.
         const int one = sms / (NEXP / 32), two = 2 * sms / (NEXP / 32);
-        if (nb <= 12 * one) launch_mid<3>(st, router_t, hS, bias, logits, nb, err, 1);
-        else if (nb <= 8 * two) launch_mid<2>(st, router_t, hS, bias, logits, nb, err, 2);
-        else if (nb <= 12 * two) launch_mid<3>(st, router_t, hS, bias, logits, nb, err, 2);
-        else launch_mid<4>(st, router_t, hS, bias, logits, nb, err, 2);
+        // Between two of these lie SMs with one of either kind: 301 tokens (12 + 8) 81.7 -> 80.3 us per layer, 352 82.8 -> 81.6, 445 (16 + 12) 91.7 -> 89.1, 504 92.8 -> 90.6.
+        // No more big rows than the tokens ask for (301 tokens with 18 of them 80.6), and one row less than fits the SMs: a full grid puts two big CTAs on one (352 82.9, 511 93.1).
+        const int big2 = (nb - 8 * (two - 1) + 3) / 4, big3 = (nb - 12 * (two - 1) + 3) / 4, half = sms / (NEXP / 32);   // rows of the bigger kind among two - 1
+        if (nb <= 12 * one) launch_mid<3, 3>(st, router_t, hS, bias, logits, nb, 0, err, 1);
+        else if (nb <= 8 * two) launch_mid<2, 2>(st, router_t, hS, bias, logits, nb, 0, err, 2);
+        else if (big2 <= half) launch_mid<3, 2>(st, router_t, hS, bias, logits, nb, big2, err, 2);
+        else if (nb <= 12 * two) launch_mid<3, 3>(st, router_t, hS, bias, logits, nb, 0, err, 2);
+        else if (big3 <= half) launch_mid<4, 3>(st, router_t, hS, bias, logits, nb, big3, err, 2);
+        else launch_mid<4, 4>(st, router_t, hS, bias, logits, nb, 0, err, 2);
         k_count_add(relaid ? 1 : 2);
         return;
     }

@@ -34,3 +34,13 @@ def test_where_eight_tokens_per_cta_begin_and_end(nb, layer, gpu, oracle, weight
     gpu.poke("hn", hn)
     gpu.stage("router", 2, nb)
     assert np.array_equal(gpu.peek("logits", nb).reshape(nb, 256).view(np.uint32), oracle.router_logits(router, hn).view(np.uint32))
+
+
+@pytest.mark.parametrize("nb", [298, 360, 361, 446, 504, 505])
+def test_where_two_kinds_of_ctas_begin_and_end(nb, layer, gpu, oracle, weights):
+    """One token past the last all-small (or all-big) grid, the last token of the mixed grids and the one after it."""
+    router, _, _ = weights.layer(2)
+    hn = weights.hidden(702, nb)
+    gpu.poke("hn", hn)
+    gpu.stage("router", 2, nb)
+    assert np.array_equal(gpu.peek("logits", nb).reshape(nb, 256).view(np.uint32), oracle.router_logits(router, hn).view(np.uint32))
