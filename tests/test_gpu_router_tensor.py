@@ -65,6 +65,30 @@ def test_ties_and_degenerate_rows_take_the_exact_path(g, clib, oracle, weights):
     assert clib.gmoe_router_flagged() >= 2
 
 
+@pytest.mark.parametrize("flag", [1, 18, 19, 37, 55, 72, 73, 100])
+def test_recomputed_tokens_are_exact_whatever_their_number(flag, g, clib, oracle, weights):
+    """Batches with a known number of tokens whose nine largest logits lie too close (a quarter of the bound apart at most; the others four times): the exact kernel
+    takes 18 groups of one to four tokens and starts over behind 72.  Exactly those rows hold the reference's logits and weights bit for bit."""
+    router, _, _ = weights.layer(2)
+    wmax = float(np.sqrt(((router.astype(np.uint32) << 16).view(np.float32).astype(np.float64) ** 2).sum(1)).max())
+    pool = weights.hidden(621, 2048)
+    logits = oracle.router_logits(router, pool)
+    top9 = -np.sort(-logits.astype(np.float64), axis=1)[:, :9]
+    gap = (top9[:, :-1] - top9[:, 1:]).min(1) / (np.sqrt((pool.astype(np.float64) ** 2).sum(1)) * wmax)
+    close, apart = np.flatnonzero(gap < 2.0 ** -20), np.flatnonzero(gap > 2.0 ** -16)
+    assert len(close) >= 4
+    nb = 512
+    rows = np.resize(apart, nb); at = np.linspace(0, nb - 1, flag).astype(int)
+    rows[at] = np.resize(close, flag)
+    g.poke("hn", np.ascontiguousarray(pool[rows]))
+    g.stage("router_tensor", 2, nb)
+    want_top, want_w = oracle_topk_all(oracle, logits[rows])
+    got_l, got_top, got_w = g.peek("logits", nb).reshape(nb, 256), g.peek("top", nb).reshape(nb, 8), g.peek("topw", nb).reshape(nb, 8)
+    assert clib.gmoe_router_flagged() == flag and np.array_equal(got_top, want_top)
+    assert np.array_equal(got_l[at].view(np.uint32), logits[rows][at].view(np.uint32)) and np.array_equal(got_w[at].view(np.uint32), want_w[at].view(np.uint32))
+    assert float((np.abs(got_w - want_w) / want_w).max()) <= TOL_W
+
+
 def test_a_million_tokens_select_the_same_experts_as_the_exact_router(g, clib, weights):
     """512 chunks of 2048 synthetic tokens (every fourth with the skewing bias): indices from the tensor-core path against the
     exact-order kernels (which other tests pin to the oracle bit for bit); also the observed error against the bound the
