@@ -76,7 +76,7 @@ static struct {
     unsigned prof_mask; cudaEvent_t *pev; int pev_n, pev_cap; unsigned char *pev_stage; long *pev_launch;
     int fwd_timed;
     /* tensor-core router (k_router_umma.cu) */
-    void *hA; float *hnorm, *rpart; int *flagged, *nflagged, *rdone; TMap amap; int router_mode;
+    void *hA; float *hnorm, *rpart; int *flagged, *nflagged; TMap amap; int router_mode;
 } S;
 
 /* The tables of a reference-shaped call are written into one page-locked block, from which one kernel distributes them to their places
@@ -180,7 +180,7 @@ static int init_common(const char *who, int maxtok, int topk) {
     ALLOC(act, P * FFN * 4); ALLOC(gate, P * FFN * 4); ALLOC(up, P * FFN * 4); ALLOC(aq, P * FFN); ALLOC(aqs, P * 4); ALLOC(aqsum, P * 4); ALLOC(down, P * HID * 4);
     ALLOC(tab_call, NEXP * sizeof(ExpertPtrs)); ALLOC(maps_seen, MAP_SLOTS * sizeof(ExpertMaps)); ALLOC(hq_sorted, P * HID); ALLOC(hqs_sorted, P * 8); S.hqsum_sorted = (int *)S.hqs_sorted + P;
     ALLOC(wire, WIRE_BYTES(P)); CU(who, cudaMemset(S.wire, 0, WIRE_BYTES(P))); ALLOC(dsp_call, NEXP * sizeof(void *));
-    ALLOC(hA, T * HID * 4); ALLOC(hnorm, T * 4); ALLOC(rpart, (size_t)8 * T * NEXP * 4); ALLOC(flagged, T * 4); ALLOC(nflagged, 16); ALLOC(rdone, T * 4); CU(who, cudaMemset(S.rdone, 0, T * 4));
+    ALLOC(hA, T * HID * 4); ALLOC(hnorm, T * 4); ALLOC(rpart, (size_t)8 * T * NEXP * 4); ALLOC(flagged, T * 4); ALLOC(nflagged, 16);
     CU(who, cudaMemset(S.hA, 0, T * HID * 4)); CU(who, cudaMemset(S.nflagged, 0, 16));
     if (tmap_init(who)) return -1;
     if (tmap_f16_2d(who, &S.amap, S.hA, 2 * HID, T, (uint64_t)2 * HID * 2, 64, 128)) return -1;
@@ -464,7 +464,7 @@ static void run_router_tensor_m(const LayerDev *l, const float *bias, int nb, in
     RouterTensorArgs r; memset(&r, 0, sizeof r);
     r.amap = S.amap; r.wmap = l->wmap; r.part = S.rpart; r.nb = nb; r.ntok_cap = S.maxtok; r.err = S.err;
     r.bias = bias; r.hnorm = S.hnorm; r.wnorm = l->wnorm; r.hn = S.hn; r.router_s = l->router_s;
-    r.logits = S.logits; r.top = S.top; r.topw = S.topw; r.flagged = S.flagged; r.nflagged = S.nflagged; r.done = S.rdone;
+    r.logits = S.logits; r.top = S.top; r.topw = S.topw; r.flagged = S.flagged; r.nflagged = S.nflagged;
     if (mark && nb > GROUP_CLUSTER_MAX) { r.mask = S.mask; r.mask_words = S.mask_words; }      /* the grouping's bits and counters come out of the routing kernels */
     k_router_tensor(S.st, &r);
 }

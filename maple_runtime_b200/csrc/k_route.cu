@@ -282,29 +282,9 @@ __global__ void __launch_bounds__(64, 1) group_one_kernel(GroupArgs g) {
     pdl_wait(); pdl_trigger();
     const float4 v0 = __ldcg(reinterpret_cast<const float4 *>(g.logits) + 2 * lane), v1 = __ldcg(reinterpret_cast<const float4 *>(g.logits) + 2 * lane + 1);
     float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-    // warp 1 adds the exponentials in the reference's order (256 dependent additions) while warp 0 selects by them
-    exact_exp_warp(p, lane, tab);
-    if (sum_warp) {
-        reinterpret_cast<float4 *>(s_row)[2 * lane] = make_float4(p[0], p[1], p[2], p[3]); reinterpret_cast<float4 *>(s_row)[2 * lane + 1] = make_float4(p[4], p[5], p[6], p[7]);
-        __syncwarp();
-        const float run = exact_sum_row(s_row);
-        if (lane == 0) s_run = run;
-        __syncthreads();
-        return;
-    }
-    int isel; float psel, tsum;                                          // lane k < 9: the k-th largest
-    top_select_warp<TOPK + 1>(p, lane, isel, psel, tsum);
-    __syncthreads();
-    const float run = s_run;
-    float wsel = __fdiv_rn(psel, run);
-    // the reference selects by the quotients: another order only where unequal exponentials have equal quotients (or are not numbers)
-    const float pn = __shfl_down_sync(0xffffffffu, psel, 1), wn = __shfl_down_sync(0xffffffffu, wsel, 1);
-    if (__any_sync(0xffffffffu, lane < TOPK && !(wsel > wn || psel == pn))) exact_topk_warp_from(p, lane, run, isel, wsel, tsum);
-    else {
-        tsum = 0.0f;
-#pragma unroll
-        for (int k = 0; k < TOPK; k++) tsum = __fadd_rn(tsum, __shfl_sync(0xffffffffu, wsel, k));
-    }
+    int isel; float wsel, tsum;
+    exact_topk_pair(p, lane, sum_warp, tab, s_row, &s_run, isel, wsel, tsum);
+    if (sum_warp) return;
     const float w = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));          // lane k < 8: the k-th selected expert
     int r = 0, st[8] = {-1, -1, -1, -1, -1, -1, -1, -1};                // st: where the pairs of experts 8 lane .. + 7 start
 #pragma unroll

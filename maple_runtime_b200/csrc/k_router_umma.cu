@@ -248,14 +248,16 @@ __global__ void __launch_bounds__(32) router_select_kernel(const float *__restri
 
 // The flagged tokens over again as the reference computes them (maple.c:870-889, 117-121, 910-923).  grid (8 expert eighths, RF_GROUPS): CTA
 // (x, y) walks flagged tokens y, y + RF_GROUPS, ... four at a time and computes 32 experts of each: 256 threads = 8 lanes x 32 experts, the
-// eight strided multiply-add chains per expert and their pairwise adds.  The last of a group's eight CTAs to finish (a counter per group
-// of four, reset by that CTA) runs the exact softmax + top-8 on the four finished rows, a warp each.
-// Bound by latency: list -> token -> hidden row -> 256 chained multiply-adds -> counter -> softmax + top-8.  So the CTA's 32 router rows come
-// into shared memory before it waits for the selection, four tokens' chains run side by side in a thread, and 144 CTAs cover 72 tokens (2% of
-// 2048 are flagged: 45) in one round.  A group's chains are as many as it has tokens (one of them up to 18 flagged, three at 45): every chain costs 1 us of
+// eight strided multiply-add chains per expert and their pairwise adds.  A group's eight CTAs are a cluster: CTA t gets the logits of the group's
+// token t through distributed shared memory and runs the exact softmax + top-8 on them.
+// Bound by latency: list -> token -> hidden row -> 256 chained multiply-adds -> cluster barrier -> softmax + top-8.  So the CTA's 32 router rows come
+// into shared memory before it waits for the selection, four tokens' chains run side by side in a thread, and as many clusters as the GPU holds at once (15) cover
+// 60 tokens (2% of 2048 are flagged: 45) in one round.  Through memory (rows, fence, a counter that the last CTA finds full) the exchange took 0.8 us more, the softmax's sum in
+// front of the selection instead of beside it (two warps) 0.5: 512 / 843 / 2048 tokens 85.7 / 95.8 / 145.4 -> 84.4 / 94.6 / 144.1 us per layer.  All 18 clusters, three of them
+// in a second wave: 85.1 / 96.0 / 148.5.  The token numbers asked for beside their count: 0.4 us slower.  A group's chains are as many as it has tokens (one up to 15 flagged, three at 45): every chain costs 1 us of
 // shared-memory reads, and all four were always read.  512 tokens 89.1 -> 85.9 us per layer, 843 99.0 -> 95.8, 2048 147.3 -> 145.7.
 // WS: the router rows re-laid as [expert][column / 32][lane j][4 steps] bf16 (k_router_pack_small, k_router_tile.cu).
-#define RF_GROUPS 18
+#define RF_GROUPS 18                     /* at most; as many as the GPU holds at once */
 #define RF_TOK 4
 #define RF_WPITCH (HID * 2 + 64)         /* rows 16 banks apart: the experts of a warp meet no bank twice */
 #define RF_SMEM (32 * RF_WPITCH + RF_TOK * HID * 4)
@@ -279,12 +281,14 @@ __device__ __forceinline__ void rf_chains(const uint8_t *wp, const float *hj, fl
 }
 __global__ void __launch_bounds__(256) router_fix_kernel(const uint8_t *__restrict__ WS, const float *__restrict__ hn, const float *__restrict__ bias,
                                                          float *__restrict__ logits, int *__restrict__ top, float *__restrict__ topw,
-                                                         const int *__restrict__ flagged, const int *__restrict__ nflagged, int *__restrict__ done,
+                                                         const int *__restrict__ flagged, const int *__restrict__ nflagged,
                                                          unsigned *__restrict__ mask, int mask_words, int nb, int *err) {
     extern __shared__ __align__(128) uint8_t rf_sm[];
     float *hrow = reinterpret_cast<float *>(rf_sm + 32 * RF_WPITCH);       // [RF_TOK][HID]
     __shared__ unsigned long long tab[32];
-    __shared__ uint64_t bar; __shared__ int s_last, abort_flag;
+    __shared__ __align__(16) float lrow[2][NEXP];                           // logits of the group's token (blockIdx.x), from all eight CTAs; even and odd groups
+    __shared__ __align__(16) float erow[NEXP]; __shared__ float s_run;
+    __shared__ uint64_t bar; __shared__ int abort_flag;
     const int tid = threadIdx.x, j = tid & 7, pos = tid >> 3, lane = tid & 31, warp = tid >> 5, e = blockIdx.x * 32 + pos;
     if (tid < 32) tab[tid] = DEV_EXP_TAB[tid];
     if (tid == 0) {
@@ -292,17 +296,21 @@ __global__ void __launch_bounds__(256) router_fix_kernel(const uint8_t *__restri
         mbar_expect_tx(&bar, 32 * HID * 2);
         for (int r = 0; r < 32; r++) rf_bulk(smem_u32(rf_sm) + r * RF_WPITCH, WS + (size_t)(blockIdx.x * 32 + r) * (HID * 2), HID * 2, &bar);
     }
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     const float be = bias ? bias[e] : 0.0f;
     __syncthreads();
-    const bool ok = mbar_wait(&bar, 0, &abort_flag);
+    if (!mbar_wait(&bar, 0, &abort_flag) && tid == 0) *(volatile int *)err = 31;
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");            // all eight CTAs run
     pdl_wait(); pdl_trigger();
-    const int total = ok ? min(*nflagged, nb) : 0;
-    if (!ok && tid == 0) *(volatile int *)err = 31;
-    for (int f0 = blockIdx.y; f0 < total; f0 += RF_GROUPS * RF_TOK) {
-        int b[RF_TOK];                                                      // the group's tokens; past the end the first one again, not stored
+    const int groups = gridDim.y;
+    const int total = min(*nflagged, nb);
+    int buf = 0;
+    for (int f0 = blockIdx.y; f0 < total; f0 += groups * RF_TOK, buf ^= 1) {
+        int b[RF_TOK];                                                      // the group's tokens; past the end the first one again, not used
 #pragma unroll
-        for (int t = 0; t < RF_TOK; t++) { const int f = f0 + t * RF_GROUPS; b[t] = flagged[f < total ? f : f0]; }
-        const int n = (min(total, f0 + RF_GROUPS * RF_TOK) - f0 + RF_GROUPS - 1) / RF_GROUPS;
+        for (int t = 0; t < RF_TOK; t++) { const int f = f0 + t * groups; b[t] = flagged[f < total ? f : f0]; }
+        const int n = min((total - f0 + groups - 1) / groups, RF_TOK);
         __syncthreads();
 #pragma unroll
         for (int t = 0; t < RF_TOK; t++)
@@ -323,27 +331,29 @@ __global__ void __launch_bounds__(256) router_fix_kernel(const uint8_t *__restri
             l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 4));
             l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 1));
             l = __fadd_rn(l, __shfl_xor_sync(0xffffffffu, l, 2));
-            if (j == 0 && t < n) logits[(size_t)b[t] * NEXP + e] = bias ? __fadd_rn(l, be) : l;
+            if (j == 0 && t < n) {
+                const float lb = bias ? __fadd_rn(l, be) : l;
+                logits[(size_t)b[t] * NEXP + e] = lb;
+                uint32_t at;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(&lrow[buf][e])), "r"(t));
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(lb) : "memory");
+            }
         }
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) s_last = atomicAdd(&done[f0], 1) == (int)gridDim.x - 1;
-        __syncthreads();
-        if (s_last && warp < n) {
-            __threadfence();
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if ((int)blockIdx.x < n && warp < 2) {
             int bt = b[0];
 #pragma unroll
-            for (int t = 1; t < RF_TOK; t++) if (warp == t) bt = b[t];
-            const float4 *lr = reinterpret_cast<const float4 *>(logits + (size_t)bt * NEXP + lane * 8);
-            const float4 v0 = __ldcg(lr), v1 = __ldcg(lr + 1);              // the other CTAs' values: read past L1
+            for (int t = 1; t < RF_TOK; t++) if ((int)blockIdx.x == t) bt = b[t];
+            const float4 *lr = reinterpret_cast<const float4 *>(lrow[buf]) + lane * 2;
+            const float4 v0 = lr[0], v1 = lr[1];
             float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
             int isel; float wsel, tsum;
-            exact_topk_warp(p, lane, tab, hrow + warp * HID, isel, wsel, tsum);      // hrow is read no more: it is the scratch of the top-8
-            if (lane < TOPK) {
+            exact_topk_pair(p, lane, warp, tab, erow, &s_run, isel, wsel, tsum);
+            if (warp == 0 && lane < TOPK) {
                 top[bt * TOPK + lane] = isel; topw[bt * TOPK + lane] = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));
                 if (mask) { atomicOr(&mask[(size_t)(bt >> 5) * NEXP + isel], 1u << (bt & 31)); atomicAdd(&mask[(size_t)NEXP * mask_words + isel], 1u); }
             }
-            if (tid == 0) done[f0] = 0;
         }
     }
 }
@@ -352,9 +362,13 @@ extern "C" void k_router_tensor(cudaStream_t st, const RouterTensorArgs *r) {
     if (r->nb <= 0) return;
     static bool attr_done = false;
     const int smem = RU_STAGES * RU_STAGE_BYTES + 1024;
-    if (!attr_done) { cudaFuncSetAttribute(router_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); cudaFuncSetAttribute(router_fix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RF_SMEM); attr_done = true; }
+    static int groups = 0;
+    if (!attr_done) {
+        cudaFuncSetAttribute(router_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); cudaFuncSetAttribute(router_fix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RF_SMEM);
+        groups = clusters_at_once(router_fix_kernel, 8, 256, RF_SMEM, RF_GROUPS); attr_done = true;
+    }
     launch_pdl(router_umma_kernel, dim3(RU_KS, (r->nb + 127) / 128), 192, smem, st, r->amap, r->wmap, r->part, r->nb, r->ntok_cap, r->err, r->nflagged, r->mask, NEXP * r->mask_words + NEXP);
     launch_pdl(router_select_kernel, (r->nb + 0) / 1, 32, 0, st, r->part, r->ntok_cap, r->bias, r->hnorm, r->wnorm, r->logits, r->top, r->topw, r->flagged, r->nflagged, r->mask, r->mask_words, r->nb);
-    launch_pdl(router_fix_kernel, dim3(8, RF_GROUPS), 256, RF_SMEM, st, (const uint8_t *)r->router_s, r->hn, r->bias, r->logits, r->top, r->topw, r->flagged, r->nflagged, r->done, r->mask, r->mask_words, r->nb, r->err);
+    launch_clusters(router_fix_kernel, dim3(8, groups), 8, 256, RF_SMEM, st, (const uint8_t *)r->router_s, r->hn, r->bias, r->logits, r->top, r->topw, r->flagged, r->nflagged, r->mask, r->mask_words, r->nb, r->err);
     k_count_add(3);
 }

@@ -152,7 +152,6 @@ typedef struct {
     float *logits; int *top; float *topw;
     int *flagged, *nflagged; /* [nb], [1]: tokens that took the exact path (left for inspection) */
     unsigned *mask; int mask_words;   /* optional: the grouping's bit words and counters (GroupArgs.mask): cleared and filled here, k_group then runs with marked = 1 */
-    int *done;               /* [nb] counters, zero between calls */
 } RouterTensorArgs;
 void k_router_w16(cudaStream_t st, const uint16_t *router, void *w16, float *wnorm);
 void k_router_tensor(cudaStream_t st, const RouterTensorArgs *r);

@@ -36,13 +36,29 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // 99.6 / 110.7 / 157.8 -> 97.5 / 107.3 / 156.4 us.  The pair-ordered int8 rows and the router's partial sums too: no further change.
 __device__ __forceinline__ void l2_discard(const void *p) { asm volatile("discard.global.L2 [%0], 128;" ::"l"(p) : "memory"); }
 #endif
-// the same, programmatically too, as one cluster of `ctas` CTAs
+// the same, programmatically too, in clusters of `ctas` CTAs along x
 template <typename... KArgs, typename... Args>
-static inline cudaError_t launch_cluster(void (*kernel)(KArgs...), unsigned ctas, dim3 block, cudaStream_t st, Args... args) {
+static inline cudaError_t launch_clusters(void (*kernel)(KArgs...), dim3 grid, unsigned ctas, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof cfg);
     cudaLaunchAttribute at[2]; memset(at, 0, sizeof at);
     at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = ctas; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = ctas; cfg.blockDim = block; cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 2;
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+// how many of them run at the same time on an empty GPU, at most `most`
+template <typename... KArgs>
+static inline int clusters_at_once(void (*kernel)(KArgs...), unsigned ctas, dim3 block, size_t smem, int most) {
+    cudaLaunchConfig_t cfg; memset(&cfg, 0, sizeof cfg);
+    cudaLaunchAttribute at; memset(&at, 0, sizeof at);
+    at.id = cudaLaunchAttributeClusterDimension; at.val.clusterDim.x = ctas; at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(ctas, most); cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.attrs = &at; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); return most; }
+    return n < most ? n : most;
+}
+// one cluster
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_cluster(void (*kernel)(KArgs...), unsigned ctas, dim3 block, cudaStream_t st, Args... args) {
+    return launch_clusters(kernel, dim3(ctas), ctas, block, 0, st, args...);
 }

@@ -69,3 +69,31 @@ __device__ __forceinline__ void exact_topk_warp(float (&p)[8], const int lane, c
     __syncwarp();
     exact_topk_warp_from(p, lane, exact_sum_row(row), isel, wsel, tsum);
 }
+// The same by two warps that hold the same logits: warp 1 adds the exponentials in the reference's order (256 dependent additions) while warp 0 selects by them;
+// warp 0 returns the result.  row, run: shared memory; the two meet at barrier 1.
+template <typename TabT>
+__device__ __forceinline__ void exact_topk_pair(float (&p)[8], const int lane, const int sum_warp, const TabT *tab, float *row, float *run_at, int &isel, float &wsel, float &tsum) {
+    exact_exp_warp(p, lane, tab);
+    isel = 0; wsel = tsum = 0.0f;
+    if (sum_warp) {
+        reinterpret_cast<float4 *>(row)[2 * lane] = make_float4(p[0], p[1], p[2], p[3]); reinterpret_cast<float4 *>(row)[2 * lane + 1] = make_float4(p[4], p[5], p[6], p[7]);
+        __syncwarp();
+        const float run = exact_sum_row(row);
+        if (lane == 0) *run_at = run;
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        return;
+    }
+    float psel;                                                          // lane k < 9: the k-th largest
+    top_select_warp<9>(p, lane, isel, psel, tsum);
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+    const float run = *run_at;
+    wsel = __fdiv_rn(psel, run);
+    // the reference selects by the quotients: another order only where unequal exponentials have equal quotients (or are not numbers)
+    const float pn = __shfl_down_sync(0xffffffffu, psel, 1), wn = __shfl_down_sync(0xffffffffu, wsel, 1);
+    if (__any_sync(0xffffffffu, lane < 8 && !(wsel > wn || psel == pn))) exact_topk_warp_from(p, lane, run, isel, wsel, tsum);
+    else {
+        tsum = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; k++) tsum = __fadd_rn(tsum, __shfl_sync(0xffffffffu, wsel, k));
+    }
+}
