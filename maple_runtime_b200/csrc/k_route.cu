@@ -143,33 +143,39 @@ extern "C" void k_norm_prep_split(cudaStream_t st, const float *x, const uint16_
 // (Router logits live in k_router_tile.cu.)
 
 // ------------------------------------------------------------------------------------------------------------
-// Softmax + top-8 (maple.c:910-923): one warp per token, lane l holds experts 8l..8l+7.
+// Softmax + top-8 (maple.c:910-923): two warps per token (topk.cuh), lane l holds experts 8l..8l+7.
 // p = expf(l - max); the sum runs over experts in index order (a chain through the lanes); p /= sum; eight rounds
 // of "first strict maximum" (lowest index wins a tie); weights divided by (their sum in selection order + 1e-20f).
-// Four tokens per CTA (eight: 65 tokens 58.4 us per layer instead of 58.1, 144 73.6 instead of 73.1; one: 160 tokens 80.9 instead of 74.0).
+// Bound by latency.  Two tokens per CTA while that is one CTA per SM, four above: 65 / 211 / 301 / 400 tokens 58.0 / 76.5 / 80.5 / 83.7 us per layer with a warp per token
+// (four per CTA) -> 57.6 / 74.8 / 80.5 / 83.1 with two warps and four tokens, 56.0 / 74.7 / 80.8 / 83.1 with two.
 // ------------------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128, 1) topk_kernel(const float *__restrict__ logits, int *__restrict__ top, float *__restrict__ topw, int nb) {
+template <int TOKENS>
+__global__ void __launch_bounds__(64 * TOKENS, 1) topk_kernel(const float *__restrict__ logits, int *__restrict__ top, float *__restrict__ topw, int nb) {
     __shared__ unsigned long long tab[32];                  // the expf table beside the arithmetic (lane-varying index)
-    __shared__ __align__(16) float s_row[4][NEXP];
+    __shared__ __align__(16) float s_row[TOKENS][NEXP]; __shared__ float s_run[TOKENS];
     if (threadIdx.x < 32) tab[threadIdx.x] = DEV_EXP_TAB[threadIdx.x];
     __syncthreads();
     pdl_wait(); pdl_trigger();
     const int lane = threadIdx.x & 31;
-    const int b = blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int pair = threadIdx.x >> 6, sum_warp = threadIdx.x >> 5 & 1, b = blockIdx.x * TOKENS + pair;
     if (b >= nb) return;
     const float4 *lr = reinterpret_cast<const float4 *>(logits + (size_t)b * NEXP + lane * 8);
     float4 v0 = lr[0], v1 = lr[1];
     float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
     int isel; float wsel, tsum;
-    exact_topk_warp(p, lane, tab, s_row[threadIdx.x >> 5], isel, wsel, tsum);
-    if (lane < TOPK) {
+    exact_topk_pair(p, lane, sum_warp, tab, s_row[pair], &s_run[pair], 1 + pair, isel, wsel, tsum);
+    if (!sum_warp && lane < TOPK) {
         top[b * TOPK + lane] = isel;
         topw[b * TOPK + lane] = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));
     }
 }
 extern "C" void k_topk(cudaStream_t st, const float *logits, int *top, float *topw, int nb) {
     if (nb <= 0) return;
-    launch_pdl(topk_kernel, (nb + 3) / 4, 128, 0, st, logits, top, topw, nb); g_launches++;
+    static int sms = 0;
+    if (!sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); if (sms < 1) sms = 148; }
+    if (nb <= 2 * sms) launch_pdl(topk_kernel<2>, (nb + 1) / 2, 128, 0, st, logits, top, topw, nb);
+    else launch_pdl(topk_kernel<4>, (nb + 3) / 4, 256, 0, st, logits, top, topw, nb);
+    g_launches++;
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -283,7 +289,7 @@ __global__ void __launch_bounds__(64, 1) group_one_kernel(GroupArgs g) {
     const float4 v0 = __ldcg(reinterpret_cast<const float4 *>(g.logits) + 2 * lane), v1 = __ldcg(reinterpret_cast<const float4 *>(g.logits) + 2 * lane + 1);
     float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
     int isel; float wsel, tsum;
-    exact_topk_pair(p, lane, sum_warp, tab, s_row, &s_run, isel, wsel, tsum);
+    exact_topk_pair(p, lane, sum_warp, tab, s_row, &s_run, 1, isel, wsel, tsum);
     if (sum_warp) return;
     const float w = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));          // lane k < 8: the k-th selected expert
     int r = 0, st[8] = {-1, -1, -1, -1, -1, -1, -1, -1};                // st: where the pairs of experts 8 lane .. + 7 start
@@ -384,7 +390,8 @@ __global__ void __launch_bounds__(NEXP, 1) group_cta_kernel(GroupArgs g) {
 // CTAs are what every GPU has to allow; from 513 tokens on sixteen share the scattered stores (2048 tokens: 14.4 -> 11.9 us).
 // Against one CTA for up to 256 tokens, a layer of the stack: 96 tokens 70.8 -> 70.0 us, 128 77.7 -> 75.9, 256 106.1 -> 100.7.
 // (One CTA per SM in the launch bounds of the grouping kernels: registers instead of reloads, 0.1 us.)
-// TOPK_IN (9 to TOPK_IN_MAX tokens): the softmax and top-8 come first, a warp per token (20 tokens 41.8 -> 41.3 us, 64 61.2 -> 60.7).
+// TOPK_IN (9 to TOPK_IN_MAX tokens): the softmax and top-8 come first, a warp per token (20 tokens 41.8 -> 41.3 us, 64 61.2 -> 60.7), two up to 32 tokens, where
+// there are enough (9 / 13 / 32 tokens 28.4 / 32.4 / 44.45 -> 28.0 / 32.0 / 44.25).
 #define GC_WORDS 8
 template <int GC_CTAS, bool TOPK_IN>
 __global__ void __launch_bounds__(NEXP, 1) group_cluster_kernel(GroupArgs g) {
@@ -397,13 +404,27 @@ __global__ void __launch_bounds__(NEXP, 1) group_cluster_kernel(GroupArgs g) {
     const bool mine = e < per && tok < nb;
     constexpr int TT = TOPK_IN ? TOPK_IN_MAX / GC_CTAS : 1;
     __shared__ __align__(16) int s_top[TT * TOPK]; __shared__ __align__(16) float s_topw[TT * TOPK];
-    __shared__ __align__(16) float s_row[TOPK_IN ? 8 : 1][NEXP];
+    __shared__ __align__(16) float s_row[TOPK_IN ? 8 : 1][NEXP]; __shared__ float s_run[4];
     __shared__ unsigned long long tab[TOPK_IN ? 32 : 1];
     if (TOPK_IN && e < 32) tab[e] = DEV_EXP_TAB[e];
     if (TOPK_IN) __syncthreads();
     pdl_wait(); pdl_trigger();
-    if (TOPK_IN) {                                              // a warp per token
-        for (int i = wid; i < per && (int)blockIdx.x * per + i < nb; i += 8) {
+    if (TOPK_IN) {
+        if (per <= 4) {                                        // up to 32 tokens: two warps each
+            const int i = wid >> 1, t = blockIdx.x * per + i;
+            if (i < per && t < nb) {
+                const float4 *lr = reinterpret_cast<const float4 *>(g.logits + (size_t)t * NEXP + lane * 8);
+                const float4 v0 = __ldcg(lr), v1 = __ldcg(lr + 1);
+                float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+                int isel; float wsel, tsum;
+                exact_topk_pair(p, lane, wid & 1, tab, s_row[i], &s_run[i], 1 + i, isel, wsel, tsum);
+                if (!(wid & 1) && lane < TOPK) {
+                    const float tw = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));
+                    s_top[i * TOPK + lane] = isel; s_topw[i * TOPK + lane] = tw;
+                    g.top_out[t * TOPK + lane] = isel; g.topw_out[t * TOPK + lane] = tw;
+                }
+            }
+        } else for (int i = wid; i < per && (int)blockIdx.x * per + i < nb; i += 8) {
             const int t = blockIdx.x * per + i;
             const float4 *lr = reinterpret_cast<const float4 *>(g.logits + (size_t)t * NEXP + lane * 8);
             const float4 v0 = __ldcg(lr), v1 = __ldcg(lr + 1);

@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(256) router_fix_kernel(const uint8_t *__restri
             const float4 v0 = lr[0], v1 = lr[1];
             float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
             int isel; float wsel, tsum;
-            exact_topk_pair(p, lane, warp, tab, erow, &s_run, isel, wsel, tsum);
+            exact_topk_pair(p, lane, warp, tab, erow, &s_run, 1, isel, wsel, tsum);
             if (warp == 0 && lane < TOPK) {
                 top[bt * TOPK + lane] = isel; topw[bt * TOPK + lane] = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));
                 if (mask) { atomicOr(&mask[(size_t)(bt >> 5) * NEXP + isel], 1u << (bt & 31)); atomicAdd(&mask[(size_t)NEXP * mask_words + isel], 1u); }

@@ -70,9 +70,9 @@ __device__ __forceinline__ void exact_topk_warp(float (&p)[8], const int lane, c
     exact_topk_warp_from(p, lane, exact_sum_row(row), isel, wsel, tsum);
 }
 // The same by two warps that hold the same logits: warp 1 adds the exponentials in the reference's order (256 dependent additions) while warp 0 selects by them;
-// warp 0 returns the result.  row, run: shared memory; the two meet at barrier 1.
+// warp 0 returns the result.  row, run: shared memory; the two meet at the named barrier `bar`.
 template <typename TabT>
-__device__ __forceinline__ void exact_topk_pair(float (&p)[8], const int lane, const int sum_warp, const TabT *tab, float *row, float *run_at, int &isel, float &wsel, float &tsum) {
+__device__ __forceinline__ void exact_topk_pair(float (&p)[8], const int lane, const int sum_warp, const TabT *tab, float *row, float *run_at, const int bar, int &isel, float &wsel, float &tsum) {
     exact_exp_warp(p, lane, tab);
     isel = 0; wsel = tsum = 0.0f;
     if (sum_warp) {
@@ -80,12 +80,12 @@ __device__ __forceinline__ void exact_topk_pair(float (&p)[8], const int lane, c
         __syncwarp();
         const float run = exact_sum_row(row);
         if (lane == 0) *run_at = run;
-        asm volatile("bar.sync 1, 64;" ::: "memory");
+        asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
         return;
     }
     float psel;                                                          // lane k < 9: the k-th largest
     top_select_warp<9>(p, lane, isel, psel, tsum);
-    asm volatile("bar.sync 1, 64;" ::: "memory");
+    asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
     const float run = *run_at;
     wsel = __fdiv_rn(psel, run);
     // the reference selects by the quotients: another order only where unequal exponentials have equal quotients (or are not numbers)
