@@ -203,11 +203,11 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
                     const uint32_t dst = smem_u32(wsm + ws * UM_WBYTES);
                     mbar_expect_tx(&sh->w_full[ws], UM_WBYTES);
                     if (GATEUP) {
-                        tma_load_2d_once(dst, &em->gate, sb * 128, mb * 128, &sh->w_full[ws], once);
-                        tma_load_2d_once(dst + 128 * 128, &em->up, sb * 128, mb * 128, &sh->w_full[ws], once);
+                        tma_load_2d(dst, &em->gate, sb * 128, mb * 128, &sh->w_full[ws], once);
+                        tma_load_2d(dst + 128 * 128, &em->up, sb * 128, mb * 128, &sh->w_full[ws], once);
                     } else {
-                        tma_load_3d_once(dst, &em->down, sb * 128, 0, mb * 128, &sh->w_full[ws], once);             // the even rows of the 256-row block
-                        tma_load_3d_once(dst + 128 * 128, &em->down, sb * 128, 1, mb * 128, &sh->w_full[ws], once);   // the odd rows
+                        tma_load_3d(dst, &em->down, sb * 128, 0, mb * 128, &sh->w_full[ws], once);             // the even rows of the 256-row block
+                        tma_load_3d(dst + 128 * 128, &em->down, sb * 128, 1, mb * 128, &sh->w_full[ws], once);   // the odd rows
                     }
                 }
             }

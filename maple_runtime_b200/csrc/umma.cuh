@@ -159,11 +159,11 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const void *tmap,
 
 // the same with an L2 policy: bytes that are read once (the weights) leave the L2 before what other kernels of the layer come back to
 __device__ __forceinline__ uint64_t l2_evict_first() { uint64_t p; asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p)); return p; }
-__device__ __forceinline__ void tma_load_2d_once(uint32_t dst_smem, const void *tmap, int x, int y, uint64_t *bar, uint64_t policy) {
+__device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const void *tmap, int x, int y, uint64_t *bar, uint64_t policy) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
                  ::"r"(dst_smem), "l"(tmap), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(policy) : "memory");
 }
-__device__ __forceinline__ void tma_load_3d_once(uint32_t dst_smem, const void *tmap, int x, int y, int z, uint64_t *bar, uint64_t policy) {
+__device__ __forceinline__ void tma_load_3d(uint32_t dst_smem, const void *tmap, int x, int y, int z, uint64_t *bar, uint64_t policy) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4}], [%5], %6;"
                  ::"r"(dst_smem), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)), "l"(policy) : "memory");
 }
