@@ -198,7 +198,7 @@ extern "C" void k_router_logits_tile(cudaStream_t st, const void *router_t, cons
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Decode batches (up to 144 tokens on 148 SMs).  The arithmetic is a handful of microseconds of dependent multiply-adds (256 per chain), so
+// Decode batches (up to 148 tokens on 148 SMs).  The arithmetic is a handful of microseconds of dependent multiply-adds (256 per chain), so
 // the kernel is about latency: a CTA owns 8 tokens x 8 experts, fetches all 2048 columns of both in two bulk copies (64 KB of
 // hidden values, 32 KB of bf16 weights, both pre-laid as [column / 32][lane j][4 steps] so that the eight lanes of a position
 // read consecutive 16-byte (8-byte) pieces), waits once, and runs the 64 x 4 steps without another synchronisation.  Two CTAs

@@ -169,14 +169,14 @@ __global__ void __launch_bounds__(192, 1) router_umma_kernel(const __grid_consta
     }
 }
 
-// one warp and CTA per token (eight warps per CTA: 2048 tokens 150.8 -> 148.9 us per layer without): lane l holds experts 8l..8l+7.  Adds the eight partial sums (fixed order) and the bias, stores the logits, takes the
+// One warp and CTA per token (2048 tokens 148.9 us per layer; with eight warps per CTA 150.8): lane l holds experts 8l..8l+7.  Adds the eight partial sums (fixed order) and the bias, stores the logits, takes the
 // nine largest (lowest index first among equals), decides whether their order is safe, and writes top-8 / weights or flags the token.
 __global__ void __launch_bounds__(32) router_select_kernel(const float *__restrict__ part, int ntok_cap, const float *__restrict__ bias,
                                                             const float *__restrict__ hnorm, const float *__restrict__ wnorm,
                                                             float *__restrict__ logits, int *__restrict__ top, float *__restrict__ topw,
                                                             int *__restrict__ flagged, int *__restrict__ nflagged,
                                                             unsigned *__restrict__ mask, int mask_words, int nb) {
-    const int lane = threadIdx.x & 31, b = blockIdx.x * 1 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31, b = blockIdx.x;
     pdl_wait(); pdl_trigger();
     if (b >= nb) return;
     float l[8];
@@ -368,7 +368,7 @@ extern "C" void k_router_tensor(cudaStream_t st, const RouterTensorArgs *r) {
         groups = clusters_at_once(router_fix_kernel, 8, 256, RF_SMEM, RF_GROUPS); attr_done = true;
     }
     launch_pdl(router_umma_kernel, dim3(RU_KS, (r->nb + 127) / 128), 192, smem, st, r->amap, r->wmap, r->part, r->nb, r->ntok_cap, r->err, r->nflagged, r->mask, NEXP * r->mask_words + NEXP);
-    launch_pdl(router_select_kernel, (r->nb + 0) / 1, 32, 0, st, r->part, r->ntok_cap, r->bias, r->hnorm, r->wnorm, r->logits, r->top, r->topw, r->flagged, r->nflagged, r->mask, r->mask_words, r->nb);
+    launch_pdl(router_select_kernel, r->nb, 32, 0, st, r->part, r->ntok_cap, r->bias, r->hnorm, r->wnorm, r->logits, r->top, r->topw, r->flagged, r->nflagged, r->mask, r->mask_words, r->nb);
     launch_clusters(router_fix_kernel, dim3(8, groups), 8, 256, RF_SMEM, st, (const uint8_t *)r->router_s, r->hn, r->bias, r->logits, r->top, r->topw, r->flagged, r->nflagged, r->mask, r->mask_words, r->nb, r->err);
     k_count_add(3);
 }
