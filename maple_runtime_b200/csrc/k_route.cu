@@ -390,8 +390,10 @@ __global__ void __launch_bounds__(NEXP, 1) group_cta_kernel(GroupArgs g) {
 // CTAs are what every GPU has to allow; from 513 tokens on sixteen share the scattered stores (2048 tokens: 14.4 -> 11.9 us).
 // Against one CTA for up to 256 tokens, a layer of the stack: 96 tokens 70.8 -> 70.0 us, 128 77.7 -> 75.9, 256 106.1 -> 100.7.
 // (One CTA per SM in the launch bounds of the grouping kernels: registers instead of reloads, 0.1 us.)
-// TOPK_IN (9 to TOPK_IN_MAX tokens): the softmax and top-8 come first, a warp per token (20 tokens 41.8 -> 41.3 us, 64 61.2 -> 60.7), two up to 32 tokens, where
-// there are enough (9 / 13 / 32 tokens 28.4 / 32.4 / 44.45 -> 28.0 / 32.0 / 44.25).
+// TOPK_IN (9 to TOPK_IN_MAX tokens): the softmax and top-8 come first, two warps per token (20 tokens 41.8 -> 41.3 us; with two warps instead of one 9 / 13 / 32 tokens
+// 28.4 / 32.4 / 44.45 -> 28.0 / 32.0 / 44.25).  Above, with one warp per token here or two in a kernel of their own: 33 / 40 / 48 / 64 tokens 47.3 / 50.2 / 52.15 / 56.1 and
+// 46.8 / 49.6 / 52.2 / 55.5; from nine tokens on in their own: 9 / 13 28.9 / 32.1.  (s_row has twice the rows it needs: with 4 KB less shared memory in the CTA, and
+// presumably another split of the SM's memory, 9 / 11 tokens took 28.8 / 30.5 instead of 27.8 / 30.0, the others the same.)
 #define GC_WORDS 8
 template <int GC_CTAS, bool TOPK_IN>
 __global__ void __launch_bounds__(NEXP, 1) group_cluster_kernel(GroupArgs g) {
@@ -403,40 +405,26 @@ __global__ void __launch_bounds__(NEXP, 1) group_cluster_kernel(GroupArgs g) {
     const int per = TOPK_IN ? (nb + GC_CTAS - 1) / GC_CTAS : (((nb + 31) / 32 + GC_CTAS - 1) / GC_CTAS) * 32, tok = blockIdx.x * per + e;      // per <= 32 GC_WORDS = one token per thread
     const bool mine = e < per && tok < nb;
     constexpr int TT = TOPK_IN ? TOPK_IN_MAX / GC_CTAS : 1;
+    static_assert(2 * TT <= 8, "two warps per token");
     __shared__ __align__(16) int s_top[TT * TOPK]; __shared__ __align__(16) float s_topw[TT * TOPK];
-    __shared__ __align__(16) float s_row[TOPK_IN ? 8 : 1][NEXP]; __shared__ float s_run[4];
+    __shared__ __align__(16) float s_row[TOPK_IN ? 8 : 1][NEXP]; __shared__ float s_run[TT];
     __shared__ unsigned long long tab[TOPK_IN ? 32 : 1];
     if (TOPK_IN && e < 32) tab[e] = DEV_EXP_TAB[e];
     if (TOPK_IN) __syncthreads();
     pdl_wait(); pdl_trigger();
     if (TOPK_IN) {
-        if (per <= 4) {                                        // up to 32 tokens: two warps each
-            const int i = wid >> 1, t = blockIdx.x * per + i;
-            if (i < per && t < nb) {
-                const float4 *lr = reinterpret_cast<const float4 *>(g.logits + (size_t)t * NEXP + lane * 8);
-                const float4 v0 = __ldcg(lr), v1 = __ldcg(lr + 1);
-                float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-                int isel; float wsel, tsum;
-                exact_topk_pair(p, lane, wid & 1, tab, s_row[i], &s_run[i], 1 + i, isel, wsel, tsum);
-                if (!(wid & 1) && lane < TOPK) {
-                    const float tw = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));
-                    s_top[i * TOPK + lane] = isel; s_topw[i * TOPK + lane] = tw;
-                    g.top_out[t * TOPK + lane] = isel; g.topw_out[t * TOPK + lane] = tw;
-                }
-            }
-        } else for (int i = wid; i < per && (int)blockIdx.x * per + i < nb; i += 8) {
-            const int t = blockIdx.x * per + i;
+        const int i = wid >> 1, t = blockIdx.x * per + i;
+        if (i < per && t < nb) {
             const float4 *lr = reinterpret_cast<const float4 *>(g.logits + (size_t)t * NEXP + lane * 8);
             const float4 v0 = __ldcg(lr), v1 = __ldcg(lr + 1);
             float p[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
             int isel; float wsel, tsum;
-            exact_topk_warp(p, lane, tab, s_row[wid], isel, wsel, tsum);
-            if (lane < TOPK) {
+            exact_topk_pair(p, lane, wid & 1, tab, s_row[i], &s_run[i], 1 + i, isel, wsel, tsum);
+            if (!(wid & 1) && lane < TOPK) {
                 const float tw = __fdiv_rn(wsel, __fadd_rn(tsum, 1e-20f));
                 s_top[i * TOPK + lane] = isel; s_topw[i * TOPK + lane] = tw;
                 g.top_out[t * TOPK + lane] = isel; g.topw_out[t * TOPK + lane] = tw;
             }
-            __syncwarp();
         }
         __syncthreads();
     }

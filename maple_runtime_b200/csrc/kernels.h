@@ -77,8 +77,7 @@ void k_topk(cudaStream_t st, const float *logits, int *top, float *topw, int nb)
 /* norm + int8 as k_norm_prep, and the normalised rows once more as two fp16 terms per value (hA: [nb][4096] fp16, hi then lo) with the
  * rows' Euclidean norms (hnorm [nb]): the A operand of the tensor-core router */
 void k_norm_prep_split(cudaStream_t st, const float *x, const uint16_t *w, float *hn, int8_t *q, float *qs, int *qsum, void *hA, float *hnorm, int nb);
-#define TOPK_IN_MAX 64              /* a warp per token in the grouping kernel: one CTA up to 8 tokens, a cluster of eight above; a second token per warp takes longer than
-                                      a kernel of its own (128 tokens: 78.0 against 75.9 us per layer) */
+#define TOPK_IN_MAX 32              /* top-8 in the grouping kernel: one CTA up to 8 tokens, a warp each; a cluster of eight above, two warps each, its eight warps' worth */
 #define GROUP_CLUSTER_MAX 4096      /* up to here k_group makes its own bits; above it the routing kernels may set them (GroupArgs.marked) */
 typedef struct {
     const int *top; const float *topw; int nb;
