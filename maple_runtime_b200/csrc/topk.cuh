@@ -88,9 +88,11 @@ __device__ __forceinline__ void exact_topk_pair(float (&p)[8], const int lane, c
     asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
     const float run = *run_at;
     wsel = __fdiv_rn(psel, run);
-    // the reference selects by the quotients: another order only where unequal exponentials have equal quotients (or are not numbers)
+    // The reference selects by the quotients, which fall with the exponentials: another order only where unequal exponentials have equal quotients (or are not numbers).
+    // Among the first nine that shows between neighbours.  Beyond the ninth it needs the ninth's own quotient above it, so the eighth has to be larger than the ninth: where
+    // the two are the same exponential, a smaller one with a lower index may have the same quotient.
     const float pn = __shfl_down_sync(0xffffffffu, psel, 1), wn = __shfl_down_sync(0xffffffffu, wsel, 1);
-    if (__any_sync(0xffffffffu, lane < 8 && !(wsel > wn || psel == pn))) exact_topk_warp_from(p, lane, run, isel, wsel, tsum);
+    if (__any_sync(0xffffffffu, lane < 8 && !(wsel > wn || (psel == pn && lane < 7)))) exact_topk_warp_from(p, lane, run, isel, wsel, tsum);
     else {
         tsum = 0.0f;
 #pragma unroll

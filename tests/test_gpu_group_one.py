@@ -20,6 +20,16 @@ def logits(kind):
         v = np.full(256, -3.0, np.float32)
         v[[200, 13, 77, 5, 250, 9]] = [1.0, 2.0, 0.5, 0.25, 3.0, 0.125]
         return v
+    if kind == "tie over a last bit":                        # the 8th and 9th exponential are equal, a smaller one has their quotient and a lower index
+        v = np.full(256, -8.0, np.float32)
+        v[100:170:10] = np.arange(1.0, 2.75, 0.25)
+        v[[200, 210]] = np.uint32(0x3f0075f7).view(np.float32)
+        v[50] = np.uint32(0x3f0075f6).view(np.float32)
+        return v
+    if kind.startswith("crowded"):                           # many ties and many last bits at the boundary
+        k = np.random.default_rng([3, int(kind.split()[1])]).integers(0, 60, 256)
+        k[0] = 0
+        return (-k * 2.0 ** -24).astype(np.float32)
     if kind == "vanishing":                                  # six exponentials above zero
         v = np.full(256, -200.0, np.float32)
         v[[31, 7, 255, 128, 64, 63]] = [0, -1, -2, -3, -4, -87]
@@ -27,10 +37,14 @@ def logits(kind):
     return rng.standard_normal(256).astype(np.float32)
 
 
-@pytest.mark.parametrize("kind", ["equal", "last bits", "pairs", "tie at the boundary", "vanishing", "ordinary"])
-def test_one_token(kind, gpu, oracle):
+@pytest.fixture(scope="module")
+def layer(gpu):                                               # once: every generation takes a region id
+    gpu.synth_layer(SEED, 0)
+
+
+@pytest.mark.parametrize("kind", ["equal", "last bits", "pairs", "tie at the boundary", "vanishing", "ordinary", "tie over a last bit", "crowded 4", "crowded 8", "crowded 33"])
+def test_one_token(kind, layer, gpu, oracle):
     g = gpu
-    g.synth_layer(SEED, 0)
     bias = logits(kind)
     top, topw, _ = oracle.topk(bias)                          # a row of zeros has no logits of its own
     nu, ue, ustart, utok, uw, tp = oracle.group(top[None, :], topw[None, :])
