@@ -125,9 +125,9 @@ __global__ void __launch_bounds__(640, 1) expert_umma_kernel(ExpertArgs a, const
     tc_fence_after();
     const uint32_t tb = sh->tmem_base;
     bool live = true;
-    // launched programmatically: the weights start to come in before the wait (the tile list is two kernels old), everything else after it
-    if (warp != 0) pdl_wait();
-    pdl_trigger();
+    // launched programmatically: the weights start to come in before the wait (the tile list is two kernels old), everything else after it.  Warp 0, which does not
+    // wait, leaves the trigger to the others: the first one counts for the CTA, and a successor may read what is two kernels old before its own wait
+    if (warp != 0) { pdl_wait(); pdl_trigger(); }
     if (DENSE && tid == 0) span_begin(a.span);
 
     // where item number i of this CTA keeps its accumulators (half 0, then half 1, n2 columns in all); over: they cover columns of the item before it

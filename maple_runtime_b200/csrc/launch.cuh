@@ -2,7 +2,8 @@
 //
 // launch_pdl: programmatic dependent launch, for the kernels of the layer loop.  Such a kernel is placed on the SMs while its predecessor in
 // the stream finishes; it does its own set-up and reads of weights, then calls pdl_wait() before it touches any memory that a predecessor
-// wrote or still reads, and pdl_trigger() after that: its own successor may then be placed.  Since a kernel triggers only after its wait,
+// wrote or still reads, and pdl_trigger() after that: its own successor may then be placed.  Since a kernel triggers only after its wait (every thread
+// that triggers has waited: the first trigger in a CTA counts for the CTA; tables_kernel, launched plainly, triggers at once: all before it is complete when it starts),
 // everything before its predecessor is complete when it starts: what was written two kernels ago may be read before pdl_wait (past L1).
 // Not every kernel gains: norm of prefill chunks, SiLU and combine of large ones, placed early, end up unevenly spread over the SMs that happen to be
 // free first (4096 tokens: combine 324 against 308 us per layer, SiLU 308 against 302; 512 tokens: norm 110 against 108); they are launched plainly.
