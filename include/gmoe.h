@@ -122,10 +122,14 @@ int gmoe_ep_received(void);               /* pairs this rank's experts received 
 int gmoe_ep_timeout_selftest(int ms);
 
 /* ---- parity hooks: named device buffers of the last call, and single stages ---------------------------------- */
-/* Names: x hn y hq hqs hqsum logits top topw nu ue ustart utok uw tp gate up act aq aqs aqsum down gu_dots dn_dots */
+/* Names: x hn y hq hqs hqsum logits top topw nu ue ustart utok uw tp gate up act aq aqs aqsum down gu_dots dn_dots
+ * Which kernels run depends on the call's size, and without kept stages they store only what a later kernel reads: gate, up, act, down, gu_dots and dn_dots hold the last
+ * call's rows after gmoe_keep_stages(1) and otherwise may be an earlier one's.  Calls of 161 tokens and more (gmoe_set_path(2): of any size) without kept stages also give up
+ * gate, up and the down rows once they are read: until a call with kept stages, a stage ("gateup", "down") or gmoe_poke writes them again, gmoe_peek of "gate" and "up" and the stages that start
+ * from them ("actq", "combine_y", "combine_x") answer -1. */
 int gmoe_peek(const char *name, void *dst, size_t bytes);
 int gmoe_poke(const char *name, const void *src, size_t bytes);
-/* keep = 1: the expert kernels also store gate, up and the int32 dot products (tot - qsum). */
+/* keep = 1: the expert kernels also store gate, up, act, down rows and the int32 dot products (tot - qsum), and nothing is given up. */
 int gmoe_keep_stages(int keep);
 /* Runs one stage on the device buffers for nb tokens of layer L: "norm" (x->hn,hq..), "prep" (hn->hq..),
  * "router", "router_tensor" (hn -> logits, top-8, weights on the tensor-core path), "topk", "group", "gateup", "actq", "down", "combine_y" (y = sum), "combine_x" (x += sum). */

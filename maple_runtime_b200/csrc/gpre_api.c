@@ -51,8 +51,12 @@ typedef struct { uint16_t *router, *post_ln; void *router_t, *router_s, *router_
                  int e0, ne;            /* the experts this GPU holds for the layer (all 256, or one rank's shard) */
                  int synth_region;      /* region index + 1 of a synthetic layer's weights, released when the layer is replaced */ } LayerDev;
 
+#define DROP_GATE 1
+#define DROP_UP 2
+#define DROP_WIRE 4
 static struct {
     int ready, maxtok, maxp, mask_words, keep, path, nb_cur, ep_on;
+    int dropped;               /* DROP_*: buffers whose rows the last call gave up after reading them (launch.cuh: l2_discard): undefined until written again */
     cudaStream_t st; cudaEvent_t e0, e1;
     void *reg[MAXREG]; size_t reg_len[MAXREG]; int nreg; double blit_s;
     LayerDev ly[GMOE_LAYERS];
@@ -425,25 +429,29 @@ static void run_experts(const ExpertPtrs *tab, const ExpertMaps *maps, const flo
         prof_begin(4);
         if (um) k_gateup_umma(S.st, &a, &S.bmap_hq); else k_gateup_mma(S.st, &a, tn);
         prof_end(4);
+        if (a.gate) S.dropped &= ~(DROP_GATE | DROP_UP);
     }
     const int fuse_q = !um && tn == 8 && which == 7;           /* decode batches: the down kernel quantises the SiLU outputs itself */
     if (fuse_q) { a.act_for_down = S.act; a.aq_out = S.aq; a.aqs_out = S.aqs; a.aqsum_out = S.aqsum; }
     if ((which & 2) && !fuse_q) {
         prof_begin(5);
-        if (um) k_silu_quant(S.st, S.gate, S.up, S.keep ? S.act : NULL, S.aq, S.aqs, S.aqsum, nb * TOPK, NULL, which == 7 && !S.keep);
-        else k_actq(S.st, S.act, S.aq, S.aqs, S.aqsum, NULL, nb * TOPK);
+        const int drop = which == 7 && !S.keep;
+        if (um) k_silu_quant(S.st, S.gate, S.up, S.keep ? S.act : NULL, S.aq, S.aqs, S.aqsum, nb * TOPK, NULL, drop);
+        if (um && drop) S.dropped |= DROP_GATE | DROP_UP;
+        if (!um) k_actq(S.st, S.act, S.aq, S.aqs, S.aqsum, NULL, nb * TOPK);
         prof_end(5);
     }
     if (which & 4) {
         prof_begin(6);
         if (um) k_down_umma(S.st, &a, &S.bmap_aq); else k_down_mma(S.st, &a, tn);
+        if (um) S.dropped &= ~DROP_WIRE;
         if (um && S.keep) k_wire_decode(S.st, S.wire, S.maxp, dsp, S.down, nb * TOPK);     /* fp32 rows for stage comparisons */
         prof_end(6);
     }
 }
 /* weighted combine of the pairs' down rows into out (init + sum): compact rows after the tcgen05 kernel (drop: not needed afterwards), fp32 rows otherwise */
 static void run_combine(const float *const *dsp, int nb, const float *init, float *out, int drop) {
-    if (use_umma(nb)) k_combine_wire(S.st, S.wire, S.maxp, dsp, S.uw, S.tp, init, out, nb, drop);
+    if (use_umma(nb)) { k_combine_wire(S.st, S.wire, S.maxp, dsp, S.uw, S.tp, init, out, nb, drop); if (drop) S.dropped |= DROP_WIRE; }
     else k_combine(S.st, S.down, S.uw, S.tp, init, out, nb);
 }
 /* router logits: large batches take the tiled kernel, small ones the kernels that read the norm's re-laid rows in place (k_router_logits_small chooses).
@@ -663,6 +671,7 @@ static int layers_enqueue_ep(int nb, int l0, int nl, const float *bd, int ep) {
         }
         r->exec = exec;
     } else k_count_add(r->launches);
+    if (use_umma(nb)) S.dropped = ep ? 0 : DROP_GATE | DROP_UP | DROP_WIRE;      /* what its layers did to the buffers when they were captured */
     CU("gmoe", cudaGraphLaunch((cudaGraphExec_t)r->exec, S.st));
     g_graph_launches++;
     return 0;
@@ -1027,11 +1036,13 @@ static int named(const char *name, void **p, size_t *cap) {
     for (size_t i = 0; i < sizeof tab / sizeof tab[0]; i++) if (!strcmp(tab[i].n, name)) { *p = tab[i].p; *cap = tab[i].cap; return 0; }
     return -1;
 }
+static int drop_bit(const char *name) { return !strcmp(name, "gate") ? DROP_GATE : !strcmp(name, "up") ? DROP_UP : 0; }
 int gmoe_peek(const char *name, void *dst, size_t bytes) {
     void *p; size_t cap;
     if (!S.ready) return fail("gmoe", "not initialised");
     if (named(name, &p, &cap)) return fail("gmoe", "no buffer named %s", name);
     if (!p) return fail("gmoe", "buffer %s is only kept after gmoe_keep_stages(1)", name);
+    if (S.dropped & drop_bit(name)) return fail("gmoe", "the last call gave up buffer %s after reading it; gmoe_keep_stages(1) keeps it", name);
     if (bytes > cap) return fail("gmoe", "%zu bytes asked of %s, which holds %zu", bytes, name, cap);
     CU("gmoe", cudaMemcpyAsync(dst, p, bytes, cudaMemcpyDeviceToHost, S.st)); CU("gmoe", cudaStreamSynchronize(S.st)); return 0;
 }
@@ -1041,11 +1052,14 @@ int gmoe_poke(const char *name, const void *src, size_t bytes) {
     if (named(name, &p, &cap)) return fail("gmoe", "no buffer named %s", name);
     if (!p) return fail("gmoe", "buffer %s is only kept after gmoe_keep_stages(1)", name);
     if (bytes > cap) return fail("gmoe", "%zu bytes given for %s, which holds %zu", bytes, name, cap);
+    S.dropped &= ~drop_bit(name);
     CU("gmoe", cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, S.st)); CU("gmoe", cudaStreamSynchronize(S.st)); return 0;
 }
 int gmoe_stage(const char *name, int L, int nb) {
     if (check_call("gmoe", L, nb)) return -1;
     LayerDev *l = &S.ly[L];
+    const int needs = !use_umma(nb) ? 0 : !strcmp(name, "actq") ? DROP_GATE | DROP_UP : !strncmp(name, "combine_", 8) ? DROP_WIRE : 0;
+    if (S.dropped & needs) return fail("gmoe", "the last call gave up the rows that stage %s starts from; gmoe_keep_stages(1) keeps them", name);
     cudaEventRecord(S.e0, S.st);
     if (!strcmp(name, "norm")) k_norm_prep(S.st, S.x, l->post_ln, S.hn, S.hq, S.hqs, S.hqsum, nb);
     else if (!strcmp(name, "prep")) k_norm_prep(S.st, S.hn, NULL, S.hn, S.hq, S.hqs, S.hqsum, nb);
@@ -1440,11 +1454,13 @@ static int run_layer_ep(int L, int nb, const float *bias) {
     if (S.keep || um) { a.gate = S.gate; a.up = S.up; }
     if (S.keep) { a.gu_dots = S.gu_dots; a.dn_dots = S.dn_dots; }
     prof_begin(4); if (um) k_gateup_umma(S.st, &a, &S.bmap_hq); else k_gateup_mma(S.st, &a, tn); prof_end(4);
+    if (a.gate) S.dropped &= ~(DROP_GATE | DROP_UP);
     prof_begin(5);
     if (um) k_silu_quant(S.st, S.gate, S.up, S.keep ? S.act : NULL, S.aq, S.aqs, S.aqsum, (int)EP.rcap, EP.total, 0);
     else k_actq(S.st, S.act, S.aq, S.aqs, S.aqsum, EP.total, (int)EP.rcap);
     prof_end(5);
     prof_begin(6); if (um) k_down_umma(S.st, &a, &S.bmap_aq); else k_down_mma(S.st, &a, tn); prof_end(6);
+    if (um) S.dropped &= ~DROP_WIRE;
     prof_begin(7);
     if (ep_barrier(NULL)) return -1;
     if (um && S.keep) k_wire_decode(S.st, S.wire, S.maxp, (const float *const *)EP.dsp[L], S.down, nb * TOPK);
