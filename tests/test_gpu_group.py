@@ -35,3 +35,27 @@ def test_cluster_grouping_equals_oracle(nb, kind, shift, gpu, clib, oracle):
     assert np.array_equal(ue.cpu().numpy()[:o_nu], o_ue[:o_nu]) and np.array_equal(ustart.cpu().numpy()[:o_nu + 1], o_ustart[:o_nu + 1])
     assert np.array_equal(utok.cpu().numpy(), o_utok.ravel()) and np.array_equal(tp.cpu().numpy(), o_tp.ravel())
     assert np.array_equal(uw.cpu().numpy().view(np.uint32), o_uw.ravel().view(np.uint32))
+
+
+@pytest.fixture(scope="module")
+def layer(gpu):                                               # once: every generation takes a region id
+    gpu.synth_layer(SEED, 0)
+
+
+@pytest.mark.parametrize("nb,kind", [(161, "even"), (256, "even"), (257, "even"), (257, "same"), (288, "skew"), (289, "even"), (512, "same"), (513, "skew"), (2047, "even"), (2048, "skew")])
+def test_grouping_of_a_layer_equals_oracle(nb, kind, layer, gpu, oracle):
+    """As a layer runs it (the stage "group"): up to 256 tokens the cluster places the pairs, from 257 the kernel that moves their rows does (k_expert_umma.cu: place_rows_kernel)."""
+    rng = np.random.default_rng(nb)
+    top, tw = routing(rng, nb, kind == "skew")
+    if kind == "same":
+        top[:] = top[0]
+    o_nu, o_ue, o_ustart, o_utok, o_uw, o_tp = oracle.group(top, tw)
+    gpu.poke("top", top.ravel())
+    gpu.poke("topw", tw.ravel())
+    gpu.poke("utok", np.full(nb * 8, -1, np.int32))
+    gpu.poke("tp", np.full(nb * 8, -1, np.int32))
+    gpu.stage("group", 0, nb)
+    assert int(gpu.peek("nu", nb)[0]) == o_nu
+    assert np.array_equal(gpu.peek("ue", nb)[:o_nu], o_ue[:o_nu]) and np.array_equal(gpu.peek("ustart", nb)[:o_nu + 1], o_ustart[:o_nu + 1])
+    assert np.array_equal(gpu.peek("utok", nb).ravel(), o_utok.ravel()) and np.array_equal(gpu.peek("tp", nb).ravel(), o_tp.ravel())
+    assert np.array_equal(gpu.peek("uw", nb).ravel().view(np.uint32), o_uw.ravel().view(np.uint32))

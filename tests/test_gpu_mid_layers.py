@@ -1,4 +1,4 @@
-"""Several layers at 209 to 511 tokens, where the combine of a layer and the norm of the next are one kernel on the compact down rows
+"""Several layers at 161 to 511 tokens, where the combine of a layer and the norm of the next are one kernel on the compact down rows
 (csrc/k_route.cu: edge_kernel<true>), against the same layers one call each, which the other tests compare with the oracle."""
 import numpy as np
 import pytest
@@ -31,7 +31,7 @@ def stacks(gpu, weights):
         gpu.set_layer(L, router, post_ln, ml.gloc_for_contiguous(0, slot=0), np.array([rid, -1, -1, -1], np.int32))
 
 
-@pytest.mark.parametrize("nb", [209, 301, 511])
+@pytest.mark.parametrize("nb", [161, 209, 301, 511])
 @pytest.mark.parametrize("l0", [0, 2])
 def test_layers_in_one_call_equal_layers_one_by_one(nb, l0, stacks, gpu, weights):
     g = gpu
@@ -51,10 +51,11 @@ def test_layers_in_one_call_equal_layers_one_by_one(nb, l0, stacks, gpu, weights
         g.keep_stages(True)
 
 
-@pytest.mark.parametrize("nb", [48, 49, 104, 105, 160, 161, 208])
+@pytest.mark.parametrize("nb", [48, 49, 104, 105, 160, 161, 208, 256, 257, 511, 512, 1152, 1153, 1307, 1308, 1536, 1537])
 def test_where_the_expert_kernels_change(nb, stacks, gpu, weights):
-    """Up to 48, 104 and 160 tokens the mma.sync down kernel takes one, two and four blocks of rows per CTA; from 161 the tcgen05 kernels run.  Either path alone
-    and the one that the size chooses: the same bits."""
+    """Up to 48, 104 and 160 tokens the mma.sync down kernel takes one, two and four blocks of rows per CTA; from 161 the tcgen05 kernels run.  From 257 the pairs are placed by the
+    kernel that moves their rows, from 512 two layers have no joint; up to 1152, 1307 and 1536 combine starts early, the tcgen05 kernels hand over blocks of 256 columns, SiLU starts
+    early.  Either path alone and the one that the size chooses: the same bits."""
     g = gpu
     x = weights.hidden(950 + nb, nb)
     out = {}
