@@ -392,8 +392,11 @@ __global__ void __launch_bounds__(NEXP, 1) group_cta_kernel(GroupArgs g) {
 // (One CTA per SM in the launch bounds of the grouping kernels: registers instead of reloads, 0.1 us.)
 // TOPK_IN (9 to TOPK_IN_MAX tokens): the softmax and top-8 come first, two warps per token (20 tokens 41.8 -> 41.3 us; with two warps instead of one 9 / 13 / 32 tokens
 // 28.4 / 32.4 / 44.45 -> 28.0 / 32.0 / 44.25).  Above, with one warp per token here or two in a kernel of their own: 33 / 40 / 48 / 64 tokens 47.3 / 50.2 / 52.15 / 56.1 and
-// 46.8 / 49.6 / 52.2 / 55.5; from nine tokens on in their own: 9 / 13 28.9 / 32.1.  (s_row has twice the rows it needs: with 4 KB less shared memory in the CTA, and
-// presumably another split of the SM's memory, 9 / 11 tokens took 28.8 / 30.5 instead of 27.8 / 30.0, the others the same.)
+// 46.8 / 49.6 / 52.2 / 55.5; from nine tokens on in their own: 9 / 13 28.9 / 32.1.
+// GC_CARVE: the split of the SM's memory, in percent of the shared memory it can have: 132 KB, the smallest that holds a CTA of the router in front of it (RS_ALONE, k_router_tile.cu).  Left
+// to the driver (or asked for 32, 64 or 100 KB) 9 / 11 tokens take 28.65 / 30.3 us per layer, with 132 KB 27.85 / 30.05, with all of it 28.2 / 30.1 but 16 / 20 34.8 / 40.9 instead of
+// 33.6 / 37.5.
+#define GC_CARVE 57
 #define GC_WORDS 8
 template <int GC_CTAS, bool TOPK_IN>
 __global__ void __launch_bounds__(NEXP, 1) group_cluster_kernel(GroupArgs g) {
@@ -407,7 +410,7 @@ __global__ void __launch_bounds__(NEXP, 1) group_cluster_kernel(GroupArgs g) {
     constexpr int TT = TOPK_IN ? TOPK_IN_MAX / GC_CTAS : 1;
     static_assert(2 * TT <= 8, "two warps per token");
     __shared__ __align__(16) int s_top[TT * TOPK]; __shared__ __align__(16) float s_topw[TT * TOPK];
-    __shared__ __align__(16) float s_row[TOPK_IN ? 8 : 1][NEXP]; __shared__ float s_run[TT];
+    __shared__ __align__(16) float s_row[TT][NEXP]; __shared__ float s_run[TT];
     __shared__ unsigned long long tab[TOPK_IN ? 32 : 1];
     if (TOPK_IN && e < 32) tab[e] = DEV_EXP_TAB[e];
     if (TOPK_IN) __syncthreads();
@@ -520,8 +523,11 @@ extern "C" void k_group(cudaStream_t st, const GroupArgs *g) {
     }
     const int np = g->nb * TOPK;
     if (g->nb <= GROUP_CLUSTER_MAX) {
-        if (g->logits) launch_cluster(group_cluster_kernel<8, true>, 8, NEXP, st, *g);
-        else if (g->nb <= 512) launch_cluster(group_cluster_kernel<8, false>, 8, NEXP, st, *g);
+        if (g->logits) {
+            static bool split_done = false;
+            if (!split_done) { cudaFuncSetAttribute(group_cluster_kernel<8, true>, cudaFuncAttributePreferredSharedMemoryCarveout, GC_CARVE); split_done = true; }
+            launch_cluster(group_cluster_kernel<8, true>, 8, NEXP, st, *g);
+        } else if (g->nb <= 512) launch_cluster(group_cluster_kernel<8, false>, 8, NEXP, st, *g);
         else {
             static bool attr_done = false;
             if (!attr_done) { cudaFuncSetAttribute(group_cluster_kernel<16, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); attr_done = true; }
