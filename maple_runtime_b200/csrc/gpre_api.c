@@ -383,8 +383,8 @@ int gmoe_profile_read(double *secs, long *launches) {
 static int tile_tn(int nb) { return nb <= 256 ? 8 : 32; }
 
 /* Which expert kernels: up to 160 tokens the mma.sync kernels on tiles of 8, above that the tcgen05 kernels, whose time hardly grows while an expert
- * has few pairs.  A layer of the stack on either: 128 tokens 73.6 and 75.6 us, 144 76.0 and 77.2, 160 76.5 and 76.5, 176 78.0 and 76.8, 208 84.0 and 78.4; a layer
- * call's kernels 85.0 and 86.0 at 160, 87.0 and 86.0 at 176, a plug-in call's 69.6 and 69.6, 73.7 and 69.6 at 192. */
+ * has few pairs.  A layer of the stack on either: 128 tokens 69.2 and 72.4 us, 144 71.6 and 73.2, 160 73.2 and 73.2, 176 74.4 and 73.5, 208 79.0 and 74.3; a layer
+ * call's kernels 80.9 and 81.9 at 160, 82.9 and 81.9 at 176, a plug-in call's 66.5 and 67.4, 68.6 and 67.7. */
 static int use_umma(int nb) { return S.path == 2 || (S.path == 0 && nb > 160); }
 static void fill_expert_args(ExpertArgs *a, const ExpertPtrs *tab, const ExpertMaps *maps, const int *ue, int nb) {
     memset(a, 0, sizeof *a);

@@ -246,9 +246,10 @@ static void launch(cudaStream_t st, const ExpertArgs *a) {
 // Where the whole list is resident at once at one or two CTAs per SM, all eight chunks go out together: one trip to memory instead of four
 // (1 token 22.1 -> 20.9 us per layer; from 4 tokens on the two are level).
 #define PF8_TILES 24
-// Eight warps per CTA share a tile's staged rows once an expert has several pairs: 192 tokens 86.2 -> 82.5 us per layer, 160 80.6 -> 79.0, 128 the same, but
-// 64 tokens 60.8 -> 61.8.  max_tiles is 256 + the tokens, as many tiles as there could be.
-#define NW8_TILES 384
+// Gate+up: eight warps per CTA share a tile's staged rows once the list of tiles is long.  max_tiles is 256 + the tokens, as many tiles as there could be.  Four / eight warps on this
+// path: 132 tokens 69.4 / 70.5 us per layer, 144 71.7 / 72.2, 160 73.2 / 73.3, 176 74.9 / 74.4, 192 77.0 / 76.4, 224 83.2 / 82.6, 256 89.4 / 88.9.  By size a layer has no such list
+// (from 161 tokens on the tcgen05 kernels run); other ranks' tokens and gmoe_set_path(1) bring them.
+#define NW8_TILES 416
 // The down kernel's CTAs each quantise the tile's activations for themselves and wait for its tile and its pointers: with more tiles than CTAs fit at once they take two
 // or four blocks of 128 rows in turn, the next one's codes on their way while the results of this one are stored.  Rounds 1 / 2 / 4: 32 tokens 44.2 / 44.2 / 47.9 us per layer,
 // 52 53.3 / 53.2 / 55.5, 64 56.4 / 55.9 / 57.8, 96 66.8 / 64.5 / 64.9, 112 71.1 / 68.4 / 68.1, 128 73.6 / 70.4 / 69.5.
