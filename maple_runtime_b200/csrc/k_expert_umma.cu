@@ -490,7 +490,7 @@ static void launch(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) {
 }
 // Blocks of 256 columns halve the hand-overs but leave the accumulators 256 columns of tensor memory instead of 320, which two items of more than 64 pairs do not share.
 // A layer with blocks of 128 and of 256: 176 tokens 76.6 and 74.4 us, 301 83.1 and 82.0, 511 94.7 and 93.5, 843 101.2 and 99.8, 1300 119.5 and 119.4, 1500 127.2 and 127.7,
-// 2048 148.9 and 155.0.
+// 2048 148.9 and 155.0.  (As many tiles as there could be: the line lies at 1307 tokens.)
 #define UM_WIDE_TILES (1300 * 8 / UMMA_TN + 256)
 template <int K, int MODE, bool FULL>
 static void launch_by_size(cudaStream_t st, const ExpertArgs *a, const TMap4 *bmap) {
